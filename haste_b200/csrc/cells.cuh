@@ -109,12 +109,6 @@ int layer_norm_lstm_backward(const LnLstmBwd& a, cudaStream_t s);
 int layer_norm_gru_forward(const LnGruFwd& a, cudaStream_t s);
 int layer_norm_gru_backward(const LnGruBwd& a, cudaStream_t s);
 
-// Persistent-kernel implementations of the recurrences (recurrent_kernels.cuh).
-// Each returns HASTE_B200_ERR_UNSUPPORTED (without touching any buffer) when the
-// shape does not fit, in which case the caller runs its step-wise path.
-// Forward: the input projection is already in a.v (LSTM) / a.tmp_Wx (GRU).
-// Backward: carries are fp32 [N,H] buffers, read at entry and written at exit.
-int lstm_forward_persistent(const LstmFwd& a, cudaStream_t s);
 // single-step (Iterate) forward in one launch (iterate_fused.cu); UNSUPPORTED: take the general path
 int lstm_forward_step_fused(const LstmFwd& a, cudaStream_t s);
 int gru_forward_step_fused(const GruFwd& a, cudaStream_t s);
@@ -125,13 +119,19 @@ struct GradPlanes {
   __nv_bfloat16* p2 = nullptr;
   long long stride = 0;
 };
-int lstm_backward_persistent(const LstmBwd& a, float* dh_carry, float* dc_carry,
-                             const GradPlanes& planes, cudaStream_t s);
-int gru_forward_persistent(const GruFwd& a, cudaStream_t s);
-int gru_backward_persistent(const GruBwd& a, float* dh_carry, const GradPlanes& planes,
-                            cudaStream_t s);
-// Tensor-core recurrence for bf16 batches of about a hundred rows and more (rec_tc_gru.cu);
-// same contract, except that the backward kernel does not sum the bias gradients.
+// Persistent implementations of the recurrences.  Each returns HASTE_B200_ERR_UNSUPPORTED
+// (without touching any buffer) when the shape is not its own, in which case the caller goes on to
+// the next one, at last to its step-wise path.
+// Chain recurrences (rec_chain_host.cu): on a thread-block cluster or the whole grid, H up to
+// 1024.  Forward: the input projection is already in a.v (LSTM) / a.tmp_Wx (GRU).  Backward:
+// complete - dh and dc are read and written in place (dc_new may be null), the bias gradients
+// added.  `few` (GRU): leave batches to the tensor-core recurrence where that is faster.
+int lstm_forward_chain(const LstmFwd& a, cudaStream_t s);
+int lstm_backward_chain(const LstmBwd& a, const GradPlanes& planes, cudaStream_t s);
+int gru_forward_chain(const GruFwd& a, bool few, cudaStream_t s);
+int gru_backward_chain(const GruBwd& a, const GradPlanes& planes, bool few, cudaStream_t s);
+// Tensor-core recurrence for bf16 batches of about a hundred rows and more (rec_tc_gru.cu).  The
+// backward kernel carries dh in an fp32 [N,H] buffer and does not sum the bias gradients.
 int gru_forward_tc(const GruFwd& a, cudaStream_t s);
 int gru_backward_tc(const GruBwd& a, float* dh_carry, cudaStream_t s);
 // LayerNormLSTM: forward expects LN(x.W) in a.act_Wx_norm; backward adds the LayerNorm

@@ -200,11 +200,12 @@ int gru_forward(const GruFwd& a, cudaStream_t s) {
     HB_TRY(gemm(g, s));
   }
   ProfScope p(PH_REC_FWD, s);
-  // large bf16 batches: the tensor-core recurrence; small batches: the register-resident one
-  int st_ = gru_forward_tc(a, s);
-  if (st_ != HASTE_B200_ERR_UNSUPPORTED) return st_;
-  st_ = a.h_out ? HASTE_B200_ERR_UNSUPPORTED : gru_forward_persistent(a, s);
-  if (st_ != HASTE_B200_ERR_UNSUPPORTED) return st_;
+  if (!a.h_out) {
+    int st_ = gru_forward_chain(a, true, s);
+    if (st_ == HASTE_B200_ERR_UNSUPPORTED) st_ = gru_forward_tc(a, s);
+    if (st_ == HASTE_B200_ERR_UNSUPPORTED) st_ = gru_forward_chain(a, false, s);
+    if (st_ != HASTE_B200_ERR_UNSUPPORTED) return st_;
+  }
   if (a.dtype == HASTE_B200_F32) return gru_forward_stepwise<float>(a, s);
   if (a.dtype == HASTE_B200_F16) return gru_forward_stepwise<__half>(a, s);
   return gru_forward_stepwise<__nv_bfloat16>(a, s);
@@ -223,15 +224,8 @@ int gru_backward(const GruBwd& a, cudaStream_t s) {
   const long long TN = (long long)a.T * N;
   HB_REQUIRE(TN < (1LL << 31), "T*N too large");
   const size_t NH = (size_t)N * H;
-  Arena ws;
-  const size_t csf = colsum_scratch_floats((int)TN, 3 * H);
-  HB_TRY(make_arena(&ws, s, Arena::pad(NH * 4) + Arena::pad(csf * 4) + 1024));
-  float* dh_carry = ws.take<float>(NH);
-  float* cs = ws.take<float>(csf);
-  HB_REQUIRE(dh_carry && cs, "scratch arena");
-  HB_TRY(to_float(a.dtype, a.dh, dh_carry, NH, s));
   GradPlanes planes;
-  bool have_planes = false, persistent_ran = false;
+  bool have_planes = false;
   if (a.dtype == HASTE_B200_F32 && ((3 * H) % 8) == 0) {
     const size_t pe = Arena::pad((size_t)TN * 3 * H * 2) / 2;  // elements per plane
     void* pw = workspace(s, 4 * pe * 2 + 256, /*slot=*/3);
@@ -241,33 +235,48 @@ int gru_backward(const GruBwd& a, cudaStream_t s) {
       planes.stride = (long long)pe;
     }
   }
-  int st_;
-  {
+  int st_ = HASTE_B200_ERR_UNSUPPORTED;
+  if (!a.iterate) {
     ProfScope p(PH_REC_BWD, s);
-    st_ = gru_backward_tc(a, dh_carry, s);
-    if (st_ == HASTE_B200_OK) {
-      // the tensor-core kernel leaves the recurrent contribution of the last processed step
-      // (t = 0) out of dh: dh += dq_0 . R^T
-      GemmDesc gd{a.dtype, HASTE_B200_F32, N, H, 3 * H, a.dq, 3LL * H, 1, a.R,
-                  a.transposed_inputs ? H : 1, a.transposed_inputs ? 1 : 3LL * H, dh_carry, H, 1};
-      st_ = gemm_small(gd, s);
-    } else if (st_ == HASTE_B200_ERR_UNSUPPORTED) {
-      st_ = a.iterate ? HASTE_B200_ERR_UNSUPPORTED
-                      : gru_backward_persistent(a, dh_carry, planes, s);
-      have_planes = st_ == HASTE_B200_OK && planes.p != nullptr;
-      persistent_ran = st_ == HASTE_B200_OK;
-    }
-    if (st_ == HASTE_B200_ERR_UNSUPPORTED) {
-    st_ = (a.dtype == HASTE_B200_F32)   ? gru_backward_stepwise<float>(a, dh_carry, s)
-          : (a.dtype == HASTE_B200_F16) ? gru_backward_stepwise<__half>(a, dh_carry, s)
-                                        : gru_backward_stepwise<__nv_bfloat16>(a, dh_carry, s);
-    }
+    st_ = gru_backward_chain(a, planes, true, s);
   }
-  HB_TRY(st_);
-  HB_TRY(from_float(a.dtype, dh_carry, a.dh, NH, s));
-  if (!persistent_ran) {  // (the persistent kernel summed the bias gradients itself)
-    HB_TRY(colsum(a.dtype, a.dp, 3LL * H, (int)TN, 3 * H, a.dtype, a.dbx, 1, cs, s));
-    HB_TRY(colsum(a.dtype, a.dq, 3LL * H, (int)TN, 3 * H, a.dtype, a.dbr, 1, cs, s));
+  if (st_ == HASTE_B200_ERR_UNSUPPORTED) {
+    Arena ws;
+    const size_t csf = colsum_scratch_floats((int)TN, 3 * H);
+    HB_TRY(make_arena(&ws, s, Arena::pad(NH * 4) + Arena::pad(csf * 4) + 1024));
+    float* dh_carry = ws.take<float>(NH);
+    float* cs = ws.take<float>(csf);
+    HB_REQUIRE(dh_carry && cs, "scratch arena");
+    bool carried = true;  // dh travels in dh_carry and the bias gradients are still to be summed
+    {
+      ProfScope p(PH_REC_BWD, s);
+      HB_TRY(to_float(a.dtype, a.dh, dh_carry, NH, s));
+      st_ = gru_backward_tc(a, dh_carry, s);
+      if (st_ == HASTE_B200_OK) {
+        // the tensor-core kernel leaves the recurrent contribution of the last processed step
+        // (t = 0) out of dh: dh += dq_0 . R^T
+        GemmDesc gd{a.dtype, HASTE_B200_F32, N, H, 3 * H, a.dq, 3LL * H, 1, a.R,
+                    a.transposed_inputs ? H : 1, a.transposed_inputs ? 1 : 3LL * H, dh_carry, H, 1};
+        st_ = gemm_small(gd, s);
+      } else if (st_ == HASTE_B200_ERR_UNSUPPORTED && !a.iterate) {
+        st_ = gru_backward_chain(a, planes, false, s);
+        have_planes = st_ == HASTE_B200_OK && planes.p != nullptr;
+        carried = st_ != HASTE_B200_OK;
+      }
+      if (st_ == HASTE_B200_ERR_UNSUPPORTED)
+        st_ = (a.dtype == HASTE_B200_F32)   ? gru_backward_stepwise<float>(a, dh_carry, s)
+              : (a.dtype == HASTE_B200_F16) ? gru_backward_stepwise<__half>(a, dh_carry, s)
+                                            : gru_backward_stepwise<__nv_bfloat16>(a, dh_carry, s);
+    }
+    HB_TRY(st_);
+    if (carried) {
+      HB_TRY(from_float(a.dtype, dh_carry, a.dh, NH, s));
+      HB_TRY(colsum(a.dtype, a.dp, 3LL * H, (int)TN, 3 * H, a.dtype, a.dbx, 1, cs, s));
+      HB_TRY(colsum(a.dtype, a.dq, 3LL * H, (int)TN, 3 * H, a.dtype, a.dbr, 1, cs, s));
+    }
+  } else {
+    HB_TRY(st_);
+    have_planes = planes.p != nullptr;
   }
   const bool tr = a.transposed_inputs != 0;
   GemmDesc gx{a.dtype, a.dtype, (int)TN, C, 3 * H, a.dp, 3LL * H, 1, a.W, tr ? C : 1,

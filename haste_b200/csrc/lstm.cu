@@ -1,7 +1,7 @@
 // LSTM forward / backward drivers and their step-wise kernels.
 //
 // Two implementations of the recurrence sit behind each driver:
-//   * the persistent kernels of recurrent_kernels.cuh (one launch per layer pass,
+//   * the persistent kernels of rec_chain_host.cu (one launch per layer pass,
 //     recurrent weights resident on chip, tensor-core step product), used
 //     whenever the shape fits; and
 //   * the step-wise path in this file (one contraction + one pointwise launch per
@@ -56,7 +56,7 @@ __global__ void lstm_pointwise_bwd(int N, int H, const T* __restrict__ c_prev, T
   if (j >= H) return;
   const long long g0 = (long long)n * 4 * H + j;
   const long long o0 = (long long)n * H + j;
-  float dc_total = ld(dc_new + o0) + dc_carry[o0];
+  float dc_total = (dc_new ? ld(dc_new + o0) : 0.f) + dc_carry[o0];
   float dh_total = ld(dh_new + o0) + dh_carry[o0];
   const float c_tanh = tanhf(ld(c_new + o0));
   const float i = ld(v + g0 + 0 * H), g = ld(v + g0 + 1 * H);
@@ -129,7 +129,7 @@ int lstm_backward_stepwise(const LstmBwd& a, float* dh_carry, float* dc_carry, c
   for (int t = a.T - 1; t >= 0; --t) {
     T* vt = v + t * NH * 4;
     const T* dh_new = (const T*)a.dh_new + (a.iterate ? 0 : (t + 1) * NH);
-    const T* dc_new = (const T*)a.dc_new + (a.iterate ? 0 : (t + 1) * NH);
+    const T* dc_new = a.dc_new ? (const T*)a.dc_new + (a.iterate ? 0 : (t + 1) * NH) : nullptr;
     const T* c_new = a.iterate ? (const T*)a.c_new : c + (t + 1) * NH;
     if (mask)
       lstm_pointwise_bwd<T, true><<<grid, block, 0, s>>>(N, H, c + t * NH, vt, c_new,
@@ -173,7 +173,7 @@ int lstm_forward(const LstmFwd& a, cudaStream_t s) {
     HB_TRY(gemm(g, s));
   }
   ProfScope p(PH_REC_FWD, s);
-  int st_ = (a.h_out || a.c_out) ? HASTE_B200_ERR_UNSUPPORTED : lstm_forward_persistent(a, s);
+  const int st_ = (a.h_out || a.c_out) ? HASTE_B200_ERR_UNSUPPORTED : lstm_forward_chain(a, s);
   if (st_ != HASTE_B200_ERR_UNSUPPORTED) return st_;
   if (a.dtype == HASTE_B200_F32) return lstm_forward_stepwise<float>(a, s);
   return lstm_forward_stepwise<__nv_bfloat16>(a, s);
@@ -183,7 +183,7 @@ int lstm_backward(const LstmBwd& a, cudaStream_t s) {
   HB_REQUIRE(a.dtype == HASTE_B200_F32 || a.dtype == HASTE_B200_BF16, "dtype");
   HB_REQUIRE(a.T >= 0 && a.N > 0 && a.C > 0 && a.H > 0, "T,N,C,H");
   if (a.T == 0) return HASTE_B200_OK;  // nothing to do; scratch pointers may be null
-  HB_REQUIRE(a.W && a.R && a.h && a.c && a.dh_new && a.dc_new && a.dW && a.dR && a.db &&
+  HB_REQUIRE(a.W && a.R && a.h && a.c && a.dh_new && a.dW && a.dR && a.db &&
                  a.dh && a.dc && a.v, "null pointer");
   if (a.T == 0) return HASTE_B200_OK;
   HB_REQUIRE(a.x && a.dx, "x/dx is null");
@@ -192,18 +192,9 @@ int lstm_backward(const LstmBwd& a, cudaStream_t s) {
   HB_REQUIRE(TN < (1LL << 31), "T*N too large");
   const size_t NH = (size_t)N * H;
 
-  Arena ws;
-  HB_TRY(make_arena(&ws, s, Arena::pad(2 * NH * 4) * 2 + Arena::pad(colsum_scratch_floats((int)TN, 4 * H) * 4) + 1024));
-  float* dh_carry = ws.take<float>(NH);
-  float* dc_carry = ws.take<float>(NH);
-  float* cs = ws.take<float>(colsum_scratch_floats((int)TN, 4 * H));
-  HB_REQUIRE(dh_carry && dc_carry && cs, "scratch arena");
-  HB_TRY(to_float(a.dtype, a.dh, dh_carry, NH, s));
-  HB_TRY(to_float(a.dtype, a.dc, dc_carry, NH, s));
-
   // fp32: room for the gate gradients as bf16 planes (written by the persistent kernel)
   GradPlanes planes;
-  bool have_planes = false, persistent_ran = false;
+  bool have_planes = false;
   if (a.dtype == HASTE_B200_F32 && ((4 * H) % 8) == 0) {
     const size_t pe = Arena::pad((size_t)TN * 4 * H * 2) / 2;  // elements per plane
     void* pw = workspace(s, 2 * pe * 2 + 256, /*slot=*/3);
@@ -215,23 +206,31 @@ int lstm_backward(const LstmBwd& a, cudaStream_t s) {
   int st_;
   {
     ProfScope p(PH_REC_BWD, s);
-    st_ = a.iterate ? HASTE_B200_ERR_UNSUPPORTED
-                    : lstm_backward_persistent(a, dh_carry, dc_carry, planes, s);
+    st_ = a.iterate ? HASTE_B200_ERR_UNSUPPORTED : lstm_backward_chain(a, planes, s);
     have_planes = st_ == HASTE_B200_OK && planes.p != nullptr;
-    persistent_ran = st_ == HASTE_B200_OK;
-    if (st_ == HASTE_B200_ERR_UNSUPPORTED) {
-    st_ = (a.dtype == HASTE_B200_F32) ? lstm_backward_stepwise<float>(a, dh_carry, dc_carry, s)
-                                      : lstm_backward_stepwise<__nv_bfloat16>(a, dh_carry, dc_carry, s);
+  }
+  if (st_ == HASTE_B200_ERR_UNSUPPORTED) {
+    Arena ws;
+    HB_TRY(make_arena(&ws, s, Arena::pad(2 * NH * 4) * 2 + Arena::pad(colsum_scratch_floats((int)TN, 4 * H) * 4) + 1024));
+    float* dh_carry = ws.take<float>(NH);
+    float* dc_carry = ws.take<float>(NH);
+    float* cs = ws.take<float>(colsum_scratch_floats((int)TN, 4 * H));
+    HB_REQUIRE(dh_carry && dc_carry && cs, "scratch arena");
+    HB_TRY(to_float(a.dtype, a.dh, dh_carry, NH, s));
+    HB_TRY(to_float(a.dtype, a.dc, dc_carry, NH, s));
+    {
+      ProfScope p(PH_REC_BWD, s);
+      st_ = (a.dtype == HASTE_B200_F32) ? lstm_backward_stepwise<float>(a, dh_carry, dc_carry, s)
+                                        : lstm_backward_stepwise<__nv_bfloat16>(a, dh_carry, dc_carry, s);
     }
+    HB_TRY(st_);
+    HB_TRY(from_float(a.dtype, dh_carry, a.dh, NH, s));
+    HB_TRY(from_float(a.dtype, dc_carry, a.dc, NH, s));
+    HB_TRY(colsum(a.dtype, a.v, 4LL * H, (int)TN, 4 * H, a.dtype, a.db, 1, cs, s));
   }
   HB_TRY(st_);
-  HB_TRY(from_float(a.dtype, dh_carry, a.dh, NH, s));
-  HB_TRY(from_float(a.dtype, dc_carry, a.dc, NH, s));
 
   // v now holds dv = d(loss)/d(pre-activation) for every step.
-  // (the persistent kernel summed the bias gradient itself)
-  if (!persistent_ran)
-    HB_TRY(colsum(a.dtype, a.v, 4LL * H, (int)TN, 4 * H, a.dtype, a.db, 1, cs, s));
   const bool tr = a.transposed_inputs != 0;
   // dW[C,4H] += x^T . dv
   GemmDesc gw{a.dtype, a.dtype, C, 4 * H, (int)TN, a.x, tr ? TN : 1, tr ? 1 : C, a.v, 4LL * H, 1,

@@ -1,0 +1,168 @@
+// Host side of the chain recurrences: what the kernels of rec_cluster_kernels.cuh and
+// rec_grid_kernels.cuh read and write, and which of the two takes a shape.
+#include <initializer_list>
+
+#include "rec_grid_launch.cuh"
+
+namespace hb {
+
+using namespace rec;
+
+namespace {
+
+// Whole-quad accesses: every row of every array starts on a multiple of four elements.
+bool aligned(std::initializer_list<const void*> ptrs, int H, int dtype) {
+  uintptr_t a = 0;
+  for (const void* q : ptrs) a |= reinterpret_cast<uintptr_t>(q);
+  return H % 4 == 0 && a % (4 * dtype_size(dtype)) == 0;
+}
+
+// Grid tiling: NMT quads of hidden units per CTA such that its slice of R fits the registers, as
+// many row groups as there are SMs for, the rest of the rows as chains - at most `most` of them: a
+// chain adds 0.7 .. 2 us to a step (H = 512 .. 1024), which the step-wise path (about 20 us plus the
+// product) undercuts from a dozen on, and from six on the tensor-core GRU recurrence (6 us forward,
+// 11 us backward at H = 1024 whatever the rows).
+constexpr int kGridChains = 12, kGridChainsBeforeTc = 5;
+
+// A handful of steps of a wide fp32 / fp16 layer stays on the step-wise path (as
+// tests/test_parity_gpu.py expects of it).
+constexpr int kWideSteps = 8;
+
+bool gl_geometry(int dtype, int T, int N, int H, int most, GlGeometry* g) {
+  if (dtype != HASTE_B200_BF16 && H > 512 && T < kWideSteps) return false;
+  g->KS16 = ceil_div(H, 16);
+  const int ks = ceil_div(g->KS16, GL_WARPS);
+  if (ks > 8) return false;
+  const int tiles = ceil_div(N, 8), sms = sm_count(), budget = sm_budget();
+  g->NMT = (dtype == HASTE_B200_BF16 || ks <= 4) ? 4 : 2;
+  g->nHS = ceil_div(H, 4 * g->NMT);
+  if (g->nHS > sms) return false;
+  const int use = (budget > 0 && budget < sms && g->nHS <= budget) ? budget : sms;
+  g->nRG = min(tiles, use / g->nHS);
+  g->CH = ceil_div(tiles, g->nRG);
+  g->nRG = ceil_div(tiles, g->CH);
+  return g->CH <= most;
+}
+
+// How many chains per CTA the cluster kernels may take before the grid kernels do better (us per
+// step, fp32 LSTM, cluster / grid).  Up to 192 units clusters are small enough that there are
+// always enough of them (H = 192, 128 rows: 1.4 / 2.2 forward).  At 256 units a cluster is 16 CTAs
+// and only seven are resident one CTA per SM: 32 rows 1.15 / 1.5 forward, 1.2 / 2.0 backward, but
+// 128 rows 2.8 / 1.8 and 3.0 / 2.4.  Five quads per CTA (to 320 units) pay in the backward pass
+// only: 2.0 / 1.7 and 1.8 / 2.2 at 19 rows.
+int cluster_chains(const ClGeometry& g, bool bwd) {
+  if (g.NW == 5) return bwd ? 1 : 0;
+  return g.CS <= 12 ? kClMaxChains : 1;
+}
+
+// Zeroed scratch: abort flag, then `words` exchange words, then `floats` that need no zeroing.
+int gl_scratch(ChainParams* p, size_t words, size_t floats, float** extra, cudaStream_t s) {
+  const size_t head = 256, bytes = head + Arena::pad(words * 4);
+  char* base = static_cast<char*>(workspace(s, bytes + Arena::pad(floats * 4), /*slot=*/2));
+  if (!base) return HASTE_B200_ERR_CUDA;
+  HB_CUDA_OK(cudaMemsetAsync(base, 0, bytes, s));
+  p->sync.abort_flag = reinterpret_cast<int*>(base);
+  p->xbuf = reinterpret_cast<uint32_t*>(base + head);
+  if (extra) *extra = reinterpret_cast<float*>(base + bytes);
+  return HASTE_B200_OK;
+}
+
+typedef int (*ClRun)(int, ChainParams&, int, int*, cudaStream_t);
+typedef int (*GlRun)(int, ChainParams&, const GlGeometry&, cudaStream_t);
+
+int run_fwd(ChainParams& p, int dtype, int grid_most, ClRun cl, GlRun gl, cudaStream_t s) {
+  p.sync.err = device_error_word();
+  HB_REQUIRE(p.sync.err, "error word");
+  ClGeometry cg;
+  if (cl_geometry(p.H, &cg)) {
+    int groups = 0;
+    const int st_ = cl(dtype, p, cluster_chains(cg, false), &groups, s);
+    if (st_ != HASTE_B200_ERR_UNSUPPORTED) return st_;
+  }
+  GlGeometry g;
+  if (!gl_geometry(dtype, p.T, p.N, p.H, grid_most, &g)) return HASTE_B200_ERR_UNSUPPORTED;
+  p.CTAS = g.nHS; p.CH = g.CH; p.K16 = g.KS16;
+  HB_TRY(gl_scratch(&p, (size_t)2 * ceil_div(p.N, 8) * g.KS16 * 128, 0, nullptr, s));
+  return gl(dtype, p, g, s);
+}
+
+int run_bwd(ChainParams& p, int dtype, int grid_most, int gates, void* db, void* db2, ClRun cl, GlRun gl,
+            cudaStream_t s) {
+  p.sync.err = device_error_word();
+  HB_REQUIRE(p.sync.err, "error word");
+  const int tiles = ceil_div(p.N, 8);
+  ClGeometry cg;
+  if (cl_geometry(p.H, &cg)) {
+    p.db_part = static_cast<float*>(workspace(s, (size_t)tiles * 4 * p.H * sizeof(float), /*slot=*/2));
+    if (!p.db_part) return HASTE_B200_ERR_CUDA;
+    int groups = 0;
+    const int st_ = cl(dtype, p, cluster_chains(cg, true), &groups, s);
+    if (st_ == HASTE_B200_OK) return bias_grad_finish(gates, p.db_part, groups, p.H, dtype, db, db2, s);
+    if (st_ != HASTE_B200_ERR_UNSUPPORTED) return st_;
+  }
+  GlGeometry g;
+  if (!gl_geometry(dtype, p.T, p.N, p.H, grid_most, &g)) return HASTE_B200_ERR_UNSUPPORTED;
+  p.CTAS = g.nHS; p.CH = g.CH; p.K16 = ceil_div(g.nHS * g.NMT, 4);
+  HB_TRY(gl_scratch(&p, (size_t)2 * tiles * g.nHS * g.nHS * g.NMT * 32, (size_t)g.nRG * 8 * p.H, &p.db_part, s));
+  HB_TRY(gl(dtype, p, g, s));
+  return bias_grad_finish(gates, p.db_part, 2 * g.nRG, p.H, dtype, db, db2, s);
+}
+
+// Rows the tensor-core GRU recurrence would take (rec_tc_gru.cu).
+bool tc_waits(int dtype, int N, int H) {
+  return dtype == HASTE_B200_BF16 && N >= 96 && H % 64 == 0 && recurrence_path() != HASTE_B200_PATH_NO_TENSOR_CORE;
+}
+
+}  // namespace
+
+int lstm_forward_chain(const LstmFwd& a, cudaStream_t s) {
+  if (recurrence_path() == HASTE_B200_PATH_STEPWISE) return HASTE_B200_ERR_UNSUPPORTED;
+  ChainParams p{};
+  p.T = a.T; p.N = a.N; p.H = a.H;
+  p.training = a.training; p.has_zoneout = a.zoneout_prob != 0.0f && a.zoneout_mask != nullptr;
+  p.zoneout_prob = a.zoneout_prob;
+  p.R = a.R; p.b = a.b; p.gin = a.v; p.gout = a.training ? a.v : nullptr; p.mask = a.zoneout_mask;
+  p.h = a.h; p.c = a.c;
+  p.wide = aligned({a.v, a.h, a.c, a.zoneout_mask}, a.H, a.dtype);
+  return run_fwd(p, a.dtype, kGridChains, run_cl_fwd_lstm, run_gl_fwd_lstm, s);
+}
+
+int gru_forward_chain(const GruFwd& a, bool few, cudaStream_t s) {
+  if (recurrence_path() == HASTE_B200_PATH_STEPWISE) return HASTE_B200_ERR_UNSUPPORTED;
+  ChainParams p{};
+  p.T = a.T; p.N = a.N; p.H = a.H;
+  p.training = a.training; p.has_zoneout = a.zoneout_prob != 0.0f && a.zoneout_mask != nullptr;
+  p.zoneout_prob = a.zoneout_prob;
+  p.R = a.R; p.b = a.bx; p.b2 = a.br; p.gin = a.tmp_Wx; p.gout = a.training ? a.v : nullptr;
+  p.mask = a.zoneout_mask; p.h = a.h;
+  p.wide = aligned({a.tmp_Wx, a.v, a.h, a.zoneout_mask}, a.H, a.dtype);
+  return run_fwd(p, a.dtype, few && tc_waits(a.dtype, a.N, a.H) ? kGridChainsBeforeTc : kGridChains,
+                 run_cl_fwd_gru, run_gl_fwd_gru, s);
+}
+
+int lstm_backward_chain(const LstmBwd& a, const GradPlanes& planes, cudaStream_t s) {
+  if (recurrence_path() == HASTE_B200_PATH_STEPWISE) return HASTE_B200_ERR_UNSUPPORTED;
+  ChainParams p{};
+  p.T = a.T; p.N = a.N; p.H = a.H;
+  p.has_zoneout = a.zoneout_mask ? 1 : 0; p.r_transposed = a.transposed_inputs;
+  p.R = a.R; p.gin = a.v; p.dv = a.v; p.c = const_cast<void*>(a.c); p.dh_new = a.dh_new; p.dc_new = a.dc_new;
+  p.mask = a.zoneout_mask; p.dh = a.dh; p.dc = a.dc;
+  p.gpl = planes.p; p.gpl_stride = planes.stride;
+  p.wide = aligned({a.v, a.c, a.dh_new, a.dc_new, a.zoneout_mask}, a.H, a.dtype);
+  return run_bwd(p, a.dtype, kGridChains, 4, a.db, nullptr, run_cl_bwd_lstm, run_gl_bwd_lstm, s);
+}
+
+int gru_backward_chain(const GruBwd& a, const GradPlanes& planes, bool few, cudaStream_t s) {
+  if (recurrence_path() == HASTE_B200_PATH_STEPWISE) return HASTE_B200_ERR_UNSUPPORTED;
+  ChainParams p{};
+  p.T = a.T; p.N = a.N; p.H = a.H;
+  p.has_zoneout = a.zoneout_mask ? 1 : 0; p.r_transposed = a.transposed_inputs;
+  p.R = a.R; p.gin = a.v; p.dp = a.dp; p.dq = a.dq; p.h = const_cast<void*>(a.h); p.dh_new = a.dh_new;
+  p.mask = a.zoneout_mask; p.dh = a.dh;
+  p.gpl = planes.p; p.gpl2 = planes.p2; p.gpl_stride = planes.stride;
+  p.wide = aligned({a.v, a.dp, a.dq, a.h, a.dh_new, a.zoneout_mask}, a.H, a.dtype);
+  return run_bwd(p, a.dtype, few && tc_waits(a.dtype, a.N, a.H) ? kGridChainsBeforeTc : kGridChains, 3, a.dbx,
+                 a.dbr, run_cl_bwd_gru, run_gl_bwd_gru, s);
+}
+
+}  // namespace hb

@@ -1,0 +1,11 @@
+// Instantiates the cluster recurrence, lstm bwd, for every storage type.
+#include "rec_cluster_launch.cuh"
+
+namespace hb {
+namespace rec {
+int run_cl_bwd_lstm(int dtype, ChainParams& p, int most, int* row_groups, cudaStream_t s) {
+  if (dtype == HASTE_B200_F32) return cl_bwd<4, 2, float>(p, most, row_groups, s);
+  return cl_bwd<4, 1, __nv_bfloat16>(p, most, row_groups, s);
+}
+}  // namespace rec
+}  // namespace hb

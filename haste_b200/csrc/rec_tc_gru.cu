@@ -1,6 +1,6 @@
 // Tensor-core GRU recurrence for large batches (bf16 storage), sm_100a.
 //
-// The register-resident kernels of recurrent_kernels.cuh are built for small batches: a CTA
+// The register-resident kernels of recurrent_common.cuh are built for small batches: a CTA
 // multiplies 16..64 batch rows with mma.sync and every row of h reaches it as tagged words.
 // From about a hundred rows per GPU the step product is a real tile for the 5th-generation
 // tensor cores, and this file runs it there:
@@ -36,7 +36,7 @@
 // (lib/gru_forward_gpu.cu.cc:214-308,345-363, lib/gru_backward_gpu.cu.cc:252-320) for
 // bf16 batches of about a hundred rows and more; math as in lib/gru_forward_gpu.cu.cc:27-85
 // and lib/gru_backward_gpu.cu.cc:26-96.
-#include "recurrent_kernels.cuh"
+#include "recurrent_common.cuh"
 #include "tcgen05.cuh"
 
 namespace hb {

@@ -1,6 +1,6 @@
 // Persistent LayerNormLSTM recurrence kernels (forward and backward), sm_100a.
 //
-// Same skeleton as recurrent_kernels.cuh - cooperative grid of (hidden slices) x (batch
+// Same skeleton as recurrent_common.cuh - cooperative grid of (hidden slices) x (batch
 // slices), the CTA's slice of R resident in registers as mma.sync fragments, self-validating
 // tagged words for every inter-CTA hand-off, bounded waits - plus what LayerNorm adds: a
 // normalisation runs over a whole row (all 4H gate columns of h.R, all H units of c'), while a
@@ -22,7 +22,7 @@
 // arithmetic; it is left out here.
 #pragma once
 
-#include "recurrent_kernels.cuh"
+#include "recurrent_common.cuh"
 
 namespace hb {
 namespace rec {
@@ -85,7 +85,7 @@ struct LnBwdParams {
 };
 
 // Statistics, partial gradients and (with fp32 storage) h travel as tagged fp32 words
-// (fword_* of recurrent_kernels.cuh): LayerNorm amplifies a relative error of the exchanged
+// (fword_* of recurrent_common.cuh): LayerNorm amplifies a relative error of the exchanged
 // value roughly tenfold, so the 17 bits of the (hi, lo) bf16 pair are not enough here.
 // h words: tagged fp32 with fp32 storage, the (hi, lo) bf16 pair with bf16 storage.
 template <int SPLIT> __device__ __forceinline__ uint32_t hword_encode(float x, uint32_t tag) {

@@ -1,0 +1,62 @@
+"""The persistent LSTM / GRU recurrences at the edges of their tiles, against the CPU oracle:
+hidden sizes on both sides of every change of tiling, batches that leave a chain of eight rows
+partly empty or give a CTA several chains, every storage type."""
+import pytest
+import torch
+
+import haste_oracle as oracle
+from helpers import TOL_BF16, TOL_F16, TOL_F32, assert_close, run_cuda
+
+pytestmark = pytest.mark.gpu
+
+# (T, N, H): cluster kernels (H <= 320)
+CLUSTER = [(1, 1, 1), (5, 2, 15), (6, 8, 16), (6, 9, 17), (7, 3, 64), (5, 33, 72), (5, 17, 129),
+           (6, 7, 200), (6, 37, 250), (5, 64, 256), (5, 5, 258), (5, 20, 320), (4, 150, 256),
+           (4, 300, 320), (3, 700, 64)]
+
+
+def _check(cell, T, N, H, dtype, tol, zoneout, transposed=False):
+    d = oracle.make_inputs(cell, T, N, 12, H, seed=T * 1000 + H + N, zoneout=zoneout)
+    dq = {k: (v.to(dtype).to(torch.float64) if v is not None else None) for k, v in d.items()}
+    ref_out, ref_grads = oracle.forward_backward(cell, dq, zoneout=zoneout)
+    out, grads = run_cuda(cell, dq, zoneout=zoneout, dtype=dtype, transposed=transposed)
+    for k, ref in list(ref_out.items()) + list(ref_grads.items()):
+        if k in out or k in grads:
+            assert_close(out[k] if k in out else grads[k], ref, tol, f"{cell} {k}")
+
+
+@pytest.mark.parametrize("zoneout", [0.0, 0.25])
+@pytest.mark.parametrize("shape", CLUSTER, ids=lambda s: "T%d_N%d_H%d" % s)
+@pytest.mark.parametrize("cell", ["lstm", "gru"])
+def test_cluster_recurrence_fp32(cell, shape, zoneout):
+    _check(cell, *shape, torch.float32, TOL_F32, zoneout, transposed=shape[1] % 2 == 0)
+
+
+@pytest.mark.parametrize("shape", [(5, 9, 17), (6, 37, 250), (5, 20, 320), (4, 150, 256)],
+                         ids=lambda s: "T%d_N%d_H%d" % s)
+@pytest.mark.parametrize("cell,dtype,tol", [("lstm", torch.bfloat16, TOL_BF16),
+                                            ("gru", torch.bfloat16, TOL_BF16),
+                                            ("gru", torch.float16, TOL_F16)])
+def test_cluster_recurrence_reduced_precision(cell, dtype, tol, shape):
+    _check(cell, *shape, dtype, tol, 0.25)
+
+
+# (T, N, H): grid kernels - every tiling of the hidden dimension, several chains per CTA
+GRID = [(5, 9, 321), (4, 20, 388), (5, 70, 512), (8, 1, 516), (8, 33, 520), (8, 12, 760),
+        (8, 17, 1020), (8, 9, 1024), (4, 300, 200)]
+
+
+@pytest.mark.parametrize("zoneout", [0.0, 0.25])
+@pytest.mark.parametrize("shape", GRID, ids=lambda s: "T%d_N%d_H%d" % s)
+@pytest.mark.parametrize("cell", ["lstm", "gru"])
+def test_grid_recurrence_fp32(cell, shape, zoneout):
+    _check(cell, *shape, torch.float32, TOL_F32, zoneout, transposed=shape[1] % 2 == 0)
+
+
+@pytest.mark.parametrize("shape", [(5, 9, 321), (8, 33, 520), (8, 17, 1020), (8, 70, 1024)],
+                         ids=lambda s: "T%d_N%d_H%d" % s)
+@pytest.mark.parametrize("cell,dtype,tol", [("lstm", torch.bfloat16, TOL_BF16),
+                                            ("gru", torch.bfloat16, TOL_BF16),
+                                            ("gru", torch.float16, TOL_F16)])
+def test_grid_recurrence_reduced_precision(cell, dtype, tol, shape):
+    _check(cell, *shape, dtype, tol, 0.25)
