@@ -4,6 +4,7 @@ The library is built in-tree by `haste_b200.build`.  There is no fallback: if th
 shared object is missing or a call fails, an exception is raised.
 """
 import ctypes
+import importlib.util
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -42,6 +43,7 @@ SIGNATURES = {
     "haste_b200_set_recurrence_path": [_i],
     "haste_b200_set_gemm_path": [_i],
     "haste_b200_set_sm_budget": [_i],
+    "haste_b200_set_assign_gradients": [_i],
     "haste_b200_sync_check": [_p],
     "haste_b200_profile_enable": [_i],
     "haste_b200_profile_read": [_p, _i],
@@ -72,6 +74,25 @@ def lib():
         L.haste_b200_launch_count.restype = _ll
         _lib = L
     return _lib
+
+
+_native = None
+
+
+def native():
+    """The compiled host path of the layers (torch_ext/native.cc), bound to `lib()`."""
+    global _native
+    if _native is None:
+        path = os.path.join(_HERE, "torch_ext", "native.so")
+        if not os.path.exists(path):
+            raise ImportError(f"{path} not found: build it with `python -m haste_b200.build`")
+        lib()
+        spec = importlib.util.spec_from_file_location("native", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.load(LIB_PATH, HasteError)
+        _native = module
+    return _native
 
 
 def call(name, *args):

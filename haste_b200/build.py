@@ -3,8 +3,9 @@
     python -m haste_b200.build            # incremental
     python -m haste_b200.build --force
 
-Only the CUDA toolkit is needed (no torch headers): the library is a plain
-C-ABI shared object that the Python layer loads with ctypes.
+The library needs only the CUDA toolkit (no torch headers): it is a plain C-ABI shared object that
+the Python ops load with ctypes.  The layers' host path (torch_ext/native.cc) is compiled against the
+installed torch.
 """
 import os
 import subprocess
@@ -69,40 +70,55 @@ def build(force=False, verbose=False):
     return LIB
 
 
-TORCH_EXT_SRC = os.path.join(HERE, "torch_ext", "haste_pytorch_lib.cc")
-TORCH_EXT = os.path.join(HERE, "torch_ext", "haste_pytorch_lib.so")
+TORCH_EXT_DIR = os.path.join(HERE, "torch_ext")
+TORCH_EXT = os.path.join(TORCH_EXT_DIR, "haste_pytorch_lib.so")
+NATIVE = os.path.join(TORCH_EXT_DIR, "native.so")
 
 
-def build_torch_ext(force=False):
-    """Compiles the pybind11 module `haste_pytorch_lib` (the reference's extension name) against
-    the installed torch and links it to libhaste_b200.so, in-tree."""
+def _build_pybind(target, link, force):
+    """Compiles torch_ext/<name>.cc against the installed torch into `target`, torch_ext/<name>.so."""
     import sysconfig
     import torch
     from torch.utils import cpp_extension as ce
+    src = target[:-3] + ".cc"
     header = os.path.join(HERE, "..", "include", "haste_b200.h")
-    if (not force and os.path.exists(TORCH_EXT) and os.path.exists(LIB)
-            and os.path.getmtime(TORCH_EXT) > max(os.path.getmtime(TORCH_EXT_SRC),
-                                                  os.path.getmtime(header))):
-        return TORCH_EXT
-    lib = build()
+    if (not force and os.path.exists(target) and os.path.exists(LIB)
+            and os.path.getmtime(target) > max(os.path.getmtime(src), os.path.getmtime(header))):
+        return target
     cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     incs = ce.include_paths() + [sysconfig.get_paths()["include"], os.path.join(HERE, "..", "include"),
                                  os.path.join(cuda_home, "include")]
     tlib = os.path.join(os.path.dirname(torch.__file__), "lib")
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
-           "-DTORCH_EXTENSION_NAME=haste_pytorch_lib", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           f"-DTORCH_EXTENSION_NAME={os.path.basename(target)[:-3]}", "-DTORCH_API_INCLUDE_EXTENSION_H",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-           *[f"-I{i}" for i in incs], TORCH_EXT_SRC, "-o", TORCH_EXT,
-           f"-L{tlib}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python",
-           f"-L{os.path.dirname(lib)}", "-lhaste_b200",
-           f"-Wl,-rpath,{tlib}", "-Wl,-rpath,$ORIGIN/.."]
+           *[f"-I{i}" for i in incs], src, "-o", target,
+           f"-L{tlib}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python", *link,
+           f"-Wl,-rpath,{tlib}"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"torch extension build failed:\n{r.stdout}\n{r.stderr}")
-    return TORCH_EXT
+    return target
+
+
+def build_native(force=False):
+    """Compiles the layers' host path (torch_ext/native.cc), in-tree; it takes the library's
+    functions from whatever shared object the ctypes binding has loaded."""
+    cuda_lib = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "lib64")
+    return _build_pybind(NATIVE, [f"-L{cuda_lib}", "-l:libcudart.so.12", "-ldl"], force)
+
+
+def build_torch_ext(force=False):
+    """Compiles the pybind11 module `haste_pytorch_lib` (the reference's extension name) against
+    the installed torch and links it to libhaste_b200.so, in-tree; with it the layers' host path."""
+    lib = build()
+    build_native(force)
+    return _build_pybind(TORCH_EXT, [f"-L{os.path.dirname(lib)}", "-lhaste_b200",
+                                     "-Wl,-rpath,$ORIGIN/.."], force)
 
 
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    print(build_native(force="--force" in sys.argv))
     if "--torch-ext" in sys.argv:
         print(build_torch_ext(force="--force" in sys.argv))

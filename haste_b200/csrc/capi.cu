@@ -13,6 +13,8 @@ static std::atomic<int> g_sm_budget{0};
 int recurrence_path() { return g_rec_path.load(); }
 int sm_budget() { return g_sm_budget.load(); }
 int gemm_path() { return g_gemm_path.load(); }
+static thread_local bool g_assign = false;
+bool assign_gradients() { return g_assign; }
 }  // namespace hb
 
 using namespace hb;
@@ -62,6 +64,10 @@ int haste_b200_set_recurrence_path(int path) {
 int haste_b200_set_sm_budget(int sms) {
   if (sms < 0) return HASTE_B200_ERR_INVALID;
   g_sm_budget.store(sms);
+  return HASTE_B200_OK;
+}
+int haste_b200_set_assign_gradients(int on) {
+  g_assign = on != 0;
   return HASTE_B200_OK;
 }
 int haste_b200_set_gemm_path(int path) {

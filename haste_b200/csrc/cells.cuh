@@ -162,5 +162,7 @@ inline int gemm_small(const GemmDesc& g, cudaStream_t s) {
 int recurrence_path();
 int sm_budget();  // 0: the whole GPU; else the SMs one recurrence launch may occupy
 int gemm_path();
+// This thread: backward passes assign parameter gradients, dh and dc instead of adding to them.
+bool assign_gradients();
 
 }  // namespace hb

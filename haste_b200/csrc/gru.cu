@@ -219,7 +219,8 @@ int gru_backward(const GruBwd& a, cudaStream_t s) {
   HB_REQUIRE(a.W && a.R && a.h && a.v && a.dh_new && a.dW && a.dR && a.dbx && a.dbr && a.dh &&
                  a.dp && a.dq, "null pointer");
   if (a.T == 0) return HASTE_B200_OK;
-  HB_REQUIRE(a.x && a.dx, "x/dx is null");
+  HB_REQUIRE(a.x, "x is null");
+  const int add = assign_gradients() ? 0 : 1;
   const int N = a.N, H = a.H, C = a.C;
   const long long TN = (long long)a.T * N;
   HB_REQUIRE(TN < (1LL << 31), "T*N too large");
@@ -250,7 +251,8 @@ int gru_backward(const GruBwd& a, cudaStream_t s) {
     bool carried = true;  // dh travels in dh_carry and the bias gradients are still to be summed
     {
       ProfScope p(PH_REC_BWD, s);
-      HB_TRY(to_float(a.dtype, a.dh, dh_carry, NH, s));
+      if (add) HB_TRY(to_float(a.dtype, a.dh, dh_carry, NH, s));
+      else HB_CUDA_OK(cudaMemsetAsync(dh_carry, 0, NH * 4, s));
       st_ = gru_backward_tc(a, dh_carry, s);
       if (st_ == HASTE_B200_OK) {
         // the tensor-core kernel leaves the recurrent contribution of the last processed step
@@ -271,8 +273,8 @@ int gru_backward(const GruBwd& a, cudaStream_t s) {
     HB_TRY(st_);
     if (carried) {
       HB_TRY(from_float(a.dtype, dh_carry, a.dh, NH, s));
-      HB_TRY(colsum(a.dtype, a.dp, 3LL * H, (int)TN, 3 * H, a.dtype, a.dbx, 1, cs, s));
-      HB_TRY(colsum(a.dtype, a.dq, 3LL * H, (int)TN, 3 * H, a.dtype, a.dbr, 1, cs, s));
+      HB_TRY(colsum(a.dtype, a.dp, 3LL * H, (int)TN, 3 * H, a.dtype, a.dbx, add, cs, s));
+      HB_TRY(colsum(a.dtype, a.dq, 3LL * H, (int)TN, 3 * H, a.dtype, a.dbr, add, cs, s));
     }
   } else {
     HB_TRY(st_);
@@ -284,11 +286,11 @@ int gru_backward(const GruBwd& a, cudaStream_t s) {
   if (have_planes) {  // dp was already split into bf16 planes by the recurrence kernel
     gx.a_pl = planes.p; gx.a_pl_ld = 3LL * H; gx.a_pl_stride = planes.stride;
   }
-  {
+  if (a.dx) {
     ProfScope p(PH_DGRAD, s);
     HB_TRY(gemm(gx, s));
   }
-  GemmDesc gr{a.dtype, a.dtype, H, 3 * H, (int)TN, a.h, 1, H, a.dq, 3LL * H, 1, a.dR, 3LL * H, 1};
+  GemmDesc gr{a.dtype, a.dtype, H, 3 * H, (int)TN, a.h, 1, H, a.dq, 3LL * H, 1, a.dR, 3LL * H, add};
   if (have_planes) {
     gr.b_pl = planes.p2; gr.b_pl_ld = 3LL * H; gr.b_pl_stride = planes.stride;
   }
@@ -297,7 +299,7 @@ int gru_backward(const GruBwd& a, cudaStream_t s) {
     HB_TRY(gemm(gr, s));
   }
   GemmDesc gw{a.dtype, a.dtype, C, 3 * H, (int)TN, a.x, tr ? TN : 1, tr ? 1 : C, a.dp, 3LL * H, 1,
-              a.dW, 3LL * H, 1};
+              a.dW, 3LL * H, add};
   if (have_planes) {
     gw.b_pl = planes.p; gw.b_pl_ld = 3LL * H; gw.b_pl_stride = planes.stride;
   }

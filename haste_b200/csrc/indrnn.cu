@@ -183,7 +183,8 @@ int indrnn_backward(const IndrnnBwd& a, cudaStream_t s) {
   const long long TN = (long long)a.T * N;
   HB_REQUIRE(TN < (1LL << 31), "T*N too large");
   if (a.T == 0) return HASTE_B200_OK;
-  HB_REQUIRE(a.x && a.dx, "x/dx is null");
+  HB_REQUIRE(a.x, "x is null");
+  const int add = assign_gradients() ? 0 : 1;
   const size_t NH = (size_t)N * H;
   const size_t csf = colsum_scratch_floats(N, H);
   const size_t lnf = a.gamma ? layer_norm_backward_scratch_floats((int)TN, H) : 0;
@@ -195,7 +196,8 @@ int indrnn_backward(const IndrnnBwd& a, cudaStream_t s) {
   float* cs = ws.take<float>(csf);
   float* lns = ws.take<float>(lnf);
   HB_REQUIRE(dh_carry && du_part && db_part && cs && (lns || !lnf), "scratch arena");
-  HB_TRY(to_float(a.dtype, a.dh, dh_carry, NH, s));
+  if (add) HB_TRY(to_float(a.dtype, a.dh, dh_carry, NH, s));
+  else HB_CUDA_OK(cudaMemsetAsync(dh_carry, 0, NH * 4, s));
   // fp32: dk = d/d(x.W) is read by both contractions below as two bf16 planes.  Without
   // LayerNorm the scan writes them next to the fp32 values; with LayerNorm its backward pass
   // does.  (Grow-only library scratch; without it the contractions split for themselves.)
@@ -213,10 +215,11 @@ int indrnn_backward(const IndrnnBwd& a, cudaStream_t s) {
     else HB_TRY(scan_bwd<__nv_bfloat16>(a, du_part, db_part, dh_carry, nullptr, 0, s));
   }
   HB_TRY(from_float(a.dtype, dh_carry, a.dh, NH, s));
-  HB_TRY(colsum(HASTE_B200_F32, du_part, H, N, H, a.dtype, a.du, 1, cs, s));
-  HB_TRY(colsum(HASTE_B200_F32, db_part, H, N, H, a.dtype, a.db, 1, cs, s));
+  HB_TRY(colsum(HASTE_B200_F32, du_part, H, N, H, a.dtype, a.du, add, cs, s));
+  HB_TRY(colsum(HASTE_B200_F32, db_part, H, N, H, a.dtype, a.db, add, cs, s));
   if (a.gamma) {
     ProfScope p(PH_OTHER, s);
+    if (!add) HB_CUDA_OK(cudaMemsetAsync(a.dgamma, 0, (size_t)H * dtype_size(a.dtype), s));
     // workspace holds dk = d/d(LN(x.W)); turn it into d/d(x.W) in place.
     HB_TRY(layer_norm_backward(a.dtype, (int)TN, H, a.gamma, a.act_Wx, a.workspace, a.workspace,
                                a.dtype, a.dgamma, nullptr, a.cache_Wx, lns, s, planes,
@@ -233,6 +236,7 @@ int indrnn_backward(const IndrnnBwd& a, cudaStream_t s) {
     ProfScope p(PH_WGRAD, s);
     HB_TRY(gemm(gw, s));
   }
+  if (!a.dx) return HASTE_B200_OK;
   GemmDesc gx{a.dtype, a.dtype, (int)TN, C, H, a.workspace, H, 1, a.W, tr ? C : 1, tr ? 1 : H,
               a.dx, C, 0};
   if (planes) { gx.a_pl = planes; gx.a_pl_ld = H; gx.a_pl_stride = plane_stride; }

@@ -120,6 +120,14 @@ int layer_norm_gru_backward(const LnGruBwd& a, cudaStream_t s) {
   const size_t NH = (size_t)N * H;
   const bool bf = a.dtype == HASTE_B200_BF16;
   const size_t es = dtype_size(a.dtype);
+  const int add = assign_gradients() ? 0 : 1;
+  if (!add) {  // everything below adds, except the two contractions at the end
+    HB_CUDA_OK(cudaMemsetAsync(a.dbx, 0, 3 * H * es, s));
+    HB_CUDA_OK(cudaMemsetAsync(a.dbr, 0, 3 * H * es, s));
+    HB_CUDA_OK(cudaMemsetAsync(a.dgamma_Wx, 0, 3 * H * es, s));
+    HB_CUDA_OK(cudaMemsetAsync(a.dgamma_Rh, 0, 3 * H * es, s));
+    HB_CUDA_OK(cudaMemsetAsync(a.dh, 0, NH * es, s));
+  }
   const size_t csf = colsum_scratch_floats((int)TN, 3 * H);
   const size_t lnf = layer_norm_backward_scratch_floats((int)TN, 3 * H);
   Arena ws;
@@ -159,10 +167,10 @@ int layer_norm_gru_backward(const LnGruBwd& a, cudaStream_t s) {
               tr ? 1 : 3LL * H, a.dx, C, 0};
   HB_TRY(gemm(gx, s));
   GemmDesc gr{a.dtype, a.dtype, H, 3 * H, (int)TN, a.h, 1, H, a.act_Rh, 3LL * H, 1, a.dR,
-              3LL * H, 1};
+              3LL * H, add};
   HB_TRY(gemm(gr, s));
   GemmDesc gw{a.dtype, a.dtype, C, 3 * H, (int)TN, a.x, tr ? TN : 1, tr ? 1 : C, a.dp, 3LL * H, 1,
-              a.dW, 3LL * H, 1};
+              a.dW, 3LL * H, add};
   HB_TRY(gemm(gw, s));
   return HASTE_B200_OK;
 }

@@ -96,7 +96,7 @@ __global__ void lnlstm_gate_grad(int N, int H, const T* __restrict__ c_prev, T* 
   const long long g0 = (long long)n * 4 * H + j;
   const long long o0 = (long long)n * H + j;
   const float i = ld(v + g0 + 0 * H), g = ld(v + g0 + 1 * H), f = ld(v + g0 + 2 * H);
-  const float dc_total = ld(dc_new + o0) + dc_carry[o0] + ld(dln + o0);
+  const float dc_total = (dc_new ? ld(dc_new + o0) : 0.f) + dc_carry[o0] + ld(dln + o0);
   const float df = ld(c_prev + o0) * dc_total;
   const float di = g * dc_total;
   const float dg = i * dc_total;
@@ -199,7 +199,8 @@ int backward_steps(const LnLstmBwd& a, float* dh_carry, float* dc_carry, void* d
                                dgamma_h, dbeta_h, (const char*)a.cache_c + (size_t)t * N * 2 * es,
                                lns, s));
     lnlstm_gate_grad<T><<<grid, block, 0, s>>>(N, H, c + t * NH, vt,
-                                               (const T*)a.dc_new + (t + 1) * NH, cn, dc_carry);
+                                               a.dc_new ? (const T*)a.dc_new + (t + 1) * NH : nullptr, cn,
+                                               dc_carry);
     HB_LAUNCH_OK();
     count_launch(2);
     // LayerNorm 2 backward: input was act_Rh[t]; result replaces it.
@@ -342,15 +343,18 @@ int backward_wide(const LnLstmBwd& a, cudaStream_t s) {
   HB_TRY(to_float(BF, a.x, x, XN, s));
   HB_TRY(to_float(BF, a.h, h, SN, s));
   HB_TRY(to_float(BF, a.c, c, SN, s));
-  HB_TRY(to_float(BF, a.dh_new, dhn, SN, s));
-  HB_TRY(to_float(BF, a.dc_new, dcn, SN, s));
+  // (slot 0 of the incoming gradients is never read)
+  HB_TRY(to_float(BF, static_cast<const char*>(a.dh_new) + NH * 2, dhn + NH, (size_t)T * NH, s));
+  if (a.dc_new) HB_TRY(to_float(BF, static_cast<const char*>(a.dc_new) + NH * 2, dcn + NH, (size_t)T * NH, s));
   HB_TRY(to_float(BF, a.dh, dh, NH, s));
   HB_TRY(to_float(BF, a.dc, dc, NH, s));
   if (mask) HB_TRY(to_float(BF, a.zoneout_mask, mask, (size_t)T * NH, s));
   // accumulated outputs: the fp32 pass adds into zeroed scratch, the sums go into the
   // caller's bf16 tensors afterwards
-  HB_CUDA_OK(cudaMemsetAsync(dR, 0, RW * 4, s));
-  HB_CUDA_OK(cudaMemsetAsync(dW, 0, WW * 4, s));
+  if (!assign_gradients()) {
+    HB_CUDA_OK(cudaMemsetAsync(dR, 0, RW * 4, s));
+    HB_CUDA_OK(cudaMemsetAsync(dW, 0, WW * 4, s));
+  }
   HB_CUDA_OK(cudaMemsetAsync(db, 0, (size_t)4 * H * 4, s));
   HB_CUDA_OK(cudaMemsetAsync(dgWx, 0, (size_t)4 * H * 4, s));
   HB_CUDA_OK(cudaMemsetAsync(dgRh, 0, (size_t)4 * H * 4, s));
@@ -360,15 +364,20 @@ int backward_wide(const LnLstmBwd& a, cudaStream_t s) {
   f.dtype = HASTE_B200_F32;
   f.W = W; f.R = R; f.gamma_Wx = gWx; f.gamma_Rh = gRh; f.gamma_h = gh;
   f.beta_h = a.beta_h ? bh : nullptr;
-  f.x = x; f.h = h; f.c = c; f.dh_new = dhn; f.dc_new = dcn; f.dx = dx; f.dW = dW; f.dR = dR;
+  f.x = x; f.h = h; f.c = c; f.dh_new = dhn; f.dc_new = a.dc_new ? dcn : nullptr; f.dx = dx; f.dW = dW; f.dR = dR;
   f.db = db; f.dgamma_Wx = dgWx; f.dgamma_Rh = dgRh; f.dgamma_h = dgh; f.dbeta_h = dbh;
   f.dh = dh; f.dc = dc; f.zoneout_mask = mask;
   HB_TRY(backward_core(f, s));
   HB_TRY(from_float(BF, dx, a.dx, XN, s));
   HB_TRY(from_float(BF, dh, a.dh, NH, s));
   HB_TRY(from_float(BF, dc, a.dc, NH, s));
-  HB_TRY(add_float_into(BF, dW, a.dW, WW, s));
-  HB_TRY(add_float_into(BF, dR, a.dR, RW, s));
+  if (assign_gradients()) {
+    HB_TRY(from_float(BF, dW, a.dW, WW, s));
+    HB_TRY(from_float(BF, dR, a.dR, RW, s));
+  } else {
+    HB_TRY(add_float_into(BF, dW, a.dW, WW, s));
+    HB_TRY(add_float_into(BF, dR, a.dR, RW, s));
+  }
   HB_TRY(add_float_into(BF, db, a.db, 4 * H, s));
   HB_TRY(add_float_into(BF, dgWx, a.dgamma_Wx, 4 * H, s));
   HB_TRY(add_float_into(BF, dgRh, a.dgamma_Rh, 4 * H, s));
@@ -410,13 +419,23 @@ int layer_norm_lstm_backward(const LnLstmBwd& a, cudaStream_t s) {
   HB_REQUIRE(a.dtype == HASTE_B200_F32 || a.dtype == HASTE_B200_BF16 ||
                  a.dtype == HASTE_B200_BF16_WIDE, "dtype");
   HB_REQUIRE(a.T >= 0 && a.N > 0 && a.C > 0 && a.H > 0, "T,N,C,H");
-  HB_REQUIRE(a.W && a.R && a.gamma_Wx && a.gamma_Rh && a.gamma_h && a.h && a.c && a.dh_new && a.dc_new && a.dW &&
+  HB_REQUIRE(a.W && a.R && a.gamma_Wx && a.gamma_Rh && a.gamma_h && a.h && a.c && a.dh_new && a.dW &&
                  a.dR && a.db && a.dgamma_Wx && a.dgamma_Rh && a.dgamma_h && a.dbeta_h && a.dh && a.dc &&
                  a.act_Wx && a.act_Wx_norm && a.cache_Wx && a.act_Rh && a.cache_Rh &&
                  a.act_c_norm && a.cache_c, "null pointer");
   if (a.T == 0) return HASTE_B200_OK;
   HB_REQUIRE(a.x && a.dx, "x/dx is null");
   HB_REQUIRE((long long)a.T * a.N < (1LL << 31), "T*N too large");
+  if (assign_gradients()) {  // everything below adds, except the two contractions of backward_core
+    const size_t es = dtype_size(a.dtype), H = a.H, NH = (size_t)a.N * H;
+    HB_CUDA_OK(cudaMemsetAsync(a.db, 0, 4 * H * es, s));
+    HB_CUDA_OK(cudaMemsetAsync(a.dgamma_Wx, 0, 4 * H * es, s));
+    HB_CUDA_OK(cudaMemsetAsync(a.dgamma_Rh, 0, 4 * H * es, s));
+    HB_CUDA_OK(cudaMemsetAsync(a.dgamma_h, 0, H * es, s));
+    HB_CUDA_OK(cudaMemsetAsync(a.dbeta_h, 0, H * es, s));
+    HB_CUDA_OK(cudaMemsetAsync(a.dh, 0, NH * es, s));
+    HB_CUDA_OK(cudaMemsetAsync(a.dc, 0, NH * es, s));
+  }
   if (a.dtype == HASTE_B200_BF16_WIDE) return backward_wide(a, s);
   return backward_core(a, s);
 }
@@ -481,13 +500,13 @@ int backward_core(const LnLstmBwd& a, cudaStream_t s) {
   }
   const bool tr = a.transposed_inputs != 0;
   GemmDesc gw{a.dtype, a.dtype, C, 4 * H, (int)TN, a.x, tr ? TN : 1, tr ? 1 : C, a.act_Wx,
-              4LL * H, 1, a.dW, 4LL * H, 1};
+              4LL * H, 1, a.dW, 4LL * H, assign_gradients() ? 0 : 1};
   {
     ProfScope p(PH_WGRAD, s);
     HB_TRY(gemm(gw, s));
   }
   GemmDesc gr{a.dtype, a.dtype, H, 4 * H, (int)TN, a.h, 1, H, a.act_Rh, 4LL * H, 1, a.dR,
-              4LL * H, 1};
+              4LL * H, assign_gradients() ? 0 : 1};
   {
     ProfScope p(PH_WGRAD, s);
     HB_TRY(gemm(gr, s));

@@ -186,7 +186,8 @@ int lstm_backward(const LstmBwd& a, cudaStream_t s) {
   HB_REQUIRE(a.W && a.R && a.h && a.c && a.dh_new && a.dW && a.dR && a.db &&
                  a.dh && a.dc && a.v, "null pointer");
   if (a.T == 0) return HASTE_B200_OK;
-  HB_REQUIRE(a.x && a.dx, "x/dx is null");
+  HB_REQUIRE(a.x, "x is null");
+  const int add = assign_gradients() ? 0 : 1;
   const int N = a.N, H = a.H, C = a.C;
   const long long TN = (long long)a.T * N;
   HB_REQUIRE(TN < (1LL << 31), "T*N too large");
@@ -216,8 +217,13 @@ int lstm_backward(const LstmBwd& a, cudaStream_t s) {
     float* dc_carry = ws.take<float>(NH);
     float* cs = ws.take<float>(colsum_scratch_floats((int)TN, 4 * H));
     HB_REQUIRE(dh_carry && dc_carry && cs, "scratch arena");
-    HB_TRY(to_float(a.dtype, a.dh, dh_carry, NH, s));
-    HB_TRY(to_float(a.dtype, a.dc, dc_carry, NH, s));
+    if (add) {
+      HB_TRY(to_float(a.dtype, a.dh, dh_carry, NH, s));
+      HB_TRY(to_float(a.dtype, a.dc, dc_carry, NH, s));
+    } else {
+      HB_CUDA_OK(cudaMemsetAsync(dh_carry, 0, NH * 4, s));
+      HB_CUDA_OK(cudaMemsetAsync(dc_carry, 0, NH * 4, s));
+    }
     {
       ProfScope p(PH_REC_BWD, s);
       st_ = (a.dtype == HASTE_B200_F32) ? lstm_backward_stepwise<float>(a, dh_carry, dc_carry, s)
@@ -226,7 +232,7 @@ int lstm_backward(const LstmBwd& a, cudaStream_t s) {
     HB_TRY(st_);
     HB_TRY(from_float(a.dtype, dh_carry, a.dh, NH, s));
     HB_TRY(from_float(a.dtype, dc_carry, a.dc, NH, s));
-    HB_TRY(colsum(a.dtype, a.v, 4LL * H, (int)TN, 4 * H, a.dtype, a.db, 1, cs, s));
+    HB_TRY(colsum(a.dtype, a.v, 4LL * H, (int)TN, 4 * H, a.dtype, a.db, add, cs, s));
   }
   HB_TRY(st_);
 
@@ -234,9 +240,9 @@ int lstm_backward(const LstmBwd& a, cudaStream_t s) {
   const bool tr = a.transposed_inputs != 0;
   // dW[C,4H] += x^T . dv
   GemmDesc gw{a.dtype, a.dtype, C, 4 * H, (int)TN, a.x, tr ? TN : 1, tr ? 1 : C, a.v, 4LL * H, 1,
-              a.dW, 4LL * H, 1};
+              a.dW, 4LL * H, add};
   // dR[H,4H] += h[0:T]^T . dv
-  GemmDesc gr{a.dtype, a.dtype, H, 4 * H, (int)TN, a.h, 1, H, a.v, 4LL * H, 1, a.dR, 4LL * H, 1};
+  GemmDesc gr{a.dtype, a.dtype, H, 4 * H, (int)TN, a.h, 1, H, a.v, 4LL * H, 1, a.dR, 4LL * H, add};
   // dx[T*N,C] = dv . W^T
   GemmDesc gx{a.dtype, a.dtype, (int)TN, C, 4 * H, a.v, 4LL * H, 1, a.W, tr ? C : 1,
               tr ? 1 : 4LL * H, a.dx, C, 0};
@@ -253,7 +259,7 @@ int lstm_backward(const LstmBwd& a, cudaStream_t s) {
     ProfScope p(PH_WGRAD, s);
     HB_TRY(gemm(gr, s));
   }
-  {
+  if (a.dx) {
     ProfScope p(PH_DGRAD, s);
     HB_TRY(gemm(gx, s));
   }

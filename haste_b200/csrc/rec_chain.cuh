@@ -23,6 +23,7 @@ struct ChainParams {
   int ring;      // grid forward: partial tiles in flight
   int throttle;  // grid forward: a slot may come round before it is known to be free
   int training, has_zoneout, r_transposed;
+  int zero_init; // backward: dh and dc start at zero instead of what they hold
   int wide;      // rows and pointers allow whole-quad accesses (H a multiple of 4)
   float zoneout_prob;
   const void *R, *b, *b2;

@@ -89,6 +89,7 @@ int run_fwd(ChainParams& p, int dtype, int grid_most, ClRun cl, GlRun gl, cudaSt
 int run_bwd(ChainParams& p, int dtype, int grid_most, int gates, void* db, void* db2, ClRun cl, GlRun gl,
             cudaStream_t s) {
   p.sync.err = device_error_word();
+  p.zero_init = assign_gradients();
   HB_REQUIRE(p.sync.err, "error word");
   const int tiles = ceil_div(p.N, 8);
   ClGeometry cg;
@@ -97,7 +98,7 @@ int run_bwd(ChainParams& p, int dtype, int grid_most, int gates, void* db, void*
     if (!p.db_part) return HASTE_B200_ERR_CUDA;
     int groups = 0;
     const int st_ = cl(dtype, p, cluster_chains(cg, true), &groups, s);
-    if (st_ == HASTE_B200_OK) return bias_grad_finish(gates, p.db_part, groups, p.H, dtype, db, db2, s);
+    if (st_ == HASTE_B200_OK) return bias_grad_finish(gates, p.db_part, groups, p.H, dtype, db, db2, !p.zero_init, s);
     if (st_ != HASTE_B200_ERR_UNSUPPORTED) return st_;
   }
   GlGeometry g;
@@ -105,7 +106,7 @@ int run_bwd(ChainParams& p, int dtype, int grid_most, int gates, void* db, void*
   p.CTAS = g.nHS; p.CH = g.CH; p.K16 = ceil_div(g.nHS * g.NMT, 4);
   HB_TRY(gl_scratch(&p, (size_t)2 * tiles * g.nHS * g.nHS * g.NMT * 32, (size_t)g.nRG * 8 * p.H, &p.db_part, s));
   HB_TRY(gl(dtype, p, g, s));
-  return bias_grad_finish(gates, p.db_part, 2 * g.nRG, p.H, dtype, db, db2, s);
+  return bias_grad_finish(gates, p.db_part, 2 * g.nRG, p.H, dtype, db, db2, !p.zero_init, s);
 }
 
 // Rows the tensor-core GRU recurrence would take (rec_tc_gru.cu).

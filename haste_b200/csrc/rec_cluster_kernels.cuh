@@ -288,8 +288,9 @@ __global__ void __launch_bounds__(NW * 32, 1) cl_bwd_kernel(const __grid_constan
     const bool ok = n < N && unit < H;
     const long long o = (long long)n * H + unit;
     float* cy = carry + (size_t)ch * 3 * NW * 32 + tid;
-    cy[0] = ok ? ld(reinterpret_cast<const T*>(p.dh) + o) : 0.f;
-    cy[NW * 32] = (G == 4 && ok) ? ld(reinterpret_cast<const T*>(p.dc) + o) : 0.f;
+    const bool given = ok && !p.zero_init;
+    cy[0] = given ? ld(reinterpret_cast<const T*>(p.dh) + o) : 0.f;
+    cy[NW * 32] = (G == 4 && given) ? ld(reinterpret_cast<const T*>(p.dc) + o) : 0.f;
     cy[2 * NW * 32] = (G == 4 && ok) ? ld(reinterpret_cast<const T*>(p.c) + (long long)p.T * N * H + o) : 0.f;
   }
   float acc_b[4] = {0.f, 0.f, 0.f, 0.f};

@@ -335,8 +335,9 @@ __global__ void __launch_bounds__(GL_THREADS, 1) gl_bwd_kernel(const __grid_cons
         const bool ok = n < N && unit < H;
         const long long o = (long long)n * H + unit;
         float* cy = carry + (size_t)ch * 3 * NMT * 32 + quad * 32 + lane;
-        cy[0] = ok ? ld(reinterpret_cast<const T*>(p.dh) + o) : 0.f;
-        cy[NMT * 32] = (G == 4 && ok) ? ld(reinterpret_cast<const T*>(p.dc) + o) : 0.f;
+        const bool given = ok && !p.zero_init;
+        cy[0] = given ? ld(reinterpret_cast<const T*>(p.dh) + o) : 0.f;
+        cy[NMT * 32] = (G == 4 && given) ? ld(reinterpret_cast<const T*>(p.dc) + o) : 0.f;
         cy[2 * NMT * 32] = (G == 4 && ok) ? ld(reinterpret_cast<const T*>(p.c) + (long long)p.T * N * H + o) : 0.f;
       }
     float acc_b[4] = {0.f, 0.f, 0.f, 0.f};

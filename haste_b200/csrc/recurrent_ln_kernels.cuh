@@ -774,7 +774,7 @@ __global__ void __launch_bounds__(THREADS, 1) ln_bwd_kernel(const LnBwdParams p)
       inv1[mt] = rok ? ld(cache1 + ((long long)t * N + n) * 2 + 1) : 0.f;
       cprev[mt] = cx3[mt] = cnv[mt] = dcv[mt] = inv3[mt] = hprev[mt] = 0.f;
       if constexpr (G == 4) {
-        dcv[mt] = ok ? ld(dcn + (long long)(t + 1) * NH + o0) : 0.f;
+        dcv[mt] = ok && dcn ? ld(dcn + (long long)(t + 1) * NH + o0) : 0.f;
         cprev[mt] = ok ? ld(cbuf + (long long)t * NH + o0) : 0.f;
         cnv[mt] = ok ? ld(cnbuf + (long long)t * NH + o0) : 0.f;
         const float mean3 = rok ? ld(cache3 + ((long long)t * N + n) * 2) : 0.f;
@@ -795,7 +795,7 @@ __global__ void __launch_bounds__(THREADS, 1) ln_bwd_kernel(const LnBwdParams p)
         prefetch_l2(dhn + (long long)t * NH + o0);
         if (p.has_zoneout) prefetch_l2(mask + (long long)(t - 1) * NH + o0);
         if constexpr (G == 4) {
-          prefetch_l2(dcn + (long long)t * NH + o0);
+          if (dcn) prefetch_l2(dcn + (long long)t * NH + o0);
           prefetch_l2(cbuf + (long long)(t - 1) * NH + o0);
           prefetch_l2(cnbuf + (long long)(t - 1) * NH + o0);
         } else {

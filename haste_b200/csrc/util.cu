@@ -219,15 +219,15 @@ __global__ void colsum_stage2(const float* __restrict__ part, int width, int chu
 
 template <typename T>
 __global__ void bias_grad_kernel(int gates, const float* __restrict__ part, int rows, int H,
-                                 T* __restrict__ db, T* __restrict__ db2) {
+                                 T* __restrict__ db, T* __restrict__ db2, int accumulate) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= 4 * H) return;
   float s = 0.f;
   for (int r = 0; r < rows; ++r) s += part[(long long)r * 4 * H + j];
-  if (gates == 4 || j < 3 * H) st(db + j, ld(db + j) + s);
+  if (gates == 4 || j < 3 * H) st(db + j, accumulate ? ld(db + j) + s : s);
   if (gates == 3 && (j < 2 * H || j >= 3 * H)) {
     T* d = db2 + (j < 2 * H ? j : j - H);
-    st(d, ld(d) + s);
+    st(d, accumulate ? ld(d) + s : s);
   }
 }
 
@@ -296,15 +296,16 @@ int colsum(int in_dtype, const void* in, long long ld_, int rows, int width, int
 }
 
 int bias_grad_finish(int gates, const float* part, int rows, int H, int dtype, void* db, void* db2,
-                     cudaStream_t stream) {
+                     int accumulate, cudaStream_t stream) {
   const int blocks = ceil_div(4LL * H, 128);
   if (dtype == HASTE_B200_F32)
-    bias_grad_kernel<float><<<blocks, 128, 0, stream>>>(gates, part, rows, H, (float*)db, (float*)db2);
+    bias_grad_kernel<float><<<blocks, 128, 0, stream>>>(gates, part, rows, H, (float*)db, (float*)db2, accumulate);
   else if (dtype == HASTE_B200_F16)
-    bias_grad_kernel<__half><<<blocks, 128, 0, stream>>>(gates, part, rows, H, (__half*)db, (__half*)db2);
+    bias_grad_kernel<__half><<<blocks, 128, 0, stream>>>(gates, part, rows, H, (__half*)db, (__half*)db2,
+                                                        accumulate);
   else
     bias_grad_kernel<__nv_bfloat16><<<blocks, 128, 0, stream>>>(gates, part, rows, H,
-                                                                (__nv_bfloat16*)db, (__nv_bfloat16*)db2);
+                                                                (__nv_bfloat16*)db, (__nv_bfloat16*)db2, accumulate);
   HB_LAUNCH_OK();
   count_launch(1);
   return HASTE_B200_OK;

@@ -47,11 +47,11 @@ size_t colsum_scratch_floats(int rows, int width);
 int colsum(int in_dtype, const void* in, long long ld, int rows, int width, int out_dtype,
            void* out, int accumulate, float* scratch, cudaStream_t stream);
 
-// Adds the bias-gradient partials [rows][4H] of a recurrence kernel to the bias gradients, in a
-// fixed order.  LSTM (gates 4): db[4H].  GRU (gates 3), partial columns dp_z, dp_r, dp_g, dq_g:
+// Adds the bias-gradient partials [rows][4H] of a recurrence kernel to the bias gradients (or
+// assigns them), in a fixed order.  LSTM (gates 4): db[4H].  GRU (gates 3), partial columns dp_z, dp_r, dp_g, dq_g:
 // db[3H] takes the first three, db2[3H] dp_z, dp_r, dq_g.
 int bias_grad_finish(int gates, const float* part, int rows, int H, int dtype, void* db, void* db2,
-                     cudaStream_t stream);
+                     int accumulate, cudaStream_t stream);
 
 // dst[i] = (float)src[i] and back, n elements.
 int to_float(int dtype, const void* src, float* dst, size_t n, cudaStream_t stream);

@@ -29,6 +29,15 @@ def _empty_mask(x):
     return x.new_empty(0, 0, 0)
 
 
+_native_forward = None
+
+
+def _load_native():
+    global _native_forward
+    _native_forward = _C.native().forward
+    return _native_forward
+
+
 class _sm_budget:
     """While active, one persistent recurrence launch occupies at most `sms` SMs (0: no
     limit), so that the two directions of a bidirectional level are co-resident."""
@@ -293,6 +302,48 @@ class BaseRNN(nn.Module):
             self._dp.recurrent_scale = scale
         return R * scale
 
+    def _native_applies(self, input, lengths):
+        """The compiled host path takes every call but three: with a data-parallel hook the
+        gradients go to its bucket, `lengths` with gradients index the state slots, and an empty
+        input returns its initial state."""
+        return (self._dp is None and (lengths is None or not torch.is_grad_enabled())
+                and input.numel() > 0)
+
+    def _native_call(self, input, state, lengths, zoneout_mask=None, dropconnect_mask=None):
+        """One call of the layer through torch_ext/native.cc.  A small batch's call is bound by
+        the Python in front of it, so this reads each attribute once and leaves state checks
+        that fail, and modules that are no plain set of parameters, to the general code."""
+        parameters = self._parameters
+        if self._modules or not all([p is not None and p.is_cuda for p in parameters.values()]):
+            self._require_cuda()
+        weights = [parameters[k] if k in parameters else getattr(self, k) for k in self._weights]
+        batch_first, H = self.batch_first, self.hidden_size
+        N = input.shape[0 if batch_first else 1]
+        if self.training and getattr(self, 'dropout', 0.0):
+            weights[1] = self._dropconnect(dropconnect_mask)
+        zoneout = self.zoneout
+        if zoneout or zoneout_mask is not None:
+            zoneout_mask = self._get_zoneout_mask(input.transpose(0, 1) if batch_first else input,
+                                                  zoneout_mask)
+        h0 = c0 = None
+        if state is not None:
+            shape = (1, N, H)
+            if not self._has_c:
+                if getattr(state, 'shape', None) != shape:
+                    _validate_state(state, [1, N, H])
+                h0 = state
+            else:
+                if (type(state) is not tuple or len(state) != 2 or state[0].shape != shape
+                        or state[1].shape != shape):
+                    _validate_state(state, ([1, N, H], [1, N, H]))
+                h0, c0 = state
+        if lengths is not None:
+            lengths = torch.as_tensor(lengths, device=input.device)
+        output, h, c = (_native_forward or _load_native())(
+            self._cell, input, h0, c0, lengths, weights, zoneout_mask, self.training, zoneout,
+            batch_first, self.return_state_sequence, self._sm_budget)
+        return output, ((h, c) if self._has_c else h)
+
     def _require_cuda(self):
         flags = [p.is_cuda for p in self.parameters()]
         if any(flags) and not all(flags):
@@ -310,6 +361,9 @@ def _check_rates(name, dropout, zoneout):
 
 class LSTM(BaseRNN):
     """Long Short-Term Memory layer (gate layout i,g,f,o)."""
+
+    _cell, _has_c = 0, True  # as torch_ext/native.cc numbers the cells
+    _weights = ('kernel', 'recurrent_kernel', 'bias')
 
     def __init__(self, input_size, hidden_size, batch_first=False, forget_bias=1.0, dropout=0.0,
                  zoneout=0.0, return_state_sequence=False):
@@ -351,6 +405,8 @@ class LSTM(BaseRNN):
         nn.init.constant_(self.bias[H * 2:H * 3], self.forget_bias)
 
     def forward(self, input, state=None, lengths=None, zoneout_mask=None, dropconnect_mask=None):
+        if self._native_applies(input, lengths):
+            return self._native_call(input, state, lengths, zoneout_mask, dropconnect_mask)
         self._require_cuda()
         input = self._permute(input)
         shape = [1, input.shape[1], self.hidden_size]
@@ -367,6 +423,9 @@ class LSTM(BaseRNN):
 class GRU(BaseRNN):
     """Gated Recurrent Unit layer (gate layout z,r,g; reset gate applied after the
     recurrent product, as in arXiv 1406.1078v1)."""
+
+    _cell, _has_c = 1, False  # as torch_ext/native.cc numbers the cells
+    _weights = ('kernel', 'recurrent_kernel', 'bias', 'recurrent_bias')
 
     def __init__(self, input_size, hidden_size, batch_first=False, dropout=0.0, zoneout=0.0,
                  return_state_sequence=False):
@@ -408,6 +467,8 @@ class GRU(BaseRNN):
         nn.init.zeros_(self.recurrent_bias)
 
     def forward(self, input, state=None, lengths=None, zoneout_mask=None, dropconnect_mask=None):
+        if self._native_applies(input, lengths):
+            return self._native_call(input, state, lengths, zoneout_mask, dropconnect_mask)
         self._require_cuda()
         input = self._permute(input)
         h0 = self._get_state(input, state, [1, input.shape[1], self.hidden_size])
@@ -422,6 +483,9 @@ class GRU(BaseRNN):
 
 class IndRNN(BaseRNN):
     """Independently Recurrent Neural Network layer: h' = tanh(xW + u*h + b)."""
+
+    _cell, _has_c = 2, False  # as torch_ext/native.cc numbers the cells
+    _weights = ('kernel', 'recurrent_scale', 'bias')
 
     def __init__(self, input_size, hidden_size, batch_first=False, zoneout=0.0,
                  return_state_sequence=False):
@@ -438,6 +502,8 @@ class IndRNN(BaseRNN):
         nn.init.zeros_(self.bias)
 
     def forward(self, input, state=None, lengths=None, zoneout_mask=None):
+        if self._native_applies(input, lengths):
+            return self._native_call(input, state, lengths, zoneout_mask)
         self._require_cuda()
         input = self._permute(input)
         h0 = self._get_state(input, state, [1, input.shape[1], self.hidden_size])
@@ -451,6 +517,9 @@ class IndRNN(BaseRNN):
 
 class LayerNormLSTM(BaseRNN):
     """LSTM with layer normalisation on x.W, h.R and the cell state."""
+
+    _cell, _has_c = 3, True  # as torch_ext/native.cc numbers the cells
+    _weights = ('kernel', 'recurrent_kernel', 'bias', 'gamma', 'gamma_h', 'beta_h')
 
     def __init__(self, input_size, hidden_size, batch_first=False, forget_bias=1.0, dropout=0.0,
                  zoneout=0.0, return_state_sequence=False):
@@ -478,6 +547,8 @@ class LayerNormLSTM(BaseRNN):
         nn.init.zeros_(self.beta_h)
 
     def forward(self, input, state=None, lengths=None, zoneout_mask=None, dropconnect_mask=None):
+        if self._native_applies(input, lengths):
+            return self._native_call(input, state, lengths, zoneout_mask, dropconnect_mask)
         self._require_cuda()
         input = self._permute(input)
         shape = [1, input.shape[1], self.hidden_size]
@@ -494,6 +565,9 @@ class LayerNormLSTM(BaseRNN):
 
 class LayerNormGRU(BaseRNN):
     """GRU with layer normalisation on x.W and h.R."""
+
+    _cell, _has_c = 4, False  # as torch_ext/native.cc numbers the cells
+    _weights = ('kernel', 'recurrent_kernel', 'bias', 'recurrent_bias', 'gamma')
 
     def __init__(self, input_size, hidden_size, batch_first=False, dropout=0.0, zoneout=0.0,
                  return_state_sequence=False):
@@ -517,6 +591,8 @@ class LayerNormGRU(BaseRNN):
         nn.init.ones_(self.gamma)
 
     def forward(self, input, state=None, lengths=None, zoneout_mask=None, dropconnect_mask=None):
+        if self._native_applies(input, lengths):
+            return self._native_call(input, state, lengths, zoneout_mask, dropconnect_mask)
         self._require_cuda()
         input = self._permute(input)
         h0 = self._get_state(input, state, [1, input.shape[1], self.hidden_size])
@@ -531,6 +607,9 @@ class LayerNormGRU(BaseRNN):
 
 class LayerNormIndRNN(BaseRNN):
     """IndRNN with layer normalisation on x.W (`gamma` is [2,H]; row 0 is used)."""
+
+    _cell, _has_c = 5, False  # as torch_ext/native.cc numbers the cells
+    _weights = ('kernel', 'recurrent_scale', 'bias', 'gamma')
 
     def __init__(self, input_size, hidden_size, batch_first=False, zoneout=0.0,
                  return_state_sequence=False):
@@ -549,6 +628,8 @@ class LayerNormIndRNN(BaseRNN):
         nn.init.ones_(self.gamma)
 
     def forward(self, input, state=None, lengths=None, zoneout_mask=None):
+        if self._native_applies(input, lengths):
+            return self._native_call(input, state, lengths, zoneout_mask)
         self._require_cuda()
         input = self._permute(input)
         h0 = self._get_state(input, state, [1, input.shape[1], self.hidden_size])

@@ -97,6 +97,11 @@ int haste_b200_profile_enable(int on);
 int haste_b200_probe_exchange_latency(int N, int H, int steps, float* us_per_step, void* stream);
 int haste_b200_profile_read(float* ms, int n);
 
+/* While on, the sequence backward entry points called from this thread ASSIGN the parameter
+ * gradients, dh and dc instead of accumulating into them, so that a caller with fresh buffers need
+ * not zero them first.  Off by default (the reference's contract). */
+int haste_b200_set_assign_gradients(int on);
+
 /* ---- LSTM -------------------------------------------------------------- */
 /* Replaces lstm::ForwardPass<T>::Run  (lib/haste/lstm.h:118-129,
  * lib/lstm_forward_gpu.cu.cc:313-366).
@@ -110,7 +115,8 @@ int haste_b200_lstm_forward(int dtype, int training, int T, int N, int C, int H,
 
 /* Replaces lstm::BackwardPass<T>::Run  (lib/haste/lstm.h:248-265,
  * lib/lstm_backward_gpu.cu.cc:319-405).
- *   dh_new, dc_new [T+1,N,H] (slot 0 is never read)  dx [T,N,C] assigned
+ *   dh_new, dc_new [T+1,N,H] (slot 0 is never read; dc_new may be NULL: no gradient of c)
+ *   dx [T,N,C] assigned (NULL: not wanted)
  *   dW [C,4H] dR [H,4H] db [4H] dh,dc [N,H] accumulated;  v is overwritten. */
 int haste_b200_lstm_backward(int dtype, int transposed_inputs, int T, int N, int C, int H,
                              const void* W, const void* R, const void* b, const void* x,
