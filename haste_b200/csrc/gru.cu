@@ -181,9 +181,8 @@ int gru_forward(const GruFwd& a, cudaStream_t s) {
              "dtype");
   HB_REQUIRE(a.T >= 0 && a.N > 0 && a.C > 0 && a.H > 0, "T,N,C,H");
   if (a.T == 0) return HASTE_B200_OK;  // nothing to do; scratch pointers may be null
-  HB_REQUIRE(a.W && a.R && a.bx && a.br && a.h && a.tmp_Wx && a.tmp_Rh, "null pointer");
+  HB_REQUIRE(a.W && a.R && a.bx && a.br && a.h, "null pointer");
   HB_REQUIRE(!a.training || a.v, "v is required when training");
-  if (a.T == 0) return HASTE_B200_OK;
   HB_REQUIRE(a.x, "x is null");
   const long long TN = (long long)a.T * a.N;
   HB_REQUIRE(TN < (1LL << 31), "T*N too large");
@@ -193,6 +192,7 @@ int gru_forward(const GruFwd& a, cudaStream_t s) {
     const int st_ = gru_forward_step_fused(a, s);
     if (st_ != HASTE_B200_ERR_UNSUPPORTED) return st_;
   }
+  HB_REQUIRE(a.tmp_Wx && a.tmp_Rh, "null pointer");
   GemmDesc g{a.dtype, a.dtype, (int)TN, 3 * a.H, a.C, a.x, a.C, 1, a.W, 3LL * a.H, 1, a.tmp_Wx,
              3LL * a.H, 0};
   {

@@ -154,9 +154,8 @@ int lstm_forward(const LstmFwd& a, cudaStream_t s) {
   HB_REQUIRE(a.dtype == HASTE_B200_F32 || a.dtype == HASTE_B200_BF16, "dtype");
   HB_REQUIRE(a.T >= 0 && a.N > 0 && a.C > 0 && a.H > 0, "T,N,C,H");
   if (a.T == 0) return HASTE_B200_OK;  // nothing to do; scratch pointers may be null
-  HB_REQUIRE(a.W && a.R && a.b && a.h && a.c && a.v && a.tmp_Rh, "null pointer");
-  HB_REQUIRE(a.T == 0 || a.x, "x is null");
-  if (a.T == 0) return HASTE_B200_OK;
+  HB_REQUIRE(a.W && a.R && a.b && a.h && a.c, "null pointer");
+  HB_REQUIRE(a.x, "x is null");
   const long long TN = (long long)a.T * a.N;
   HB_REQUIRE(TN < (1LL << 31), "T*N too large");
   if (a.T == 1 && a.h_out && recurrence_path() != HASTE_B200_PATH_STEPWISE) {
@@ -165,6 +164,7 @@ int lstm_forward(const LstmFwd& a, cudaStream_t s) {
     const int st_ = lstm_forward_step_fused(a, s);
     if (st_ != HASTE_B200_ERR_UNSUPPORTED) return st_;
   }
+  HB_REQUIRE(a.v && a.tmp_Rh, "null pointer");
   // v = x . W for all steps at once
   GemmDesc g{a.dtype, a.dtype, (int)TN, 4 * a.H, a.C, a.x, a.C, 1, a.W, 4LL * a.H, 1, a.v,
              4LL * a.H, 0};

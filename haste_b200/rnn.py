@@ -311,38 +311,36 @@ class BaseRNN(nn.Module):
 
     def _native_call(self, input, state, lengths, zoneout_mask=None, dropconnect_mask=None):
         """One call of the layer through torch_ext/native.cc.  A small batch's call is bound by
-        the Python in front of it, so this reads each attribute once and leaves state checks
-        that fail, and modules that are no plain set of parameters, to the general code."""
+        the Python in front of it, so this reads each attribute once, and the checks that name
+        what is wrong with a call run after the compiled ones have refused it."""
         parameters = self._parameters
-        if self._modules or not all([p is not None and p.is_cuda for p in parameters.values()]):
-            self._require_cuda()
-        weights = [parameters[k] if k in parameters else getattr(self, k) for k in self._weights]
-        batch_first, H = self.batch_first, self.hidden_size
-        N = input.shape[0 if batch_first else 1]
+        try:
+            weights = [parameters[k] for k in self._weights]
+        except KeyError:  # parametrised modules
+            weights = [getattr(self, k) for k in self._weights]
+        batch_first = self.batch_first
         if self.training and getattr(self, 'dropout', 0.0):
             weights[1] = self._dropconnect(dropconnect_mask)
         zoneout = self.zoneout
         if zoneout or zoneout_mask is not None:
             zoneout_mask = self._get_zoneout_mask(input.transpose(0, 1) if batch_first else input,
                                                   zoneout_mask)
-        h0 = c0 = None
-        if state is not None:
-            shape = (1, N, H)
-            if not self._has_c:
-                if getattr(state, 'shape', None) != shape:
-                    _validate_state(state, [1, N, H])
-                h0 = state
-            else:
-                if (type(state) is not tuple or len(state) != 2 or state[0].shape != shape
-                        or state[1].shape != shape):
-                    _validate_state(state, ([1, N, H], [1, N, H]))
-                h0, c0 = state
         if lengths is not None:
             lengths = torch.as_tensor(lengths, device=input.device)
-        output, h, c = (_native_forward or _load_native())(
-            self._cell, input, h0, c0, lengths, weights, zoneout_mask, self.training, zoneout,
-            batch_first, self.return_state_sequence, self._sm_budget)
-        return output, ((h, c) if self._has_c else h)
+        has_c = self._has_c
+        if has_c and state is not None and type(state) is not tuple:
+            _validate_state(state, ([1, None, None], [1, None, None]))
+        try:
+            h0, c0 = (None, None) if state is None else state if has_c else (state, None)
+            output, h, c = (_native_forward or _load_native())(
+                self._cell, input, h0, c0, lengths, weights, zoneout_mask, self.training, zoneout,
+                batch_first, self.return_state_sequence, self._sm_budget)
+        except (RuntimeError, TypeError, ValueError):
+            self._require_cuda()
+            shape = [1, input.shape[0 if batch_first else 1], self.hidden_size]
+            self._get_state(input, state, (shape, shape) if has_c else shape)
+            raise
+        return output, ((h, c) if has_c else h)
 
     def _require_cuda(self):
         flags = [p.is_cuda for p in self.parameters()]

@@ -103,7 +103,7 @@ struct AssignGradients {
   ~AssignGradients() { lib.set_assign_gradients(0); }
 };
 
-void check(const Tensor& x, at::TensorList ts) {
+void check(const Tensor& x, at::ArrayRef<Tensor> ts) {
   TORCH_CHECK(x.is_cuda(), "haste_b200: tensor must be a CUDA tensor");
   for (const Tensor& t : ts) {
     if (!t.defined() || !t.numel()) continue;
@@ -356,6 +356,7 @@ std::tuple<Tensor, Tensor, c10::optional<Tensor>> forward(
   const int64_t H = cell == INDRNN || cell == LN_INDRNN ? params[0].size(1) : params[1].size(0);
   auto state = [&](const c10::optional<Tensor>& t) {
     if (!t) return Tensor();
+    TORCH_CHECK(t->dim() == 3 && t->size(0) == 1 && t->size(1) == N && t->size(2) == H, "haste_b200: state must be [1,N,H]");
     return t->requires_grad() ? t->select(0, 0).contiguous() : t->contiguous();  // [1,N,H] lies like [N,H]
   };
   Tensor h0 = state(h0_), c0 = state(c0_);
@@ -386,17 +387,23 @@ std::tuple<Tensor, Tensor, c10::optional<Tensor>> forward(
     const void* mp = zo ? mask.data_ptr() : nullptr;
     y = at::empty({1, N, H}, x.options());
     if (!h0.defined()) h0 = at::zeros({N, H}, x.options());
-    Tensor tmp = at::empty({2, N, G * H}, x.options());
-    void* t1 = static_cast<char*>(tmp.data_ptr()) + N * G * H * tmp.element_size();
     if (cell == LSTM) {
       if (!c0.defined()) c0 = at::zeros({N, H}, x.options());
       c = at::empty({1, N, H}, x.options());
-      CALL(lstm_forward_iterate, dt, 0, n, cc, hh, ptr(params[0]), ptr(params[1]), ptr(params[2]), ptr(x), ptr(h0),
-           ptr(c0), ptr(y), ptr(c), ptr(tmp), t1, zp, mp, s);
-    } else {
-      CALL(gru_forward_iterate, dt, 0, n, cc, hh, ptr(params[0]), ptr(params[1]), ptr(params[2]), ptr(params[3]),
-           ptr(x), ptr(h0), ptr(y), nullptr, ptr(tmp), t1, zp, mp, s);
     }
+    auto step = [&](void* t0, void* t1) {
+      return cell == LSTM ? lib.lstm_forward_iterate(dt, 0, n, cc, hh, ptr(params[0]), ptr(params[1]), ptr(params[2]),
+                                                     ptr(x), ptr(h0), ptr(c0), ptr(y), ptr(c), t0, t1, zp, mp, s)
+                          : lib.gru_forward_iterate(dt, 0, n, cc, hh, ptr(params[0]), ptr(params[1]), ptr(params[2]),
+                                                    ptr(params[3]), ptr(x), ptr(h0), ptr(y), nullptr, t0, t1, zp, mp, s);
+    };
+    // up to 64 rows the step is one kernel without scratch; what it does not take comes back at once
+    int status = N > 64 ? HASTE_B200_ERR_INVALID : step(nullptr, nullptr);
+    if (status == HASTE_B200_ERR_INVALID) {
+      Tensor tmp = at::empty({2, N, G * H}, x.options());
+      status = step(tmp.data_ptr(), static_cast<char*>(tmp.data_ptr()) + N * G * H * tmp.element_size());
+    }
+    ok(cell == LSTM ? "lstm_forward_iterate" : "gru_forward_iterate", status);
   } else {
     Forward f = run_forward(cell, training, zoneout, x, h0, c0, mask, params);
     y = f.y;
@@ -404,7 +411,7 @@ std::tuple<Tensor, Tensor, c10::optional<Tensor>> forward(
   }
   auto final_state = [&](const Tensor& seq) {
     if (state_sequence) return (batch_first ? seq.transpose(0, 1) : seq).unsqueeze(0);
-    if (!lengths) return seq.narrow(0, T - 1, 1);
+    if (!lengths) return T == 1 && !graph ? seq : seq.narrow(0, T - 1, 1);
     // the state after lengths[n] steps: slot 0, the initial state, belongs to length 0
     const Tensor slots = seq.as_strided({T + 1, N, H}, {N * H, H, 1}, 0);
     return at::index(slots, {*lengths, at::arange(N, lengths->options().dtype(at::kLong))}).unsqueeze(0);

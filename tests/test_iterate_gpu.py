@@ -144,3 +144,39 @@ def test_fused_single_launch_step_equals_the_general_path(cell, N, C, H, dtype, 
     if training:
         ref_out, _ = oracle.forward_backward(cell, d, zoneout=zoneout)
         assert_close(outs["fused"][0], ref_out["h"][1], tol if bf16 else TOL_F32, "h vs oracle")
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,C,H", [(1, 1, 1), (1, 300, 1024), (4, 7, 18), (3, 65, 250), (5, 16, 33), (8, 129, 16),
+                                   (9, 64, 64), (17, 31, 520), (33, 200, 96), (64, 1024, 40), (65, 24, 32)])
+@pytest.mark.parametrize("cell", ["LSTM", "GRU"])
+def test_single_step_sizes(cell, N, C, H, dtype):
+    """One step in evaluation mode at the edges of the step kernels' tiles, against fp64."""
+    import haste_b200
+    torch.manual_seed(N * 7 + H)
+    layer = getattr(haste_b200, cell)(C, H).cuda().to(dtype).eval()
+    with torch.no_grad():
+        for p in layer.parameters():
+            p.copy_(torch.randn_like(p) * (0.5 if p.dim() == 1 else p.shape[0] ** -0.5))
+    x = torch.randn(1, N, C, device="cuda", dtype=dtype)
+    state = torch.randn(1, N, H, device="cuda", dtype=dtype)
+    state = (state, torch.randn_like(state)) if cell == "LSTM" else state
+    with torch.no_grad():
+        y, final = layer(x, state)
+    d = lambda t: t.double()
+    W, R, b = d(layer.kernel), d(layer.recurrent_kernel), d(layer.bias)
+    if cell == "LSTM":
+        h, c = d(state[0][0]), d(state[1][0])
+        i, g, f, o = (d(x[0]) @ W + h @ R + b).chunk(4, 1)
+        c = f.sigmoid() * c + i.sigmoid() * g.tanh()
+        want = [o.sigmoid() * c.tanh(), c]
+        got = [y[0], final[1][0]]
+    else:
+        h = d(state[0])
+        zx, rx, gx = (d(x[0]) @ W + b).chunk(3, 1)
+        zh, rh, gh = (h @ R + d(layer.recurrent_bias)).chunk(3, 1)
+        z, r = (zx + zh).sigmoid(), (rx + rh).sigmoid()
+        want, got = [z * h + (1 - z) * (gx + r * gh).tanh()], [y[0]]
+    tol = 3e-6 if dtype == torch.float32 else 1e-2
+    for a, ref in zip(got, want):
+        torch.testing.assert_close(a.double(), ref, rtol=tol, atol=tol)
