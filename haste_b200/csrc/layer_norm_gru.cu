@@ -141,7 +141,8 @@ int layer_norm_gru_backward(const LnGruBwd& a, cudaStream_t s) {
   HB_TRY(to_float(a.dtype, a.dh, dh_carry, NH, s));
   // Persistent recurrence first; it adds dgamma_Rh into `acc`.
   HB_CUDA_OK(cudaMemsetAsync(acc, 0, 3 * H * sizeof(float), s));
-  int st_ = layer_norm_gru_backward_persistent(a, dh_carry, acc, GradPlanes{}, s);
+  bool bias_done = false;
+  int st_ = layer_norm_gru_backward_persistent(a, dh_carry, acc, GradPlanes{}, &bias_done, s);
   bool use_acc = st_ == HASTE_B200_OK;
   if (st_ == HASTE_B200_ERR_UNSUPPORTED) {
     void* dgamma1 = a.dgamma_Rh;
@@ -157,8 +158,10 @@ int layer_norm_gru_backward(const LnGruBwd& a, cudaStream_t s) {
   HB_TRY(from_float(a.dtype, dh_carry, a.dh, NH, s));
 
   // dp/dq hold gradients w.r.t. the normalised projections (+ bias).
-  HB_TRY(colsum(a.dtype, a.dp, 3LL * H, (int)TN, 3 * H, a.dtype, a.dbx, 1, cs, s));
-  HB_TRY(colsum(a.dtype, a.dq, 3LL * H, (int)TN, 3 * H, a.dtype, a.dbr, 1, cs, s));
+  if (!bias_done) {
+    HB_TRY(colsum(a.dtype, a.dp, 3LL * H, (int)TN, 3 * H, a.dtype, a.dbx, 1, cs, s));
+    HB_TRY(colsum(a.dtype, a.dq, 3LL * H, (int)TN, 3 * H, a.dtype, a.dbr, 1, cs, s));
+  }
   // LayerNorm 1 backward over all steps, in place on dp.
   HB_TRY(layer_norm_backward(a.dtype, (int)TN, 3 * H, a.gamma_Wx, a.act_Wx, a.dp, a.dp, a.dtype,
                              a.dgamma_Wx, nullptr, a.cache_Wx, lns, s));

@@ -463,7 +463,8 @@ int backward_core(const LnLstmBwd& a, cudaStream_t s) {
   // Persistent recurrence first; it adds its LayerNorm parameter gradients into `acc`.
   HB_CUDA_OK(cudaMemsetAsync(acc, 0, 6 * H * sizeof(float), s));
   if (profile_enabled()) profile_mark(PH_REC_BWD, true, s);
-  int st_ = layer_norm_lstm_backward_persistent(a, dh_carry, dc_carry, acc, GradPlanes{}, s);
+  bool bias_done = false;
+  int st_ = layer_norm_lstm_backward_persistent(a, dh_carry, dc_carry, acc, GradPlanes{}, &bias_done, s);
   bool use_acc = st_ == HASTE_B200_OK;
   if (st_ == HASTE_B200_ERR_UNSUPPORTED) {
     void* dgamma1 = a.dgamma_Rh;
@@ -493,7 +494,8 @@ int backward_core(const LnLstmBwd& a, cudaStream_t s) {
   {
     ProfScope p(PH_OTHER, s);
     // act_Wx_norm now holds the gradient w.r.t. (LN1(x.W) + LN2(h.R) + b).
-    HB_TRY(colsum(a.dtype, a.act_Wx_norm, 4LL * H, (int)TN, 4 * H, a.dtype, a.db, 1, cs, s));
+    if (!bias_done)
+      HB_TRY(colsum(a.dtype, a.act_Wx_norm, 4LL * H, (int)TN, 4 * H, a.dtype, a.db, 1, cs, s));
     // LayerNorm 1 backward over all steps: act_Wx <- d/d(x.W).
     HB_TRY(layer_norm_backward(a.dtype, (int)TN, 4 * H, a.gamma_Wx, a.act_Wx, a.act_Wx_norm,
                                a.act_Wx, a.dtype, a.dgamma_Wx, nullptr, a.cache_Wx, lns, s));

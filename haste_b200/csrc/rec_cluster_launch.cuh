@@ -36,7 +36,8 @@ constexpr int kClMaxChains = 6;
 // carries is the smallest that lets all clusters be resident at once (further clusters would
 // queue behind whole passes); more than `most` (below kClMaxChains) is not taken.  `smem_chain` / `smem_fixed`: dynamic shared memory per chain and
 // besides.  `slots`: resident clusters per (device, cluster size), asked once.
-inline int cl_launch(void (*kernel)(ChainParams), ChainParams& p, int threads, size_t smem_chain, size_t smem_fixed,
+template <typename P>
+int cl_launch(void (*kernel)(P), P& p, int threads, size_t smem_chain, size_t smem_fixed,
                      std::atomic<int> (*slots)[17], int most, int* row_groups, cudaStream_t s) {
   int dev = 0;
   HB_CUDA_OK(cudaGetDevice(&dev));

@@ -183,23 +183,60 @@ int exchange_probe(int N, int H, int steps, float* us_per_step, cudaStream_t s) 
 
 using namespace rec;
 
+namespace {
+
+// The cluster kernels (rec_ln_cluster.cuh), where they take the shape.
+int cluster_forward(LnFwdParams& p, int (*run)(const LnFwdParams&, cudaStream_t), cudaStream_t s) {
+  if (recurrence_path() == HASTE_B200_PATH_STEPWISE) return HASTE_B200_ERR_UNSUPPORTED;
+  p.sync.err = device_error_word();
+  HB_REQUIRE(p.sync.err, "error word");
+  return run(p, s);
+}
+// Adds the LayerNorm parameter gradients into `acc` and the bias gradients into db (GRU: db2 too).
+int cluster_backward(LnBwdParams& p, int gates, float* acc, int dtype, void* db, void* db2,
+                     int (*run)(const LnBwdParams&, float*, int*, cudaStream_t), cudaStream_t s) {
+  if (recurrence_path() == HASTE_B200_PATH_STEPWISE || p.H > 256) return HASTE_B200_ERR_UNSUPPORTED;
+  p.sync.err = device_error_word();
+  HB_REQUIRE(p.sync.err, "error word");
+  const int H = p.H, tiles = ceil_div(p.N, 8);
+  const size_t cwords = colsum_scratch_floats(tiles, gates * H);
+  float* part = static_cast<float*>(workspace(s, ((size_t)tiles * 10 * H + cwords) * sizeof(float), /*slot=*/2));
+  if (!part) return HASTE_B200_ERR_CUDA;
+  float* cs = part + (size_t)tiles * 10 * H;
+  float* db_part = part + (size_t)tiles * 6 * H;
+  p.dgRh_part = part;
+  p.dgh_part = part + (size_t)tiles * 4 * H;
+  p.dbh_part = part + (size_t)tiles * 5 * H;
+  int rows = 0;
+  HB_TRY(run(p, db_part, &rows, s));
+  HB_TRY(bias_grad_finish(gates, db_part, rows, H, dtype, db, db2, 1, s));
+  HB_TRY(colsum(HASTE_B200_F32, part, (long long)gates * H, rows, gates * H, HASTE_B200_F32, acc, 1, cs, s));
+  if (gates == 3) return HASTE_B200_OK;
+  HB_TRY(colsum(HASTE_B200_F32, p.dgh_part, H, rows, H, HASTE_B200_F32, acc + 4 * H, 1, cs, s));
+  return colsum(HASTE_B200_F32, p.dbh_part, H, rows, H, HASTE_B200_F32, acc + 5 * H, 1, cs, s);
+}
+
+}  // namespace
+
 // ---- LayerNormLSTM (recurrent_ln_kernels.cuh) ------------------------------------------
 // Forward: LN(x.W) is already in a.act_Wx_norm.  Four source slices per thread in the
 // statistic exchange limit the kernels to 64 hidden slices, which `supported` guarantees.
 int layer_norm_lstm_forward_persistent(const LnLstmFwd& a, cudaStream_t s) {
+  const bool zo = a.zoneout_prob != 0.0f && a.zoneout_mask != nullptr;
+  LnFwdParams p{a.T, a.N, a.H, 0, 0, 0, a.training, zo ? 1 : 0, a.zoneout_prob, a.R, a.b,
+                nullptr, a.act_Wx_norm, a.gamma_Rh, a.gamma_h, a.beta_h, a.act_Wx_norm, a.act_Rh, a.cache_Rh,
+                a.act_c_norm, a.cache_c, a.h, a.c, a.zoneout_mask, nullptr, nullptr, Sync{}, debug_skip()};
+  const int cl = cluster_forward(p, a.dtype == HASTE_B200_F32 ? run_ln_cl_fwd_f32 : run_ln_cl_fwd_bf16, s);
+  if (cl != HASTE_B200_ERR_UNSUPPORTED) return cl;
   Geometry g;
   if (!supported(a.dtype, a.N, a.H, &g) || g.nHS > 64) return HASTE_B200_ERR_UNSUPPORTED;
-  const int Hx = (a.H + 3) & ~3;
-  const size_t xwords = (size_t)2 * a.N * Hx;
+  p.Hx = (a.H + 3) & ~3;
+  p.nHS = g.nHS;
+  p.MT = g.MT;
+  const size_t xwords = (size_t)2 * a.N * p.Hx;
   const size_t swords = (size_t)2 * 2 * g.nBS * g.MT * 16 * g.nHS * 2;
-  Sync sync;
-  uint32_t* words = nullptr;
-  HB_TRY(make_scratch(xwords + swords + 64, &sync, &words, s));
-  const bool zo = a.zoneout_prob != 0.0f && a.zoneout_mask != nullptr;
-  LnFwdParams p{a.T, a.N, a.H, Hx, g.nHS, g.MT, a.training, zo ? 1 : 0, a.zoneout_prob, a.R, a.b,
-                nullptr, a.act_Wx_norm, a.gamma_Rh, a.gamma_h, a.beta_h, a.act_Wx_norm, a.act_Rh, a.cache_Rh,
-                a.act_c_norm, a.cache_c, a.h, a.c, a.zoneout_mask, words,
-                words + ((xwords + 63) & ~size_t(63)), sync, debug_skip()};
+  HB_TRY(make_scratch(xwords + swords + 64, &p.sync, &p.xbuf, s));
+  p.sbuf = p.xbuf + ((xwords + 63) & ~size_t(63));
   return a.dtype == HASTE_B200_F32 ? run_ln_fwd_f32(p, g, s) : run_ln_fwd_bf16(p, g, s);
 }
 
@@ -207,26 +244,33 @@ int layer_norm_lstm_forward_persistent(const LnLstmFwd& a, cudaStream_t s) {
 // per-row-group partial sums of the kernel are added into (fixed order).  As for the plain
 // LSTM, the recurrent contribution of step 0 to dh is added here by one small contraction.
 int layer_norm_lstm_backward_persistent(const LnLstmBwd& a, float* dh_carry, float* dc_carry,
-                                        float* acc, const GradPlanes& planes, cudaStream_t s) {
+                                        float* acc, const GradPlanes& planes, bool* bias_done, cudaStream_t s) {
+  const int H = a.H;
+  LnBwdParams p{a.T, a.N, H, 0, 0, a.zoneout_mask ? 1 : 0, a.transposed_inputs, a.R,
+                a.gamma_Rh, a.gamma_h, a.c, nullptr, nullptr, nullptr, a.act_Wx_norm, a.act_Rh,
+                a.cache_Rh, a.act_c_norm,
+                a.cache_c, a.dh_new, a.dc_new, a.zoneout_mask, dh_carry, dc_carry, nullptr, nullptr, nullptr,
+                nullptr, nullptr, Sync{}, planes.p, planes.p2, planes.stride, debug_skip()};
+  const int cl = cluster_backward(p, 4, acc, a.dtype, a.db, nullptr,
+                                  a.dtype == HASTE_B200_F32 ? run_ln_cl_bwd_f32 : run_ln_cl_bwd_bf16, s);
+  *bias_done = cl == HASTE_B200_OK;
+  if (cl != HASTE_B200_ERR_UNSUPPORTED) return cl;
   Geometry g;
   if (!supported(a.dtype, a.N, a.H, &g) || g.nHS > 64) return HASTE_B200_ERR_UNSUPPORTED;
-  const int H = a.H;
+  p.nHS = g.nHS;
+  p.MT = g.MT;
   const size_t ewords = ((size_t)2 * g.nBS * g.nHS * g.nHS * g.MT * 16 * U + 63) & ~size_t(63);
   const size_t swords = ((size_t)2 * 2 * g.nBS * g.MT * 16 * g.nHS * 2 + 63) & ~size_t(63);
   const int prow = g.nBS * 16;
   const size_t pwords = (size_t)prow * 6 * H;
   const size_t cwords = colsum_scratch_floats(prow, 4 * H);
-  Sync sync;
-  uint32_t* words = nullptr;
-  HB_TRY(make_scratch(ewords + swords + pwords + cwords + 64, &sync, &words, s));
-  float* part = reinterpret_cast<float*>(words + ewords + swords);
+  HB_TRY(make_scratch(ewords + swords + pwords + cwords + 64, &p.sync, &p.exch, s));
+  p.sbuf = p.exch + ewords;
+  float* part = reinterpret_cast<float*>(p.sbuf + swords);
   float* cs = part + pwords;
-  LnBwdParams p{a.T, a.N, H, g.nHS, g.MT, a.zoneout_mask ? 1 : 0, a.transposed_inputs, a.R,
-                a.gamma_Rh, a.gamma_h, a.c, nullptr, nullptr, nullptr, a.act_Wx_norm, a.act_Rh,
-                a.cache_Rh, a.act_c_norm,
-                a.cache_c, a.dh_new, a.dc_new, a.zoneout_mask, dh_carry, dc_carry, part,
-                part + (size_t)prow * 4 * H, part + (size_t)prow * 5 * H, words, words + ewords,
-                sync, planes.p, planes.p2, planes.stride, debug_skip()};
+  p.dgRh_part = part;
+  p.dgh_part = part + (size_t)prow * 4 * H;
+  p.dbh_part = part + (size_t)prow * 5 * H;
   int st_ = a.dtype == HASTE_B200_F32 ? run_ln_bwd_f32(p, g, s) : run_ln_bwd_bf16(p, g, s);
   if (st_ != HASTE_B200_OK) return st_;
   HB_TRY(colsum(HASTE_B200_F32, part, 4LL * H, prow, 4 * H, HASTE_B200_F32, acc, 1, cs, s));
@@ -243,44 +287,51 @@ int layer_norm_lstm_backward_persistent(const LnLstmBwd& a, float* dh_carry, flo
 // ---- LayerNormGRU (the G = 3 instantiation of the same kernels) ---------------------------
 // Forward: LN(x.W) is already in a.tmp_Wx_norm.
 int layer_norm_gru_forward_persistent(const LnGruFwd& a, cudaStream_t s) {
+  const bool zo = a.zoneout_prob != 0.0f && a.zoneout_mask != nullptr;
+  LnFwdParams p{a.T, a.N, a.H, 0, 0, 0, a.training, zo ? 1 : 0, a.zoneout_prob, a.R, a.bx,
+                a.br, a.tmp_Wx_norm, a.gamma_Rh, nullptr, nullptr, a.v, a.act_Rh, a.cache_Rh,
+                nullptr, nullptr, a.h, nullptr, a.zoneout_mask, nullptr, nullptr, Sync{}};
+  const int cl = cluster_forward(p, a.dtype == HASTE_B200_F32 ? run_lngru_cl_fwd_f32 : run_lngru_cl_fwd_bf16, s);
+  if (cl != HASTE_B200_ERR_UNSUPPORTED) return cl;
   Geometry g;
   if (!supported(a.dtype, a.N, a.H, &g) || g.nHS > 64) return HASTE_B200_ERR_UNSUPPORTED;
-  const int Hx = (a.H + 3) & ~3;
-  const size_t xwords = (size_t)2 * a.N * Hx;
+  p.Hx = (a.H + 3) & ~3;
+  p.nHS = g.nHS;
+  p.MT = g.MT;
+  const size_t xwords = (size_t)2 * a.N * p.Hx;
   const size_t swords = (size_t)2 * 2 * g.nBS * g.MT * 16 * g.nHS * 2;
-  Sync sync;
-  uint32_t* words = nullptr;
-  HB_TRY(make_scratch(xwords + swords + 64, &sync, &words, s));
-  const bool zo = a.zoneout_prob != 0.0f && a.zoneout_mask != nullptr;
-  LnFwdParams p{a.T, a.N, a.H, Hx, g.nHS, g.MT, a.training, zo ? 1 : 0, a.zoneout_prob, a.R, a.bx,
-                a.br, a.tmp_Wx_norm, a.gamma_Rh, nullptr, nullptr, a.v, a.act_Rh, a.cache_Rh,
-                nullptr, nullptr, a.h, nullptr, a.zoneout_mask, words,
-                words + ((xwords + 63) & ~size_t(63)), sync};
+  HB_TRY(make_scratch(xwords + swords + 64, &p.sync, &p.xbuf, s));
+  p.sbuf = p.xbuf + ((xwords + 63) & ~size_t(63));
   return a.dtype == HASTE_B200_F32 ? run_lngru_fwd_f32(p, g, s) : run_lngru_fwd_bf16(p, g, s);
 }
 
 // Backward.  `acc` is the fp32 accumulator [3H] for dgamma_Rh.  a.act_Rh is overwritten with
 // d(h.R); a.dp / a.dq receive the gradients w.r.t. the normalised projections (+ biases).
 int layer_norm_gru_backward_persistent(const LnGruBwd& a, float* dh_carry, float* acc,
-                                       const GradPlanes& planes, cudaStream_t s) {
+                                       const GradPlanes& planes, bool* bias_done, cudaStream_t s) {
+  const int H = a.H;
+  LnBwdParams p{a.T, a.N, H, 0, 0, a.zoneout_mask ? 1 : 0, a.transposed_inputs, a.R,
+                a.gamma_Rh, nullptr, nullptr, a.h, a.dp, a.dq, const_cast<void*>(a.v), a.act_Rh,
+                a.cache_Rh, nullptr, nullptr, a.dh_new, nullptr, a.zoneout_mask, dh_carry, nullptr,
+                nullptr, nullptr, nullptr, nullptr, nullptr, Sync{}, planes.p, planes.p2, planes.stride};
+  const int cl = cluster_backward(p, 3, acc, a.dtype, a.dbx, a.dbr,
+                                  a.dtype == HASTE_B200_F32 ? run_lngru_cl_bwd_f32 : run_lngru_cl_bwd_bf16, s);
+  *bias_done = cl == HASTE_B200_OK;
+  if (cl != HASTE_B200_ERR_UNSUPPORTED) return cl;
   Geometry g;
   if (!supported(a.dtype, a.N, a.H, &g) || g.nHS > 64) return HASTE_B200_ERR_UNSUPPORTED;
-  const int H = a.H;
+  p.nHS = g.nHS;
+  p.MT = g.MT;
   const size_t ewords = ((size_t)2 * g.nBS * g.nHS * g.nHS * g.MT * 16 * U + 63) & ~size_t(63);
   const size_t swords = ((size_t)2 * 2 * g.nBS * g.MT * 16 * g.nHS * 2 + 63) & ~size_t(63);
   const int prow = g.nBS * 16;
   const size_t pwords = (size_t)prow * 3 * H;
   const size_t cwords = colsum_scratch_floats(prow, 3 * H);
-  Sync sync;
-  uint32_t* words = nullptr;
-  HB_TRY(make_scratch(ewords + swords + pwords + cwords + 64, &sync, &words, s));
-  float* part = reinterpret_cast<float*>(words + ewords + swords);
+  HB_TRY(make_scratch(ewords + swords + pwords + cwords + 64, &p.sync, &p.exch, s));
+  p.sbuf = p.exch + ewords;
+  float* part = reinterpret_cast<float*>(p.sbuf + swords);
   float* cs = part + pwords;
-  LnBwdParams p{a.T, a.N, H, g.nHS, g.MT, a.zoneout_mask ? 1 : 0, a.transposed_inputs, a.R,
-                a.gamma_Rh, nullptr, nullptr, a.h, a.dp, a.dq, const_cast<void*>(a.v), a.act_Rh,
-                a.cache_Rh, nullptr, nullptr, a.dh_new, nullptr, a.zoneout_mask, dh_carry, nullptr,
-                part, nullptr, nullptr, words, words + ewords, sync, planes.p, planes.p2,
-                planes.stride};
+  p.dgRh_part = part;
   int st_ = a.dtype == HASTE_B200_F32 ? run_lngru_bwd_f32(p, g, s) : run_lngru_bwd_bf16(p, g, s);
   if (st_ != HASTE_B200_OK) return st_;
   HB_TRY(colsum(HASTE_B200_F32, part, 3LL * H, prow, 3 * H, HASTE_B200_F32, acc, 1, cs, s));

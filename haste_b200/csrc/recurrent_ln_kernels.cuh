@@ -1174,6 +1174,15 @@ int run_ln_bwd(LnBwdParams& p, const Geometry& g, cudaStream_t s) {
   return HASTE_B200_ERR_UNSUPPORTED;
 }
 
+// Clusters (rec_ln_cluster.cuh): HASTE_B200_ERR_UNSUPPORTED beyond 256 units.
+int run_ln_cl_fwd_f32(const LnFwdParams& p, cudaStream_t s);
+int run_ln_cl_fwd_bf16(const LnFwdParams& p, cudaStream_t s);
+int run_lngru_cl_fwd_f32(const LnFwdParams& p, cudaStream_t s);
+int run_lngru_cl_fwd_bf16(const LnFwdParams& p, cudaStream_t s);
+int run_ln_cl_bwd_f32(const LnBwdParams& p, float* db_part, int* row_groups, cudaStream_t s);
+int run_ln_cl_bwd_bf16(const LnBwdParams& p, float* db_part, int* row_groups, cudaStream_t s);
+int run_lngru_cl_bwd_f32(const LnBwdParams& p, float* db_part, int* row_groups, cudaStream_t s);
+int run_lngru_cl_bwd_bf16(const LnBwdParams& p, float* db_part, int* row_groups, cudaStream_t s);
 int run_ln_fwd_f32(LnFwdParams& p, const Geometry& g, cudaStream_t s);
 int run_ln_fwd_bf16(LnFwdParams& p, const Geometry& g, cudaStream_t s);
 int run_ln_bwd_f32(LnBwdParams& p, const Geometry& g, cudaStream_t s);
