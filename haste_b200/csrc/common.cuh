@@ -127,6 +127,8 @@ struct GemmDesc {
 };
 int gemm(const GemmDesc& g, cudaStream_t stream);
 int gemm_simt(const GemmDesc& g, cudaStream_t stream);
+// Whether a contraction with a_pl / b_pl reads nothing but the planes (its a / b may then be null).
+bool gemm_reads_planes(const GemmDesc& g);
 // fp32 [rows, cols] -> two bf16 planes (hi, lo), the a_pl / b_pl form, for an operand that
 // more than one contraction reads (gemm_sm100.cu).
 int gemm_split_planes(const float* src, long long ld_src, int rows, int cols,

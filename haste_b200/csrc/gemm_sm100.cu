@@ -24,6 +24,7 @@
 // Replaces the cuBLAS calls of the reference (lib/blas.h:48-61 and the call sites in
 // lib/*_gpu.cu.cc).
 #include <atomic>
+#include <type_traits>
 
 #include "cells.cuh"
 #include "tcgen05.cuh"
@@ -47,7 +48,8 @@ struct Params {
   int c_is_bf16, accumulate;   // direct epilogue only; c_is_bf16: 0 fp32, 1 bf16, 2 fp16 output
   void* c;
   long long ldc;
-  float* partial;              // non-null: write fp32 partial tiles [split][M][N]
+  float* partial;              // non-null: write fp32 partial tiles [split][M][partial_ld]
+  int partial_ld;              // N rounded up to whole 32-column chunks
   int* err;
 };
 
@@ -78,17 +80,13 @@ struct Cfg {
 __device__ __forceinline__ void store_chunk(const Params& p, int sp, int m, int nb,
                                       const uint32_t (&r)[32]) {
   if (m < p.M && nb < p.N) {
-    if (p.partial) {
-      float* dst = p.partial + ((long long)sp * p.M + m) * p.N + nb;
-      if (nb + 32 <= p.N && (p.N & 3) == 0) {
+    if (p.partial) {  // rows of whole chunks, 16-byte aligned
+      float* dst = p.partial + ((long long)sp * p.M + m) * p.partial_ld + nb;
 #pragma unroll
-        for (int j = 0; j < 32; j += 4)
-          *reinterpret_cast<float4*>(dst + j) =
-              make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
-                          __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
-      } else {
-        for (int j = 0; j < 32 && nb + j < p.N; ++j) dst[j] = __uint_as_float(r[j]);
-      }
+      for (int j = 0; j < 32; j += 4)
+        *reinterpret_cast<float4*>(dst + j) =
+            make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
+                        __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
     } else if (p.c_is_bf16) {
       __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.c) + (long long)m * p.ldc + nb;
       if (nb + 32 <= p.N && (p.ldc & 7) == 0 &&
@@ -639,9 +637,10 @@ __global__ void split_planes_kernel(const TS* __restrict__ src, long long ld_src
         const float4 f = *reinterpret_cast<const float4*>(sp);
         x[0] = f.x; x[1] = f.y; x[2] = f.z; x[3] = f.w;
       } else {
+        typedef typename std::conditional<std::is_same<TS, __half>::value, __half2, __nv_bfloat162>::type Pair;
         const uint2 u = *reinterpret_cast<const uint2*>(sp);
-        const __half2 h0 = *reinterpret_cast<const __half2*>(&u.x);
-        const __half2 h1 = *reinterpret_cast<const __half2*>(&u.y);
+        const Pair h0 = *reinterpret_cast<const Pair*>(&u.x);
+        const Pair h1 = *reinterpret_cast<const Pair*>(&u.y);
         x[0] = __low2float(h0); x[1] = __high2float(h0);
         x[2] = __low2float(h1); x[3] = __high2float(h1);
       }
@@ -665,13 +664,17 @@ __global__ void split_planes_kernel(const TS* __restrict__ src, long long ld_src
   }
 }
 
-// `half_src`: the source is __half (its 11 significant bits split exactly into two planes).
-int launch_split(const void* src, bool half_src, long long ld_src, int rows, int cols,
+// `dtype` of the source.  __half: its 11 significant bits split exactly into two planes.  bf16: one
+// plane, a copy with rows that TMA can address.
+int launch_split(const void* src, int dtype, long long ld_src, int rows, int cols,
                  __nv_bfloat16* dst, long long ld_dst, long long plane_stride, int planes,
                  int blocks, cudaStream_t stream) {
   const int vec_ok = ((ld_src & 3) == 0) &&
-                     ((reinterpret_cast<uintptr_t>(src) & (half_src ? 7 : 15)) == 0);
-  if (half_src) {
+                     ((reinterpret_cast<uintptr_t>(src) & (dtype == HASTE_B200_F32 ? 15 : 7)) == 0);
+  if (dtype == HASTE_B200_BF16) {
+    split_planes_kernel<1, __nv_bfloat16><<<blocks, 256, 0, stream>>>(
+        static_cast<const __nv_bfloat16*>(src), ld_src, rows, cols, dst, ld_dst, plane_stride, vec_ok);
+  } else if (dtype == HASTE_B200_F16) {
     const __half* hs = static_cast<const __half*>(src);
     if (planes == 3)
       split_planes_kernel<3, __half><<<blocks, 256, 0, stream>>>(hs, ld_src, rows, cols, dst, ld_dst,
@@ -692,15 +695,19 @@ int launch_split(const void* src, bool half_src, long long ld_src, int rows, int
   return HASTE_B200_OK;
 }
 
+// Adds up the partial tiles of a K split ([splits][M][ld]) into C.
 template <typename TC>
-__global__ void splitk_reduce_kernel(const float* __restrict__ part, int splits, long long MN,
-                                     int N, TC* __restrict__ c, long long ldc, int accumulate) {
+__global__ void splitk_reduce_kernel(const float* __restrict__ part, int splits, long long split_stride,
+                                     int M, int N, int ld_part, TC* __restrict__ c, long long ldc, int accumulate) {
+  const long long MN = (long long)M * N;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < MN;
        i += (long long)gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int k = 0; k < splits; ++k) s += part[k * MN + i];
     const long long m = i / N;
-    TC* dst = c + m * ldc + (i - m * N);
+    const int n = (int)(i - m * N);
+    const float* src = part + m * ld_part + n;
+    float s = 0.f;
+    for (int k = 0; k < splits; ++k) s += src[k * split_stride];
+    TC* dst = c + m * ldc + n;
     if (accumulate) s += ld(dst);
     st(dst, s);
   }
@@ -778,27 +785,36 @@ int max_pairs() {
 int gemm_split_planes(const float* src, long long ld_src, int rows, int cols,
                       __nv_bfloat16* dst, long long ld_dst, long long plane_stride,
                       cudaStream_t stream) {
-  return launch_split(src, false, ld_src, rows, cols, dst, ld_dst, plane_stride, 2,
+  return launch_split(src, HASTE_B200_F32, ld_src, rows, cols, dst, ld_dst, plane_stride, 2,
                       8 * sm_count(), stream);
 }
+
+namespace {
+// Why this file's kernels do not take a contraction; null if they do.
+const char* refusal(const GemmDesc& g) {
+  if (!encode_fn()) return "cuTensorMapEncodeTiled not available";
+  if (g.K <= 0) return "K == 0";
+  // Small problems are launch-bound either way; keep them on the generic kernel.
+  if ((long long)g.M * g.N * g.K < (1LL << 21) || g.M < 32 || g.N < 32)
+    return "problem too small for the tensor-core path";
+  if ((g.a_cs != 1 && g.a_rs != 1) || (g.b_rs != 1 && g.b_cs != 1)) return "operand has no unit stride";
+  return nullptr;
+}
+}  // namespace
+
+bool gemm_reads_planes(const GemmDesc& g) { return gemm_path() != HASTE_B200_GEMM_SIMT && !refusal(g); }
 
 int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
   auto unsupported = [](const char* why) {
     set_last_error("gemm_sm100: %s", why);
     return HASTE_B200_ERR_UNSUPPORTED;
   };
-  if (!encode_fn()) return unsupported("cuTensorMapEncodeTiled not available");
   if (g.M <= 0 || g.N <= 0) return HASTE_B200_OK;
-  if (g.K <= 0) return unsupported("K == 0");
-  // Small problems are launch-bound either way; keep them on the generic kernel.
-  if ((long long)g.M * g.N * g.K < (1LL << 21) || g.M < 32 || g.N < 32)
-    return unsupported("problem too small for the tensor-core path");
+  if (const char* why = refusal(g)) return unsupported(why);
   // __half storage takes the split path too: a half splits exactly into two bf16 planes
   const bool half_src = g.dtype == HASTE_B200_F16;
   const bool f32 = g.dtype == HASTE_B200_F32 || half_src;
-  const bool a_k = g.a_cs == 1, a_m = g.a_rs == 1 && !a_k;
-  const bool b_k = g.b_rs == 1, b_n = g.b_cs == 1 && !b_k;
-  if (!(a_k || a_m) || !(b_k || b_n)) return unsupported("operand has no unit stride");
+  const bool a_k = g.a_cs == 1, b_k = g.b_rs == 1;
 
   const int M = g.M, N = g.N, K = g.K;
   Operand A, B;
@@ -848,44 +864,48 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
   };
   const bool a_pre = planes_usable(g.a_pl, g.a_pl_ld) && (g.a_pl_stride % 8) == 0;
   const bool b_pre = planes_usable(g.b_pl, g.b_pl_ld) && (g.b_pl_stride % 8) == 0;
-  const long long a_ld = a_pre ? g.a_pl_ld : (f32 ? ((a_cols + 7) & ~7LL) : a_ld_src);
-  const long long b_ld = b_pre ? g.b_pl_ld : (f32 ? ((b_cols + 7) & ~7LL) : b_ld_src);
-  if (!f32) {
-    if ((a_ld % 8) || (b_ld % 8) || ((uintptr_t)g.a & 15) || ((uintptr_t)g.b & 15))
-      return unsupported("bf16 operand not 16-byte aligned for TMA");
-  }
+  // An operand goes through scratch if it has to be split or if TMA cannot address its rows
+  // (bf16 with a row or a start that is no multiple of 16 bytes: the copy costs two passes over the
+  // operand, the CUDA-core kernel that would take it as it is twenty times the contraction).
+  const bool a_copy = f32 ? !a_pre : (a_ld_src % 8) != 0 || ((uintptr_t)g.a & 15) != 0;
+  const bool b_copy = f32 ? !b_pre : (b_ld_src % 8) != 0 || ((uintptr_t)g.b & 15) != 0;
+  const long long a_ld = a_pre ? g.a_pl_ld : (a_copy ? ((a_cols + 7) & ~7LL) : a_ld_src);
+  const long long b_ld = b_pre ? g.b_pl_ld : (b_copy ? ((b_cols + 7) & ~7LL) : b_ld_src);
   const int planes = f32 ? (g.precise ? 3 : 2) : 1;
-  const size_t a_plane = (f32 && !a_pre) ? Arena::pad((size_t)a_rows * a_ld * 2) : 0;
-  const size_t b_plane = (f32 && !b_pre) ? Arena::pad((size_t)b_rows * b_ld * 2) : 0;
-  const size_t part_bytes = splits > 1 ? Arena::pad((size_t)splits * M * N * 4) : 0;
+  const size_t a_plane = a_copy ? Arena::pad((size_t)a_rows * a_ld * 2) : 0;
+  const size_t b_plane = b_copy ? Arena::pad((size_t)b_rows * b_ld * 2) : 0;
+  // The epilogue stores a row per lane in 16-byte pieces.  Element by element - a C whose rows do
+  // not start on 16 bytes - each store touches 32 lines and the epilogue took five times the MMAs
+  // ([12321 x 161] . [161 x 750] in fp32: 56 us), so such a C goes through a padded fp32 tile as
+  // the parts of a K split do, and the reduction writes it row by row.
+  const bool c_rows = (g.ldc % (g.dtype_c == HASTE_B200_F32 ? 4 : 8)) == 0 && ((uintptr_t)g.c & 15) == 0;
+  const bool via_partial = splits > 1 || (!c_rows && M >= 64);
+  const int part_ld = (N + 31) & ~31;
+  const size_t part_bytes = via_partial ? Arena::pad((size_t)splits * M * part_ld * 4) : 0;
   const size_t bytes = planes * (a_plane + b_plane) + part_bytes + 1024;
   Arena ws;
   HB_TRY(make_arena(&ws, stream, bytes, /*slot=*/1));
   int* err = device_error_word();
   if (!err) return unsupported("error word allocation failed");
-  if (f32) {
-    __nv_bfloat16* ap = ws.take<__nv_bfloat16>(planes * a_plane / 2);
-    __nv_bfloat16* bp = ws.take<__nv_bfloat16>(planes * b_plane / 2);
-    if (!ap || !bp) return unsupported("scratch arena");
-    const int blocks = 8 * sms;
-    if (!a_pre)
-      HB_TRY(launch_split(g.a, half_src, a_ld_src, (int)a_rows, (int)a_cols, ap, a_ld,
-                          a_plane / 2, planes, blocks, stream));
-    if (!b_pre)
-      HB_TRY(launch_split(g.b, half_src, b_ld_src, (int)b_rows, (int)b_cols, bp, b_ld,
-                          b_plane / 2, planes, blocks, stream));
-    A.base = ap; A.plane_stride = a_plane / 2;
-    B.base = bp; B.plane_stride = b_plane / 2;
-    if (a_pre) { A.base = g.a_pl; A.plane_stride = g.a_pl_stride; }
-    if (b_pre) { B.base = g.b_pl; B.plane_stride = g.b_pl_stride; }
-  } else {
-    A.base = g.a; A.plane_stride = 0;
-    B.base = g.b; B.plane_stride = 0;
-  }
+  A.base = a_pre ? g.a_pl : g.a;
+  A.plane_stride = a_pre ? g.a_pl_stride : 0;
+  B.base = b_pre ? g.b_pl : g.b;
+  B.plane_stride = b_pre ? g.b_pl_stride : 0;
+  auto through_scratch = [&](const void* src, long long ld_src, long long rows, long long cols, size_t plane,
+                             long long ld, Operand* o) -> int {
+    __nv_bfloat16* to = ws.take<__nv_bfloat16>(planes * plane / 2);
+    if (!to) return unsupported("scratch arena");
+    HB_TRY(launch_split(src, g.dtype, ld_src, (int)rows, (int)cols, to, ld, plane / 2, planes, 8 * sms, stream));
+    o->base = to;
+    o->plane_stride = plane / 2;
+    return HASTE_B200_OK;
+  };
+  if (a_copy) HB_TRY(through_scratch(g.a, a_ld_src, a_rows, a_cols, a_plane, a_ld, &A));
+  if (b_copy) HB_TRY(through_scratch(g.b, b_ld_src, b_rows, b_cols, b_plane, b_ld, &B));
   A.ld = a_ld;
   B.ld = b_ld;
   float* partial = nullptr;
-  if (splits > 1) {
+  if (via_partial) {
     partial = ws.take<float>(part_bytes / 4);
     if (!partial) return unsupported("scratch arena");
   }
@@ -908,6 +928,7 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
   p.accumulate = g.accumulate;
   p.c = g.c; p.ldc = g.ldc;
   p.partial = partial;
+  p.partial_ld = part_ld;
   p.err = err;
 
   HB_TRY(set_kernel_attributes());
@@ -944,18 +965,18 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
   }
   HB_LAUNCH_OK();
   count_launch(1);
-  if (splits > 1) {
-    const long long MN = (long long)M * N;
-    const int blocks = min(ceil_div(MN, 256), 8 * sms);
+  if (via_partial) {
+    const int blocks = min(ceil_div((long long)M * N, 256), 8 * sms);
+    const long long stride = (long long)M * part_ld;
     if (g.dtype_c == HASTE_B200_BF16)
-      splitk_reduce_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(
-          partial, splits, MN, N, (__nv_bfloat16*)g.c, g.ldc, g.accumulate);
+      splitk_reduce_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(partial, splits, stride, M, N, part_ld,
+                                                                      (__nv_bfloat16*)g.c, g.ldc, g.accumulate);
     else if (g.dtype_c == HASTE_B200_F16)
-      splitk_reduce_kernel<__half><<<blocks, 256, 0, stream>>>(partial, splits, MN, N,
-                                                                (__half*)g.c, g.ldc, g.accumulate);
+      splitk_reduce_kernel<__half><<<blocks, 256, 0, stream>>>(partial, splits, stride, M, N, part_ld,
+                                                               (__half*)g.c, g.ldc, g.accumulate);
     else
-      splitk_reduce_kernel<float><<<blocks, 256, 0, stream>>>(partial, splits, MN, N, (float*)g.c,
-                                                              g.ldc, g.accumulate);
+      splitk_reduce_kernel<float><<<blocks, 256, 0, stream>>>(partial, splits, stride, M, N, part_ld,
+                                                              (float*)g.c, g.ldc, g.accumulate);
     HB_LAUNCH_OK();
     count_launch(1);
   }
