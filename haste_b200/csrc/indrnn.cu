@@ -12,10 +12,14 @@
 namespace hb {
 namespace {
 
-constexpr int AHEAD = 8;  // independent loads in flight per thread
+constexpr int AHEAD = 8;  // steps whose inputs are loaded together
 
-template <typename T, bool Training, bool Zoneout>
-__global__ void indrnn_scan_fwd(int T_, long long NH, int H, const T* __restrict__ Wx,
+// Piped: a group's loads are issued before the group in front of it is computed.  With few (batch,
+// unit) pairs the GPU has too little in flight to hide a group's latency behind other threads, and
+// the scan took T / 8 latencies; with many, the registers cost more threads than that wins.  The
+// line lies where the pairs no longer fit in half of the resident threads (see scan_blocks).
+template <typename T, bool Training, bool Zoneout, bool Piped>
+__global__ void __launch_bounds__(128) indrnn_scan_fwd(int T_, long long NH, int H, const T* __restrict__ Wx,
                                 const T* __restrict__ u, const T* __restrict__ b,
                                 T* __restrict__ h, float zoneout_prob,
                                 const T* __restrict__ mask) {
@@ -24,14 +28,20 @@ __global__ void indrnn_scan_fwd(int T_, long long NH, int H, const T* __restrict
   const int j = (int)(idx % H);
   const float uj = ld(u + j), bj = ld(b + j);
   float hp = ld(h + idx);
-  for (int t0 = 0; t0 < T_; t0 += AHEAD) {
-    float wx[AHEAD], m[AHEAD];
+  float wx[AHEAD], m[AHEAD];
+  auto load = [&](int t0, float (&x)[AHEAD], float (&z)[AHEAD]) {
 #pragma unroll
     for (int k = 0; k < AHEAD; ++k) {
       const int t = t0 + k;
-      wx[k] = (t < T_) ? ld(Wx + t * NH + idx) : 0.f;
-      m[k] = (Zoneout && Training && t < T_) ? ld(mask + t * NH + idx) : 0.f;
+      x[k] = (t < T_) ? ld(Wx + t * NH + idx) : 0.f;
+      z[k] = (Zoneout && Training && t < T_) ? ld(mask + t * NH + idx) : 0.f;
     }
+  };
+  if (Piped) load(0, wx, m);
+  for (int t0 = 0; t0 < T_; t0 += AHEAD) {
+    float wn[AHEAD], mn[AHEAD];
+    if (Piped) load(t0 + AHEAD, wn, mn);
+    else load(t0, wx, m);
 #pragma unroll
     for (int k = 0; k < AHEAD; ++k) {
       const int t = t0 + k;
@@ -42,14 +52,21 @@ __global__ void indrnn_scan_fwd(int T_, long long NH, int H, const T* __restrict
         hp = hn;  // the carried state stays fp32 whatever the storage type
       }
     }
+    if (Piped) {
+#pragma unroll
+      for (int k = 0; k < AHEAD; ++k) {
+        wx[k] = wn[k];
+        m[k] = mn[k];
+      }
+    }
   }
 }
 
-// Planes: dk is also written as two bf16 planes (hi, lo; `dk_planes`, the lo plane
-// `plane_stride` elements later) - the form the two contractions that read it take their
-// fp32 operands in, so that neither splits it again.
-template <typename T, bool Zoneout, bool Planes>
-__global__ void indrnn_scan_bwd(int T_, long long NH, int H, const T* __restrict__ u,
+// Planes: dk is written as two bf16 planes (hi, lo; `dk_planes`, the lo plane `plane_stride`
+// elements later) - the form the two contractions that read it take their fp32 operands in, so
+// that neither splits it again.  dk_out: null if nothing reads the fp32 values.
+template <typename T, bool Zoneout, bool Planes, bool Piped>
+__global__ void __launch_bounds__(128) indrnn_scan_bwd(int T_, long long NH, int H, const T* __restrict__ u,
                                 const T* __restrict__ h, const T* __restrict__ dh_new,
                                 float* __restrict__ du_part, float* __restrict__ db_part,
                                 float* __restrict__ dh_carry, T* __restrict__ dk_out,
@@ -61,17 +78,23 @@ __global__ void indrnn_scan_bwd(int T_, long long NH, int H, const T* __restrict
   const float uj = ld(u + j);
   float carry = dh_carry[idx];
   float du = 0.f, db = 0.f;
-  for (int t0 = T_ - 1; t0 >= 0; t0 -= AHEAD) {
-    float hn[AHEAD], hpv[AHEAD], dn[AHEAD], m[AHEAD];
+  float hn = ld(h + (long long)T_ * NH + idx);  // h after the step at hand
+  float hv[AHEAD], dn[AHEAD], m[AHEAD];
+  auto load = [&](int t0, float (&hp)[AHEAD], float (&d)[AHEAD], float (&z)[AHEAD]) {
 #pragma unroll
     for (int k = 0; k < AHEAD; ++k) {
       const int t = t0 - k;
       const bool ok = t >= 0;
-      hn[k] = ok ? ld(h + (t + 1) * NH + idx) : 0.f;
-      hpv[k] = ok ? ld(h + t * NH + idx) : 0.f;
-      dn[k] = ok ? ld(dh_new + (t + 1) * NH + idx) : 0.f;
-      m[k] = (Zoneout && ok) ? ld(mask + t * NH + idx) : 0.f;
+      hp[k] = ok ? ld(h + t * NH + idx) : 0.f;
+      d[k] = ok ? ld(dh_new + (t + 1) * NH + idx) : 0.f;
+      z[k] = (Zoneout && ok) ? ld(mask + t * NH + idx) : 0.f;
     }
+  };
+  if (Piped) load(T_ - 1, hv, dn, m);
+  for (int t0 = T_ - 1; t0 >= 0; t0 -= AHEAD) {
+    float hx[AHEAD], dx[AHEAD], mx[AHEAD];
+    if (Piped) load(t0 - AHEAD, hx, dx, mx);
+    else load(t0, hv, dn, m);
 #pragma unroll
     for (int k = 0; k < AHEAD; ++k) {
       const int t = t0 - k;
@@ -82,16 +105,25 @@ __global__ void indrnn_scan_bwd(int T_, long long NH, int H, const T* __restrict
           keep = (1.0f - m[k]) * dh_total;
           dh_total = m[k] * dh_total;
         }
-        const float dk = d_tanh(hn[k]) * dh_total;
-        st(dk_out + t * NH + idx, dk);
+        const float dk = d_tanh(hn) * dh_total;
+        if (!Planes || dk_out) st(dk_out + t * NH + idx, dk);
         if (Planes) {
           const __nv_bfloat16 hi = __float2bfloat16_rn(dk);
           dk_planes[t * NH + idx] = hi;
           dk_planes[plane_stride + t * NH + idx] = __float2bfloat16_rn(dk - __bfloat162float(hi));
         }
         carry = keep + uj * dk;
-        du += hpv[k] * dk;
+        du += hv[k] * dk;
         db += dk;
+        hn = hv[k];
+      }
+    }
+    if (Piped) {
+#pragma unroll
+      for (int k = 0; k < AHEAD; ++k) {
+        hv[k] = hx[k];
+        dn[k] = dx[k];
+        m[k] = mx[k];
       }
     }
   }
@@ -100,45 +132,65 @@ __global__ void indrnn_scan_bwd(int T_, long long NH, int H, const T* __restrict
   db_part[idx] = db;
 }
 
-template <typename T>
-int scan_fwd(const IndrnnFwd& a, const void* Wx, cudaStream_t s) {
+// Threads per block and whether the piped form runs: half of 2048 threads on every SM.
+struct ScanShape {
+  int blocks, threads;
+  bool piped;
+  explicit ScanShape(long long NH)
+      : threads(NH < 64LL * 4 * sm_count() ? 32 : 128), piped(NH <= 1024LL * sm_count() / 2) {
+    blocks = ceil_div(NH, threads);
+  }
+};
+
+template <typename T, bool Piped>
+int scan_fwd_p(const IndrnnFwd& a, const void* Wx, const ScanShape& sc, cudaStream_t s) {
   const long long NH = (long long)a.N * a.H;
   const T* mask = (const T*)a.zoneout_mask;
   const bool zo = a.zoneout_prob != 0.0f && mask != nullptr;
-  const int blocks = ceil_div(NH, 128);
 #define HB_ARGS a.T, NH, a.H, (const T*)Wx, (const T*)a.u, (const T*)a.b, (T*)a.h, \
                 a.zoneout_prob, zo ? mask : nullptr
   if (a.training) {
-    if (zo) indrnn_scan_fwd<T, true, true><<<blocks, 128, 0, s>>>(HB_ARGS);
-    else    indrnn_scan_fwd<T, true, false><<<blocks, 128, 0, s>>>(HB_ARGS);
+    if (zo) indrnn_scan_fwd<T, true, true, Piped><<<sc.blocks, sc.threads, 0, s>>>(HB_ARGS);
+    else    indrnn_scan_fwd<T, true, false, Piped><<<sc.blocks, sc.threads, 0, s>>>(HB_ARGS);
   } else {
-    if (zo) indrnn_scan_fwd<T, false, true><<<blocks, 128, 0, s>>>(HB_ARGS);
-    else    indrnn_scan_fwd<T, false, false><<<blocks, 128, 0, s>>>(HB_ARGS);
+    if (zo) indrnn_scan_fwd<T, false, true, Piped><<<sc.blocks, sc.threads, 0, s>>>(HB_ARGS);
+    else    indrnn_scan_fwd<T, false, false, Piped><<<sc.blocks, sc.threads, 0, s>>>(HB_ARGS);
   }
 #undef HB_ARGS
   HB_LAUNCH_OK();
   count_launch(1);
   return HASTE_B200_OK;
 }
-
 template <typename T>
-int scan_bwd(const IndrnnBwd& a, float* du_part, float* db_part, float* dh_carry,
-             __nv_bfloat16* planes, long long plane_stride, cudaStream_t s) {
+int scan_fwd(const IndrnnFwd& a, const void* Wx, cudaStream_t s) {
+  const ScanShape sc((long long)a.N * a.H);
+  return sc.piped ? scan_fwd_p<T, true>(a, Wx, sc, s) : scan_fwd_p<T, false>(a, Wx, sc, s);
+}
+
+template <typename T, bool Piped>
+int scan_bwd_p(const IndrnnBwd& a, float* du_part, float* db_part, float* dh_carry, void* dk,
+               __nv_bfloat16* planes, long long plane_stride, const ScanShape& sc, cudaStream_t s) {
   const long long NH = (long long)a.N * a.H;
-  const int blocks = ceil_div(NH, 128);
 #define HB_ARGS a.T, NH, a.H, (const T*)a.u, (const T*)a.h, (const T*)a.dh_new, du_part, db_part, \
-                dh_carry, (T*)a.workspace, (const T*)a.zoneout_mask, planes, plane_stride
+                dh_carry, (T*)dk, (const T*)a.zoneout_mask, planes, plane_stride
   if (planes) {
-    if (a.zoneout_mask) indrnn_scan_bwd<T, true, true><<<blocks, 128, 0, s>>>(HB_ARGS);
-    else                indrnn_scan_bwd<T, false, true><<<blocks, 128, 0, s>>>(HB_ARGS);
+    if (a.zoneout_mask) indrnn_scan_bwd<T, true, true, Piped><<<sc.blocks, sc.threads, 0, s>>>(HB_ARGS);
+    else                indrnn_scan_bwd<T, false, true, Piped><<<sc.blocks, sc.threads, 0, s>>>(HB_ARGS);
   } else {
-    if (a.zoneout_mask) indrnn_scan_bwd<T, true, false><<<blocks, 128, 0, s>>>(HB_ARGS);
-    else                indrnn_scan_bwd<T, false, false><<<blocks, 128, 0, s>>>(HB_ARGS);
+    if (a.zoneout_mask) indrnn_scan_bwd<T, true, false, Piped><<<sc.blocks, sc.threads, 0, s>>>(HB_ARGS);
+    else                indrnn_scan_bwd<T, false, false, Piped><<<sc.blocks, sc.threads, 0, s>>>(HB_ARGS);
   }
 #undef HB_ARGS
   HB_LAUNCH_OK();
   count_launch(1);
   return HASTE_B200_OK;
+}
+template <typename T>
+int scan_bwd(const IndrnnBwd& a, float* du_part, float* db_part, float* dh_carry, void* dk,
+             __nv_bfloat16* planes, long long plane_stride, cudaStream_t s) {
+  const ScanShape sc((long long)a.N * a.H);
+  return sc.piped ? scan_bwd_p<T, true>(a, du_part, db_part, dh_carry, dk, planes, plane_stride, sc, s)
+                  : scan_bwd_p<T, false>(a, du_part, db_part, dh_carry, dk, planes, plane_stride, sc, s);
 }
 
 }  // namespace
@@ -208,11 +260,29 @@ int indrnn_backward(const IndrnnBwd& a, cudaStream_t s) {
     planes = static_cast<__nv_bfloat16*>(workspace(s, 2 * pe * 2 + 256, /*slot=*/3));
     plane_stride = (long long)pe;
   }
+  const bool tr = a.transposed_inputs != 0;
+  // dW[C,H] = x^T . dk   (assigned, as in the reference)
+  GemmDesc gw{a.dtype, a.dtype, C, H, (int)TN, a.x, tr ? TN : 1, tr ? 1 : C, a.workspace, H, 1,
+              a.dW, H, 0};
+  // the backward contractions feed no recurrence: the three-product form is enough also for
+  // the LayerNorm variant (six products measured the same 2.6e-5 on a six-layer stack)
+  if (planes) { gw.b_pl = planes; gw.b_pl_ld = H; gw.b_pl_stride = plane_stride; }
+  GemmDesc gx{a.dtype, a.dtype, (int)TN, C, H, a.workspace, H, 1, a.W, tr ? C : 1, tr ? 1 : H,
+              a.dx, C, 0};
+  if (planes) { gx.a_pl = planes; gx.a_pl_ld = H; gx.a_pl_stride = plane_stride; }
+  // The fp32 values then go nowhere, unless LayerNorm works on them or a contraction is one for
+  // the CUDA cores: a fifth of the scan's traffic.
+  void* dk = a.workspace;
+  if (planes && !a.gamma && gemm_reads_planes(gw) && (!a.dx || gemm_reads_planes(gx))) {
+    dk = nullptr;
+    gw.b = nullptr;
+    gx.a = nullptr;
+  }
   {
     ProfScope p(PH_REC_BWD, s);
     __nv_bfloat16* sp = a.gamma ? nullptr : planes;
-    if (a.dtype == HASTE_B200_F32) HB_TRY(scan_bwd<float>(a, du_part, db_part, dh_carry, sp, plane_stride, s));
-    else HB_TRY(scan_bwd<__nv_bfloat16>(a, du_part, db_part, dh_carry, nullptr, 0, s));
+    if (a.dtype == HASTE_B200_F32) HB_TRY(scan_bwd<float>(a, du_part, db_part, dh_carry, dk, sp, plane_stride, s));
+    else HB_TRY(scan_bwd<__nv_bfloat16>(a, du_part, db_part, dh_carry, dk, nullptr, 0, s));
   }
   HB_TRY(from_float(a.dtype, dh_carry, a.dh, NH, s));
   HB_TRY(colsum(HASTE_B200_F32, du_part, H, N, H, a.dtype, a.du, add, cs, s));
@@ -225,21 +295,11 @@ int indrnn_backward(const IndrnnBwd& a, cudaStream_t s) {
                                a.dtype, a.dgamma, nullptr, a.cache_Wx, lns, s, planes,
                                plane_stride));
   }
-  const bool tr = a.transposed_inputs != 0;
-  // dW[C,H] = x^T . dk   (assigned, as in the reference)
-  GemmDesc gw{a.dtype, a.dtype, C, H, (int)TN, a.x, tr ? TN : 1, tr ? 1 : C, a.workspace, H, 1,
-              a.dW, H, 0};
-  // the backward contractions feed no recurrence: the three-product form is enough also for
-  // the LayerNorm variant (six products measured the same 2.6e-5 on a six-layer stack)
-  if (planes) { gw.b_pl = planes; gw.b_pl_ld = H; gw.b_pl_stride = plane_stride; }
   {
     ProfScope p(PH_WGRAD, s);
     HB_TRY(gemm(gw, s));
   }
   if (!a.dx) return HASTE_B200_OK;
-  GemmDesc gx{a.dtype, a.dtype, (int)TN, C, H, a.workspace, H, 1, a.W, tr ? C : 1, tr ? 1 : H,
-              a.dx, C, 0};
-  if (planes) { gx.a_pl = planes; gx.a_pl_ld = H; gx.a_pl_stride = plane_stride; }
   {
     ProfScope p(PH_DGRAD, s);
     HB_TRY(gemm(gx, s));
