@@ -273,8 +273,11 @@ int gru_backward(const GruBwd& a, cudaStream_t s) {
     HB_TRY(st_);
     if (carried) {
       HB_TRY(from_float(a.dtype, dh_carry, a.dh, NH, s));
-      HB_TRY(colsum(a.dtype, a.dp, 3LL * H, (int)TN, 3 * H, a.dtype, a.dbx, add, cs, s));
-      HB_TRY(colsum(a.dtype, a.dq, 3LL * H, (int)TN, 3 * H, a.dtype, a.dbr, add, cs, s));
+      // dq differs from dp in the third gate only
+      HB_TRY(colsum(a.dtype, a.dp, 3LL * H, (int)TN, 3 * H, a.dtype, a.dbx, add, cs, s, a.dbr, 2 * H));
+      const size_t third = 2 * (size_t)H * dtype_size(a.dtype);
+      HB_TRY(colsum(a.dtype, static_cast<const char*>(a.dq) + third, 3LL * H, (int)TN, H, a.dtype,
+                    static_cast<char*>(a.dbr) + third, add, cs, s));
     }
   } else {
     HB_TRY(st_);

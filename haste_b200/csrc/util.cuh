@@ -45,7 +45,8 @@ int make_arena(Arena* a, cudaStream_t stream, size_t bytes, int slot = 0);
 // HASTE_B200_F32 / HASTE_B200_BF16.  `scratch` needs colsum_scratch_floats().
 size_t colsum_scratch_floats(int rows, int width);
 int colsum(int in_dtype, const void* in, long long ld, int rows, int width, int out_dtype,
-           void* out, int accumulate, float* scratch, cudaStream_t stream);
+           void* out, int accumulate, float* scratch, cudaStream_t stream, void* out2 = nullptr,
+           int w2 = 0);  // the first w2 columns go to out2 as well
 
 // Adds the bias-gradient partials [rows][4H] of a recurrence kernel to the bias gradients (or
 // assigns them), in a fixed order.  LSTM (gates 4): db[4H].  GRU (gates 3), partial columns dp_z, dp_r, dp_g, dq_g:
