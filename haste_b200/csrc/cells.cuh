@@ -138,13 +138,15 @@ int gru_backward_tc(const GruBwd& a, float* dh_carry, cudaStream_t s);
 // parameter gradients of the recurrence into the fp32 accumulators acc = [dgamma_Rh 4H |
 // dgamma_h H | dbeta_h H]; planes.p / p2 receive the gate gradient and d(h.R).
 int layer_norm_lstm_forward_persistent(const LnLstmFwd& a, cudaStream_t s);
+int layer_norm_lstm_backward_cluster(const LnLstmBwd& a, float* dh_carry, float* dc_carry, cudaStream_t s);
 int layer_norm_lstm_backward_persistent(const LnLstmBwd& a, float* dh_carry, float* dc_carry,
-                                        float* acc, const GradPlanes& planes, bool* bias_done, cudaStream_t s);
+                                        float* acc, const GradPlanes& planes, cudaStream_t s);
 // LayerNormGRU: forward expects LN(x.W) in a.tmp_Wx_norm; backward adds dgamma_Rh into the
 // fp32 accumulator acc [3H] and leaves d(h.R) in a.act_Rh.
 int layer_norm_gru_forward_persistent(const LnGruFwd& a, cudaStream_t s);
+int layer_norm_gru_backward_cluster(const LnGruBwd& a, float* dh_carry, cudaStream_t s);
 int layer_norm_gru_backward_persistent(const LnGruBwd& a, float* dh_carry, float* acc,
-                                       const GradPlanes& planes, bool* bias_done, cudaStream_t s);
+                                       const GradPlanes& planes, cudaStream_t s);
 
 // Exchange-only probe (recurrent_host.cu): device microseconds per step of the forward
 // recurrence's hand-off alone, for the tiling (N, H) would get.

@@ -121,13 +121,6 @@ int layer_norm_gru_backward(const LnGruBwd& a, cudaStream_t s) {
   const bool bf = a.dtype == HASTE_B200_BF16;
   const size_t es = dtype_size(a.dtype);
   const int add = assign_gradients() ? 0 : 1;
-  if (!add) {  // everything below adds, except the two contractions at the end
-    HB_CUDA_OK(cudaMemsetAsync(a.dbx, 0, 3 * H * es, s));
-    HB_CUDA_OK(cudaMemsetAsync(a.dbr, 0, 3 * H * es, s));
-    HB_CUDA_OK(cudaMemsetAsync(a.dgamma_Wx, 0, 3 * H * es, s));
-    HB_CUDA_OK(cudaMemsetAsync(a.dgamma_Rh, 0, 3 * H * es, s));
-    HB_CUDA_OK(cudaMemsetAsync(a.dh, 0, NH * es, s));
-  }
   const size_t csf = colsum_scratch_floats((int)TN, 3 * H);
   const size_t lnf = layer_norm_backward_scratch_floats((int)TN, 3 * H);
   Arena ws;
@@ -138,12 +131,26 @@ int layer_norm_gru_backward(const LnGruBwd& a, cudaStream_t s) {
   float* lns = ws.take<float>(lnf);
   float* acc = ws.take<float>(3 * H);
   HB_REQUIRE(dh_carry && cs && lns && acc, "scratch arena");
-  HB_TRY(to_float(a.dtype, a.dh, dh_carry, NH, s));
-  // Persistent recurrence first; it adds dgamma_Rh into `acc`.
-  HB_CUDA_OK(cudaMemsetAsync(acc, 0, 3 * H * sizeof(float), s));
-  bool bias_done = false;
-  int st_ = layer_norm_gru_backward_persistent(a, dh_carry, acc, GradPlanes{}, &bias_done, s);
-  bool use_acc = st_ == HASTE_B200_OK;
+  if (add) {
+    HB_TRY(to_float(a.dtype, a.dh, dh_carry, NH, s));
+  } else {
+    HB_CUDA_OK(cudaMemsetAsync(dh_carry, 0, NH * 4, s));
+    HB_CUDA_OK(cudaMemsetAsync(a.dgamma_Wx, 0, 3 * H * es, s));  // LayerNorm 1 below adds
+  }
+  int st_ = layer_norm_gru_backward_cluster(a, dh_carry, s);
+  const bool done = st_ == HASTE_B200_OK;  // biases and gamma_Rh included
+  bool use_acc = false;
+  if (st_ == HASTE_B200_ERR_UNSUPPORTED) {
+    if (!add) {  // the rest adds
+      HB_CUDA_OK(cudaMemsetAsync(a.dbx, 0, 3 * H * es, s));
+      HB_CUDA_OK(cudaMemsetAsync(a.dbr, 0, 3 * H * es, s));
+      HB_CUDA_OK(cudaMemsetAsync(a.dgamma_Rh, 0, 3 * H * es, s));
+    }
+    // Persistent recurrence first; it adds dgamma_Rh into `acc`.
+    HB_CUDA_OK(cudaMemsetAsync(acc, 0, 3 * H * sizeof(float), s));
+    st_ = layer_norm_gru_backward_persistent(a, dh_carry, acc, GradPlanes{}, s);
+    use_acc = st_ == HASTE_B200_OK;
+  }
   if (st_ == HASTE_B200_ERR_UNSUPPORTED) {
     void* dgamma1 = a.dgamma_Rh;
     if (bf) {
@@ -158,9 +165,12 @@ int layer_norm_gru_backward(const LnGruBwd& a, cudaStream_t s) {
   HB_TRY(from_float(a.dtype, dh_carry, a.dh, NH, s));
 
   // dp/dq hold gradients w.r.t. the normalised projections (+ bias).
-  if (!bias_done) {
-    HB_TRY(colsum(a.dtype, a.dp, 3LL * H, (int)TN, 3 * H, a.dtype, a.dbx, 1, cs, s));
-    HB_TRY(colsum(a.dtype, a.dq, 3LL * H, (int)TN, 3 * H, a.dtype, a.dbr, 1, cs, s));
+  if (!done) {
+    // dq differs from dp in the third gate only
+    HB_TRY(colsum(a.dtype, a.dp, 3LL * H, (int)TN, 3 * H, a.dtype, a.dbx, 1, cs, s, a.dbr, 2 * H));
+    const size_t third = 2 * (size_t)H * dtype_size(a.dtype);
+    HB_TRY(colsum(a.dtype, static_cast<const char*>(a.dq) + third, 3LL * H, (int)TN, H, a.dtype,
+                  static_cast<char*>(a.dbr) + third, 1, cs, s));
   }
   // LayerNorm 1 backward over all steps, in place on dp.
   HB_TRY(layer_norm_backward(a.dtype, (int)TN, 3 * H, a.gamma_Wx, a.act_Wx, a.dp, a.dp, a.dtype,

@@ -346,20 +346,21 @@ int backward_wide(const LnLstmBwd& a, cudaStream_t s) {
   // (slot 0 of the incoming gradients is never read)
   HB_TRY(to_float(BF, static_cast<const char*>(a.dh_new) + NH * 2, dhn + NH, (size_t)T * NH, s));
   if (a.dc_new) HB_TRY(to_float(BF, static_cast<const char*>(a.dc_new) + NH * 2, dcn + NH, (size_t)T * NH, s));
-  HB_TRY(to_float(BF, a.dh, dh, NH, s));
-  HB_TRY(to_float(BF, a.dc, dc, NH, s));
   if (mask) HB_TRY(to_float(BF, a.zoneout_mask, mask, (size_t)T * NH, s));
-  // accumulated outputs: the fp32 pass adds into zeroed scratch, the sums go into the
-  // caller's bf16 tensors afterwards
-  if (!assign_gradients()) {
+  // accumulated outputs: the fp32 pass adds into zeroed scratch, the sums go into the caller's bf16
+  // tensors afterwards (assigned gradients: it assigns, and so do the conversions)
+  const bool assign = assign_gradients();
+  if (!assign) {
+    HB_TRY(to_float(BF, a.dh, dh, NH, s));
+    HB_TRY(to_float(BF, a.dc, dc, NH, s));
     HB_CUDA_OK(cudaMemsetAsync(dR, 0, RW * 4, s));
     HB_CUDA_OK(cudaMemsetAsync(dW, 0, WW * 4, s));
+    HB_CUDA_OK(cudaMemsetAsync(db, 0, (size_t)4 * H * 4, s));
+    HB_CUDA_OK(cudaMemsetAsync(dgWx, 0, (size_t)4 * H * 4, s));
+    HB_CUDA_OK(cudaMemsetAsync(dgRh, 0, (size_t)4 * H * 4, s));
+    HB_CUDA_OK(cudaMemsetAsync(dgh, 0, (size_t)H * 4, s));
+    HB_CUDA_OK(cudaMemsetAsync(dbh, 0, (size_t)H * 4, s));
   }
-  HB_CUDA_OK(cudaMemsetAsync(db, 0, (size_t)4 * H * 4, s));
-  HB_CUDA_OK(cudaMemsetAsync(dgWx, 0, (size_t)4 * H * 4, s));
-  HB_CUDA_OK(cudaMemsetAsync(dgRh, 0, (size_t)4 * H * 4, s));
-  HB_CUDA_OK(cudaMemsetAsync(dgh, 0, (size_t)H * 4, s));
-  HB_CUDA_OK(cudaMemsetAsync(dbh, 0, (size_t)H * 4, s));
   LnLstmBwd f = a;
   f.dtype = HASTE_B200_F32;
   f.W = W; f.R = R; f.gamma_Wx = gWx; f.gamma_Rh = gRh; f.gamma_h = gh;
@@ -371,18 +372,16 @@ int backward_wide(const LnLstmBwd& a, cudaStream_t s) {
   HB_TRY(from_float(BF, dx, a.dx, XN, s));
   HB_TRY(from_float(BF, dh, a.dh, NH, s));
   HB_TRY(from_float(BF, dc, a.dc, NH, s));
-  if (assign_gradients()) {
-    HB_TRY(from_float(BF, dW, a.dW, WW, s));
-    HB_TRY(from_float(BF, dR, a.dR, RW, s));
-  } else {
-    HB_TRY(add_float_into(BF, dW, a.dW, WW, s));
-    HB_TRY(add_float_into(BF, dR, a.dR, RW, s));
-  }
-  HB_TRY(add_float_into(BF, db, a.db, 4 * H, s));
-  HB_TRY(add_float_into(BF, dgWx, a.dgamma_Wx, 4 * H, s));
-  HB_TRY(add_float_into(BF, dgRh, a.dgamma_Rh, 4 * H, s));
-  HB_TRY(add_float_into(BF, dgh, a.dgamma_h, H, s));
-  HB_TRY(add_float_into(BF, dbh, a.dbeta_h, H, s));
+  auto hand_over = [&](const float* src, void* dst, size_t n) {
+    return assign ? from_float(BF, src, dst, n, s) : add_float_into(BF, src, dst, n, s);
+  };
+  HB_TRY(hand_over(dW, a.dW, WW));
+  HB_TRY(hand_over(dR, a.dR, RW));
+  HB_TRY(hand_over(db, a.db, 4 * H));
+  HB_TRY(hand_over(dgWx, a.dgamma_Wx, 4 * H));
+  HB_TRY(hand_over(dgRh, a.dgamma_Rh, 4 * H));
+  HB_TRY(hand_over(dgh, a.dgamma_h, H));
+  HB_TRY(hand_over(dbh, a.dbeta_h, H));
   return HASTE_B200_OK;
 }
 
@@ -426,16 +425,6 @@ int layer_norm_lstm_backward(const LnLstmBwd& a, cudaStream_t s) {
   if (a.T == 0) return HASTE_B200_OK;
   HB_REQUIRE(a.x && a.dx, "x/dx is null");
   HB_REQUIRE((long long)a.T * a.N < (1LL << 31), "T*N too large");
-  if (assign_gradients()) {  // everything below adds, except the two contractions of backward_core
-    const size_t es = dtype_size(a.dtype), H = a.H, NH = (size_t)a.N * H;
-    HB_CUDA_OK(cudaMemsetAsync(a.db, 0, 4 * H * es, s));
-    HB_CUDA_OK(cudaMemsetAsync(a.dgamma_Wx, 0, 4 * H * es, s));
-    HB_CUDA_OK(cudaMemsetAsync(a.dgamma_Rh, 0, 4 * H * es, s));
-    HB_CUDA_OK(cudaMemsetAsync(a.dgamma_h, 0, H * es, s));
-    HB_CUDA_OK(cudaMemsetAsync(a.dbeta_h, 0, H * es, s));
-    HB_CUDA_OK(cudaMemsetAsync(a.dh, 0, NH * es, s));
-    HB_CUDA_OK(cudaMemsetAsync(a.dc, 0, NH * es, s));
-  }
   if (a.dtype == HASTE_B200_BF16_WIDE) return backward_wide(a, s);
   return backward_core(a, s);
 }
@@ -457,15 +446,32 @@ int backward_core(const LnLstmBwd& a, cudaStream_t s) {
   float* lns = ws.take<float>(lnf);
   float* acc = ws.take<float>(6 * H);  // fp32 accumulators for bf16 runs: dgamma1, dgamma_h, dbeta_h
   HB_REQUIRE(dh_carry && dc_carry && cs && lns && acc, "scratch arena");
-  HB_TRY(to_float(a.dtype, a.dh, dh_carry, NH, s));
-  HB_TRY(to_float(a.dtype, a.dc, dc_carry, NH, s));
+  const bool assign = assign_gradients();
+  const size_t es = dtype_size(a.dtype);
+  if (assign) {
+    HB_CUDA_OK(cudaMemsetAsync(dh_carry, 0, (char*)(dc_carry + NH) - (char*)dh_carry, s));
+    HB_CUDA_OK(cudaMemsetAsync(a.dgamma_Wx, 0, 4 * H * es, s));  // LayerNorm 1 below adds
+  } else {
+    HB_TRY(to_float(a.dtype, a.dh, dh_carry, NH, s));
+    HB_TRY(to_float(a.dtype, a.dc, dc_carry, NH, s));
+  }
 
-  // Persistent recurrence first; it adds its LayerNorm parameter gradients into `acc`.
-  HB_CUDA_OK(cudaMemsetAsync(acc, 0, 6 * H * sizeof(float), s));
   if (profile_enabled()) profile_mark(PH_REC_BWD, true, s);
-  bool bias_done = false;
-  int st_ = layer_norm_lstm_backward_persistent(a, dh_carry, dc_carry, acc, GradPlanes{}, &bias_done, s);
-  bool use_acc = st_ == HASTE_B200_OK;
+  int st_ = layer_norm_lstm_backward_cluster(a, dh_carry, dc_carry, s);
+  const bool done = st_ == HASTE_B200_OK;  // bias, gamma_Rh, gamma_h, beta_h included
+  bool use_acc = false;
+  if (st_ == HASTE_B200_ERR_UNSUPPORTED) {
+    if (assign) {  // the rest adds
+      HB_CUDA_OK(cudaMemsetAsync(a.db, 0, 4 * H * es, s));
+      HB_CUDA_OK(cudaMemsetAsync(a.dgamma_Rh, 0, 4 * H * es, s));
+      HB_CUDA_OK(cudaMemsetAsync(a.dgamma_h, 0, H * es, s));
+      HB_CUDA_OK(cudaMemsetAsync(a.dbeta_h, 0, H * es, s));
+    }
+    // Persistent recurrence first; it adds its LayerNorm parameter gradients into `acc`.
+    HB_CUDA_OK(cudaMemsetAsync(acc, 0, 6 * H * sizeof(float), s));
+    st_ = layer_norm_lstm_backward_persistent(a, dh_carry, dc_carry, acc, GradPlanes{}, s);
+    use_acc = st_ == HASTE_B200_OK;
+  }
   if (st_ == HASTE_B200_ERR_UNSUPPORTED) {
     void* dgamma1 = a.dgamma_Rh;
     void* dgamma_h = a.dgamma_h;
@@ -494,7 +500,7 @@ int backward_core(const LnLstmBwd& a, cudaStream_t s) {
   {
     ProfScope p(PH_OTHER, s);
     // act_Wx_norm now holds the gradient w.r.t. (LN1(x.W) + LN2(h.R) + b).
-    if (!bias_done)
+    if (!done)
       HB_TRY(colsum(a.dtype, a.act_Wx_norm, 4LL * H, (int)TN, 4 * H, a.dtype, a.db, 1, cs, s));
     // LayerNorm 1 backward over all steps: act_Wx <- d/d(x.W).
     HB_TRY(layer_norm_backward(a.dtype, (int)TN, 4 * H, a.gamma_Wx, a.act_Wx, a.act_Wx_norm,
@@ -502,13 +508,13 @@ int backward_core(const LnLstmBwd& a, cudaStream_t s) {
   }
   const bool tr = a.transposed_inputs != 0;
   GemmDesc gw{a.dtype, a.dtype, C, 4 * H, (int)TN, a.x, tr ? TN : 1, tr ? 1 : C, a.act_Wx,
-              4LL * H, 1, a.dW, 4LL * H, assign_gradients() ? 0 : 1};
+              4LL * H, 1, a.dW, 4LL * H, assign ? 0 : 1};
   {
     ProfScope p(PH_WGRAD, s);
     HB_TRY(gemm(gw, s));
   }
   GemmDesc gr{a.dtype, a.dtype, H, 4 * H, (int)TN, a.h, 1, H, a.act_Rh, 4LL * H, 1, a.dR,
-              4LL * H, assign_gradients() ? 0 : 1};
+              4LL * H, assign ? 0 : 1};
   {
     ProfScope p(PH_WGRAD, s);
     HB_TRY(gemm(gr, s));

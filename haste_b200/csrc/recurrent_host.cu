@@ -192,28 +192,63 @@ int cluster_forward(LnFwdParams& p, int (*run)(const LnFwdParams&, cudaStream_t)
   HB_REQUIRE(p.sync.err, "error word");
   return run(p, s);
 }
-// Adds the LayerNorm parameter gradients into `acc` and the bias gradients into db (GRU: db2 too).
-int cluster_backward(LnBwdParams& p, int gates, float* acc, int dtype, void* db, void* db2,
+// Sums of the row groups' partial parameter gradients, into the caller's tensors: bias (as
+// bias_grad_finish), gains of h.R and, LSTM, gain and offset of the cell state.
+struct LnGrads {
+  void *db, *db2, *dgRh, *dgh, *dbh;
+};
+template <typename T>
+__global__ void ln_grad_finish(int G, const float* db_part, const float* dgRh_part, const float* dgh_part,
+                               const float* dbh_part, int rows, int H, LnGrads out, int accumulate) {
+  int j = blockIdx.x * blockDim.x + threadIdx.x;
+  const float* part = nullptr;
+  int width = 0;
+  T *d = nullptr, *d2 = nullptr;
+  if (j < 4 * H) {
+    part = db_part; width = 4 * H;
+    if (G == 4 || j < 3 * H) d = static_cast<T*>(out.db) + j;
+    if (G == 3 && (j < 2 * H || j >= 3 * H)) d2 = static_cast<T*>(out.db2) + (j < 2 * H ? j : j - H);
+  } else if ((j -= 4 * H) < G * H) {
+    part = dgRh_part; width = G * H;
+    d = static_cast<T*>(out.dgRh) + j;
+  } else if (G == 4 && (j -= G * H) < 2 * H) {
+    part = j < H ? dgh_part : dbh_part; width = H;
+    d = static_cast<T*>(j < H ? out.dgh : out.dbh);
+    j = j < H ? j : j - H;
+    d += j;
+  } else {
+    return;
+  }
+  float s = 0.f;
+  for (int r = 0; r < rows; ++r) s += part[(long long)r * width + j];
+  if (d) st(d, accumulate ? s + ld(d) : s);
+  if (d2) st(d2, accumulate ? s + ld(d2) : s);
+}
+
+int cluster_backward(LnBwdParams& p, int gates, int dtype, const LnGrads& out,
                      int (*run)(const LnBwdParams&, float*, int*, cudaStream_t), cudaStream_t s) {
   if (recurrence_path() == HASTE_B200_PATH_STEPWISE || p.H > 256) return HASTE_B200_ERR_UNSUPPORTED;
   p.sync.err = device_error_word();
   HB_REQUIRE(p.sync.err, "error word");
-  const int H = p.H, tiles = ceil_div(p.N, 8);
-  const size_t cwords = colsum_scratch_floats(tiles, gates * H);
-  float* part = static_cast<float*>(workspace(s, ((size_t)tiles * 10 * H + cwords) * sizeof(float), /*slot=*/2));
+  const int H = p.H;
+  const size_t tiles = ceil_div(p.N, 8);
+  float* part = static_cast<float*>(workspace(s, tiles * 10 * H * sizeof(float), /*slot=*/2));
   if (!part) return HASTE_B200_ERR_CUDA;
-  float* cs = part + (size_t)tiles * 10 * H;
-  float* db_part = part + (size_t)tiles * 6 * H;
+  float* db_part = part + tiles * 6 * H;
   p.dgRh_part = part;
-  p.dgh_part = part + (size_t)tiles * 4 * H;
-  p.dbh_part = part + (size_t)tiles * 5 * H;
+  p.dgh_part = part + tiles * 4 * H;
+  p.dbh_part = part + tiles * 5 * H;
   int rows = 0;
   HB_TRY(run(p, db_part, &rows, s));
-  HB_TRY(bias_grad_finish(gates, db_part, rows, H, dtype, db, db2, 1, s));
-  HB_TRY(colsum(HASTE_B200_F32, part, (long long)gates * H, rows, gates * H, HASTE_B200_F32, acc, 1, cs, s));
-  if (gates == 3) return HASTE_B200_OK;
-  HB_TRY(colsum(HASTE_B200_F32, p.dgh_part, H, rows, H, HASTE_B200_F32, acc + 4 * H, 1, cs, s));
-  return colsum(HASTE_B200_F32, p.dbh_part, H, rows, H, HASTE_B200_F32, acc + 5 * H, 1, cs, s);
+  const int blocks = ceil_div((gates == 4 ? 10LL : 7LL) * H, 128), add = assign_gradients() ? 0 : 1;
+  if (dtype == HASTE_B200_F32)
+    ln_grad_finish<float><<<blocks, 128, 0, s>>>(gates, db_part, p.dgRh_part, p.dgh_part, p.dbh_part, rows, H, out, add);
+  else
+    ln_grad_finish<__nv_bfloat16><<<blocks, 128, 0, s>>>(gates, db_part, p.dgRh_part, p.dgh_part, p.dbh_part, rows, H,
+                                                         out, add);
+  HB_LAUNCH_OK();
+  count_launch(1);
+  return HASTE_B200_OK;
 }
 
 }  // namespace
@@ -240,21 +275,31 @@ int layer_norm_lstm_forward_persistent(const LnLstmFwd& a, cudaStream_t s) {
   return a.dtype == HASTE_B200_F32 ? run_ln_fwd_f32(p, g, s) : run_ln_fwd_bf16(p, g, s);
 }
 
+namespace {
+LnBwdParams ln_lstm_params(const LnLstmBwd& a, float* dh_carry, float* dc_carry, const GradPlanes& planes) {
+  return LnBwdParams{a.T, a.N, a.H, 0, 0, a.zoneout_mask ? 1 : 0, a.transposed_inputs, a.R,
+                     a.gamma_Rh, a.gamma_h, a.c, nullptr, nullptr, nullptr, a.act_Wx_norm, a.act_Rh,
+                     a.cache_Rh, a.act_c_norm,
+                     a.cache_c, a.dh_new, a.dc_new, a.zoneout_mask, dh_carry, dc_carry, nullptr, nullptr, nullptr,
+                     nullptr, nullptr, Sync{}, planes.p, planes.p2, planes.stride, debug_skip()};
+}
+}  // namespace
+
+// The cluster kernels, up to 256 units: dh and dc come back complete, and the bias and LayerNorm
+// gradients of h.R and c go into the caller's tensors (added or assigned).
+int layer_norm_lstm_backward_cluster(const LnLstmBwd& a, float* dh_carry, float* dc_carry, cudaStream_t s) {
+  LnBwdParams p = ln_lstm_params(a, dh_carry, dc_carry, GradPlanes{});
+  return cluster_backward(p, 4, a.dtype, LnGrads{a.db, nullptr, a.dgamma_Rh, a.dgamma_h, a.dbeta_h},
+                          a.dtype == HASTE_B200_F32 ? run_ln_cl_bwd_f32 : run_ln_cl_bwd_bf16, s);
+}
+
 // Backward.  `acc` holds fp32 accumulators [dgamma_Rh 4H | dgamma_h H | dbeta_h H] that the
 // per-row-group partial sums of the kernel are added into (fixed order).  As for the plain
 // LSTM, the recurrent contribution of step 0 to dh is added here by one small contraction.
 int layer_norm_lstm_backward_persistent(const LnLstmBwd& a, float* dh_carry, float* dc_carry,
-                                        float* acc, const GradPlanes& planes, bool* bias_done, cudaStream_t s) {
+                                        float* acc, const GradPlanes& planes, cudaStream_t s) {
   const int H = a.H;
-  LnBwdParams p{a.T, a.N, H, 0, 0, a.zoneout_mask ? 1 : 0, a.transposed_inputs, a.R,
-                a.gamma_Rh, a.gamma_h, a.c, nullptr, nullptr, nullptr, a.act_Wx_norm, a.act_Rh,
-                a.cache_Rh, a.act_c_norm,
-                a.cache_c, a.dh_new, a.dc_new, a.zoneout_mask, dh_carry, dc_carry, nullptr, nullptr, nullptr,
-                nullptr, nullptr, Sync{}, planes.p, planes.p2, planes.stride, debug_skip()};
-  const int cl = cluster_backward(p, 4, acc, a.dtype, a.db, nullptr,
-                                  a.dtype == HASTE_B200_F32 ? run_ln_cl_bwd_f32 : run_ln_cl_bwd_bf16, s);
-  *bias_done = cl == HASTE_B200_OK;
-  if (cl != HASTE_B200_ERR_UNSUPPORTED) return cl;
+  LnBwdParams p = ln_lstm_params(a, dh_carry, dc_carry, planes);
   Geometry g;
   if (!supported(a.dtype, a.N, a.H, &g) || g.nHS > 64) return HASTE_B200_ERR_UNSUPPORTED;
   p.nHS = g.nHS;
@@ -305,19 +350,27 @@ int layer_norm_gru_forward_persistent(const LnGruFwd& a, cudaStream_t s) {
   return a.dtype == HASTE_B200_F32 ? run_lngru_fwd_f32(p, g, s) : run_lngru_fwd_bf16(p, g, s);
 }
 
+namespace {
+LnBwdParams ln_gru_params(const LnGruBwd& a, float* dh_carry, const GradPlanes& planes) {
+  return LnBwdParams{a.T, a.N, a.H, 0, 0, a.zoneout_mask ? 1 : 0, a.transposed_inputs, a.R,
+                     a.gamma_Rh, nullptr, nullptr, a.h, a.dp, a.dq, const_cast<void*>(a.v), a.act_Rh,
+                     a.cache_Rh, nullptr, nullptr, a.dh_new, nullptr, a.zoneout_mask, dh_carry, nullptr,
+                     nullptr, nullptr, nullptr, nullptr, nullptr, Sync{}, planes.p, planes.p2, planes.stride};
+}
+}  // namespace
+
+int layer_norm_gru_backward_cluster(const LnGruBwd& a, float* dh_carry, cudaStream_t s) {
+  LnBwdParams p = ln_gru_params(a, dh_carry, GradPlanes{});
+  return cluster_backward(p, 3, a.dtype, LnGrads{a.dbx, a.dbr, a.dgamma_Rh, nullptr, nullptr},
+                          a.dtype == HASTE_B200_F32 ? run_lngru_cl_bwd_f32 : run_lngru_cl_bwd_bf16, s);
+}
+
 // Backward.  `acc` is the fp32 accumulator [3H] for dgamma_Rh.  a.act_Rh is overwritten with
 // d(h.R); a.dp / a.dq receive the gradients w.r.t. the normalised projections (+ biases).
 int layer_norm_gru_backward_persistent(const LnGruBwd& a, float* dh_carry, float* acc,
-                                       const GradPlanes& planes, bool* bias_done, cudaStream_t s) {
+                                       const GradPlanes& planes, cudaStream_t s) {
   const int H = a.H;
-  LnBwdParams p{a.T, a.N, H, 0, 0, a.zoneout_mask ? 1 : 0, a.transposed_inputs, a.R,
-                a.gamma_Rh, nullptr, nullptr, a.h, a.dp, a.dq, const_cast<void*>(a.v), a.act_Rh,
-                a.cache_Rh, nullptr, nullptr, a.dh_new, nullptr, a.zoneout_mask, dh_carry, nullptr,
-                nullptr, nullptr, nullptr, nullptr, nullptr, Sync{}, planes.p, planes.p2, planes.stride};
-  const int cl = cluster_backward(p, 3, acc, a.dtype, a.dbx, a.dbr,
-                                  a.dtype == HASTE_B200_F32 ? run_lngru_cl_bwd_f32 : run_lngru_cl_bwd_bf16, s);
-  *bias_done = cl == HASTE_B200_OK;
-  if (cl != HASTE_B200_ERR_UNSUPPORTED) return cl;
+  LnBwdParams p = ln_gru_params(a, dh_carry, planes);
   Geometry g;
   if (!supported(a.dtype, a.N, a.H, &g) || g.nHS > 64) return HASTE_B200_ERR_UNSUPPORTED;
   p.nHS = g.nHS;
