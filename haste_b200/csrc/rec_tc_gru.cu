@@ -223,6 +223,9 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int hs = blockIdx.x % p.nHS, rg = blockIdx.x / p.nHS;
   const int u0 = hs * UC;
+  // two 64-row tiles per CTA: the second one's rows are rows 64..127 of its MMAs and belong to
+  // epilogue warps of their own, so that the tiles are two chains that only share the streams
+  const bool halves = p.RB == 64 && p.MT == 2;
   constexpr int ACC_COLS = NB <= 32 ? 32 : 64;   // tensor-memory columns per accumulator
   constexpr uint32_t TMEM_COLS = 2 * NI * ACC_COLS;  // two buffers x one accumulator per issuer
 
@@ -234,7 +237,7 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(accf_bar(a), NI);
-      mbar_init(acce_bar(a), 128);
+      mbar_init(acce_bar(a), halves ? 64 : 128);
     }
     *s_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -293,7 +296,8 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
   const uint32_t tmem_base = *tmem_slot;
 
   const int tiles_total = (N + p.RB - 1) / p.RB;
-  const unsigned int arrivals = (unsigned int)p.nHS * 4u;  // per step: four epilogue warps per CTA
+  // per step: the epilogue warps of every CTA
+  const unsigned int arrivals = (unsigned int)p.nHS * (halves ? 2u : 4u);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -350,7 +354,7 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
         if (!FWD && it == 0) continue;
         for (int mt = 0; mt < p.MT && ok; ++mt) {
           if (rg * p.MT + mt >= tiles_total) break;
-          const int acc = n_acc & 1;
+          const int acc = halves ? mt : n_acc & 1;
           ++n_acc;
           if (!mbar_wait(acce_bar(acc), acc_phase[acc] ^ 1u, s_abort, p.err, 53)) { ok = false; break; }
           acc_phase[acc] ^= 1u;
@@ -365,7 +369,7 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
             if (!mbar_wait(full_bar(stage), phase, s_abort, p.err, 54)) { ok = false; break; }
             tc_fence_after();
             if (kb == 0) HB_STAMP(p, it, mt, 2);  // first k-block has landed
-            const uint64_t ad = a_desc0 + (uint64_t)stage * a_stage_inc;
+            const uint64_t ad = a_desc0 + (uint64_t)stage * a_stage_inc - (halves && mt ? a_stage_inc : 0);
             const uint64_t bd = b_desc0 + (uint64_t)kb * (R_TILE >> 4);
             tc_mma_bf16(d_tmem, ad, bd, idesc, kb >= NI ? 1u : 0u);
             tc_mma_bf16(d_tmem, ad + 2, bd + 2, idesc, 1u);
@@ -382,14 +386,14 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
   } else {
     // ------------------------------------------------------------------ epilogue
     const int quad = warp & 3;
-    const int r = quad * 32 + lane;  // row of the tile = tensor-memory lane
+    const int r = (halves ? quad & 1 : quad) * 32 + lane;  // row of the tile
     uint32_t acc_phase[2] = {0, 0};
     int n_acc = 0;
     bool ok = true;
     const long long NH = (long long)N * H;
     for (int it = 0; it < p.T && ok; ++it) {
       const int t = FWD ? it : (p.T - 1 - it);
-      for (int mt = 0; mt < p.MT && ok; ++mt) {
+      for (int mt = halves ? quad >> 1 : 0; mt < p.MT && ok; mt += halves ? 2 : 1) {
         const int tile = rg * p.MT + mt;
         if (tile >= tiles_total) break;
         const int n = tile * p.RB + r;
@@ -432,7 +436,7 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
         // ---- wait for the step product
         int acc = 0;
         if (have_acc) {
-          acc = n_acc & 1;
+          acc = halves ? mt : n_acc & 1;
           ++n_acc;
           bool got = mbar_wait(accf_bar(acc), acc_phase[acc], s_abort, p.err, 55);
           got = __all_sync(0xffffffffu, got);
@@ -593,7 +597,8 @@ bool tc_geometry_for(int N, int H, bool fwd, int sms, TcGeometry* g) {
   for (int rb = 64; rb <= 128; rb *= 2) {
     const int tiles = ceil_div(N, rb);
     const int mt = ceil_div(tiles, groups_max);
-    if (rb == 64 && mt > 1) continue;
+    // (the second 64-row tile's MMAs read 8 KB in front of their stage: there has to be as much R)
+    if (rb == 64 && (mt > 2 || (mt == 2 && r_bytes < (size_t)rb * 128))) continue;
     if (mt > 2) return false;
     g->RB = rb;
     g->MT = mt;
