@@ -37,11 +37,17 @@ bool gl_geometry(int dtype, int T, int N, int H, int most, GlGeometry* g) {
   g->NMT = (dtype == HASTE_B200_BF16 || ks <= 4) ? 4 : 2;
   g->nHS = ceil_div(H, 4 * g->NMT);
   if (g->nHS > sms) return false;
-  const int use = (budget > 0 && budget < sms && g->nHS <= budget) ? budget : sms;
-  g->nRG = min(tiles, use / g->nHS);
-  g->CH = ceil_div(tiles, g->nRG);
-  g->nRG = ceil_div(tiles, g->CH);
-  return g->CH <= most;
+  // Under an SM budget (two directions side by side) first within it; if that takes too many chains,
+  // the whole GPU for one direction after the other still beats the step-wise path (bf16 LSTM, two
+  // directions of 139 rows, H = 696: 18 chains within the budget, 6 without).
+  for (int use : {budget, sms}) {
+    if (use < g->nHS || use > sms) continue;
+    g->nRG = min(tiles, use / g->nHS);
+    g->CH = ceil_div(tiles, g->nRG);
+    g->nRG = ceil_div(tiles, g->CH);
+    if (g->CH <= most) return true;
+  }
+  return false;
 }
 
 // How many chains per CTA the cluster kernels may take before the grid kernels do better (us per
