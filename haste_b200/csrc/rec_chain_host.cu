@@ -55,8 +55,10 @@ bool gl_geometry(int dtype, int T, int N, int H, int most, GlGeometry* g) {
 // always enough of them (H = 192, 128 rows: 1.4 / 2.2 forward).  At 256 units a cluster is 16 CTAs
 // and only seven are resident one CTA per SM: 32 rows 1.15 / 1.5 forward, 1.2 / 2.0 backward, but
 // 128 rows 2.8 / 1.8 and 3.0 / 2.4.  Five quads per CTA (to 320 units) pay in the backward pass
-// only: 2.0 / 1.7 and 1.8 / 2.2 at 19 rows.
+// only: 2.0 / 1.7 and 1.8 / 2.2 at 19 rows.  Eight (bf16, backward, to 512 units): one chain 1.47 / 1.96
+// at H = 384 and 1.58 / 2.41 at H = 512 (48 and 56 rows), two chains 2.87 / 2.31 and 3.0 / 2.4.
 int cluster_chains(const ClGeometry& g, bool bwd) {
+  if (g.NW == 8) return 1;
   if (g.NW == 5) return bwd ? 1 : 0;
   return g.CS <= 12 ? kClMaxChains : 1;
 }
@@ -80,7 +82,7 @@ int run_fwd(ChainParams& p, int dtype, int grid_most, ClRun cl, GlRun gl, cudaSt
   p.sync.err = device_error_word();
   HB_REQUIRE(p.sync.err, "error word");
   ClGeometry cg;
-  if (cl_geometry(p.H, &cg)) {
+  if (cl_geometry(p.H, false, &cg)) {
     int groups = 0;
     const int st_ = cl(dtype, p, cluster_chains(cg, false), &groups, s);
     if (st_ != HASTE_B200_ERR_UNSUPPORTED) return st_;
@@ -99,7 +101,7 @@ int run_bwd(ChainParams& p, int dtype, int grid_most, int gates, void* db, void*
   HB_REQUIRE(p.sync.err, "error word");
   const int tiles = ceil_div(p.N, 8);
   ClGeometry cg;
-  if (cl_geometry(p.H, &cg)) {
+  if (cl_geometry(p.H, dtype == HASTE_B200_BF16, &cg)) {
     p.db_part = static_cast<float*>(workspace(s, (size_t)tiles * 4 * p.H * sizeof(float), /*slot=*/2));
     if (!p.db_part) return HASTE_B200_ERR_CUDA;
     int groups = 0;

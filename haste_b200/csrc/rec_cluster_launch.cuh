@@ -15,8 +15,15 @@ struct ClGeometry {
 
 // 16 units per CTA up to H = 256 (one quad per tensor-core sub-partition); from there to 320 five
 // quads keep the cluster at 16 CTAs - the largest there is - and R in registers.
-inline bool cl_geometry(int H, ClGeometry* g) {
-  if (H <= 256) {
+// Backward with bf16 storage - half the weights, a third of the MMAs - 32 units per CTA reach 512.
+// (In the other places that would fit, halving the cluster that way loses to the doubled work per
+// sub-partition: H = 256, 32 rows 1.05 -> 1.30 us per step forward, 0.97 -> 1.21 backward, and
+// forward at 512 units 1.65 -> 2.09 against the grid.)
+inline bool cl_geometry(int H, bool wide_bwd, ClGeometry* g) {
+  if (wide_bwd && H > 256 && H <= 512) {
+    g->NW = 8;
+    g->CS = ceil_div(H, 32);
+  } else if (H <= 256) {
     g->NW = 4;
     g->CS = ceil_div(H, 16);
   } else if (H <= 320) {
@@ -91,7 +98,7 @@ int cl_fwd_go(ChainParams& p, int most, int* row_groups, cudaStream_t s) {
 template <int G, int SPLIT, typename T>
 int cl_fwd(ChainParams& p, int most, int* row_groups, cudaStream_t s) {
   ClGeometry g;
-  if (!cl_geometry(p.H, &g)) return HASTE_B200_ERR_UNSUPPORTED;
+  if (!cl_geometry(p.H, false, &g)) return HASTE_B200_ERR_UNSUPPORTED;
   p.CTAS = g.CS;
   p.K16 = g.K16;
   if (g.NW == 5) return cl_fwd_go<G, 5, 20, SPLIT, T>(p, most, row_groups, s);
@@ -112,9 +119,13 @@ int cl_bwd_go(ChainParams& p, int most, int* row_groups, cudaStream_t s) {
 template <int G, int SPLIT, typename T>
 int cl_bwd(ChainParams& p, int most, int* row_groups, cudaStream_t s) {
   ClGeometry g;
-  if (!cl_geometry(p.H, &g)) return HASTE_B200_ERR_UNSUPPORTED;
+  if (!cl_geometry(p.H, SPLIT == 1, &g)) return HASTE_B200_ERR_UNSUPPORTED;
   p.CTAS = g.CS;
   p.K16 = g.K16;
+  if constexpr (SPLIT == 1) {
+    if (g.NW == 8 && g.CS <= 12) return cl_bwd_go<G, 8, 3, SPLIT, T>(p, most, row_groups, s);
+    if (g.NW == 8) return cl_bwd_go<G, 8, 4, SPLIT, T>(p, most, row_groups, s);
+  }
   if (g.NW == 5) return cl_bwd_go<G, 5, 4, SPLIT, T>(p, most, row_groups, s);
   if (g.K16 <= 4) return cl_bwd_go<G, 4, 1, SPLIT, T>(p, most, row_groups, s);
   if (g.K16 <= 8) return cl_bwd_go<G, 4, 2, SPLIT, T>(p, most, row_groups, s);
