@@ -23,6 +23,7 @@
 //
 // Replaces the cuBLAS calls of the reference (lib/blas.h:48-61 and the call sites in
 // lib/*_gpu.cu.cc).
+#include <algorithm>
 #include <atomic>
 #include <type_traits>
 
@@ -620,19 +621,31 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
 // same orientation as the source, leading dimension ld_dst (a multiple of 8), planes
 // `plane_stride` elements apart.  One thread converts 4 consecutive elements of a row:
 // a 16-byte load and one 8-byte store per plane when the source allows it.
+// One launch takes up to two operands (blockIdx.y).
+struct SplitJob {
+  const void* src = nullptr;
+  long long ld_src = 0;
+  int rows = 0, cols = 0;
+  __nv_bfloat16* dst = nullptr;
+  long long ld_dst = 0, plane_stride = 0;
+  int vec_ok = 0;
+};
 template <int PLANES, typename TS>
-__global__ void split_planes_kernel(const TS* __restrict__ src, long long ld_src, int rows,
-                                    int cols, __nv_bfloat16* __restrict__ dst, long long ld_dst,
-                                    long long plane_stride, int vec_ok) {
+__global__ void split_planes_kernel(const SplitJob job0, const SplitJob job1) {
+  const SplitJob& job = blockIdx.y ? job1 : job0;
+  const TS* __restrict__ src = static_cast<const TS*>(job.src);
+  __nv_bfloat16* __restrict__ dst = job.dst;
+  const long long ld_src = job.ld_src, ld_dst = job.ld_dst, plane_stride = job.plane_stride;
+  const int cols = job.cols;
   const int quads = (int)(ld_dst / 4);
-  const long long total = (long long)rows * quads;
+  const long long total = (long long)job.rows * quads;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
     const long long r = i / quads;
     const int c = (int)(i - r * quads) * 4;
     float x[4] = {0.f, 0.f, 0.f, 0.f};
     const TS* sp = src + r * ld_src + c;
-    if (vec_ok && c + 3 < cols) {
+    if (job.vec_ok && c + 3 < cols) {
       if constexpr (sizeof(TS) == 4) {
         const float4 f = *reinterpret_cast<const float4*>(sp);
         x[0] = f.x; x[1] = f.y; x[2] = f.z; x[3] = f.w;
@@ -664,32 +677,22 @@ __global__ void split_planes_kernel(const TS* __restrict__ src, long long ld_src
   }
 }
 
-// `dtype` of the source.  __half: its 11 significant bits split exactly into two planes.  bf16: one
-// plane, a copy with rows that TMA can address.
-int launch_split(const void* src, int dtype, long long ld_src, int rows, int cols,
-                 __nv_bfloat16* dst, long long ld_dst, long long plane_stride, int planes,
-                 int blocks, cudaStream_t stream) {
-  const int vec_ok = ((ld_src & 3) == 0) &&
-                     ((reinterpret_cast<uintptr_t>(src) & (dtype == HASTE_B200_F32 ? 15 : 7)) == 0);
-  if (dtype == HASTE_B200_BF16) {
-    split_planes_kernel<1, __nv_bfloat16><<<blocks, 256, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(src), ld_src, rows, cols, dst, ld_dst, plane_stride, vec_ok);
-  } else if (dtype == HASTE_B200_F16) {
-    const __half* hs = static_cast<const __half*>(src);
-    if (planes == 3)
-      split_planes_kernel<3, __half><<<blocks, 256, 0, stream>>>(hs, ld_src, rows, cols, dst, ld_dst,
-                                                                 plane_stride, vec_ok);
-    else
-      split_planes_kernel<2, __half><<<blocks, 256, 0, stream>>>(hs, ld_src, rows, cols, dst, ld_dst,
-                                                                 plane_stride, vec_ok);
-  } else if (planes == 3)
-    split_planes_kernel<3, float><<<blocks, 256, 0, stream>>>(static_cast<const float*>(src), ld_src,
-                                                              rows, cols, dst, ld_dst, plane_stride,
-                                                              vec_ok);
-  else
-    split_planes_kernel<2, float><<<blocks, 256, 0, stream>>>(static_cast<const float*>(src), ld_src,
-                                                              rows, cols, dst, ld_dst, plane_stride,
-                                                              vec_ok);
+// `dtype` of the sources.  __half: its 11 significant bits split exactly into two planes.  bf16: one
+// plane, a copy with rows that TMA can address.  jobs: one or two.
+int launch_split(SplitJob* jobs, int n, int dtype, int planes, cudaStream_t stream) {
+  long long most = 0;
+  for (int i = 0; i < n; ++i) {
+    jobs[i].vec_ok = (jobs[i].ld_src & 3) == 0 &&
+                     (reinterpret_cast<uintptr_t>(jobs[i].src) & (dtype == HASTE_B200_F32 ? 15 : 7)) == 0;
+    most = std::max(most, (long long)jobs[i].rows * (jobs[i].ld_dst / 4));
+  }
+  const dim3 grid(min(ceil_div(most, 256), 8 * sm_count()), n);
+  const SplitJob a = jobs[0], b = jobs[n - 1];
+  if (dtype == HASTE_B200_BF16) split_planes_kernel<1, __nv_bfloat16><<<grid, 256, 0, stream>>>(a, b);
+  else if (dtype == HASTE_B200_F16 && planes == 3) split_planes_kernel<3, __half><<<grid, 256, 0, stream>>>(a, b);
+  else if (dtype == HASTE_B200_F16) split_planes_kernel<2, __half><<<grid, 256, 0, stream>>>(a, b);
+  else if (planes == 3) split_planes_kernel<3, float><<<grid, 256, 0, stream>>>(a, b);
+  else split_planes_kernel<2, float><<<grid, 256, 0, stream>>>(a, b);
   HB_LAUNCH_OK();
   count_launch(1);
   return HASTE_B200_OK;
@@ -785,8 +788,8 @@ int max_pairs() {
 int gemm_split_planes(const float* src, long long ld_src, int rows, int cols,
                       __nv_bfloat16* dst, long long ld_dst, long long plane_stride,
                       cudaStream_t stream) {
-  return launch_split(src, HASTE_B200_F32, ld_src, rows, cols, dst, ld_dst, plane_stride, 2,
-                      8 * sm_count(), stream);
+  SplitJob job{src, ld_src, rows, cols, dst, ld_dst, plane_stride};
+  return launch_split(&job, 1, HASTE_B200_F32, 2, stream);
 }
 
 namespace {
@@ -891,17 +894,19 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
   A.plane_stride = a_pre ? g.a_pl_stride : 0;
   B.base = b_pre ? g.b_pl : g.b;
   B.plane_stride = b_pre ? g.b_pl_stride : 0;
+  SplitJob jobs[2];
+  int n_jobs = 0;
   auto through_scratch = [&](const void* src, long long ld_src, long long rows, long long cols, size_t plane,
-                             long long ld, Operand* o) -> int {
+                             long long ld, Operand* o) {
     __nv_bfloat16* to = ws.take<__nv_bfloat16>(planes * plane / 2);
-    if (!to) return unsupported("scratch arena");
-    HB_TRY(launch_split(src, g.dtype, ld_src, (int)rows, (int)cols, to, ld, plane / 2, planes, 8 * sms, stream));
+    jobs[n_jobs++] = SplitJob{src, ld_src, (int)rows, (int)cols, to, ld, (long long)(plane / 2)};
     o->base = to;
     o->plane_stride = plane / 2;
-    return HASTE_B200_OK;
+    return to != nullptr;
   };
-  if (a_copy) HB_TRY(through_scratch(g.a, a_ld_src, a_rows, a_cols, a_plane, a_ld, &A));
-  if (b_copy) HB_TRY(through_scratch(g.b, b_ld_src, b_rows, b_cols, b_plane, b_ld, &B));
+  if (a_copy && !through_scratch(g.a, a_ld_src, a_rows, a_cols, a_plane, a_ld, &A)) return unsupported("scratch arena");
+  if (b_copy && !through_scratch(g.b, b_ld_src, b_rows, b_cols, b_plane, b_ld, &B)) return unsupported("scratch arena");
+  if (n_jobs) HB_TRY(launch_split(jobs, n_jobs, g.dtype, planes, stream));
   A.ld = a_ld;
   B.ld = b_ld;
   float* partial = nullptr;
