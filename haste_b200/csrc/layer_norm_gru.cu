@@ -172,18 +172,29 @@ int layer_norm_gru_backward(const LnGruBwd& a, cudaStream_t s) {
     HB_TRY(colsum(a.dtype, static_cast<const char*>(a.dq) + third, 3LL * H, (int)TN, H, a.dtype,
                   static_cast<char*>(a.dbr) + third, 1, cs, s));
   }
+  // fp32: LayerNorm 1 leaves d(x.W) as the bf16 planes that both contractions below read as well
+  // (without this scratch they split it for themselves)
+  __nv_bfloat16* planes = nullptr;
+  long long plane_stride = 0;
+  if (a.dtype == HASTE_B200_F32 && (3 * H) % 8 == 0) {
+    const size_t pe = Arena::pad((size_t)TN * 3 * H * 2) / 2;  // elements per plane
+    planes = static_cast<__nv_bfloat16*>(workspace(s, 2 * pe * 2 + 256, /*slot=*/3));
+    plane_stride = (long long)pe;
+  }
   // LayerNorm 1 backward over all steps, in place on dp.
   HB_TRY(layer_norm_backward(a.dtype, (int)TN, 3 * H, a.gamma_Wx, a.act_Wx, a.dp, a.dp, a.dtype,
-                             a.dgamma_Wx, nullptr, a.cache_Wx, lns, s));
+                             a.dgamma_Wx, nullptr, a.cache_Wx, lns, s, planes, plane_stride));
   const bool tr = a.transposed_inputs != 0;
   GemmDesc gx{a.dtype, a.dtype, (int)TN, C, 3 * H, a.dp, 3LL * H, 1, a.W, tr ? C : 1,
               tr ? 1 : 3LL * H, a.dx, C, 0};
+  if (planes) { gx.a_pl = planes; gx.a_pl_ld = 3LL * H; gx.a_pl_stride = plane_stride; }
   HB_TRY(gemm(gx, s));
   GemmDesc gr{a.dtype, a.dtype, H, 3 * H, (int)TN, a.h, 1, H, a.act_Rh, 3LL * H, 1, a.dR,
               3LL * H, add};
   HB_TRY(gemm(gr, s));
   GemmDesc gw{a.dtype, a.dtype, C, 3 * H, (int)TN, a.x, tr ? TN : 1, tr ? 1 : C, a.dp, 3LL * H, 1,
               a.dW, 3LL * H, add};
+  if (planes) { gw.b_pl = planes; gw.b_pl_ld = 3LL * H; gw.b_pl_stride = plane_stride; }
   HB_TRY(gemm(gw, s));
   return HASTE_B200_OK;
 }

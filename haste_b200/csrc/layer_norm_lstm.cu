@@ -497,6 +497,15 @@ int backward_core(const LnLstmBwd& a, cudaStream_t s) {
   HB_TRY(from_float(a.dtype, dh_carry, a.dh, NH, s));
   HB_TRY(from_float(a.dtype, dc_carry, a.dc, NH, s));
 
+  // fp32: LayerNorm 1 leaves d(x.W) as the bf16 planes that both contractions below read as well
+  // (without this scratch they split it for themselves)
+  __nv_bfloat16* planes = nullptr;
+  long long plane_stride = 0;
+  if (a.dtype == HASTE_B200_F32 && (4 * H) % 8 == 0) {
+    const size_t pe = Arena::pad((size_t)TN * 4 * H * 2) / 2;  // elements per plane
+    planes = static_cast<__nv_bfloat16*>(workspace(s, 2 * pe * 2 + 256, /*slot=*/3));
+    plane_stride = (long long)pe;
+  }
   {
     ProfScope p(PH_OTHER, s);
     // act_Wx_norm now holds the gradient w.r.t. (LN1(x.W) + LN2(h.R) + b).
@@ -504,11 +513,13 @@ int backward_core(const LnLstmBwd& a, cudaStream_t s) {
       HB_TRY(colsum(a.dtype, a.act_Wx_norm, 4LL * H, (int)TN, 4 * H, a.dtype, a.db, 1, cs, s));
     // LayerNorm 1 backward over all steps: act_Wx <- d/d(x.W).
     HB_TRY(layer_norm_backward(a.dtype, (int)TN, 4 * H, a.gamma_Wx, a.act_Wx, a.act_Wx_norm,
-                               a.act_Wx, a.dtype, a.dgamma_Wx, nullptr, a.cache_Wx, lns, s));
+                               a.act_Wx, a.dtype, a.dgamma_Wx, nullptr, a.cache_Wx, lns, s, planes,
+                               plane_stride));
   }
   const bool tr = a.transposed_inputs != 0;
   GemmDesc gw{a.dtype, a.dtype, C, 4 * H, (int)TN, a.x, tr ? TN : 1, tr ? 1 : C, a.act_Wx,
               4LL * H, 1, a.dW, 4LL * H, assign ? 0 : 1};
+  if (planes) { gw.b_pl = planes; gw.b_pl_ld = 4LL * H; gw.b_pl_stride = plane_stride; }
   {
     ProfScope p(PH_WGRAD, s);
     HB_TRY(gemm(gw, s));
@@ -521,6 +532,7 @@ int backward_core(const LnLstmBwd& a, cudaStream_t s) {
   }
   GemmDesc gx{a.dtype, a.dtype, (int)TN, C, 4 * H, a.act_Wx, 4LL * H, 1, a.W, tr ? C : 1,
               tr ? 1 : 4LL * H, a.dx, C, 0};
+  if (planes) { gx.a_pl = planes; gx.a_pl_ld = 4LL * H; gx.a_pl_stride = plane_stride; }
   {
     ProfScope p(PH_DGRAD, s);
     HB_TRY(gemm(gx, s));
