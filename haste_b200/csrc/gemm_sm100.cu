@@ -25,6 +25,7 @@
 // lib/*_gpu.cu.cc).
 #include <algorithm>
 #include <atomic>
+#include <cstring>
 #include <type_traits>
 
 #include "cells.cuh"
@@ -637,11 +638,11 @@ __global__ void split_planes_kernel(const SplitJob job0, const SplitJob job1) {
   __nv_bfloat16* __restrict__ dst = job.dst;
   const long long ld_src = job.ld_src, ld_dst = job.ld_dst, plane_stride = job.plane_stride;
   const int cols = job.cols;
-  const int quads = (int)(ld_dst / 4);
+  const unsigned quads = (unsigned)(ld_dst / 4);
   const long long total = (long long)job.rows * quads;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
-    const long long r = i / quads;
+    const long long r = total >> 32 ? i / quads : (long long)((unsigned)i / quads);
     const int c = (int)(i - r * quads) * 4;
     float x[4] = {0.f, 0.f, 0.f, 0.f};
     const TS* sp = src + r * ld_src + c;
@@ -698,22 +699,53 @@ int launch_split(SplitJob* jobs, int n, int dtype, int planes, cudaStream_t stre
   return HASTE_B200_OK;
 }
 
-// Adds up the partial tiles of a K split ([splits][M][ld]) into C.
-template <typename TC>
-__global__ void splitk_reduce_kernel(const float* __restrict__ part, int splits, long long split_stride,
-                                     int M, int N, int ld_part, TC* __restrict__ c, long long ldc, int accumulate) {
-  const long long MN = (long long)M * N;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < MN;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long m = i / N;
-    const int n = (int)(i - m * N);
-    const float* src = part + m * ld_part + n;
-    float s = 0.f;
-    for (int k = 0; k < splits; ++k) s += src[k * split_stride];
-    TC* dst = c + m * ldc + n;
-    if (accumulate) s += ld(dst);
-    st(dst, s);
+// Adds up the partial tiles of a K split ([splits][M][ld], ld a multiple of 32) into C: four columns
+// per thread, eight threads per 32-column chunk.  Vec: C's rows take 16-byte (8-byte) stores.
+template <typename TC, bool Vec>
+__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restrict__ part, int splits,
+                                                            long long split_stride, int M, int N, int ld_part,
+                                                            TC* __restrict__ c, long long ldc, int accumulate) {
+  const unsigned quads = ld_part / 4, total = (unsigned)M * quads;
+  for (unsigned i = blockIdx.x * 256 + threadIdx.x; i < total; i += gridDim.x * 256) {
+    const unsigned m = i / quads, n = (i - m * quads) * 4;
+    if ((int)n >= N) continue;
+    const float4* src = reinterpret_cast<const float4*>(part + (long long)m * ld_part + n);
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (int k = 0; k < splits; ++k) {
+      const float4 f = src[k * (split_stride / 4)];
+      s.x += f.x; s.y += f.y; s.z += f.z; s.w += f.w;
+    }
+    float v[4] = {s.x, s.y, s.z, s.w};
+    TC* dst = c + (long long)m * ldc + n;
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (accumulate && (Vec || (int)n + e < N)) v[e] += ld(dst + e);
+    if constexpr (Vec) {
+      TC out[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) st(out + e, v[e]);
+      typedef typename std::conditional<sizeof(TC) == 4, uint4, uint2>::type Word;
+      Word w;
+      memcpy(&w, out, sizeof(w));
+      *reinterpret_cast<Word*>(dst) = w;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if ((int)n + e < N) st(dst + e, v[e]);
+    }
   }
+}
+template <typename TC>
+void launch_reduce(const float* part, int splits, int M, int N, int ld_part, void* c, long long ldc, int accumulate,
+                   int most, cudaStream_t stream) {
+  const long long stride = (long long)M * ld_part;
+  const int blocks = min(ceil_div(stride / 4, 256), most);
+  const bool vec = N % 4 == 0 && ldc % 4 == 0 && reinterpret_cast<uintptr_t>(c) % (4 * sizeof(TC)) == 0;
+  if (vec)
+    splitk_reduce_kernel<TC, true><<<blocks, 256, 0, stream>>>(part, splits, stride, M, N, ld_part, (TC*)c, ldc, accumulate);
+  else
+    splitk_reduce_kernel<TC, false><<<blocks, 256, 0, stream>>>(part, splits, stride, M, N, ld_part, (TC*)c, ldc, accumulate);
 }
 
 // ----------------------------------------------------------------------------
@@ -831,8 +863,14 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
 
   // scratch: planes for fp32 operands, partial tiles for split-K
   const int sms = sm_count();
-  // CTA pairs on 256 x 256 tiles where the output is wide enough to fill them
-  const int pairs = (gemm_path() == HASTE_B200_GEMM_TCGEN05_SINGLE || M < 192 || N < 192)
+  // CTA pairs on 256 x 256 tiles where the output is wide enough to fill them and the work is
+  // worth the cluster launch and the coarser waves: 4 .. 7 us below 16 G multiply-adds, where only a
+  // long K lets the pair's better rate make up for it (us, pair / single: fp32 2000 x 512 x 512 31 / 17,
+  // 20000 x 512 x 512 66 / 58, 6400 x 512 x 2048 66 / 70, 30000 x 1024 x 1024 206 / 222; bf16 29 / 25 for the
+  // second, 22 / 27 for the third).
+  const double macs = (double)M * N * K;
+  const bool large = macs >= 16e9 || (macs >= 4e9 && K >= 1024);
+  const int pairs = (gemm_path() == HASTE_B200_GEMM_TCGEN05_SINGLE || M < 192 || N < 192 || !large)
                         ? 0 : max_pairs();
   const bool pair = pairs > 0;
   const int units = pair ? pairs : sms;
@@ -882,8 +920,8 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
   // ([12321 x 161] . [161 x 750] in fp32: 56 us), so such a C goes through a padded fp32 tile as
   // the parts of a K split do, and the reduction writes it row by row.
   const bool c_rows = (g.ldc % (g.dtype_c == HASTE_B200_F32 ? 4 : 8)) == 0 && ((uintptr_t)g.c & 15) == 0;
-  const bool via_partial = splits > 1 || (!c_rows && M >= 64);
   const int part_ld = (N + 31) & ~31;
+  const bool via_partial = splits > 1 || (!c_rows && M >= 64 && (long long)M * (part_ld / 4) < (1LL << 31));
   const size_t part_bytes = via_partial ? Arena::pad((size_t)splits * M * part_ld * 4) : 0;
   const size_t bytes = planes * (a_plane + b_plane) + part_bytes + 1024;
   Arena ws;
@@ -971,17 +1009,10 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
   HB_LAUNCH_OK();
   count_launch(1);
   if (via_partial) {
-    const int blocks = min(ceil_div((long long)M * N, 256), 8 * sms);
-    const long long stride = (long long)M * part_ld;
-    if (g.dtype_c == HASTE_B200_BF16)
-      splitk_reduce_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(partial, splits, stride, M, N, part_ld,
-                                                                      (__nv_bfloat16*)g.c, g.ldc, g.accumulate);
-    else if (g.dtype_c == HASTE_B200_F16)
-      splitk_reduce_kernel<__half><<<blocks, 256, 0, stream>>>(partial, splits, stride, M, N, part_ld,
-                                                               (__half*)g.c, g.ldc, g.accumulate);
-    else
-      splitk_reduce_kernel<float><<<blocks, 256, 0, stream>>>(partial, splits, stride, M, N, part_ld,
-                                                              (float*)g.c, g.ldc, g.accumulate);
+    auto reduce = g.dtype_c == HASTE_B200_BF16  ? launch_reduce<__nv_bfloat16>
+                  : g.dtype_c == HASTE_B200_F16 ? launch_reduce<__half>
+                                                : launch_reduce<float>;
+    reduce(partial, splits, M, N, part_ld, g.c, g.ldc, g.accumulate, 16 * sms, stream);
     HB_LAUNCH_OK();
     count_launch(1);
   }
