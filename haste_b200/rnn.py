@@ -669,6 +669,21 @@ def _flip_time(x):
     return _FlipTime.apply(x)
 
 
+_side_streams = {}
+
+
+def _side_stream(device, main):
+    """The stream beside `main` for the second direction of a bidirectional level: one per stream
+    that a program works on, whatever the number of its `Stack`s, because the library keeps
+    scratch per stream (a stream of its own for every Stack made the first pass of a
+    three-layer LayerNormLSTM stack 58 ms, four times a pass, most of it allocation)."""
+    key = (device.index, main.cuda_stream)
+    side = _side_streams.get(key)
+    while side is None or side.cuda_stream == main.cuda_stream:  # (torch hands out a fixed set in turn)
+        side = _side_streams[key] = torch.cuda.Stream(device=device)
+    return side
+
+
 class Stack(nn.Module):
     """`num_layers` layers of one cell type, optionally bidirectional.
 
@@ -696,7 +711,6 @@ class Stack(nn.Module):
             layers.append(nn.ModuleList([cell(in_size, hidden_size, **cell_kwargs)
                                          for _ in range(dirs)]))
         self.layers = nn.ModuleList(layers)
-        self._side = None
         self._budget_set = False
 
     def forward(self, x, masks=None):
@@ -705,8 +719,6 @@ class Stack(nn.Module):
             if not self.bidirectional:
                 x, _ = level[0](x, **kw[0])
                 continue
-            if self._side is None:
-                self._side = torch.cuda.Stream(device=x.device)
             if not self._budget_set and self.concurrent_directions:
                 # half of the GPU per direction: the two directions' persistent kernels, issued
                 # on two streams, then run at the same time instead of one after the other
@@ -716,17 +728,18 @@ class Stack(nn.Module):
                         layer._sm_budget = sms
                 self._budget_set = True
             main = torch.cuda.current_stream()
+            side = _side_stream(x.device, main)
             # the side stream starts after everything queued so far (x included) and makes its
             # own reversed copy, so no kernel of the backward-direction layer can run ahead
             # of the flip that produces its input
-            self._side.wait_stream(main)
-            with torch.cuda.stream(self._side):
-                x.record_stream(self._side)
+            side.wait_stream(main)
+            with torch.cuda.stream(side):
+                x.record_stream(side)
                 x_rev = _flip_time(x)
                 y_bw, _ = level[1](x_rev, **kw[1])
                 y_bw = _flip_time(y_bw)
             y_fw, _ = level[0](x, **kw[0])
-            main.wait_stream(self._side)
+            main.wait_stream(side)
             y_bw.record_stream(main)
             x = torch.cat([y_fw, y_bw], dim=-1)
         return x
