@@ -160,6 +160,11 @@ inline int gemm_small(const GemmDesc& g, cudaStream_t s) {
   return gemm_simt(g, s);
 }
 
+// fp32 [rows, width] -> planes for several contractions, in the scratch the recurrence kernels would
+// have written them to; *have stays false if `wanted` is or the scratch cannot be had.
+int split_once(const void* src, long long rows, int width, bool wanted, GradPlanes* planes, long long* ld, bool* have,
+               cudaStream_t s);
+
 // Process-wide knobs (set through the C ABI).
 int recurrence_path();
 int sm_budget();  // 0: the whole GPU; else the SMs one recurrence launch may occupy

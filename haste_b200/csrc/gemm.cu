@@ -16,4 +16,17 @@ int gemm(const GemmDesc& g, cudaStream_t stream) {
   return gemm_simt(g, stream);
 }
 
+int split_once(const void* src, long long rows, int width, bool wanted, GradPlanes* planes, long long* ld, bool* have,
+               cudaStream_t s) {
+  if (!wanted) return HASTE_B200_OK;
+  const long long pad = (width + 7) & ~7LL;
+  const size_t pe = Arena::pad((size_t)rows * pad * 2) / 2;  // elements per plane
+  planes->p = static_cast<__nv_bfloat16*>(workspace(s, 2 * pe * 2 + 256, /*slot=*/3));
+  if (!planes->p) return HASTE_B200_OK;
+  planes->stride = (long long)pe;
+  *ld = pad;
+  *have = true;
+  return gemm_split_planes(static_cast<const float*>(src), width, (int)rows, width, planes->p, pad, planes->stride, s);
+}
+
 }  // namespace hb

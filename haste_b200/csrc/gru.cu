@@ -286,8 +286,13 @@ int gru_backward(const GruBwd& a, cudaStream_t s) {
   const bool tr = a.transposed_inputs != 0;
   GemmDesc gx{a.dtype, a.dtype, (int)TN, C, 3 * H, a.dp, 3LL * H, 1, a.W, tr ? C : 1,
               tr ? 1 : 3LL * H, a.dx, C, 0};
-  if (have_planes) {  // dp was already split into bf16 planes by the recurrence kernel
-    gx.a_pl = planes.p; gx.a_pl_ld = 3LL * H; gx.a_pl_stride = planes.stride;
+  // two contractions read dp: without planes from the recurrence it is split once
+  long long pl_ld = 3LL * H;
+  bool dp_planes = have_planes;
+  if (!have_planes && a.dtype == HASTE_B200_F32 && a.dx)
+    HB_TRY(split_once(a.dp, TN, 3 * H, !a.iterate && gemm_reads_planes(gx), &planes, &pl_ld, &dp_planes, s));
+  if (dp_planes) {
+    gx.a_pl = planes.p; gx.a_pl_ld = pl_ld; gx.a_pl_stride = planes.stride;
   }
   if (a.dx) {
     ProfScope p(PH_DGRAD, s);
@@ -303,8 +308,8 @@ int gru_backward(const GruBwd& a, cudaStream_t s) {
   }
   GemmDesc gw{a.dtype, a.dtype, C, 3 * H, (int)TN, a.x, tr ? TN : 1, tr ? 1 : C, a.dp, 3LL * H, 1,
               a.dW, 3LL * H, add};
-  if (have_planes) {
-    gw.b_pl = planes.p; gw.b_pl_ld = 3LL * H; gw.b_pl_stride = planes.stride;
+  if (dp_planes) {
+    gw.b_pl = planes.p; gw.b_pl_ld = pl_ld; gw.b_pl_stride = planes.stride;
   }
   {
     ProfScope p(PH_WGRAD, s);

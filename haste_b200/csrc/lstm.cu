@@ -246,10 +246,13 @@ int lstm_backward(const LstmBwd& a, cudaStream_t s) {
   // dx[T*N,C] = dv . W^T
   GemmDesc gx{a.dtype, a.dtype, (int)TN, C, 4 * H, a.v, 4LL * H, 1, a.W, tr ? C : 1,
               tr ? 1 : 4LL * H, a.dx, C, 0};
-  if (have_planes) {  // dv was already split into bf16 planes by the recurrence kernel
-    gw.b_pl = planes.p; gw.b_pl_ld = 4LL * H; gw.b_pl_stride = planes.stride;
-    gr.b_pl = planes.p; gr.b_pl_ld = 4LL * H; gr.b_pl_stride = planes.stride;
-    gx.a_pl = planes.p; gx.a_pl_ld = 4LL * H; gx.a_pl_stride = planes.stride;
+  long long pl_ld = 4LL * H;
+  if (!have_planes && a.dtype == HASTE_B200_F32)  // three contractions read dv: split it once
+    HB_TRY(split_once(a.v, TN, 4 * H, !a.iterate && gemm_reads_planes(gr), &planes, &pl_ld, &have_planes, s));
+  if (have_planes) {  // dv as bf16 planes
+    gw.b_pl = planes.p; gw.b_pl_ld = pl_ld; gw.b_pl_stride = planes.stride;
+    gr.b_pl = planes.p; gr.b_pl_ld = pl_ld; gr.b_pl_stride = planes.stride;
+    gx.a_pl = planes.p; gx.a_pl_ld = pl_ld; gx.a_pl_stride = planes.stride;
   }
   {
     ProfScope p(PH_WGRAD, s);
