@@ -20,9 +20,10 @@ bool aligned(std::initializer_list<const void*> ptrs, int H, int dtype) {
 // Grid tiling: NMT quads of hidden units per CTA such that its slice of R fits the registers, as
 // many row groups as there are SMs for, the rest of the rows as chains - at most `most` of them: a
 // chain adds 0.7 .. 2 us to a step (H = 512 .. 1024), which the step-wise path (about 20 us plus the
-// product) undercuts from a dozen on, and from six on the tensor-core GRU recurrence (6 us forward,
-// 11 us backward at H = 1024 whatever the rows).
-constexpr int kGridChains = 12, kGridChainsBeforeTc = 5;
+// product) undercuts from a dozen on, and beyond six the tensor-core GRU recurrence (6 us
+// forward, 11 us backward at H = 1024 whatever the rows; both passes of a bidirectional layer of 200
+// steps, chains / tensor-core: 48 rows, six chains, 3.5 / 4.0 ms; 64 rows, eight chains, 4.9 / 4.6).
+constexpr int kGridChains = 12, kGridChainsBeforeTc = 6;
 
 // A handful of steps of a wide fp32 / fp16 layer stays on the step-wise path (as
 // tests/test_parity_gpu.py expects of it).
@@ -119,7 +120,7 @@ int run_bwd(ChainParams& p, int dtype, int grid_most, int gates, void* db, void*
 
 // Rows the tensor-core GRU recurrence would take (rec_tc_gru.cu).
 bool tc_waits(int dtype, int N, int H) {
-  return dtype == HASTE_B200_BF16 && N >= 96 && H % 64 == 0 && recurrence_path() != HASTE_B200_PATH_NO_TENSOR_CORE;
+  return dtype == HASTE_B200_BF16 && N >= 64 && H % 64 == 0 && recurrence_path() != HASTE_B200_PATH_NO_TENSOR_CORE;
 }
 
 }  // namespace

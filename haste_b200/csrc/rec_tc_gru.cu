@@ -195,6 +195,20 @@ __device__ __forceinline__ uint32_t swz_off(int n, int kk) {
   return (uint32_t)((n >> 3) * 1024 + (n & 7) * 128 + ((((kk >> 3) ^ (n & 7)) & 7) << 4) + (kk & 7) * 2);
 }
 
+// The ring's stages belong to NI lanes / issuers for good: `own` has stages own, own + NI, ...  (If
+// they took k-blocks in turn whatever the stage, one of them a whole ring ahead of another would
+// take a phase of a stage for the one two further on, which a barrier's parity does not tell
+// apart.)  From one block of `own` to its next.
+__device__ __forceinline__ void next_block(int& stage, uint32_t& phase, int& kb, int own, int stages) {
+  stage += NI;
+  kb += NI;
+  if (stage >= stages) {
+    kb += stages + own - stage;
+    stage = own;
+    phase ^= 1u;
+  }
+}
+
 template <int NB, bool FWD>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const int stages) {
@@ -301,13 +315,14 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    // PL lanes issue the k-blocks of a tile in turn (lane l takes k-blocks l, l + PL, ...): a
-    // cp.async.bulk.tensor holds its issuing thread for about 0.1 us, which would otherwise
-    // be the rate of the whole ring.
-    constexpr int PL = 4;
+    // PL lanes issue the k-blocks (lane l fills stages l, l + PL, ...): a cp.async.bulk.tensor
+    // holds its issuing thread for about 0.1 us, which would otherwise be the rate of the whole
+    // ring.
+    constexpr int PL = NI;
     constexpr unsigned PMASK = (1u << PL) - 1u;
     if (lane < PL) {
-      uint32_t g0 = 0;  // k-blocks issued before this tile (the same in every lane)
+      int stage = lane, kb = lane;  // this lane's next stage, and its k-block counted from this tile
+      uint32_t phase = 0;
       bool ok = true;
       const uint32_t box_bytes = (uint32_t)p.RB * 128u;
       for (int it = 0; it < p.T && ok; ++it) {
@@ -324,14 +339,13 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
           fence_proxy_async_all();
           const int trow = FWD ? it : (p.T - it);  // time slot of the streamed tensor
           const int row = trow * N + tile * p.RB;
-          for (int kb = lane; kb < KB && ok; kb += PL) {
-            const uint32_t g = g0 + (uint32_t)kb;
-            const uint32_t stage = g % (uint32_t)stages, phase = (g / (uint32_t)stages) & 1u;
+          while (kb < KB) {
             if (!mbar_wait(empty_bar(stage), phase ^ 1u, s_abort, p.err, 52)) { ok = false; break; }
             mbar_expect_tx(full_bar(stage), box_bytes);
             tma_load_3d(ring + stage * p.stage_bytes, &map_a, full_bar(stage), kb * BK, row, 0);
+            next_block(stage, phase, kb, lane, stages);
           }
-          g0 += (uint32_t)KB;
+          kb -= KB;
           ok = __all_sync(PMASK, ok);  // all producer lanes leave together
           HB_STAMP(p, it, mt, 1);  // all TMA loads of the tile issued
         }
@@ -340,10 +354,11 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
   } else if (warp <= NI) {
     // ------------------------------------------------------------------ MMA issuers
     if (lane == 0) {
-      const int iss = warp - 1;  // this issuer takes k-blocks iss, iss + NI, ...
+      const int iss = warp - 1;  // this issuer takes what lies in stages iss, iss + NI, ...
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NB >> 3) << 17) |
                              ((uint32_t)(128 >> 4) << 24);
-      uint32_t g0 = 0;  // k-blocks consumed before this tile
+      int stage = iss, kb = iss;
+      uint32_t phase = 0;
       uint32_t acc_phase[2] = {0, 0};
       int n_acc = 0;
       bool ok = true;
@@ -363,21 +378,20 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
           // Descriptors differ only in their 14-bit start-address field (bytes >> 4): one add
           // per MMA instead of rebuilding them.
 #pragma unroll 1
-          for (int kb = iss; kb < KB; kb += NI) {
-            const uint32_t g = g0 + (uint32_t)kb;
-            const uint32_t stage = g % (uint32_t)stages, phase = (g / (uint32_t)stages) & 1u;
+          for (uint32_t more = 0; kb < KB; more = 1) {
             if (!mbar_wait(full_bar(stage), phase, s_abort, p.err, 54)) { ok = false; break; }
             tc_fence_after();
             if (kb == 0) HB_STAMP(p, it, mt, 2);  // first k-block has landed
             const uint64_t ad = a_desc0 + (uint64_t)stage * a_stage_inc - (halves && mt ? a_stage_inc : 0);
             const uint64_t bd = b_desc0 + (uint64_t)kb * (R_TILE >> 4);
-            tc_mma_bf16(d_tmem, ad, bd, idesc, kb >= NI ? 1u : 0u);
+            tc_mma_bf16(d_tmem, ad, bd, idesc, more);
             tc_mma_bf16(d_tmem, ad + 2, bd + 2, idesc, 1u);
             tc_mma_bf16(d_tmem, ad + 4, bd + 4, idesc, 1u);
             tc_mma_bf16(d_tmem, ad + 6, bd + 6, idesc, 1u);
             tc_commit(empty_bar(stage));
+            next_block(stage, phase, kb, iss, stages);
           }
-          g0 += (uint32_t)KB;
+          kb -= KB;
           if (iss == 0) HB_STAMP(p, it, mt, 3);  // last MMA issued
           if (ok) tc_commit(accf_bar(acc));
         }
@@ -433,7 +447,13 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
             }
           }
         }
-        // ---- wait for the step product
+        // ---- wait for the step product; which issuers had a part in it (all, unless K is short)
+        uint32_t have = (1u << NI) - 1u;
+        if (KB < 2 * NI) {
+          const int first = ((it - (FWD ? 0 : 1)) * min(p.MT, tiles_total - rg * p.MT) + mt) * KB;
+          have = 0;
+          for (int kb = 0; kb < KB; ++kb) have |= 1u << ((first + kb) % stages % NI);
+        }
         int acc = 0;
         if (have_acc) {
           acc = halves ? mt : n_acc & 1;
@@ -462,7 +482,7 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
 #pragma unroll
               for (int k = 0; k < GRP; ++k) {
                 const int i2 = g0 + k;
-                if (i2 < NI && KB > i2) {
+                if (i2 < NI && (have >> i2 & 1u)) {
                   tc_ld8(taddr + i2 * ACC_COLS + uo, b0[k]);
                   if (FWD) {
                     tc_ld8(taddr + i2 * ACC_COLS + 16 + uo, b1[k]);
@@ -474,7 +494,7 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
 #pragma unroll
               for (int k = 0; k < GRP; ++k) {
                 const int i2 = g0 + k;
-                if (i2 < NI && KB > i2) {
+                if (i2 < NI && (have >> i2 & 1u)) {
 #pragma unroll
                   for (int i = 0; i < 8; ++i) {
                     s0[i] += __uint_as_float(b0[k][i]);
@@ -576,7 +596,7 @@ struct TcGeometry {
 };
 
 // Shapes this path takes: bf16, H a multiple of 64 up to 1024 (the resident slice of R and a
-// useful ring must fit shared memory), at least 96 batch rows (below that the register
+// useful ring must fit shared memory), at least 64 batch rows (below that the register
 // kernels are faster) and at most two row tiles per CTA: every CTA of a row group streams
 // the group's whole h (or dq), H / 16 copies of it per step out of L2, which is what bounds
 // the step from a few hundred rows per GPU on - there the per-step contraction + pointwise
@@ -620,7 +640,7 @@ bool tc_geometry_for(int N, int H, bool fwd, int sms, TcGeometry* g) {
 // bidirectional layer are co-resident).
 bool tc_geometry(int N, int H, bool fwd, TcGeometry* g, bool* budgeted) {
   *budgeted = false;
-  if (H % 64 != 0 || H < 64 || H > 1024 || N < 96) return false;
+  if (H % 64 != 0 || H < 64 || H > 1024 || N < 64) return false;
   const int budget = sm_budget();
   if (budget > 0 && budget < sm_count() && tc_geometry_for(N, H, fwd, budget, g)) {
     *budgeted = true;

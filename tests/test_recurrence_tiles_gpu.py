@@ -60,3 +60,16 @@ def test_grid_recurrence_fp32(cell, shape, zoneout):
                                             ("gru", torch.float16, TOL_F16)])
 def test_grid_recurrence_reduced_precision(cell, dtype, tol, shape):
     _check(cell, *shape, dtype, tol, 0.25)
+
+
+# tensor-core GRU recurrence: two 64-row tiles per CTA with a ragged second one, rings whose stage
+# count is no multiple of the issuers, fewer k-blocks than issuers have turns
+@pytest.mark.parametrize("T,N,H,sms", [(40, 90, 1024, 74), (40, 65, 1024, 74), (60, 128, 768, 74), (8, 700, 320, 0)])
+def test_tensor_core_gru_tiles(T, N, H, sms):
+    from haste_b200 import _C
+    _C.set_sm_budget(sms)
+    try:
+        _check("gru", T, N, H, torch.bfloat16, TOL_BF16, 0.25)
+        _C.sync_check(torch.cuda.current_stream().cuda_stream)
+    finally:
+        _C.set_sm_budget(0)
