@@ -1,11 +1,11 @@
-// LayerNormLSTM / LayerNormGRU recurrences on thread-block clusters, sm_100a: up to 256 units.
+// LayerNormLSTM / LayerNormGRU recurrences on thread-block clusters, sm_100a: up to 320 units.
 //
 // A LayerNorm step is a chain of hand-offs: besides the new state, the row statistics of h.R (and,
 // LSTM, of the cell state) have to meet from all columns before any of them can go on.  Through L2
 // (recurrent_ln_kernels.cuh) each hand-off costs 1.3 .. 1.5 us; here the layer's row group lives in
-// one cluster - 16 hidden units per CTA, R in registers, chains of eight rows, as in
+// one cluster - 16 or 20 hidden units per CTA, R in registers, chains of eight rows, as in
 // rec_cluster_kernels.cuh, whose layouts and tagged words these kernels use - and a hand-off is a
-// store into the peers' shared memory.  The statistics of a CTA's four warps meet in its own
+// store into the peers' shared memory.  The statistics of a CTA's warps meet in its own
 // shared memory first, so that a peer receives one 64-byte line (8 rows x 2 words) per CTA: a
 // remote store is paid per line.
 //
@@ -36,7 +36,6 @@ struct LnClBwd : LnBwdParams {
   float* db_part;  // [row groups][4][H] sums of the gate gradients (GRU: z, r, g of dp, g of dq)
 };
 
-constexpr int LC_NW = 4, LC_THREADS = LC_NW * 32, LC_U = 4 * LC_NW;
 constexpr int LC_FWD_STASH = 9, LC_BWD_STASH = 16;  // floats per thread and chain
 
 __device__ __forceinline__ uint2 lc_poll2(uint32_t a) {
@@ -101,6 +100,7 @@ __device__ __forceinline__ float plane_sum(const float (&a)[PL][4], int j) {
 
 // The exchange of row statistics: buffers of the CTA ([stat][parity][chain][source][row] pairs of
 // tagged words) and the meeting place of its warps ([stat][parity][warp][row]).
+template <int NW>
 struct Stats {
   uint32_t buf, dst, SB;  // own buffers; this lane's place in its destination's; bytes per buffer
   float2* part;
@@ -110,7 +110,7 @@ struct Stats {
   __device__ __forceinline__ uint32_t area(int stat, int par, int ch) const {
     return (uint32_t)((stat * 2 + par) * CH + ch) * SB;
   }
-  __device__ __forceinline__ float2* meet(int stat, int par) const { return part + (stat * 2 + par) * LC_NW * 8; }
+  __device__ __forceinline__ float2* meet(int stat, int par) const { return part + (stat * 2 + par) * NW * 8; }
   // Pairs of this lane's quarter of the sources for `row`; zeros beyond the cluster.
   __device__ __forceinline__ bool collect(int stat, int par, int ch, int row, int quarter, uint32_t tag, float (&a)[4],
                                           float (&b)[4], const Sync& sync, volatile int* s_abort, int code) const {
@@ -140,38 +140,39 @@ struct Stats {
 };
 
 // ---------------------------------------------------------------------------------------
-template <int G, int KS, int SPLIT, typename T>
-__global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_fwd_kernel(const __grid_constant__ LnClFwd p) {
-  constexpr int PL = SPLIT == 2 ? 3 : 1;
+template <int G, int NW, int KS, int SPLIT, typename T>
+__global__ void __launch_bounds__(NW * 32, 1) ln_cl_fwd_kernel(const __grid_constant__ LnClFwd p) {
+  constexpr int PL = SPLIT == 2 ? 3 : 1, U = 4 * NW, THREADS_ = NW * 32;
   extern __shared__ __align__(16) uint8_t smem[];
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
   const int CS = p.CTAS, my = (int)cl_rank(), rg = blockIdx.x / CS;
-  const int H = p.H, N = p.N, u0 = my * LC_U, tile0 = rg * p.CH, ch_n = min(p.CH, ((N + 7) >> 3) - tile0);
+  const int H = p.H, N = p.N, u0 = my * U, tile0 = rg * p.CH, ch_n = min(p.CH, ((N + 7) >> 3) - tile0);
   const long long NH = (long long)N * H;
-  const uint32_t XB = (uint32_t)CS * 512;  // one buffer of h words
+  const int KSR = CS * NW / 4, rot = my * NW / 4;  // k-steps of 16 units; the first to arrive
+  const uint32_t XB = (uint32_t)KSR * 512;  // one buffer of h words
   const uint32_t xb = smem_u32(smem);      // [CH][2][XB]
-  Stats st_;
+  Stats<NW> st_;
   st_.SB = (uint32_t)CS * 64;
   st_.CS = CS;
   st_.CH = p.CH;
   const size_t stats_at = (size_t)p.CH * 2 * XB, pl_at = stats_at + (size_t)4 * p.CH * st_.SB;
   st_.buf = xb + (uint32_t)stats_at;
   const uint32_t pl3 = xb + (uint32_t)pl_at + (uint32_t)(w * KS) * 512 + lane * 16;  // third plane of R
-  uint8_t* after = smem + pl_at + (PL == 3 ? (size_t)LC_NW * KS * 512 : 0);
+  uint8_t* after = smem + pl_at + (PL == 3 ? (size_t)NW * KS * 512 : 0);
   st_.part = reinterpret_cast<float2*>(after);
-  float* carry = reinterpret_cast<float*>(after + 4 * LC_NW * 8 * 8);  // [CH][h, c][threads]
-  float* stash = carry + p.CH * 2 * LC_THREADS;                        // [CH][LC_FWD_STASH][threads]
+  float* carry = reinterpret_cast<float*>(after + 4 * NW * 8 * 8);  // [CH][h, c][threads]
+  float* stash = carry + p.CH * 2 * THREADS_;                        // [CH][LC_FWD_STASH][threads]
   __shared__ int s_abort_;
   volatile int* s_abort = &s_abort_;
 
   if (tid == 0) *s_abort = 0;
-  for (size_t i = tid; i < pl_at / 16; i += LC_THREADS)
+  for (size_t i = tid; i < pl_at / 16; i += THREADS_)
     reinterpret_cast<uint4*>(smem)[i] = make_uint4(0u, 0u, 0u, 0u);
   __syncthreads();
   {
     const T* h0 = reinterpret_cast<const T*>(p.h);
-    const int units = CS * LC_U;
-    for (int i = tid; i < ch_n * 8 * units; i += LC_THREADS) {
+    const int units = CS * U;
+    for (int i = tid; i < ch_n * 8 * units; i += THREADS_) {
       const int r = i / units, k = i - r * units, n = tile0 * 8 + r, Q = k >> 2;
       const float x = (n < N && k < H) ? ld(h0 + (long long)n * H + k) : 0.f;
       *reinterpret_cast<uint32_t*>(smem + (size_t)(r >> 3) * 2 * XB + (Q >> 2) * 512 + quad_piece(Q & 3, r & 7) +
@@ -179,18 +180,18 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_fwd_kernel(const __grid_c
     }
   }
 
-  // ---- weights, in the order of arrival (slot s: k-step my - s)
+  // ---- weights, in the order of arrival (slot s: k-step rot - s)
   const int gq = lane >> 2, q = lane & 3;
   uint32_t wf[SPLIT][KS][4];
 #pragma unroll
   for (int s = 0; s < KS; ++s) {
-    int ks = my - s;
-    if (ks < 0) ks += CS;
+    int ks = rot - s;
+    if (ks < 0) ks += KSR;
     const int unit = u0 + 4 * w + (gq >> 1), ga = gq & 1, k = (ks * 4 + q) * 4;
     float x[2][4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const bool ok = s < CS && unit < H && k + i < H;
+      const bool ok = s < KSR && unit < H && k + i < H;
       const T* r = reinterpret_cast<const T*>(p.R) + (long long)(k + i) * G * H + unit;
       x[0][i] = ok ? ld(r + (long long)ga * H) : 0.f;
       x[1][i] = (ok && ga + 2 < G) ? ld(r + (long long)(ga + 2) * H) : 0.f;
@@ -227,23 +228,22 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_fwd_kernel(const __grid_c
   for (int ch = 0; ch < ch_n; ++ch) {
     const int n = (tile0 + ch) * 8 + row;
     const bool ok = n < N && uok;
-    carry[(ch * 2 + 0) * LC_THREADS + tid] = ok ? ld(hb + (long long)n * H + unit) : 0.f;
-    carry[(ch * 2 + 1) * LC_THREADS + tid] = (G == 4 && ok) ? ld(cb + (long long)n * H + unit) : 0.f;
+    carry[(ch * 2 + 0) * THREADS_ + tid] = ok ? ld(hb + (long long)n * H + unit) : 0.f;
+    carry[(ch * 2 + 1) * THREADS_ + tid] = (G == 4 && ok) ? ld(cb + (long long)n * H + unit) : 0.f;
   }
   // ---- how many values lie behind a mean: of a warp, of a CTA (per gate), and of the row
   const float units_w = (float)max(0, min(4, H - (u0 + 4 * w)));
   const float rec_w = units_w > 0.f ? 1.0f / units_w : 0.f;
-  float units_v[LC_NW], units_s[4];  // of the CTA's warps; of this lane's quarter of the CTAs
+  float units_v[NW], units_s[4];  // of the CTA's warps; of this lane's quarter of the CTAs
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    units_v[k] = (float)max(0, min(4, H - (u0 + 4 * k)));
-    units_s[k] = ul * 4 + k < CS ? (float)max(0, min(LC_U, H - (ul * 4 + k) * LC_U)) : 0.f;
-  }
-  const float rec_c = 1.0f / (float)max(1, min(LC_U, H - u0)), rec_H = 1.0f / (float)H;
+  for (int k = 0; k < NW; ++k) units_v[k] = (float)max(0, min(4, H - (u0 + 4 * k)));
+#pragma unroll
+  for (int k = 0; k < 4; ++k) units_s[k] = ul * 4 + k < CS ? (float)max(0, min(U, H - (ul * 4 + k) * U)) : 0.f;
+  const float rec_c = 1.0f / (float)max(1, min(U, H - u0)), rec_H = 1.0f / (float)H;
   // ---- destinations: lines of h to peers my + ul, my + ul + 4, ...; statistics to peer 4w + ul
   uint32_t dst[4];
   {
-    const int Q = my * LC_NW + w;
+    const int Q = my * NW + w;
     const uint32_t off = (Q >> 2) * 512 + quad_piece(Q & 3, row);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -278,19 +278,19 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_fwd_kernel(const __grid_c
     float2* at = st_.meet(stat, turn[stat]);
     turn[stat] ^= 1;
     if (ul == 0) at[w * 8 + row] = make_float2(m, d);
-    stop = stage_barrier_or<LC_NW>(!alive);
+    stop = stage_barrier_or<NW>(!alive);
     if (stop) return;
-    float2 y[LC_NW];
+    float2 y[NW];
     float mc = 0.f;
 #pragma unroll
-    for (int k = 0; k < LC_NW; ++k) {
+    for (int k = 0; k < NW; ++k) {
       y[k] = at[k * 8 + (lane & 7)];
       mc += units_v[k] * y[k].x;
     }
     mc *= rec_c;
     float m2 = 0.f;
 #pragma unroll
-    for (int k = 0; k < LC_NW; ++k) m2 += y[k].y + units_v[k] * (float)nv * (y[k].x - mc) * (y[k].x - mc);
+    for (int k = 0; k < NW; ++k) m2 += y[k].y + units_v[k] * (float)nv * (y[k].x - mc) * (y[k].x - mc);
     if (st_.sends) lc_store2(st_.dst + st_.area(stat, t & 1, ch), fword_encode(mc, tag), fword_encode(m2, tag));
   };
   auto collect = [&](int stat, int t, int ch, int nv, uint32_t tag, float& mean, float& inv, int code) {
@@ -328,9 +328,9 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_fwd_kernel(const __grid_c
     const uint32_t wtag = (((uint32_t)(t + 1) >> 1) & 1u) ^ 1u;    // of h_{t+1}
     // ---- stage A: h.R, its statistics
     for (int ch = 0; ch < ch_n; ++ch) {
-      float* sh = stash + (size_t)ch * LC_FWD_STASH * LC_THREADS + tid;
+      float* sh = stash + (size_t)ch * LC_FWD_STASH * THREADS_ + tid;
 #pragma unroll
-      for (int g = 0; g <= G; ++g) sh[(4 + g) * LC_THREADS] = nx[g];
+      for (int g = 0; g <= G; ++g) sh[(4 + g) * THREADS_] = nx[g];
       fetch_inputs(ch + 1 < ch_n ? t : t + 1, ch + 1 < ch_n ? ch + 1 : 0);
       float acc[2][PL][4];
 #pragma unroll
@@ -342,9 +342,9 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_fwd_kernel(const __grid_c
       auto fetch = [&](int b0, uint4 (&y)[4]) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          int ks = my - (b0 + k);
-          if (ks < 0) ks += CS;
-          if (b0 + k < KS - 3 || b0 + k < CS) y[k] = cl_poll(src + (uint32_t)ks * 512);
+          int ks = rot - (b0 + k);
+          if (ks < 0) ks += KSR;
+          if (b0 + k < KS - 3 || b0 + k < KSR) y[k] = cl_poll(src + (uint32_t)ks * 512);
           else y[k] = make_uint4(rtag, rtag, rtag, rtag);
         }
       };
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_fwd_kernel(const __grid_c
       if (stop) break;
 #pragma unroll
       for (int g = 0; g < G; ++g) {
-        sh[g * LC_THREADS] = rh[g];
+        sh[g * THREADS_] = rh[g];
         if (ok) st(rhb + (((long long)t * N + n) * G + g) * H + unit, rh[g]);
       }
     }
@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_fwd_kernel(const __grid_c
     // ---- stage B (LSTM): gates and the new cell state, its statistics
     if constexpr (G == 4) {
       for (int ch = 0; ch < ch_n; ++ch) {
-        float* sh = stash + (size_t)ch * LC_FWD_STASH * LC_THREADS + tid;
+        float* sh = stash + (size_t)ch * LC_FWD_STASH * THREADS_ + tid;
         const int n = (tile0 + ch) * 8 + row;
         const bool ok = n < N && uok;
         float mean1, inv1;
@@ -409,14 +409,14 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_fwd_kernel(const __grid_c
         float pre[4];
 #pragma unroll
         for (int g = 0; g < 4; ++g)
-          pre[g] = (sh[g * LC_THREADS] - mean1) * inv1 * g1[g % G] + sh[(4 + g) * LC_THREADS] + bias[g % G];
+          pre[g] = (sh[g * THREADS_] - mean1) * inv1 * g1[g % G] + sh[(4 + g) * THREADS_] + bias[g % G];
         const float i = ln_sigmoid<SPLIT>(pre[0]), gg = ln_tanh<SPLIT>(pre[1]), f = ln_sigmoid<SPLIT>(pre[2]),
                     o = ln_sigmoid<SPLIT>(pre[3]);
-        float c_new[1] = {f * carry[(ch * 2 + 1) * LC_THREADS + tid] + i * gg};
+        float c_new[1] = {f * carry[(ch * 2 + 1) * THREADS_ + tid] + i * gg};
         publish(1, t, ch, c_new, 1, ok, rt);
         if (stop) break;
         sh[0] = o;
-        sh[LC_THREADS] = c_new[0];
+        sh[THREADS_] = c_new[0];
         if (ok) {
           st(cb + (long long)(t + 1) * NH + (long long)n * H + unit, c_new[0]);
           if (p.training) {
@@ -433,25 +433,25 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_fwd_kernel(const __grid_c
     }
     // ---- last stage: the new state, on its way to every peer
     for (int ch = 0; ch < ch_n; ++ch) {
-      float* sh = stash + (size_t)ch * LC_FWD_STASH * LC_THREADS + tid;
-      float* cy = carry + (size_t)ch * 2 * LC_THREADS + tid;
+      float* sh = stash + (size_t)ch * LC_FWD_STASH * THREADS_ + tid;
+      float* cy = carry + (size_t)ch * 2 * THREADS_ + tid;
       const int n = (tile0 + ch) * 8 + row;
       const bool ok = n < N && uok;
       float mean, inv;
       collect(G == 4 ? 1 : 0, t, ch, G == 4 ? 1 : G, rt, mean, inv, 65);
-      const float hp = cy[0], m = sh[(4 + G) * LC_THREADS];
+      const float hp = cy[0], m = sh[(4 + G) * THREADS_];
       float h_new, c_norm = 0.f, z = 0.f, r = 0.f, gg = 0.f, qg = 0.f;
       if (G == 4) {
-        c_norm = (sh[LC_THREADS] - mean) * inv * gh + bh;
+        c_norm = (sh[THREADS_] - mean) * inv * gh + bh;
         h_new = sh[0] * ln_tanh<SPLIT>(c_norm);
       } else {
         float rn[3];
 #pragma unroll
-        for (int g = 0; g < 3; ++g) rn[g] = (sh[g * LC_THREADS] - mean) * inv * g1[g] + bias2[g];
-        z = ln_sigmoid<SPLIT>(sh[4 * LC_THREADS] + bias[0] + rn[0]);
-        r = ln_sigmoid<SPLIT>(sh[5 * LC_THREADS] + bias[1] + rn[1]);
+        for (int g = 0; g < 3; ++g) rn[g] = (sh[g * THREADS_] - mean) * inv * g1[g] + bias2[g];
+        z = ln_sigmoid<SPLIT>(sh[4 * THREADS_] + bias[0] + rn[0]);
+        r = ln_sigmoid<SPLIT>(sh[5 * THREADS_] + bias[1] + rn[1]);
         qg = rn[2];
-        gg = ln_tanh<SPLIT>(sh[6 * LC_THREADS] + bias[2] + r * qg);
+        gg = ln_tanh<SPLIT>(sh[6 * THREADS_] + bias[2] + r * qg);
         h_new = z * hp + (1.0f - z) * gg;
       }
       if (p.has_zoneout)
@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_fwd_kernel(const __grid_c
             cl_store(dst[i] + off, o2 ? f0 : e0, o2 ? f1 : e1, o2 ? e0 : f0, o2 ? e1 : f1);
       }
       cy[0] = h_new;
-      if (G == 4) cy[LC_THREADS] = sh[LC_THREADS];
+      if (G == 4) cy[THREADS_] = sh[THREADS_];
       if (ok) {
         const long long e = (long long)t * N + n;
         st(hb + NH + e * H + unit, h_new);
@@ -494,18 +494,18 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_fwd_kernel(const __grid_c
 }
 
 // ---------------------------------------------------------------------------------------
-template <int G, int TPW, int SPLIT, typename T>
-__global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_bwd_kernel(const __grid_constant__ LnClBwd p) {
-  constexpr int PL = SPLIT == 2 ? 3 : 1;
-  constexpr int KSB = G;  // k-steps: the four unit quads of a gate
+template <int G, int NW, int TPW, int SPLIT, typename T>
+__global__ void __launch_bounds__(NW * 32, 1) ln_cl_bwd_kernel(const __grid_constant__ LnClBwd p) {
+  constexpr int PL = SPLIT == 2 ? 3 : 1, U = 4 * NW, THREADS_ = NW * 32;
+  constexpr int KSB = (G * NW + 3) / 4;  // k-steps: G * NW unit quads of own gate columns
   extern __shared__ __align__(16) uint8_t smem[];
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
   const int CS = p.CTAS, my = (int)cl_rank(), rg = blockIdx.x / CS;
-  const int H = p.H, N = p.N, u0 = my * LC_U, tile0 = rg * p.CH, ch_n = min(p.CH, ((N + 7) >> 3) - tile0);
+  const int H = p.H, N = p.N, u0 = my * U, tile0 = rg * p.CH, ch_n = min(p.CH, ((N + 7) >> 3) - tile0);
   const long long NH = (long long)N * H;
-  const uint32_t XB = (uint32_t)CS * LC_NW * 128;  // one exchange buffer: [source][own quad][128]
+  const uint32_t XB = (uint32_t)CS * NW * 128;  // one exchange buffer: [source][own quad][128]
   const uint32_t xb = smem_u32(smem);              // [CH][2][XB]
-  Stats st_;
+  Stats<NW> st_;
   st_.SB = (uint32_t)CS * 64;
   st_.CS = CS;
   st_.CH = p.CH;
@@ -515,39 +515,39 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_bwd_kernel(const __grid_c
   uint8_t* gsm3 = gsm + 2 * KSB * 512;            // its third plane: [2][KSB][256]
   const size_t pl_at = g_at + 2 * KSB * 512 + (PL == 3 ? 2 * KSB * 256 : 0);
   const uint32_t pl3 = xb + (uint32_t)pl_at + (uint32_t)(w * TPW * KSB) * 512 + lane * 16;
-  uint8_t* after = smem + pl_at + (PL == 3 ? (size_t)LC_NW * TPW * KSB * 512 : 0);
+  uint8_t* after = smem + pl_at + (PL == 3 ? (size_t)NW * TPW * KSB * 512 : 0);
   st_.part = reinterpret_cast<float2*>(after);
-  float* carry = reinterpret_cast<float*>(after + 4 * LC_NW * 8 * 8);  // [CH][dh, dc, c][threads]
-  float* stash = carry + p.CH * 3 * LC_THREADS;                        // [CH][LC_BWD_STASH][threads]
+  float* carry = reinterpret_cast<float*>(after + 4 * NW * 8 * 8);  // [CH][dh, dc, c][threads]
+  float* stash = carry + p.CH * 3 * THREADS_;                        // [CH][LC_BWD_STASH][threads]
   __shared__ int s_abort_;
   volatile int* s_abort = &s_abort_;
   if (tid == 0) *s_abort = 0;
-  for (size_t i = tid; i < pl_at / 16; i += LC_THREADS)
+  for (size_t i = tid; i < pl_at / 16; i += THREADS_)
     reinterpret_cast<uint4*>(smem)[i] = make_uint4(0u, 0u, 0u, 0u);
 
-  // ---- weights: slot i of warp w is output tile (w + 4 i + my) mod CS (see cl_bwd_kernel)
-  const int gq = lane >> 2, q = lane & 3;
+  // ---- weights: slot i of warp w is output tile (w + NW i + my NW / 4) mod MTR (see cl_bwd_kernel)
+  const int gq = lane >> 2, q = lane & 3, MTR = CS * NW / 4;
   uint32_t wf[SPLIT][TPW][KSB][4];
   uint32_t dst[TPW];
 #pragma unroll
   for (int i = 0; i < TPW; ++i) {
-    const int Lt = w + LC_NW * i;
-    int tile = Lt + my;
-    while (tile >= CS) tile -= CS;
-    const int Q = tile * 4 + (gq >> 1), d = Q / LC_NW, qw = Q - d * LC_NW;
-    const bool live = Lt < CS;
-    dst[i] = live ? cl_mapa(xb + (uint32_t)(my * LC_NW + qw) * 128 + ((gq & 1) * 4 + q) * 16, (uint32_t)d) : 0u;
+    const int Lt = w + NW * i;
+    int tile = Lt + my * NW / 4;
+    while (tile >= MTR) tile -= MTR;
+    const int Q = tile * 4 + (gq >> 1), d = Q / NW, qw = Q - d * NW;
+    const bool live = Lt < MTR;
+    dst[i] = live ? cl_mapa(xb + (uint32_t)(my * NW + qw) * 128 + ((gq & 1) * 4 + q) * 16, (uint32_t)d) : 0u;
 #pragma unroll
     for (int kk = 0; kk < KSB; ++kk) {
-      const int j = Q * 4 + (gq & 1), k = u0 + 4 * q;
+      const int lq = kk * 4 + q, gate = lq / NW, j = Q * 4 + (gq & 1), k = u0 + 4 * (lq - gate * NW);
       const T* R = reinterpret_cast<const T*>(p.R);
       float x[2][4];
 #pragma unroll
       for (int hf = 0; hf < 2; ++hf)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const bool ok = live && j + 2 * hf < H && k + e < H;
-          const long long col = (long long)kk * H + k + e;
+          const bool ok = live && gate < G && j + 2 * hf < H && k + e < H;
+          const long long col = (long long)gate * H + k + e;
           x[hf][e] = ok ? ld(p.r_transposed ? R + col * H + j + 2 * hf : R + (long long)(j + 2 * hf) * G * H + col) : 0.f;
         }
       uint32_t f[PL][4];
@@ -583,10 +583,10 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_bwd_kernel(const __grid_c
     const int n = (tile0 + ch) * 8 + row;
     const bool ok = n < N && uok;
     const long long o = (long long)n * H + unit;
-    float* cy = carry + (size_t)ch * 3 * LC_THREADS + tid;
+    float* cy = carry + (size_t)ch * 3 * THREADS_ + tid;
     cy[0] = ok ? p.dh_carry[o] : 0.f;
-    cy[LC_THREADS] = (G == 4 && ok) ? p.dc_carry[o] : 0.f;
-    cy[2 * LC_THREADS] = (G == 4 && ok) ? ld(cb + (long long)p.T * NH + o) : 0.f;
+    cy[THREADS_] = (G == 4 && ok) ? p.dc_carry[o] : 0.f;
+    cy[2 * THREADS_] = (G == 4 && ok) ? ld(cb + (long long)p.T * NH + o) : 0.f;
   }
   st_.sends = w * 4 + (lane >> 3) < CS;
   st_.dst = st_.sends ? cl_mapa(st_.buf + my * 64 + (lane & 7) * 8, (uint32_t)(w * 4 + (lane >> 3))) : 0u;
@@ -607,11 +607,11 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_bwd_kernel(const __grid_c
     float2* at = st_.meet(stat, turn[stat]);
     turn[stat] ^= 1;
     if (ul == 0) at[w * 8 + row] = make_float2(x, y);
-    stop = stage_barrier_or<LC_NW>(!alive);
+    stop = stage_barrier_or<NW>(!alive);
     if (stop) return;
     float sx = 0.f, sy = 0.f;
 #pragma unroll
-    for (int k = 0; k < LC_NW; ++k) {
+    for (int k = 0; k < NW; ++k) {
       const float2 v = at[k * 8 + (lane & 7)];
       sx += v.x;
       sy += v.y;
@@ -644,7 +644,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_bwd_kernel(const __grid_c
       for (int k = 0; k < TPW; ++k) {
         const int j = sub * TPW + k;
         y[k] = make_uint4(want, want, want, want);
-        if (j < CS) y[k] = cl_poll(src + (uint32_t)(j * LC_NW) * 128);
+        if (j < CS) y[k] = cl_poll(src + (uint32_t)(j * NW) * 128);
         bad |= stale4(y[k], want);
       }
       if (__all_sync(0xffffffffu, (bad & 1u) == 0)) break;
@@ -717,8 +717,8 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_bwd_kernel(const __grid_c
     };
     // ---- stage A
     for (int ch = 0; ch < ch_n; ++ch) {
-      float* sh = stash + (size_t)ch * LC_BWD_STASH * LC_THREADS + tid;
-      float* cy = carry + (size_t)ch * 3 * LC_THREADS + tid;
+      float* sh = stash + (size_t)ch * LC_BWD_STASH * THREADS_ + tid;
+      float* cy = carry + (size_t)ch * 3 * THREADS_ + tid;
       float in[NI];
 #pragma unroll
       for (int i = 0; i < NI; ++i) in[i] = nx[i];
@@ -736,22 +736,22 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_bwd_kernel(const __grid_c
 #pragma unroll
       for (int g = 0; g < G; ++g) {
         cx[g] = in[I_RH + g] - in[I_C1];
-        sh[(4 + g) * LC_THREADS] = cx[g];
+        sh[(4 + g) * THREADS_] = cx[g];
       }
-      sh[8 * LC_THREADS] = in[I_C1 + 1];
+      sh[8 * THREADS_] = in[I_C1 + 1];
       if constexpr (G == 4) {
         const float o = in[3], inv3 = in[NI - 1];
-        const float cx3 = ok ? cy[2 * LC_THREADS] - in[NI - 2] : 0.f;
+        const float cx3 = ok ? cy[2 * THREADS_] - in[NI - 2] : 0.f;
         const float c_tanh = ln_tanh<SPLIT>(in[I_S + 2]);
         const float d_norm = ok ? d_tanh(c_tanh) * (o * dh_total) : 0.f;  // gradient w.r.t. LayerNorm(c')
         acc_gh += cx3 * inv3 * d_norm;
         acc_bh += d_norm;
         const float db3 = gh * d_norm;
         cy[0] = ok ? keep : 0.f;
-        sh[0] = in[0]; sh[LC_THREADS] = in[1]; sh[2 * LC_THREADS] = in[2];
-        sh[3 * LC_THREADS] = d_sigmoid(o) * (c_tanh * dh_total);
-        sh[9 * LC_THREADS] = in[I_S]; sh[10 * LC_THREADS] = in[I_S + 1];
-        sh[11 * LC_THREADS] = cx3; sh[12 * LC_THREADS] = inv3; sh[13 * LC_THREADS] = db3;
+        sh[0] = in[0]; sh[THREADS_] = in[1]; sh[2 * THREADS_] = in[2];
+        sh[3 * THREADS_] = d_sigmoid(o) * (c_tanh * dh_total);
+        sh[9 * THREADS_] = in[I_S]; sh[10 * THREADS_] = in[I_S + 1];
+        sh[11 * THREADS_] = cx3; sh[12 * THREADS_] = inv3; sh[13 * THREADS_] = db3;
         publish(1, ti, ch, cx3 * db3, db3, tag);
         if (stop) break;
       } else {
@@ -765,7 +765,7 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_bwd_kernel(const __grid_c
         norm_sums(dg, cx, in[I_C1 + 1], ok, ch);
         if (stop) break;
 #pragma unroll
-        for (int g = 0; g < G; ++g) sh[g * LC_THREADS] = dg[g];
+        for (int g = 0; g < G; ++g) sh[g * THREADS_] = dg[g];
         if (ok) {
           const long long w0 = ((long long)t * N + n) * 3 * H + unit;
           st(dpb + w0, dg[0]); st(dpb + w0 + H, dg[1]); st(dpb + w0 + 2 * H, dp_g);
@@ -778,31 +778,31 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_bwd_kernel(const __grid_c
     // ---- stage B (LSTM): the cell state's LayerNorm, the gate gradients
     if constexpr (G == 4) {
       for (int ch = 0; ch < ch_n; ++ch) {
-        float* sh = stash + (size_t)ch * LC_BWD_STASH * LC_THREADS + tid;
-        float* cy = carry + (size_t)ch * 3 * LC_THREADS + tid;
+        float* sh = stash + (size_t)ch * LC_BWD_STASH * THREADS_ + tid;
+        float* cy = carry + (size_t)ch * 3 * THREADS_ + tid;
         const int n = (tile0 + ch) * 8 + row;
         const bool ok = n < N && uok;
         float S1, S2;
         collect(1, ti, ch, tag, S1, S2, 67);
-        const float r = sh[12 * LC_THREADS];
+        const float r = sh[12 * THREADS_];
         const float dsigma = -0.5f * S1 * r * r * r, dmu = -S2 * r;
-        const float dcl = 2.0f * sh[11 * LC_THREADS] * dsigma * inv_H + r * sh[13 * LC_THREADS] + dmu * inv_H;
-        const float i = sh[0], gg = sh[LC_THREADS], f = sh[2 * LC_THREADS], cprev = sh[10 * LC_THREADS];
-        const float dc_total = ok ? sh[9 * LC_THREADS] + cy[LC_THREADS] + dcl : 0.f;
+        const float dcl = 2.0f * sh[11 * THREADS_] * dsigma * inv_H + r * sh[13 * THREADS_] + dmu * inv_H;
+        const float i = sh[0], gg = sh[THREADS_], f = sh[2 * THREADS_], cprev = sh[10 * THREADS_];
+        const float dc_total = ok ? sh[9 * THREADS_] + cy[THREADS_] + dcl : 0.f;
         float dg[G], cx[G];
         dg[0] = d_sigmoid(i) * (gg * dc_total);
         dg[1] = d_tanh(gg) * (i * dc_total);
         dg[2] = d_sigmoid(f) * (cprev * dc_total);
-        dg[G - 1] = ok ? sh[3 * LC_THREADS] : 0.f;
-        cy[LC_THREADS] = f * dc_total;
-        cy[2 * LC_THREADS] = cprev;
+        dg[G - 1] = ok ? sh[3 * THREADS_] : 0.f;
+        cy[THREADS_] = f * dc_total;
+        cy[2 * THREADS_] = cprev;
 #pragma unroll
-        for (int g = 0; g < G; ++g) cx[g] = sh[(4 + g) * LC_THREADS];
-        norm_sums(dg, cx, sh[8 * LC_THREADS], ok, ch);
+        for (int g = 0; g < G; ++g) cx[g] = sh[(4 + g) * THREADS_];
+        norm_sums(dg, cx, sh[8 * THREADS_], ok, ch);
         if (stop) break;
 #pragma unroll
         for (int g = 0; g < G; ++g) {
-          sh[g * LC_THREADS] = dg[g];
+          sh[g * THREADS_] = dg[g];
           acc_b[g] += dg[g];
           if (ok) st(vb + (((long long)t * N + n) * 4 + g) * H + unit, dg[g]);
         }
@@ -811,18 +811,18 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_bwd_kernel(const __grid_c
     }
     // ---- stage C: d(h.R), and what it makes of dh for every unit
     for (int ch = 0; ch < ch_n; ++ch) {
-      float* sh = stash + (size_t)ch * LC_BWD_STASH * LC_THREADS + tid;
+      float* sh = stash + (size_t)ch * LC_BWD_STASH * THREADS_ + tid;
       const int n = (tile0 + ch) * 8 + row;
       const bool ok = n < N && uok;
       float S1, S2;
       collect(0, ti, ch, tag, S1, S2, 68);
-      const float r = sh[8 * LC_THREADS];
+      const float r = sh[8 * THREADS_];
       const float dsigma = -0.5f * S1 * r * r * r, dmu = -S2 * r;
       uint8_t *gb = gsm + gpar * KSB * 512, *gb3 = gsm3 + gpar * KSB * 256;
       gpar ^= 1;
 #pragma unroll
       for (int g = 0; g < G; ++g) {
-        const float x = ok ? 2.0f * sh[(4 + g) * LC_THREADS] * dsigma * inv_GH + r * (g1[g] * sh[g * LC_THREADS]) +
+        const float x = ok ? 2.0f * sh[(4 + g) * THREADS_] * dsigma * inv_GH + r * (g1[g] * sh[g * THREADS_]) +
                                  dmu * inv_GH
                            : 0.f;
         if (ok) st(rhb + (((long long)t * N + n) * G + g) * H + unit, x);
@@ -832,14 +832,15 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_bwd_kernel(const __grid_c
         if (PL == 3) split3_bf16(x, pl);
         const uint32_t own = pack_bf16(pl[0], pl[1]);
         const uint32_t other = __shfl_xor_sync(0xffffffffu, own, 4);
-        *reinterpret_cast<uint32_t*>(gb + g * 512 + quad_piece(w, row) + (second ? 8 : 0) + (sub >> 1) * 4) =
+        const int lq = g * NW + w;
+        *reinterpret_cast<uint32_t*>(gb + (lq >> 2) * 512 + quad_piece(lq & 3, row) + (second ? 8 : 0) + (sub >> 1) * 4) =
             second ? __byte_perm(other, own, 0x7632) : __byte_perm(own, other, 0x5410);
         if (PL == 3) {
           const float third = __shfl_xor_sync(0xffffffffu, pl[2], 4);
-          if (!second) *reinterpret_cast<uint32_t*>(gb3 + g * 256 + w * 64 + row * 8 + (sub >> 1) * 4) = pack_bf16(pl[2], third);
+          if (!second) *reinterpret_cast<uint32_t*>(gb3 + lq * 64 + row * 8 + (sub >> 1) * 4) = pack_bf16(pl[2], third);
         }
       }
-      stop = stage_barrier_or<LC_NW>(!alive);
+      stop = stage_barrier_or<NW>(!alive);
       if (stop) break;
       const uint32_t off = (uint32_t)ch * 2 * XB + (ti & 1) * XB;
       uint32_t b0[KSB][PL], b1[KSB][PL];
@@ -882,12 +883,12 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_bwd_kernel(const __grid_c
   // ---- what is left of dh: the recurrent part of step 0, then the carries go out
   for (int ch = 0; ch < ch_n && alive && !stop; ++ch) {
     const int n = (tile0 + ch) * 8 + row;
-    float* cy = carry + (size_t)ch * 3 * LC_THREADS + tid;
+    float* cy = carry + (size_t)ch * 3 * THREADS_ + tid;
     float dh_c = cy[0];
     gather(ch, p.T - 1, dh_c);
     if (alive && n < N && uok) {
       p.dh_carry[(long long)n * H + unit] = dh_c;
-      if (G == 4) p.dc_carry[(long long)n * H + unit] = cy[LC_THREADS];
+      if (G == 4) p.dc_carry[(long long)n * H + unit] = cy[THREADS_];
     }
   }
   // ---- parameter gradients of this row group: sums over the eight rows
@@ -919,48 +920,56 @@ __global__ void __launch_bounds__(LC_THREADS, 1) ln_cl_bwd_kernel(const __grid_c
 }
 
 // ---------------------------------------------------------------------------------------
-// Host side.  `row_groups` receives the number of partial rows in db_part and the others.
-template <int G, int KS, int SPLIT, typename T>
-int ln_cl_fwd_go(LnClFwd& p, cudaStream_t s) {
+// Host side.  Sixteen CTAs of 16 units (four warps) reach 256, of 20 units (five warps) 320; these only
+// while the chains of a CTA stay few, as seven such clusters are resident and the fifth warp shares a
+// sub-partition (LSTM fp32, us per step, these / the grid kernels: one chain, 45 rows H = 296 5.1 / 11.7
+// forward, 4.4 / 11.9 backward; two chains, 64 rows H = 320 9.7 / 8.0 and 8.2 / 11.7).
+constexpr int kLnClMost = 320, kLnWideFwdChains = 1, kLnWideBwdChains = 2;
+// `row_groups` receives the number of partial rows in db_part and the others.
+template <int G, int NW, int KS, int SPLIT, typename T>
+int ln_cl_fwd_go(LnClFwd& p, int most, cudaStream_t s) {
   static std::atomic<int> slots[kChainMaxDevices][17];
-  const size_t chain = (size_t)2 * p.CTAS * 512 + (size_t)4 * p.CTAS * 64 +
-                       (size_t)(2 + LC_FWD_STASH) * LC_THREADS * 4;
-  const size_t fixed = (SPLIT == 2 ? (size_t)LC_NW * KS * 512 : 0) + 4 * LC_NW * 8 * 8;
+  const size_t chain = (size_t)2 * (p.CTAS * NW / 4) * 512 + (size_t)4 * p.CTAS * 64 +
+                       (size_t)(2 + LC_FWD_STASH) * NW * 32 * 4;
+  const size_t fixed = (SPLIT == 2 ? (size_t)NW * KS * 512 : 0) + 4 * NW * 8 * 8;
   int groups = 0;
-  return cl_launch(ln_cl_fwd_kernel<G, KS, SPLIT, T>, p, LC_THREADS, chain, fixed, slots, kClMaxChains, &groups, s);
+  return cl_launch(ln_cl_fwd_kernel<G, NW, KS, SPLIT, T>, p, NW * 32, chain, fixed, slots, most, &groups, s);
 }
 template <int G, int SPLIT, typename T>
 int run_ln_cl_fwd(const LnFwdParams& q, cudaStream_t s) {
-  if (q.H > 16 * LC_U) return HASTE_B200_ERR_UNSUPPORTED;
+  if (q.H > kLnClMost) return HASTE_B200_ERR_UNSUPPORTED;
   LnClFwd p;
   static_cast<LnFwdParams&>(p) = q;
-  p.CTAS = ceil_div(q.H, LC_U);
-  if (p.CTAS <= 4) return ln_cl_fwd_go<G, 4, SPLIT, T>(p, s);
-  if (p.CTAS <= 8) return ln_cl_fwd_go<G, 8, SPLIT, T>(p, s);
-  if (p.CTAS <= 12) return ln_cl_fwd_go<G, 12, SPLIT, T>(p, s);
-  return ln_cl_fwd_go<G, 16, SPLIT, T>(p, s);
+  p.CTAS = q.H > 256 ? 16 : ceil_div(q.H, 16);
+  if (q.H > 256) return ln_cl_fwd_go<G, 5, 20, SPLIT, T>(p, kLnWideFwdChains, s);
+  if (p.CTAS <= 4) return ln_cl_fwd_go<G, 4, 4, SPLIT, T>(p, kClMaxChains, s);
+  if (p.CTAS <= 8) return ln_cl_fwd_go<G, 4, 8, SPLIT, T>(p, kClMaxChains, s);
+  if (p.CTAS <= 12) return ln_cl_fwd_go<G, 4, 12, SPLIT, T>(p, kClMaxChains, s);
+  return ln_cl_fwd_go<G, 4, 16, SPLIT, T>(p, kClMaxChains, s);
 }
 
-template <int G, int TPW, int SPLIT, typename T>
-int ln_cl_bwd_go(LnClBwd& p, int* row_groups, cudaStream_t s) {
+template <int G, int NW, int TPW, int SPLIT, typename T>
+int ln_cl_bwd_go(LnClBwd& p, int most, int* row_groups, cudaStream_t s) {
+  constexpr int KSB = (G * NW + 3) / 4;
   static std::atomic<int> slots[kChainMaxDevices][17];
-  const size_t chain = (size_t)2 * p.CTAS * LC_NW * 128 + (size_t)4 * p.CTAS * 64 +
-                       (size_t)(3 + LC_BWD_STASH) * LC_THREADS * 4;
-  const size_t fixed = (size_t)2 * G * 512 + (SPLIT == 2 ? (size_t)2 * G * 256 + (size_t)LC_NW * TPW * G * 512 : 0) +
-                       4 * LC_NW * 8 * 8;
-  return cl_launch(ln_cl_bwd_kernel<G, TPW, SPLIT, T>, p, LC_THREADS, chain, fixed, slots, kClMaxChains, row_groups, s);
+  const size_t chain = (size_t)2 * p.CTAS * NW * 128 + (size_t)4 * p.CTAS * 64 +
+                       (size_t)(3 + LC_BWD_STASH) * NW * 32 * 4;
+  const size_t fixed = (size_t)2 * KSB * 512 + (SPLIT == 2 ? (size_t)2 * KSB * 256 + (size_t)NW * TPW * KSB * 512 : 0) +
+                       4 * NW * 8 * 8;
+  return cl_launch(ln_cl_bwd_kernel<G, NW, TPW, SPLIT, T>, p, NW * 32, chain, fixed, slots, most, row_groups, s);
 }
 template <int G, int SPLIT, typename T>
 int run_ln_cl_bwd(const LnBwdParams& q, float* db_part, int* row_groups, cudaStream_t s) {
-  if (q.H > 16 * LC_U) return HASTE_B200_ERR_UNSUPPORTED;
+  if (q.H > kLnClMost) return HASTE_B200_ERR_UNSUPPORTED;
   LnClBwd p;
   static_cast<LnBwdParams&>(p) = q;
-  p.CTAS = ceil_div(q.H, LC_U);
+  p.CTAS = q.H > 256 ? 16 : ceil_div(q.H, 16);
   p.db_part = db_part;
-  if (p.CTAS <= 4) return ln_cl_bwd_go<G, 1, SPLIT, T>(p, row_groups, s);
-  if (p.CTAS <= 8) return ln_cl_bwd_go<G, 2, SPLIT, T>(p, row_groups, s);
-  if (p.CTAS <= 12) return ln_cl_bwd_go<G, 3, SPLIT, T>(p, row_groups, s);
-  return ln_cl_bwd_go<G, 4, SPLIT, T>(p, row_groups, s);
+  if (q.H > 256) return ln_cl_bwd_go<G, 5, 4, SPLIT, T>(p, kLnWideBwdChains, row_groups, s);
+  if (p.CTAS <= 4) return ln_cl_bwd_go<G, 4, 1, SPLIT, T>(p, kClMaxChains, row_groups, s);
+  if (p.CTAS <= 8) return ln_cl_bwd_go<G, 4, 2, SPLIT, T>(p, kClMaxChains, row_groups, s);
+  if (p.CTAS <= 12) return ln_cl_bwd_go<G, 4, 3, SPLIT, T>(p, kClMaxChains, row_groups, s);
+  return ln_cl_bwd_go<G, 4, 4, SPLIT, T>(p, kClMaxChains, row_groups, s);
 }
 
 }  // namespace rec

@@ -227,7 +227,7 @@ __global__ void ln_grad_finish(int G, const float* db_part, const float* dgRh_pa
 
 int cluster_backward(LnBwdParams& p, int gates, int dtype, const LnGrads& out,
                      int (*run)(const LnBwdParams&, float*, int*, cudaStream_t), cudaStream_t s) {
-  if (recurrence_path() == HASTE_B200_PATH_STEPWISE || p.H > 256) return HASTE_B200_ERR_UNSUPPORTED;
+  if (recurrence_path() == HASTE_B200_PATH_STEPWISE || p.H > 320) return HASTE_B200_ERR_UNSUPPORTED;
   p.sync.err = device_error_word();
   HB_REQUIRE(p.sync.err, "error word");
   const int H = p.H;
@@ -326,7 +326,8 @@ int layer_norm_lstm_backward_persistent(const LnLstmBwd& a, float* dh_carry, flo
   GemmDesc gd{a.dtype, HASTE_B200_F32, a.N, H, 4 * H, a.act_Rh, 4LL * H, 1, a.R,
               a.transposed_inputs ? H : 1, a.transposed_inputs ? 1 : 4LL * H, dh_carry, H, 1};
   gd.precise = 1;
-  return gemm_small(gd, s);
+  // (once per pass, not once per step: the CUDA-core kernel would take 92 us for 45 rows, H = 296)
+  return gemm(gd, s);
 }
 
 // ---- LayerNormGRU (the G = 3 instantiation of the same kernels) ---------------------------
@@ -391,7 +392,8 @@ int layer_norm_gru_backward_persistent(const LnGruBwd& a, float* dh_carry, float
   GemmDesc gd{a.dtype, HASTE_B200_F32, a.N, H, 3 * H, a.act_Rh, 3LL * H, 1, a.R,
               a.transposed_inputs ? H : 1, a.transposed_inputs ? 1 : 3LL * H, dh_carry, H, 1};
   gd.precise = 1;
-  return gemm_small(gd, s);
+  // (once per pass, not once per step: the CUDA-core kernel would take 92 us for 45 rows, H = 296)
+  return gemm(gd, s);
 }
 
 }  // namespace hb

@@ -9,7 +9,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("T,N,H", [(1, 1, 3), (3, 8, 16), (5, 9, 17), (6, 3, 64), (5, 17, 100), (4, 70, 128),
-                                   (7, 33, 200), (4, 130, 250), (6, 8, 256)])
+                                   (7, 33, 200), (4, 130, 250), (6, 8, 256),
+                                   (5, 9, 257), (4, 70, 301), (6, 3, 320)])
 @pytest.mark.parametrize("cell", ["layer_norm_lstm", "layer_norm_gru"])
 def test_tiles_f32(cell, T, N, H):
     d = oracle.make_inputs(cell, T, N, 12, H, seed=H + N, zoneout=0.2)
@@ -20,7 +21,7 @@ def test_tiles_f32(cell, T, N, H):
         assert_close(g[k], r, TOL_F32, "d" + k)
 
 
-@pytest.mark.parametrize("N,H", [(9, 40), (20, 256)])
+@pytest.mark.parametrize("N,H", [(9, 40), (20, 256), (11, 300)])
 def test_tiles_bf16(N, H):
     d = oracle.make_inputs("layer_norm_gru", 5, N, 16, H, seed=H, zoneout=0.2)
     dq = {k: (v.to(torch.bfloat16).to(torch.float64) if v is not None else None) for k, v in d.items()}
