@@ -47,6 +47,7 @@ bool gl_geometry(int dtype, int T, int N, int H, int most, GlGeometry* g) {
     g->CH = ceil_div(tiles, g->nRG);
     g->nRG = ceil_div(tiles, g->CH);
     if (g->CH <= most) return true;
+    if (most < kGridChains) break;  // the tensor-core recurrence comes next, within the budget too
   }
   return false;
 }
@@ -120,7 +121,7 @@ int run_bwd(ChainParams& p, int dtype, int grid_most, int gates, void* db, void*
 
 // Rows the tensor-core GRU recurrence would take (rec_tc_gru.cu).
 bool tc_waits(int dtype, int N, int H) {
-  return dtype == HASTE_B200_BF16 && N >= 64 && H % 64 == 0 && recurrence_path() != HASTE_B200_PATH_NO_TENSOR_CORE;
+  return dtype == HASTE_B200_BF16 && N >= 64 && H % 8 == 0 && recurrence_path() != HASTE_B200_PATH_NO_TENSOR_CORE;
 }
 
 }  // namespace

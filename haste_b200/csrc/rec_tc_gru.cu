@@ -140,28 +140,6 @@ __device__ __forceinline__ bool wait_count(const unsigned int* c, unsigned int t
   return true;
 }
 
-// 16 consecutive bf16 (32 bytes, 16-byte aligned) <-> floats
-__device__ __forceinline__ void ld16(const bf16* p, float (&x)[16]) {
-  const uint4 a = *reinterpret_cast<const uint4*>(p);
-  const uint4 b = *reinterpret_cast<const uint4*>(p + 8);
-  const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    x[2 * i] = __uint_as_float(w[i] << 16);
-    x[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
-  }
-}
-__device__ __forceinline__ void st16(bf16* p, const float (&x)[16]) {
-  uint32_t w[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    __nv_bfloat162 t2 = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
-    w[i] = *reinterpret_cast<uint32_t*>(&t2);
-  }
-  *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
-  *reinterpret_cast<uint4*>(p + 8) = make_uint4(w[4], w[5], w[6], w[7]);
-}
-
 // 8 consecutive bf16 as one 16-byte load, and element u of such a group as a float
 __device__ __forceinline__ uint4 ldq(const bf16* p) { return *reinterpret_cast<const uint4*>(p); }
 __device__ __forceinline__ float bfq(const uint4& q, int u) {
@@ -217,7 +195,7 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
   uint8_t* aligned = smem_raw + (base - smem_u32(smem_raw));
   const int H = p.H, N = p.N;
   const int K = FWD ? H : 3 * H;
-  const int KB = K / BK;
+  const int KB = (K + BK - 1) / BK;  // (TMA fills what lies beyond K with zeros)
   constexpr int R_TILE = NB * 128;  // bytes of the resident operand per k-block
   const uint32_t r_bytes = (uint32_t)KB * R_TILE;
   const uint32_t ring = base + r_bytes;  // r_bytes is a multiple of 1024
@@ -266,39 +244,47 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
   // ---- streamed-operand ring: zero once, so that rows a 64-row box never writes are zeros
   for (int i = threadIdx.x; i < p.ring_bytes / 16; i += TC_THREADS)
     reinterpret_cast<uint4*>(ring_ptr)[i] = make_uint4(0u, 0u, 0u, 0u);
-  // ---- resident operand: this CTA's slice of R, K-major and swizzled
+  // ---- resident operand: this CTA's slice of R, K-major and swizzled; zeros beyond K and beyond H
+  // (H is a multiple of 8: a slice has 16 units or, the last one, 8)
+  for (int i = threadIdx.x; i < (int)(r_bytes / 16); i += TC_THREADS)
+    reinterpret_cast<uint4*>(aligned)[i] = make_uint4(0u, 0u, 0u, 0u);
+  __syncthreads();
   if (FWD) {
     // B^T[n = gate*16 + u][k] = R[k][gate*H + u0 + u]
-    for (int item = threadIdx.x; item < K * 3; item += TC_THREADS) {
-      const int k = item / 3, gate = item % 3;
-      float x[16];
-      ld16(p.R + (size_t)k * 3 * H + (size_t)gate * H + u0, x);
+    for (int item = threadIdx.x; item < K * 6; item += TC_THREADS) {
+      const int k = item / 6, gate = item % 6 / 2, uo = item % 2 * 8;
+      if (u0 + uo >= H) continue;
+      float x[8];
+      ld8(p.R + (size_t)k * 3 * H + (size_t)gate * H + u0 + uo, x);
       uint8_t* tile = aligned + (size_t)(k / BK) * R_TILE;
 #pragma unroll
-      for (int u = 0; u < 16; ++u)
-        *reinterpret_cast<bf16*>(tile + swz_off(gate * 16 + u, k % BK)) = __float2bfloat16_rn(x[u]);
+      for (int u = 0; u < 8; ++u)
+        *reinterpret_cast<bf16*>(tile + swz_off(gate * 16 + uo + u, k % BK)) = __float2bfloat16_rn(x[u]);
     }
     for (int i = threadIdx.x; i < 96; i += TC_THREADS) {
       const int which = i / 48, c = i % 48, gate = c / 16, u = c % 16;
-      s_bias[i] = __bfloat162float((which ? p.br : p.bx)[gate * H + u0 + u]);
+      s_bias[i] = u0 + u < H ? __bfloat162float((which ? p.br : p.bx)[gate * H + u0 + u]) : 0.f;
     }
   } else {
     // B^T[n = unit j][k = gate column c] = R[u0 + j][c]   (R_t[c][u0 + j] when transposed)
     if (!p.r_transposed) {
       for (int item = threadIdx.x; item < 16 * (K / 8); item += TC_THREADS) {
         const int j = item / (K / 8), c8 = (item % (K / 8)) * 8;
+        if (u0 + j >= H) continue;
         const uint4 w = *reinterpret_cast<const uint4*>(p.R + (size_t)(u0 + j) * K + c8);
         uint8_t* tile = aligned + (size_t)(c8 / BK) * R_TILE;
         *reinterpret_cast<uint4*>(tile + swz_off(j, c8 % BK)) = w;  // one whole 16-byte chunk
       }
     } else {
-      for (int c = threadIdx.x; c < K; c += TC_THREADS) {
-        float x[16];
-        ld16(p.R + (size_t)c * H + u0, x);
+      for (int item = threadIdx.x; item < K * 2; item += TC_THREADS) {
+        const int c = item / 2, uo = item % 2 * 8;
+        if (u0 + uo >= H) continue;
+        float x[8];
+        ld8(p.R + (size_t)c * H + u0 + uo, x);
         uint8_t* tile = aligned + (size_t)(c / BK) * R_TILE;
 #pragma unroll
-        for (int j = 0; j < 16; ++j)
-          *reinterpret_cast<bf16*>(tile + swz_off(j, c % BK)) = __float2bfloat16_rn(x[j]);
+        for (int j = 0; j < 8; ++j)
+          *reinterpret_cast<bf16*>(tile + swz_off(uo + j, c % BK)) = __float2bfloat16_rn(x[j]);
       }
     }
   }
@@ -424,6 +410,7 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
 #pragma unroll
           for (int hf = 0; hf < 2; ++hf) {
             const int uo = hf * 8;
+            if (u0 + uo >= H) break;
             if (FWD) {
               const bf16* wx = p.Wx + ((long long)t * N + n) * 3 * H + u0 + uo;
               in0[hf] = ldq(wx);
@@ -512,7 +499,7 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
               if (warp == NI + 1 && lane == 0) HB_STAMP(p, it, mt, 5);
             }
           }
-          if (valid) {
+          if (valid && u0 + uo < H) {
             if (FWD) {
               float hn[8], vz[8], vr[8], vg[8], vq[8];
 #pragma unroll
@@ -595,7 +582,7 @@ struct TcGeometry {
   size_t ring, smem;
 };
 
-// Shapes this path takes: bf16, H a multiple of 64 up to 1024 (the resident slice of R and a
+// Shapes this path takes: bf16, H a multiple of 8 up to 1024 (the resident slice of R and a
 // useful ring must fit shared memory), at least 64 batch rows (below that the register
 // kernels are faster) and at most two row tiles per CTA: every CTA of a row group streams
 // the group's whole h (or dq), H / 16 copies of it per step out of L2, which is what bounds
@@ -607,10 +594,10 @@ struct TcGeometry {
 // when the budget would need more than two tiles per CTA, the whole GPU is used.
 bool tc_geometry_for(int N, int H, bool fwd, int sms, TcGeometry* g) {
   const int K = fwd ? H : 3 * H;
-  const size_t r_bytes = (size_t)(K / BK) * (fwd ? 48 : 16) * 128;
+  const size_t r_bytes = (size_t)ceil_div(K, BK) * (fwd ? 48 : 16) * 128;
   const size_t fixed = 1024 /*alignment*/ + r_bytes + 1024 /*barriers, bias*/;
   if (fixed + 2 * (size_t)A_STAGE > (size_t)MAX_SMEM) return false;
-  g->nHS = H / UC;
+  g->nHS = ceil_div(H, UC);
   const int groups_max = sms / g->nHS;
   if (groups_max < 1) return false;
   // 64-row tiles when that still gives one tile per CTA (more CTAs, less to stream per CTA)
@@ -640,7 +627,7 @@ bool tc_geometry_for(int N, int H, bool fwd, int sms, TcGeometry* g) {
 // bidirectional layer are co-resident).
 bool tc_geometry(int N, int H, bool fwd, TcGeometry* g, bool* budgeted) {
   *budgeted = false;
-  if (H % 64 != 0 || H < 64 || H > 1024 || N < 64) return false;
+  if (H % 8 != 0 || H < 64 || H > 1024 || N < 64) return false;
   const int budget = sm_budget();
   if (budget > 0 && budget < sm_count() && tc_geometry_for(N, H, fwd, budget, g)) {
     *budgeted = true;
