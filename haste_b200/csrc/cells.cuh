@@ -126,12 +126,15 @@ struct GradPlanes {
 // 1024.  Forward: the input projection is already in a.v (LSTM) / a.tmp_Wx (GRU).  Backward:
 // complete - dh and dc are read and written in place (dc_new may be null), the bias gradients
 // added.  `few` (GRU): leave batches to the tensor-core recurrence where that is faster.
-int lstm_forward_chain(const LstmFwd& a, cudaStream_t s);
-int lstm_backward_chain(const LstmBwd& a, const GradPlanes& planes, cudaStream_t s);
+int lstm_forward_chain(const LstmFwd& a, bool few, cudaStream_t s);
+int lstm_backward_chain(const LstmBwd& a, const GradPlanes& planes, bool few, cudaStream_t s);
 int gru_forward_chain(const GruFwd& a, bool few, cudaStream_t s);
 int gru_backward_chain(const GruBwd& a, const GradPlanes& planes, bool few, cudaStream_t s);
-// Tensor-core recurrence for bf16 batches of about a hundred rows and more (rec_tc_gru.cu).  The
+// Tensor-core recurrence for bf16 batches of about a hundred rows and more (rec_tc.cu).  The
 // backward kernel carries dh in an fp32 [N,H] buffer and does not sum the bias gradients.
+bool lstm_tc_takes(int dtype, int N, int H, bool fwd);
+int lstm_forward_tc(const LstmFwd& a, float* c_carry, cudaStream_t s);
+int lstm_backward_tc(const LstmBwd& a, float* dh_carry, float* dc_carry, cudaStream_t s);
 int gru_forward_tc(const GruFwd& a, cudaStream_t s);
 int gru_backward_tc(const GruBwd& a, float* dh_carry, cudaStream_t s);
 // LayerNormLSTM: forward expects LN(x.W) in a.act_Wx_norm; backward adds the LayerNorm

@@ -173,8 +173,20 @@ int lstm_forward(const LstmFwd& a, cudaStream_t s) {
     HB_TRY(gemm(g, s));
   }
   ProfScope p(PH_REC_FWD, s);
-  const int st_ = (a.h_out || a.c_out) ? HASTE_B200_ERR_UNSUPPORTED : lstm_forward_chain(a, s);
-  if (st_ != HASTE_B200_ERR_UNSUPPORTED) return st_;
+  if (!a.h_out && !a.c_out) {
+    int st_ = lstm_forward_chain(a, /*few=*/true, s);
+    if (st_ != HASTE_B200_ERR_UNSUPPORTED) return st_;
+    if (lstm_tc_takes(a.dtype, a.N, a.H, true)) {
+      const size_t NH = (size_t)a.N * a.H;
+      float* c_carry = static_cast<float*>(workspace(s, NH * sizeof(float)));
+      if (!c_carry) return HASTE_B200_ERR_CUDA;
+      HB_TRY(to_float(a.dtype, a.c, c_carry, NH, s));
+      st_ = lstm_forward_tc(a, c_carry, s);
+      if (st_ != HASTE_B200_ERR_UNSUPPORTED) return st_;
+    }
+    st_ = lstm_forward_chain(a, /*few=*/false, s);
+    if (st_ != HASTE_B200_ERR_UNSUPPORTED) return st_;
+  }
   if (a.dtype == HASTE_B200_F32) return lstm_forward_stepwise<float>(a, s);
   return lstm_forward_stepwise<__nv_bfloat16>(a, s);
 }
@@ -207,7 +219,7 @@ int lstm_backward(const LstmBwd& a, cudaStream_t s) {
   int st_;
   {
     ProfScope p(PH_REC_BWD, s);
-    st_ = a.iterate ? HASTE_B200_ERR_UNSUPPORTED : lstm_backward_chain(a, planes, s);
+    st_ = a.iterate ? HASTE_B200_ERR_UNSUPPORTED : lstm_backward_chain(a, planes, /*few=*/true, s);
     have_planes = st_ == HASTE_B200_OK && planes.p != nullptr;
   }
   if (st_ == HASTE_B200_ERR_UNSUPPORTED) {
@@ -224,15 +236,29 @@ int lstm_backward(const LstmBwd& a, cudaStream_t s) {
       HB_CUDA_OK(cudaMemsetAsync(dh_carry, 0, NH * 4, s));
       HB_CUDA_OK(cudaMemsetAsync(dc_carry, 0, NH * 4, s));
     }
+    bool carried = true;  // dh, dc travel in the carries and the bias gradients are still to be summed
     {
       ProfScope p(PH_REC_BWD, s);
-      st_ = (a.dtype == HASTE_B200_F32) ? lstm_backward_stepwise<float>(a, dh_carry, dc_carry, s)
-                                        : lstm_backward_stepwise<__nv_bfloat16>(a, dh_carry, dc_carry, s);
+      if (!a.iterate) st_ = lstm_backward_tc(a, dh_carry, dc_carry, s);
+      if (st_ == HASTE_B200_OK) {
+        // the tensor-core kernel leaves the recurrent contribution of step 0 out of dh
+        GemmDesc gd{a.dtype, HASTE_B200_F32, N, H, 4 * H, a.v, 4LL * H, 1, a.R, a.transposed_inputs ? H : 1,
+                    a.transposed_inputs ? 1 : 4LL * H, dh_carry, H, 1};
+        st_ = gemm(gd, s);
+      } else if (st_ == HASTE_B200_ERR_UNSUPPORTED && !a.iterate) {
+        st_ = lstm_backward_chain(a, planes, /*few=*/false, s);
+        carried = st_ != HASTE_B200_OK;
+      }
+      if (st_ == HASTE_B200_ERR_UNSUPPORTED)
+        st_ = (a.dtype == HASTE_B200_F32) ? lstm_backward_stepwise<float>(a, dh_carry, dc_carry, s)
+                                          : lstm_backward_stepwise<__nv_bfloat16>(a, dh_carry, dc_carry, s);
     }
     HB_TRY(st_);
-    HB_TRY(from_float(a.dtype, dh_carry, a.dh, NH, s));
-    HB_TRY(from_float(a.dtype, dc_carry, a.dc, NH, s));
-    HB_TRY(colsum(a.dtype, a.v, 4LL * H, (int)TN, 4 * H, a.dtype, a.db, add, cs, s));
+    if (carried) {
+      HB_TRY(from_float(a.dtype, dh_carry, a.dh, NH, s));
+      HB_TRY(from_float(a.dtype, dc_carry, a.dc, NH, s));
+      HB_TRY(colsum(a.dtype, a.v, 4LL * H, (int)TN, 4 * H, a.dtype, a.db, add, cs, s));
+    }
   }
   HB_TRY(st_);
 

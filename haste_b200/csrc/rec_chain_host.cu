@@ -22,8 +22,10 @@ bool aligned(std::initializer_list<const void*> ptrs, int H, int dtype) {
 // chain adds 0.7 .. 2 us to a step (H = 512 .. 1024), which the step-wise path (about 20 us plus the
 // product) undercuts from a dozen on, and beyond six the tensor-core GRU recurrence (6 us
 // forward, 11 us backward at H = 1024 whatever the rows; both passes of a bidirectional layer of 200
-// steps, chains / tensor-core: 48 rows, six chains, 3.5 / 4.0 ms; 64 rows, eight chains, 4.9 / 4.6).
-constexpr int kGridChains = 12, kGridChainsBeforeTc = 6;
+// steps, chains / tensor-core: 48 rows, six chains, 3.5 / 4.0 ms; 64 rows, eight chains, 4.9 / 4.0).  The
+// LSTM's has a third more to stream and to compute: beyond eight (H = 1024, 64 rows, eight chains, 4.7 / 5.2 ms;
+// 90 rows, twelve, 8.1 / 6.4).
+constexpr int kGridChains = 12, kGruChainsBeforeTc = 6, kLstmChainsBeforeTc = 8;
 
 // A handful of steps of a wide fp32 / fp16 layer stays on the step-wise path (as
 // tests/test_parity_gpu.py expects of it).
@@ -119,14 +121,14 @@ int run_bwd(ChainParams& p, int dtype, int grid_most, int gates, void* db, void*
   return bias_grad_finish(gates, p.db_part, 2 * g.nRG, p.H, dtype, db, db2, !p.zero_init, s);
 }
 
-// Rows the tensor-core GRU recurrence would take (rec_tc_gru.cu).
+// Rows the tensor-core GRU recurrence would take (rec_tc.cu).
 bool tc_waits(int dtype, int N, int H) {
   return dtype == HASTE_B200_BF16 && N >= 64 && H % 8 == 0 && recurrence_path() != HASTE_B200_PATH_NO_TENSOR_CORE;
 }
 
 }  // namespace
 
-int lstm_forward_chain(const LstmFwd& a, cudaStream_t s) {
+int lstm_forward_chain(const LstmFwd& a, bool few, cudaStream_t s) {
   if (recurrence_path() == HASTE_B200_PATH_STEPWISE) return HASTE_B200_ERR_UNSUPPORTED;
   ChainParams p{};
   p.T = a.T; p.N = a.N; p.H = a.H;
@@ -135,7 +137,8 @@ int lstm_forward_chain(const LstmFwd& a, cudaStream_t s) {
   p.R = a.R; p.b = a.b; p.gin = a.v; p.gout = a.training ? a.v : nullptr; p.mask = a.zoneout_mask;
   p.h = a.h; p.c = a.c;
   p.wide = aligned({a.v, a.h, a.c, a.zoneout_mask}, a.H, a.dtype);
-  return run_fwd(p, a.dtype, kGridChains, run_cl_fwd_lstm, run_gl_fwd_lstm, s);
+  const int most = few && lstm_tc_takes(a.dtype, a.N, a.H, true) ? kLstmChainsBeforeTc : kGridChains;
+  return run_fwd(p, a.dtype, most, run_cl_fwd_lstm, run_gl_fwd_lstm, s);
 }
 
 int gru_forward_chain(const GruFwd& a, bool few, cudaStream_t s) {
@@ -147,11 +150,11 @@ int gru_forward_chain(const GruFwd& a, bool few, cudaStream_t s) {
   p.R = a.R; p.b = a.bx; p.b2 = a.br; p.gin = a.tmp_Wx; p.gout = a.training ? a.v : nullptr;
   p.mask = a.zoneout_mask; p.h = a.h;
   p.wide = aligned({a.tmp_Wx, a.v, a.h, a.zoneout_mask}, a.H, a.dtype);
-  return run_fwd(p, a.dtype, few && tc_waits(a.dtype, a.N, a.H) ? kGridChainsBeforeTc : kGridChains,
+  return run_fwd(p, a.dtype, few && tc_waits(a.dtype, a.N, a.H) ? kGruChainsBeforeTc : kGridChains,
                  run_cl_fwd_gru, run_gl_fwd_gru, s);
 }
 
-int lstm_backward_chain(const LstmBwd& a, const GradPlanes& planes, cudaStream_t s) {
+int lstm_backward_chain(const LstmBwd& a, const GradPlanes& planes, bool few, cudaStream_t s) {
   if (recurrence_path() == HASTE_B200_PATH_STEPWISE) return HASTE_B200_ERR_UNSUPPORTED;
   ChainParams p{};
   p.T = a.T; p.N = a.N; p.H = a.H;
@@ -160,7 +163,8 @@ int lstm_backward_chain(const LstmBwd& a, const GradPlanes& planes, cudaStream_t
   p.mask = a.zoneout_mask; p.dh = a.dh; p.dc = a.dc;
   p.gpl = planes.p; p.gpl_stride = planes.stride;
   p.wide = aligned({a.v, a.c, a.dh_new, a.dc_new, a.zoneout_mask}, a.H, a.dtype);
-  return run_bwd(p, a.dtype, kGridChains, 4, a.db, nullptr, run_cl_bwd_lstm, run_gl_bwd_lstm, s);
+  const int most = few && lstm_tc_takes(a.dtype, a.N, a.H, false) ? kLstmChainsBeforeTc : kGridChains;
+  return run_bwd(p, a.dtype, most, 4, a.db, nullptr, run_cl_bwd_lstm, run_gl_bwd_lstm, s);
 }
 
 int gru_backward_chain(const GruBwd& a, const GradPlanes& planes, bool few, cudaStream_t s) {
@@ -172,7 +176,7 @@ int gru_backward_chain(const GruBwd& a, const GradPlanes& planes, bool few, cuda
   p.mask = a.zoneout_mask; p.dh = a.dh;
   p.gpl = planes.p; p.gpl2 = planes.p2; p.gpl_stride = planes.stride;
   p.wide = aligned({a.v, a.dp, a.dq, a.h, a.dh_new, a.zoneout_mask}, a.H, a.dtype);
-  return run_bwd(p, a.dtype, few && tc_waits(a.dtype, a.N, a.H) ? kGridChainsBeforeTc : kGridChains, 3, a.dbx,
+  return run_bwd(p, a.dtype, few && tc_waits(a.dtype, a.N, a.H) ? kGruChainsBeforeTc : kGridChains, 3, a.dbx,
                  a.dbr, run_cl_bwd_gru, run_gl_bwd_gru, s);
 }
 

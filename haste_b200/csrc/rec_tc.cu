@@ -1,12 +1,19 @@
-// Tensor-core GRU recurrence for large batches (bf16 storage), sm_100a.
+// Tensor-core GRU and LSTM recurrences for large batches (bf16 storage), sm_100a.
 //
-// The register-resident kernels of recurrent_common.cuh are built for small batches: a CTA
-// multiplies 16..64 batch rows with mma.sync and every row of h reaches it as tagged words.
-// From about a hundred rows per GPU the step product is a real tile for the 5th-generation
-// tensor cores, and this file runs it there:
+// The chain kernels (rec_grid_kernels.cuh) take eight batch rows at a time and pay for every chain
+// of a CTA.  Where they would need more than six (LSTM: eight) - a hundred rows of a wide layer, or
+// half of that on half of the GPU - the step product is a real tile for the 5th-generation tensor
+// cores, and this file runs it there:
 //
-//   forward   gates[rows, 3*16] = h_{t-1}[rows, 0:H] . R[0:H, slice]            K = H
-//   backward  dh_rec[rows, 16]  = dq_{t+1}[rows, 0:3H] . R[slice, 0:3H]^T       K = 3H
+//   forward   gates[rows, G*16] = h_{t-1}[rows, 0:H] . R[0:H, slice]            K = H
+//   backward  dh_rec[rows, 16]  = dq_{t+1}[rows, 0:GH] . R[slice, 0:GH]^T       K = GH
+//
+// (G = 3 for the GRU; G = 4 for the LSTM, where "dq" is the gate gradient in the cache's place.)
+// A step is bound by its chain - counter, TMA, MMA issue (65 cycles each), tensor-memory read, gate
+// math, publish - and, with many rows per CTA, by the stream of h or dq at 64 bytes per clock and SM.
+// GRU, H = 1024, us per step forward / backward: 128 rows 6.5 / 9.8, 256 rows 7.5 / 11.9 (one 128-row tile
+// per CTA before: 7.6 / 13.3).  Two directions of 200 steps side by side, chain kernels -> this: GRU 90
+// rows 8.2 -> 5.0 ms, LSTM 90 rows 8.1 -> 6.4, LSTM 178 rows H = 808 9.4 -> 6.9.
 //
 // * Grid = (H / 16 hidden slices) x (row groups), one cooperative launch per layer pass; a
 //   CTA owns 16 hidden units for MT tiles of RB (64 or 128) batch rows.
@@ -36,7 +43,7 @@
 // (lib/gru_forward_gpu.cu.cc:214-308,345-363, lib/gru_backward_gpu.cu.cc:252-320) for
 // bf16 batches of about a hundred rows and more; math as in lib/gru_forward_gpu.cu.cc:27-85
 // and lib/gru_backward_gpu.cu.cc:26-96.
-#include "recurrent_common.cuh"
+#include "rec_chain.cuh"
 #include "tcgen05.cuh"
 
 namespace hb {
@@ -45,7 +52,7 @@ namespace {
 using namespace tc;
 typedef __nv_bfloat16 bf16;
 
-// Gate functions of this bf16-only path: one MUFU.TANH each (relative error 2^-11, a
+// Gate functions of the GRU here (the LSTM uses those of rec_chain.cuh): one MUFU.TANH each (relative error 2^-11, a
 // fraction of a bf16 ulp; the parity bar of bf16 storage is 2e-2).
 __device__ __forceinline__ float tanh_fast(float x) {
   float y;
@@ -80,6 +87,9 @@ struct TcParams {
   bf16* dp;            // backward out [T,N,3H]
   bf16* dq;            // backward out [T,N,3H], also the streamed operand
   float* dh_carry;     // backward [N,H] fp32 in/out
+  bf16* c;             // LSTM [T+1,N,H] (backward: read only)
+  float* c_carry;      // LSTM [N,H] fp32: forward c, backward its gradient, in/out
+  const bf16* dc_new;  // LSTM backward [T+1,N,H] or null
   unsigned int* cnt;   // [row tiles] arrival counters, zeroed before launch
   int* abort_flag;     // device-global, zeroed before launch
   int* err;            // process error word
@@ -167,6 +177,16 @@ __device__ __forceinline__ void st8(bf16* p, const float (&x)[8]) {
   *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+__device__ __forceinline__ void ld_carry(const float* p, float (&x)[8]) {
+  const float4 a = reinterpret_cast<const float4*>(p)[0], b = reinterpret_cast<const float4*>(p)[1];
+  x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
+  x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+}
+__device__ __forceinline__ void st_carry(float* p, const float (&x)[8]) {
+  reinterpret_cast<float4*>(p)[0] = make_float4(x[0], x[1], x[2], x[3]);
+  reinterpret_cast<float4*>(p)[1] = make_float4(x[4], x[5], x[6], x[7]);
+}
+
 // Byte offset of element (row n, k) inside one K-major, 128-byte-swizzled k-block tile
 // (rows of 64 bf16 = 128 bytes; 16-byte chunk c of row n sits at chunk c ^ (n & 7)).
 __device__ __forceinline__ uint32_t swz_off(int n, int kk) {
@@ -187,14 +207,16 @@ __device__ __forceinline__ void next_block(int& stage, uint32_t& phase, int& kb,
   }
 }
 
-template <int NB, bool FWD>
+// G: gates, 3 GRU, 4 LSTM.
+template <int G, bool FWD>
 __global__ void __launch_bounds__(TC_THREADS, 1)
-gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const int stages) {
+tc_recurrence_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const int stages) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* aligned = smem_raw + (base - smem_u32(smem_raw));
   const int H = p.H, N = p.N;
-  const int K = FWD ? H : 3 * H;
+  constexpr int NB = FWD ? G * UC : UC;  // columns of the step product
+  const int K = FWD ? H : G * H;
   const int KB = (K + BK - 1) / BK;  // (TMA fills what lies beyond K with zeros)
   constexpr int R_TILE = NB * 128;  // bytes of the resident operand per k-block
   const uint32_t r_bytes = (uint32_t)KB * R_TILE;
@@ -251,18 +273,19 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
   __syncthreads();
   if (FWD) {
     // B^T[n = gate*16 + u][k] = R[k][gate*H + u0 + u]
-    for (int item = threadIdx.x; item < K * 6; item += TC_THREADS) {
-      const int k = item / 6, gate = item % 6 / 2, uo = item % 2 * 8;
+    for (int item = threadIdx.x; item < K * 2 * G; item += TC_THREADS) {
+      const int k = item / (2 * G), gate = item % (2 * G) / 2, uo = item % 2 * 8;
       if (u0 + uo >= H) continue;
       float x[8];
-      ld8(p.R + (size_t)k * 3 * H + (size_t)gate * H + u0 + uo, x);
+      ld8(p.R + (size_t)k * G * H + (size_t)gate * H + u0 + uo, x);
       uint8_t* tile = aligned + (size_t)(k / BK) * R_TILE;
 #pragma unroll
       for (int u = 0; u < 8; ++u)
         *reinterpret_cast<bf16*>(tile + swz_off(gate * 16 + uo + u, k % BK)) = __float2bfloat16_rn(x[u]);
     }
-    for (int i = threadIdx.x; i < 96; i += TC_THREADS) {
-      const int which = i / 48, c = i % 48, gate = c / 16, u = c % 16;
+    // (the GRU's bx, then br)
+    for (int i = threadIdx.x; i < (G == 3 ? 96 : 64); i += TC_THREADS) {
+      const int which = i / NB, c = i % NB, gate = c / 16, u = c % 16;
       s_bias[i] = u0 + u < H ? __bfloat162float((which ? p.br : p.bx)[gate * H + u0 + u]) : 0.f;
     }
   } else {
@@ -404,19 +427,21 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
         // pairs) until they are used, so that the live state of a thread stays within its
         // share of the register file (nine warps per CTA).
         // ---- inputs that do not depend on the recurrence: issued before the wait below
-        uint4 in0[2], in1[2], in2[2], in3[2], hp[2], mk[2], dhn[2];
-        float carry[2][8];
+        uint4 in0[2], in1[2], in2[2], in3[2], hp[2], mk[2], dhn[2], cn[2], dcn[2];
+        float carry[2][8];  // backward: dh; LSTM forward: c
         if (valid) {
 #pragma unroll
           for (int hf = 0; hf < 2; ++hf) {
             const int uo = hf * 8;
             if (u0 + uo >= H) break;
             if (FWD) {
-              const bf16* wx = p.Wx + ((long long)t * N + n) * 3 * H + u0 + uo;
+              const bf16* wx = p.Wx + ((long long)t * N + n) * G * H + u0 + uo;
               in0[hf] = ldq(wx);
               in1[hf] = ldq(wx + H);
               in2[hf] = ldq(wx + 2 * H);
-              hp[hf] = ldq(p.h + (long long)t * NH + o0 + uo);
+              if (G == 4) in3[hf] = ldq(wx + 3 * H);
+              if (G == 3 || p.has_zoneout) hp[hf] = ldq(p.h + (long long)t * NH + o0 + uo);
+              if (G == 4) ld_carry(p.c_carry + o0 + uo, carry[hf]);
               if (p.has_zoneout && p.training) mk[hf] = ldq(p.mask + (long long)t * NH + o0 + uo);
             } else {
               const bf16* vt = p.v + ((long long)t * N + n) * 4 * H + u0 + uo;
@@ -424,13 +449,12 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
               in1[hf] = ldq(vt + H);
               in2[hf] = ldq(vt + 2 * H);
               in3[hf] = ldq(vt + 3 * H);
-              hp[hf] = ldq(p.h + (long long)t * NH + o0 + uo);
+              hp[hf] = ldq((G == 4 ? p.c : p.h) + (long long)t * NH + o0 + uo);  // before the step
+              if (G == 4) cn[hf] = ldq(p.c + (long long)(t + 1) * NH + o0 + uo);
+              if (G == 4 && p.dc_new) dcn[hf] = ldq(p.dc_new + (long long)(t + 1) * NH + o0 + uo);
               dhn[hf] = ldq(p.dh_new + (long long)(t + 1) * NH + o0 + uo);
               if (p.has_zoneout) mk[hf] = ldq(p.mask + (long long)t * NH + o0 + uo);
-              const float4* cp = reinterpret_cast<const float4*>(p.dh_carry + o0 + uo);
-              const float4 f0 = cp[0], f1 = cp[1];
-              carry[hf][0] = f0.x; carry[hf][1] = f0.y; carry[hf][2] = f0.z; carry[hf][3] = f0.w;
-              carry[hf][4] = f1.x; carry[hf][5] = f1.y; carry[hf][6] = f1.z; carry[hf][7] = f1.w;
+              ld_carry(p.dh_carry + o0 + uo, carry[hf]);
             }
           }
         }
@@ -457,15 +481,15 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
         for (int hf = 0; hf < 2; ++hf) {
           const int uo = hf * 8;
           // this half's columns of the accumulators (one per issuer), summed
-          float s0[8], s1[8], s2[8];
+          float s0[8], s1[8], s2[8], s3[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) s0[i] = s1[i] = s2[i] = 0.f;
+          for (int i = 0; i < 8; ++i) s0[i] = s1[i] = s2[i] = s3[i] = 0.f;
           if (have_acc) {
             // the issuers' accumulators, GRP of them per wait (all loads of a group in flight)
-            constexpr int GRP = FWD ? 2 : NI;
+            constexpr int GRP = FWD ? (G == 4 ? 1 : 2) : NI;
 #pragma unroll
             for (int g0 = 0; g0 < NI; g0 += GRP) {
-              uint32_t b0[GRP][8], b1[GRP][8], b2[GRP][8];
+              uint32_t b0[GRP][8], b1[GRP][8], b2[GRP][8], b3[GRP][8];
 #pragma unroll
               for (int k = 0; k < GRP; ++k) {
                 const int i2 = g0 + k;
@@ -474,6 +498,7 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
                   if (FWD) {
                     tc_ld8(taddr + i2 * ACC_COLS + 16 + uo, b1[k]);
                     tc_ld8(taddr + i2 * ACC_COLS + 32 + uo, b2[k]);
+                    if (G == 4) tc_ld8(taddr + i2 * ACC_COLS + 48 + uo, b3[k]);
                   }
                 }
               }
@@ -488,6 +513,7 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
                     if (FWD) {
                       s1[i] += __uint_as_float(b1[k][i]);
                       s2[i] += __uint_as_float(b2[k][i]);
+                      if (G == 4) s3[i] += __uint_as_float(b3[k][i]);
                     }
                   }
                 }
@@ -500,7 +526,29 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
             }
           }
           if (valid && u0 + uo < H) {
-            if (FWD) {
+            if (FWD && G == 4) {
+              float hn[8], vi[8], vg[8], vf[8], vo[8];
+#pragma unroll
+              for (int u = 0; u < 8; ++u) {
+                vi[u] = rec::chain_sigmoid(bfq(in0[hf], u) + s0[u] + s_bias[uo + u]);
+                vg[u] = rec::chain_tanh(bfq(in1[hf], u) + s1[u] + s_bias[16 + uo + u]);
+                vf[u] = rec::chain_sigmoid(bfq(in2[hf], u) + s2[u] + s_bias[32 + uo + u]);
+                vo[u] = rec::chain_sigmoid(bfq(in3[hf], u) + s3[u] + s_bias[48 + uo + u]);
+                carry[hf][u] = vf[u] * carry[hf][u] + vi[u] * vg[u];
+                float x = vo[u] * rec::chain_tanh(carry[hf][u]);
+                if (p.has_zoneout)
+                  x = p.training ? zoneout<true>(x, bfq(hp[hf], u), p.zoneout_prob, bfq(mk[hf], u))
+                                 : zoneout<false>(x, bfq(hp[hf], u), p.zoneout_prob, 0.f);
+                hn[u] = x;
+              }
+              st8(p.h + (long long)(t + 1) * NH + o0 + uo, hn);  // the next step streams it
+              st8(p.c + (long long)(t + 1) * NH + o0 + uo, carry[hf]);
+              st_carry(p.c_carry + o0 + uo, carry[hf]);
+              if (p.training) {
+                bf16* vt = p.v + ((long long)t * N + n) * 4 * H + u0 + uo;
+                st8(vt, vi); st8(vt + H, vg); st8(vt + 2 * H, vf); st8(vt + 3 * H, vo);
+              }
+            } else if (FWD) {
               float hn[8], vz[8], vr[8], vg[8], vq[8];
 #pragma unroll
               for (int u = 0; u < 8; ++u) {
@@ -520,6 +568,22 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
                 bf16* vt = p.v + ((long long)t * N + n) * 4 * H + u0 + uo;
                 st8(vt, vz); st8(vt + H, vr); st8(vt + 2 * H, vg); st8(vt + 3 * H, vq);
               }
+            } else if (G == 4) {
+              float di[8], dg[8], df[8], d_o[8], dcc[8];
+              ld_carry(p.c_carry + o0 + uo, dcc);  // the carried gradient of c
+#pragma unroll
+              for (int u = 0; u < 8; ++u) {
+                const float gv[4] = {bfq(in0[hf], u), bfq(in1[hf], u), bfq(in2[hf], u), bfq(in3[hf], u)};
+                float d[4];
+                const float dh_total = bfq(dhn[hf], u) + carry[hf][u] + s0[u];
+                rec::cell_bwd<4>(gv, bfq(hp[hf], u), bfq(cn[hf], u), dh_total, p.dc_new ? bfq(dcn[hf], u) : 0.f,
+                                 p.has_zoneout != 0, p.has_zoneout ? bfq(mk[hf], u) : 1.f, carry[hf][u], dcc[u], d);
+                di[u] = d[0]; dg[u] = d[1]; df[u] = d[2]; d_o[u] = d[3];
+              }
+              bf16* vt = p.v + ((long long)t * N + n) * 4 * H + u0 + uo;  // streamed next
+              st8(vt, di); st8(vt + H, dg); st8(vt + 2 * H, df); st8(vt + 3 * H, d_o);
+              st_carry(p.dh_carry + o0 + uo, carry[hf]);
+              st_carry(p.c_carry + o0 + uo, dcc);
             } else {
               float dpz[8], dpr[8], dpg[8], dqg[8];
 #pragma unroll
@@ -545,9 +609,7 @@ gru_tc_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const
               const long long w0 = ((long long)t * N + n) * 3 * H + u0 + uo;
               st8(p.dq + w0, dpz); st8(p.dq + w0 + H, dpr); st8(p.dq + w0 + 2 * H, dqg);  // streamed next
               st8(p.dp + w0, dpz); st8(p.dp + w0 + H, dpr); st8(p.dp + w0 + 2 * H, dpg);
-              float4* cp = reinterpret_cast<float4*>(p.dh_carry + o0 + uo);
-              cp[0] = make_float4(carry[hf][0], carry[hf][1], carry[hf][2], carry[hf][3]);
-              cp[1] = make_float4(carry[hf][4], carry[hf][5], carry[hf][6], carry[hf][7]);
+              st_carry(p.dh_carry + o0 + uo, carry[hf]);
             }
           }
         }
@@ -592,9 +654,9 @@ struct TcGeometry {
 // (register kernel) / 18.4 / 20.5 us; backward 20.6 / 22.4 / 30.4 against 16.4 / 18.6 / 24.6).
 // `half` asks for the geometry under the SM budget (concurrent directions); without it, or
 // when the budget would need more than two tiles per CTA, the whole GPU is used.
-bool tc_geometry_for(int N, int H, bool fwd, int sms, TcGeometry* g) {
-  const int K = fwd ? H : 3 * H;
-  const size_t r_bytes = (size_t)ceil_div(K, BK) * (fwd ? 48 : 16) * 128;
+bool tc_geometry_for(int G, int N, int H, bool fwd, int sms, TcGeometry* g) {
+  const int K = fwd ? H : G * H;
+  const size_t r_bytes = (size_t)ceil_div(K, BK) * (fwd ? G * UC : UC) * 128;
   const size_t fixed = 1024 /*alignment*/ + r_bytes + 1024 /*barriers, bias*/;
   if (fixed + 2 * (size_t)A_STAGE > (size_t)MAX_SMEM) return false;
   g->nHS = ceil_div(H, UC);
@@ -625,22 +687,22 @@ bool tc_geometry_for(int N, int H, bool fwd, int sms, TcGeometry* g) {
 
 // `budgeted` reports whether the geometry honours the SM budget (then the two directions of a
 // bidirectional layer are co-resident).
-bool tc_geometry(int N, int H, bool fwd, TcGeometry* g, bool* budgeted) {
+bool tc_geometry(int G, int N, int H, bool fwd, TcGeometry* g, bool* budgeted) {
   *budgeted = false;
   if (H % 8 != 0 || H < 64 || H > 1024 || N < 64) return false;
   const int budget = sm_budget();
-  if (budget > 0 && budget < sm_count() && tc_geometry_for(N, H, fwd, budget, g)) {
+  if (budget > 0 && budget < sm_count() && tc_geometry_for(G, N, H, fwd, budget, g)) {
     *budgeted = true;
     return true;
   }
-  return tc_geometry_for(N, H, fwd, sm_count(), g);
+  return tc_geometry_for(G, N, H, fwd, sm_count(), g);
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-template <int NB, bool FWD>
+template <int G, bool FWD>
 int launch_tc(const CUtensorMap& map, TcParams& p, const TcGeometry& g, cudaStream_t s) {
-  auto kernel = gru_tc_kernel<NB, FWD>;
+  auto kernel = tc_recurrence_kernel<G, FWD>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)g.smem);
   if (e != cudaSuccess) {
@@ -695,6 +757,14 @@ int tc_scratch(int tiles, TcParams* p, cudaStream_t s) {
 
 }  // namespace
 
+bool lstm_tc_takes(int dtype, int N, int H, bool fwd) {
+  TcGeometry g;
+  bool budgeted = false;
+  return dtype == HASTE_B200_BF16 && recurrence_path() != HASTE_B200_PATH_STEPWISE &&
+         recurrence_path() != HASTE_B200_PATH_NO_TENSOR_CORE && encode_fn() &&
+         tc_geometry(4, N, H, fwd, &g, &budgeted);
+}
+
 // Forward: x.W is already in a.tmp_Wx.  HASTE_B200_ERR_UNSUPPORTED (nothing touched) when the
 // shape is not this path's.
 int gru_forward_tc(const GruFwd& a, cudaStream_t s) {
@@ -702,7 +772,7 @@ int gru_forward_tc(const GruFwd& a, cudaStream_t s) {
   bool budgeted = false;
   if (a.dtype != HASTE_B200_BF16 || recurrence_path() == HASTE_B200_PATH_STEPWISE ||
       recurrence_path() == HASTE_B200_PATH_NO_TENSOR_CORE || a.h_out ||
-      !encode_fn() || !tc_geometry(a.N, a.H, true, &g, &budgeted))
+      !encode_fn() || !tc_geometry(3, a.N, a.H, true, &g, &budgeted))
     return HASTE_B200_ERR_UNSUPPORTED;
   if (!aligned16(a.R) || !aligned16(a.tmp_Wx) || !aligned16(a.h) || !aligned16(a.v) ||
       !aligned16(a.zoneout_mask) || !aligned16(a.bx) || !aligned16(a.br))
@@ -719,7 +789,7 @@ int gru_forward_tc(const GruFwd& a, cudaStream_t s) {
   p.Wx = (const bf16*)a.tmp_Wx; p.mask = (const bf16*)a.zoneout_mask;
   p.h = (bf16*)a.h; p.v = (bf16*)a.v;
   HB_TRY(tc_scratch(ceil_div(a.N, g.RB), &p, s));
-  return launch_tc<48, true>(map, p, g, s);
+  return launch_tc<3, true>(map, p, g, s);
 }
 
 // Backward: dh_carry (fp32 [N,H]) holds the incoming gradient of the final state and receives
@@ -730,7 +800,7 @@ int gru_backward_tc(const GruBwd& a, float* dh_carry, cudaStream_t s) {
   bool budgeted = false;
   if (a.dtype != HASTE_B200_BF16 || recurrence_path() == HASTE_B200_PATH_STEPWISE ||
       recurrence_path() == HASTE_B200_PATH_NO_TENSOR_CORE || a.iterate ||
-      !encode_fn() || !tc_geometry(a.N, a.H, false, &g, &budgeted))
+      !encode_fn() || !tc_geometry(3, a.N, a.H, false, &g, &budgeted))
     return HASTE_B200_ERR_UNSUPPORTED;
   if (!aligned16(a.R) || !aligned16(a.h) || !aligned16(a.v) || !aligned16(a.dh_new) ||
       !aligned16(a.dp) || !aligned16(a.dq) || !aligned16(a.zoneout_mask) || !aligned16(dh_carry))
@@ -747,7 +817,50 @@ int gru_backward_tc(const GruBwd& a, float* dh_carry, cudaStream_t s) {
   p.dh_new = (const bf16*)a.dh_new; p.dp = (bf16*)a.dp; p.dq = (bf16*)a.dq;
   p.dh_carry = dh_carry;
   HB_TRY(tc_scratch(ceil_div(a.N, g.RB), &p, s));
-  return launch_tc<16, false>(map, p, g, s);
+  return launch_tc<3, false>(map, p, g, s);
+}
+
+// LSTM, in the same way: x.W is in a.v; c_carry (fp32 [N,H]) holds c_0.
+int lstm_forward_tc(const LstmFwd& a, float* c_carry, cudaStream_t s) {
+  TcGeometry g;
+  bool budgeted = false;
+  if (!lstm_tc_takes(a.dtype, a.N, a.H, true) || !tc_geometry(4, a.N, a.H, true, &g, &budgeted) || !aligned16(a.R) ||
+      !aligned16(a.h) || !aligned16(a.c) || !aligned16(a.v) || !aligned16(a.zoneout_mask) || !aligned16(c_carry))
+    return HASTE_B200_ERR_UNSUPPORTED;
+  CUtensorMap map;
+  if (!make_map(&map, a.h, a.H, (long long)(a.T + 1) * a.N, a.H, 0, 1, BK, g.RB))
+    return HASTE_B200_ERR_UNSUPPORTED;
+  TcParams p{};
+  p.T = a.T; p.N = a.N; p.H = a.H; p.nHS = g.nHS; p.MT = g.MT; p.RB = g.RB;
+  p.stage_bytes = g.RB * 128; p.ring_bytes = (int)g.ring;
+  p.training = a.training; p.has_zoneout = a.zoneout_prob != 0.0f && a.zoneout_mask != nullptr;
+  p.zoneout_prob = a.zoneout_prob;
+  p.R = (const bf16*)a.R; p.bx = (const bf16*)a.b; p.Wx = (const bf16*)a.v; p.mask = (const bf16*)a.zoneout_mask;
+  p.h = (bf16*)a.h; p.c = (bf16*)a.c; p.v = (bf16*)a.v; p.c_carry = c_carry;
+  HB_TRY(tc_scratch(ceil_div(a.N, g.RB), &p, s));
+  return launch_tc<4, true>(map, p, g, s);
+}
+
+// v: gates in, gate gradients out.  dh_carry, dc_carry as dh_carry of gru_backward_tc.
+int lstm_backward_tc(const LstmBwd& a, float* dh_carry, float* dc_carry, cudaStream_t s) {
+  TcGeometry g;
+  bool budgeted = false;
+  if (!lstm_tc_takes(a.dtype, a.N, a.H, false) || !tc_geometry(4, a.N, a.H, false, &g, &budgeted) || !aligned16(a.R) ||
+      !aligned16(a.c) || !aligned16(a.v) || !aligned16(a.dh_new) || !aligned16(a.dc_new) ||
+      !aligned16(a.zoneout_mask) || !aligned16(dh_carry) || !aligned16(dc_carry))
+    return HASTE_B200_ERR_UNSUPPORTED;
+  CUtensorMap map;
+  if (!make_map(&map, a.v, 4LL * a.H, (long long)a.T * a.N, 4LL * a.H, 0, 1, BK, g.RB))
+    return HASTE_B200_ERR_UNSUPPORTED;
+  TcParams p{};
+  p.T = a.T; p.N = a.N; p.H = a.H; p.nHS = g.nHS; p.MT = g.MT; p.RB = g.RB;
+  p.stage_bytes = g.RB * 128; p.ring_bytes = (int)g.ring;
+  p.has_zoneout = a.zoneout_mask ? 1 : 0; p.r_transposed = a.transposed_inputs;
+  p.R = (const bf16*)a.R; p.mask = (const bf16*)a.zoneout_mask;
+  p.c = (bf16*)const_cast<void*>(a.c); p.v = (bf16*)a.v; p.dh_new = (const bf16*)a.dh_new;
+  p.dc_new = (const bf16*)a.dc_new; p.dh_carry = dh_carry; p.c_carry = dc_carry;
+  HB_TRY(tc_scratch(ceil_div(a.N, g.RB), &p, s));
+  return launch_tc<4, false>(map, p, g, s);
 }
 
 #ifdef HASTE_B200_TIMING_EXPERIMENTS

@@ -1,5 +1,5 @@
 // Inline-PTX wrappers for the sm_100a tensor-core path shared by the contraction kernel
-// (gemm_sm100.cu) and the tensor-core recurrence kernels (rec_tc_gru.cu): mbarriers with
+// (gemm_sm100.cu) and the tensor-core recurrence kernels (rec_tc.cu): mbarriers with
 // bounded waits, TMA tile loads, tcgen05 MMA / commit / tensor-memory loads, shared-memory
 // matrix descriptors, and the host-side tensor-map encoder.
 #pragma once

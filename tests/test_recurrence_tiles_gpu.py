@@ -62,15 +62,16 @@ def test_grid_recurrence_reduced_precision(cell, dtype, tol, shape):
     _check(cell, *shape, dtype, tol, 0.25)
 
 
-# tensor-core GRU recurrence: two 64-row tiles per CTA with a ragged second one, a last slice of eight units, rings whose stage
+# tensor-core recurrence: two 64-row tiles per CTA with a ragged second one, a last slice of eight units, rings whose stage
 # count is no multiple of the issuers, fewer k-blocks than issuers have turns
 @pytest.mark.parametrize("T,N,H,sms", [(40, 90, 1024, 74), (40, 65, 1024, 74), (60, 128, 768, 74), (8, 700, 320, 0),
                                         (20, 90, 1000, 74), (8, 700, 328, 0), (12, 130, 808, 74)])
-def test_tensor_core_gru_tiles(T, N, H, sms):
+@pytest.mark.parametrize("cell", ["lstm", "gru"])
+def test_tensor_core_tiles(cell, T, N, H, sms):
     from haste_b200 import _C
     _C.set_sm_budget(sms)
     try:
-        _check("gru", T, N, H, torch.bfloat16, TOL_BF16, 0.25, transposed=N % 4 == 0)
+        _check(cell, T, N, H, torch.bfloat16, TOL_BF16, 0.25, transposed=N % 4 == 0)
         _C.sync_check(torch.cuda.current_stream().cuda_stream)
     finally:
         _C.set_sm_budget(0)
