@@ -1143,15 +1143,13 @@ int run_ln_fwd(LnFwdParams& p, const Geometry& g, cudaStream_t s) {
       return launch_coop(ln_fwd_kernel<G, KSW, SPLIT, 1, T>, grid, smem_for(KSW), &p, s);    \
     return launch_coop(ln_fwd_kernel<G, KSW, SPLIT, 4, T>, grid, smem_for(KSW), &p, s);      \
   }
-  HB_FWD(1)
-  HB_FWD(2)
-  HB_FWD(4)
+  HB_FWD(4)  // (up to 256 units the cluster kernels take every shape)
   if constexpr (SPLIT == 1) { HB_FWD(8) }
 #undef HB_FWD
   return HASTE_B200_ERR_UNSUPPORTED;
 }
 
-inline int ntw_pad(int ntw) { return ntw <= 1 ? 1 : ntw <= 2 ? 2 : ntw <= 4 ? 4 : ntw <= 8 ? 8 : 16; }
+inline int ntw_pad(int ntw) { return ntw <= 8 ? 8 : 16; }
 
 template <int G, int SPLIT, typename T>
 int run_ln_bwd(LnBwdParams& p, const Geometry& g, cudaStream_t s) {
@@ -1165,9 +1163,6 @@ int run_ln_bwd(LnBwdParams& p, const Geometry& g, cudaStream_t s) {
       return launch_coop(ln_bwd_kernel<G, NTW, SPLIT, 1, T>, grid, smem, &p, s);      \
     return launch_coop(ln_bwd_kernel<G, NTW, SPLIT, 4, T>, grid, smem, &p, s);        \
   }
-  HB_BWD(1)
-  HB_BWD(2)
-  HB_BWD(4)
   HB_BWD(8)
   if constexpr (SPLIT == 1) { HB_BWD(16) }
 #undef HB_BWD
