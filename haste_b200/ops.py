@@ -48,6 +48,22 @@ def _check(*tensors):
             raise RuntimeError("haste_b200: all tensors must share one device and dtype")
 
 
+def _sizes(T, N, C, H, G, kernel, recurrent, bias, mask, steps=(), **others):
+    """The library takes pointers and sizes, so what the tensors hold is checked here: G gates,
+    `bias` [G*H] each, `steps` [T+1,N,H], `others` name=(tensor, values); the mask and `others` may
+    be empty.  (Initial states are copied with torch, which checks them itself.)"""
+    want = [("kernel", kernel, C * G * H), ("recurrent weights", recurrent, H * G * H if G > 1 else H)]
+    want += [("bias", t, G * H) for t in bias]
+    want += [("sequence", t, (T + 1) * N * H) for t in steps]
+    if mask is not None:
+        others["zoneout mask"] = mask, T * N * H
+    want += [(name, t, n) for name, (t, n) in others.items() if t.numel()]
+    for name, t, n in want:
+        if t.numel() != n:
+            raise RuntimeError(f"haste_b200: {name} must hold {n} values for an input of {T} steps, "
+                               f"{N} rows and {C} columns, got {tuple(t.shape)}")
+
+
 def _p(t):
     return None if t is None or t.numel() == 0 else t.data_ptr()
 
@@ -59,6 +75,11 @@ def _stream():
 def _mask_ptr(zoneout_prob, mask):
     has = bool(zoneout_prob) and mask is not None and mask.numel() > 0
     return (mask.data_ptr() if has else None), (float(zoneout_prob) if has else 0.0)
+
+
+def _read(training, zoneout_prob, mask):
+    """The mask where the forward pass reads it."""
+    return mask if training and zoneout_prob else None
 
 
 def _zeros(grads, like, *shape):
@@ -88,6 +109,7 @@ def _dims_bwd(x, transposed, H):
 def lstm_forward(training, zoneout_prob, x, h0, c0, kernel, recurrent_kernel, bias, zoneout_mask):
     _check(x, h0, c0, kernel, recurrent_kernel, bias, zoneout_mask)
     T, N, C, H = _dims_fwd(x, recurrent_kernel)
+    _sizes(T, N, C, H, 4, kernel, recurrent_kernel, [bias], _read(training, zoneout_prob, zoneout_mask))
     with torch.cuda.device(x.device):
         h = x.new_empty(T + 1, N, H)
         c = x.new_empty(T + 1, N, H)
@@ -107,6 +129,8 @@ def lstm_backward(x, kernel, recurrent_kernel, bias, zoneout_mask, h, c, cache, 
     _check(x, kernel, recurrent_kernel, bias, zoneout_mask, h, c, cache, dh_new, dc_new)
     H = h.shape[2]
     T, N, C, H = _dims_bwd(x, transposed, H)
+    _sizes(T, N, C, H, 4, kernel, recurrent_kernel, [], zoneout_mask,
+           [h, c, dh_new, dc_new], cache=(cache, T * N * 4 * H))
     with torch.cuda.device(h.device):
         dx = h.new_empty(T, N, C)
         dW = _zeros(grads, h, C, 4 * H)
@@ -145,6 +169,7 @@ def lstm_forward_from_host(training, zoneout_prob, x_host, h0, c0, kernel, recur
         raise RuntimeError("haste_b200: x_host must be a pinned CPU tensor")
     T, N, C = x_host.shape
     H = recurrent_kernel.shape[0]
+    _sizes(T, N, C, H, 4, kernel, recurrent_kernel, [bias], _read(training, zoneout_prob, zoneout_mask))
     dev = h0.device
     with torch.cuda.device(dev):
         main = torch.cuda.current_stream()
@@ -209,6 +234,8 @@ def lstm_backward_from_host(x, kernel, recurrent_kernel, bias, zoneout_mask, h, 
     T, N, C = x.shape
     H = h.shape[2]
     dev = h.device
+    _sizes(T, N, C, H, 4, kernel, recurrent_kernel, [], zoneout_mask,
+           [h, c, dh_new_host, dc_new], cache=(cache, T * N * 4 * H))
     with torch.cuda.device(dev):
         main = torch.cuda.current_stream()
         side = _copy_streams.get(dev.index)
@@ -260,6 +287,8 @@ def gru_forward(training, zoneout_prob, x, h0, kernel, recurrent_kernel, bias, r
                 zoneout_mask):
     _check(x, h0, kernel, recurrent_kernel, bias, recurrent_bias, zoneout_mask)
     T, N, C, H = _dims_fwd(x, recurrent_kernel)
+    _sizes(T, N, C, H, 3, kernel, recurrent_kernel, [bias, recurrent_bias],
+           _read(training, zoneout_prob, zoneout_mask))
     with torch.cuda.device(x.device):
         h = x.new_empty(T + 1, N, H)
         h[0] = h0
@@ -278,6 +307,8 @@ def gru_backward(x, kernel, recurrent_kernel, bias, recurrent_bias, zoneout_mask
     _check(x, kernel, recurrent_kernel, bias, recurrent_bias, zoneout_mask, h, cache, dh_new)
     H = h.shape[2]
     T, N, C, H = _dims_bwd(x, transposed, H)
+    _sizes(T, N, C, H, 3, kernel, recurrent_kernel, [], zoneout_mask,
+           [h, dh_new], cache=(cache, T * N * 4 * H))
     with torch.cuda.device(h.device):
         dx = h.new_empty(T, N, C)
         dW = _zeros(grads, h, C, 3 * H)
@@ -299,6 +330,7 @@ def indrnn_forward(training, zoneout_prob, x, h0, kernel, recurrent_scale, bias,
     _check(x, h0, kernel, recurrent_scale, bias, zoneout_mask)
     T, N, C = x.shape
     H = kernel.shape[1]
+    _sizes(T, N, C, H, 1, kernel, recurrent_scale, [bias], _read(training, zoneout_prob, zoneout_mask))
     with torch.cuda.device(x.device):
         h = x.new_empty(T + 1, N, H)
         h[0] = h0
@@ -313,6 +345,7 @@ def indrnn_backward(x, kernel, recurrent_scale, bias, zoneout_mask, h, dh_new, t
     _check(x, kernel, recurrent_scale, bias, zoneout_mask, h, dh_new)
     H = h.shape[2]
     T, N, C, H = _dims_bwd(x, transposed, H)
+    _sizes(T, N, C, H, 1, kernel, recurrent_scale, [], zoneout_mask, [h, dh_new])
     with torch.cuda.device(h.device):
         dx = h.new_empty(T, N, C)
         dW = _zeros(grads, h, C, H)
@@ -331,6 +364,8 @@ def layer_norm_lstm_forward(training, zoneout_prob, x, h0, c0, kernel, recurrent
                             gamma, gamma_h, beta_h, zoneout_mask, saved_dtype=torch.float32):
     _check(x, h0, c0, kernel, recurrent_kernel, bias, gamma, gamma_h, beta_h, zoneout_mask)
     T, N, C, H = _dims_fwd(x, recurrent_kernel)
+    _sizes(T, N, C, H, 4, kernel, recurrent_kernel, [bias], _read(training, zoneout_prob, zoneout_mask),
+           gamma=(gamma, 8 * H), gamma_h=(gamma_h, H), beta_h=(beta_h, H))
     with torch.cuda.device(x.device):
         h = x.new_empty(T + 1, N, H)
         c = x.new_empty(T + 1, N, H)
@@ -367,6 +402,13 @@ def layer_norm_lstm_backward(x, kernel, recurrent_kernel, bias, gamma, gamma_h, 
     _check(act_Wx, act_Wx_norm, cache_Wx, act_Rh, cache_Rh, act_c_norm, cache_c)
     H = h.shape[2]
     T, N, C, H = _dims_bwd(x, transposed, H)
+    rows = T * N
+    _sizes(T, N, C, H, 4, kernel, recurrent_kernel, [], zoneout_mask,
+           [h, c, dh_new, dc_new], gamma=(gamma, 8 * H), gamma_h=(gamma_h, H), beta_h=(beta_h, H),
+           act_Wx=(act_Wx, rows * 4 * H), act_Wx_norm=(act_Wx_norm, rows * 4 * H),
+           cache_Wx=(cache_Wx, rows * 2), act_Rh=(act_Rh, rows * 4 * H),
+           cache_Rh=(cache_Rh, rows * 2), act_c_norm=(act_c_norm, rows * H),
+           cache_c=(cache_c, rows * 2))
     with torch.cuda.device(h.device):
         dx = h.new_empty(T, N, C)
         dW = _zeros(grads, h, C, 4 * H)
@@ -392,6 +434,9 @@ def layer_norm_gru_forward(training, zoneout_prob, x, h0, kernel, recurrent_kern
                            recurrent_bias, gamma, zoneout_mask):
     _check(x, h0, kernel, recurrent_kernel, bias, recurrent_bias, gamma, zoneout_mask)
     T, N, C, H = _dims_fwd(x, recurrent_kernel)
+    _sizes(T, N, C, H, 3, kernel, recurrent_kernel, [bias, recurrent_bias],
+           _read(training, zoneout_prob, zoneout_mask),
+           gamma=(gamma, 6 * H))
     with torch.cuda.device(x.device):
         h = x.new_empty(T + 1, N, H)
         h[0] = h0
@@ -418,6 +463,11 @@ def layer_norm_gru_backward(x, kernel, recurrent_kernel, bias, recurrent_bias, g
            act_Wx, cache_Wx, act_Rh, cache_Rh, dh_new)
     H = h.shape[2]
     T, N, C, H = _dims_bwd(x, transposed, H)
+    rows = T * N
+    _sizes(T, N, C, H, 3, kernel, recurrent_kernel, [], zoneout_mask,
+           [h, dh_new], gamma=(gamma, 6 * H), cache=(cache, rows * 4 * H),
+           act_Wx=(act_Wx, rows * 3 * H), cache_Wx=(cache_Wx, rows * 2),
+           act_Rh=(act_Rh, rows * 3 * H), cache_Rh=(cache_Rh, rows * 2))
     with torch.cuda.device(h.device):
         dx = h.new_empty(T, N, C)
         dW = _zeros(grads, h, C, 3 * H)
@@ -443,6 +493,9 @@ def layer_norm_indrnn_forward(training, zoneout_prob, x, h0, kernel, recurrent_s
     _check(x, h0, kernel, recurrent_scale, bias, gamma, zoneout_mask)
     T, N, C = x.shape
     H = kernel.shape[1]
+    _sizes(T, N, C, H, 1, kernel, recurrent_scale, [bias], _read(training, zoneout_prob, zoneout_mask))
+    if gamma.numel() < H:
+        raise RuntimeError(f"haste_b200: gamma must hold {H} values, got {tuple(gamma.shape)}")
     with torch.cuda.device(x.device):
         h = x.new_empty(T + 1, N, H)
         h[0] = h0
@@ -462,6 +515,10 @@ def layer_norm_indrnn_backward(x, kernel, recurrent_scale, bias, gamma, zoneout_
     _check(x, kernel, recurrent_scale, bias, gamma, zoneout_mask, h, act_Wx, cache_Wx, dh_new)
     H = h.shape[2]
     T, N, C, H = _dims_bwd(x, transposed, H)
+    _sizes(T, N, C, H, 1, kernel, recurrent_scale, [], zoneout_mask, [h, dh_new],
+           act_Wx=(act_Wx, T * N * H), cache_Wx=(cache_Wx, T * N * 2))
+    if gamma.numel() < H:
+        raise RuntimeError(f"haste_b200: gamma must hold {H} values, got {tuple(gamma.shape)}")
     with torch.cuda.device(h.device):
         dx = h.new_empty(T, N, C)
         dW = _zeros(grads, h, C, H)

@@ -114,6 +114,45 @@ void check(const Tensor& x, at::ArrayRef<Tensor> ts) {
   }
 }
 
+// (Numbers are put into messages with std::to_string: an ostream of this object may meet the locale
+// of another copy of the C++ library.)
+std::string shape_of(const Tensor& t) {
+  std::string s = "[";
+  for (int64_t n : t.sizes()) s += (s.size() > 1 ? "," : "") + std::to_string(n);
+  return s + "]";
+}
+
+// The library takes pointers and sizes, so what the tensors hold has to be said here: x [T,N,C] with
+// the layer's weights, and the mask where it is read.  (The states are checked where they are taken.)
+void check_sizes(int cell, const Tensor& x, int64_t H, const std::vector<Tensor>& P, const Tensor* mask) {
+  static const int kGates[] = {4, 3, 1, 4, 3, 1};
+  const int64_t GH = kGates[cell] * H, C = x.size(2);
+  auto wrong = [&](const Tensor& t, const char* name, const std::string& want) {
+    TORCH_CHECK(false, "haste_b200: " + std::string(name) + " must be " + want + " for an input " + shape_of(x) +
+                           " and " + std::to_string(H) + " units, got " + shape_of(t));
+  };
+  auto matrix = [&](const Tensor& t, const char* name, int64_t rows, int64_t cols) {
+    if (t.dim() != 2 || t.size(0) != rows || t.size(1) != cols)
+      wrong(t, name, "[" + std::to_string(rows) + "," + std::to_string(cols) + "]");
+  };
+  auto holds = [&](const Tensor& t, const char* name, int64_t n) {
+    if (t.numel() != n) wrong(t, name, std::to_string(n) + " values");
+  };
+  matrix(P[0], "kernel", C, GH);
+  if (GH != H) matrix(P[1], "recurrent kernel", H, GH);
+  else holds(P[1], "recurrent scale", H);
+  holds(P[2], "bias", GH);
+  if (cell == GRU || cell == LN_GRU) holds(P[3], "recurrent bias", GH);
+  if (cell == LN_LSTM) {
+    holds(P[3], "gamma", 2 * GH);
+    holds(P[4], "gamma_h", H);
+    holds(P[5], "beta_h", H);
+  }
+  if (cell == LN_GRU) holds(P[4], "gamma", 2 * GH);
+  if (cell == LN_INDRNN && P[3].numel() < H) wrong(P[3], "gamma", "[2,H]");  // only its first row is read
+  if (mask && mask->defined() && mask->numel()) holds(*mask, "zoneout mask", x.size(0) * x.size(1) * H);
+}
+
 struct Dims { int T, N, C, H; };
 
 // A sequence [T,N,H] with room for the state before it: slot 0 of the buffer, filled with `s0` or
@@ -350,6 +389,7 @@ std::tuple<Tensor, Tensor, c10::optional<Tensor>> forward(
     int cell, Tensor x, const c10::optional<Tensor>& h0_, const c10::optional<Tensor>& c0_,
     const c10::optional<Tensor>& lengths, std::vector<Tensor> params, const c10::optional<Tensor>& mask_, bool training,
     double zoneout, bool batch_first, bool state_sequence, int budget) {
+  TORCH_CHECK(x.dim() == 3, "haste_b200: input must have three dimensions, got " + shape_of(x));
   if (batch_first) x = x.transpose(0, 1);
   x = x.contiguous();
   const int64_t T = x.size(0), N = x.size(1);
@@ -369,6 +409,7 @@ std::tuple<Tensor, Tensor, c10::optional<Tensor>> forward(
   }
   check(x, params);
   check(x, {h0, c0, mask});
+  check_sizes(cell, x, H, params, training && zoneout != 0.0 ? &mask : nullptr);
   const c10::cuda::CUDAGuard guard(x.device());
   const SmBudget sm(budget);
   Tensor y, c;
