@@ -156,8 +156,7 @@ void check_sizes(int cell, const Tensor& x, int64_t H, const std::vector<Tensor>
 struct Dims { int T, N, C, H; };
 
 // A sequence [T,N,H] with room for the state before it: slot 0 of the buffer, filled with `s0` or
-// zeros.  The returned tensor starts at slot 1 (and is no view of the buffer to autograd, which
-// checks its version like that of any other output).
+// zeros.  The returned tensor starts at slot 1 and is no view of the buffer to autograd.
 Tensor sequence(const Dims& d, const Tensor& like, const Tensor& s0, cudaStream_t stream) {
   const int64_t slot = (int64_t)d.N * d.H;
   Tensor buf = at::empty({d.T + 1, d.N, d.H}, like.options());
@@ -171,6 +170,16 @@ Tensor sequence(const Dims& d, const Tensor& like, const Tensor& s0, cudaStream_
 // Start of the buffer behind a tensor of sequence().
 void* slot0(const Tensor& y) {
   return static_cast<char*>(y.data_ptr()) - y.size(1) * y.size(2) * y.element_size();
+}
+// The whole buffer [T+1,N,H] behind a tensor of sequence(), as the backward pass keeps it: slot 0 is
+// part of what saved-tensor hooks (offloading, checkpointing) copy, and the version counter is that
+// of `y`, so that a change of the output in place is noticed.
+Tensor whole(const Tensor& y) {
+  Tensor buf = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(y.storage()), y.key_set(), y.dtype());
+  c10::TensorImpl* impl = buf.unsafeGetTensorImpl();
+  impl->set_sizes_and_strides(c10::IntArrayRef{y.size(0) + 1, y.size(1), y.size(2)}, y.strides(), 0);
+  impl->set_version_counter(y.unsafeGetTensorImpl()->version_counter());
+  return buf;
 }
 
 struct Forward {
@@ -255,10 +264,10 @@ Forward run_forward(int cell, bool training, double zoneout, const Tensor& x, co
 
 // Incoming gradient of a sequence as the library takes it: a pointer one slot before it (the library
 // never reads that slot).  Undefined: `zero` makes it zeros, else null.
-void* incoming(Tensor& g, const Tensor& y, bool zero) {
+void* incoming(Tensor& g, const Tensor& hs, bool zero) {
   if (!g.defined()) {
     if (!zero) return nullptr;
-    g = at::zeros(y.sizes(), y.options());
+    g = at::zeros({hs.size(0) - 1, hs.size(1), hs.size(2)}, hs.options());
   }
   g = g.contiguous();
   return slot0(g);
@@ -270,10 +279,15 @@ struct RnnNode : public torch::autograd::Function<RnnNode> {
                                c10::optional<Tensor> mask_, at::TensorList params) {
     const Tensor mask = mask_.value_or(Tensor());
     Forward f = run_forward((int)cell, training, zoneout, x, h0.value_or(Tensor()), c0.value_or(Tensor()), mask, params);
-    variable_list save = {x, mask, f.y};
-    if (f.c.defined()) save.push_back(f.c);
+    variable_list save = {x, mask, whole(f.y)};
+    if (f.c.defined()) save.push_back(whole(f.c));
     for (const Tensor& t : params) save.push_back(t);
-    for (const Tensor& t : f.saved) save.push_back(t);
+    int64_t kept = 0;
+    for (const Tensor& t : f.saved) {
+      save.push_back(t);
+      kept += t.defined() ? t.numel() : 0;
+    }
+    ctx->saved_data["kept"] = kept;
     ctx->save_for_backward(std::move(save));
     ctx->saved_data["cell"] = cell;
     ctx->saved_data["training"] = training;
@@ -306,18 +320,31 @@ struct RnnNode : public torch::autograd::Function<RnnNode> {
     const SmBudget sm((int)ctx->saved_data["budget"].toInt());
     const size_t np = (size_t)ctx->saved_data["params"].toInt();
     variable_list sv = ctx->get_saved_variables();
-    const Tensor x = sv[0], mask = sv[1], y = sv[2];
+    for (Tensor& t : sv)  // hooks may hand back tensors of their own
+      if (t.defined()) t = t.contiguous();
+    const Tensor x = sv[0], mask = sv[1], hs = sv[2];
     size_t i = 3;
     const Tensor cs = has_c(cell) ? sv[i++] : Tensor();
     const variable_list P(sv.begin() + i, sv.begin() + i + np);
     const variable_list S(sv.begin() + i + np, sv.end());
+    const int T = (int)x.size(0), N = (int)x.size(1), C = (int)x.size(2), H = (int)hs.size(2);
+    check(x, P);
+    check(x, {mask, hs, cs});
+    check_sizes(cell, x, H, P, &mask);
+    const int64_t values = (int64_t)(T + 1) * N * H;
+    bool same = hs.numel() == values && (!cs.defined() || cs.numel() == values);
+    int64_t kept = 0;
+    for (const Tensor& t : S) {
+      kept += t.defined() ? t.numel() : 0;
+      same &= !t.defined() || (t.device() == x.device() && t.dtype() == saved_options(x, cell).dtype());
+    }
+    TORCH_CHECK(same && kept == ctx->saved_data["kept"].toInt(), "haste_b200: a saved tensor has changed its kind");
     const c10::cuda::CUDAGuard guard(x.device());
     void* s = (void*)c10::cuda::getCurrentCUDAStream().stream();
-    const int T = (int)x.size(0), N = (int)x.size(1), C = (int)x.size(2), H = (int)y.size(2);
     const auto o = x.options();
     const int dt = lib_dtype(x, cell);
-    void* gh = incoming(grad[0], y, true);
-    void* gc = has_c(cell) ? incoming(grad[1], cs, false) : nullptr;
+    void* gh = incoming(grad[0], hs, true);
+    void* gc = has_c(cell) ? incoming(grad[1], hs, false) : nullptr;
     const bool want_x = cell == LN_LSTM || cell == LN_GRU || ctx->needs_input_grad(0);
     Tensor dx = want_x ? at::empty(x.sizes(), o) : Tensor();
     Tensor dh = at::empty({N, H}, o), dc = has_c(cell) ? at::empty({N, H}, o) : Tensor();
@@ -326,20 +353,20 @@ struct RnnNode : public torch::autograd::Function<RnnNode> {
     const AssignGradients assign;
     switch (cell) {
       case LSTM:
-        CALL(lstm_backward, dt, 0, T, N, C, H, ptr(P[0]), ptr(P[1]), ptr(P[2]), ptr(x), slot0(y), slot0(cs), gh,
+        CALL(lstm_backward, dt, 0, T, N, C, H, ptr(P[0]), ptr(P[1]), ptr(P[2]), ptr(x), ptr(hs), ptr(cs), gh,
                                     gc, ptr(dx), ptr(D[0]), ptr(D[1]), ptr(D[2]), ptr(dh), ptr(dc), ptr(S[0]), ptr(mask),
                                     s);
         break;
       case GRU: {
         Tensor dp = at::empty({T, N, 3 * H}, o), dq = at::empty({T, N, 3 * H}, o);
-        CALL(gru_backward, dt, 0, T, N, C, H, ptr(P[0]), ptr(P[1]), ptr(P[2]), ptr(P[3]), ptr(x), slot0(y),
+        CALL(gru_backward, dt, 0, T, N, C, H, ptr(P[0]), ptr(P[1]), ptr(P[2]), ptr(P[3]), ptr(x), ptr(hs),
                                    ptr(S[0]), gh, ptr(dx), ptr(D[0]), ptr(D[1]), ptr(D[2]), ptr(D[3]), ptr(dh), ptr(dp),
                                    ptr(dq), ptr(mask), s);
         break;
       }
       case INDRNN: {
         Tensor ws = at::empty({T, N, H}, o);
-        CALL(indrnn_backward, dt, 0, T, N, C, H, ptr(P[0]), ptr(P[1]), ptr(P[2]), ptr(x), slot0(y), gh, ptr(dx),
+        CALL(indrnn_backward, dt, 0, T, N, C, H, ptr(P[0]), ptr(P[1]), ptr(P[2]), ptr(x), ptr(hs), gh, ptr(dx),
                                       ptr(D[0]), ptr(D[1]), ptr(D[2]), ptr(dh), ptr(ws), ptr(mask), s);
         break;
       }
@@ -347,7 +374,7 @@ struct RnnNode : public torch::autograd::Function<RnnNode> {
         const size_t row = (size_t)4 * H * P[3].element_size();
         char *g = static_cast<char*>(P[3].data_ptr()), *dg = static_cast<char*>(D[3].data_ptr());
         CALL(layer_norm_lstm_backward, dt, 0, T, N, C, H, ptr(P[0]), ptr(P[1]), ptr(P[2]), g, g + row, ptr(P[4]),
-                                               ptr(P[5]), ptr(x), slot0(y), slot0(cs), gh, gc, ptr(dx), ptr(D[0]),
+                                               ptr(P[5]), ptr(x), ptr(hs), ptr(cs), gh, gc, ptr(dx), ptr(D[0]),
                                                ptr(D[1]), ptr(D[2]), dg, dg + row, ptr(D[4]), ptr(D[5]), ptr(dh), ptr(dc),
                                                ptr(S[0]), ptr(S[1]), ptr(S[2]), ptr(S[3]), ptr(S[4]), ptr(S[5]),
                                                ptr(S[6]), ptr(mask), s);
@@ -358,7 +385,7 @@ struct RnnNode : public torch::autograd::Function<RnnNode> {
         const size_t row = (size_t)3 * H * P[4].element_size();
         char *g = static_cast<char*>(P[4].data_ptr()), *dg = static_cast<char*>(D[4].data_ptr());
         CALL(layer_norm_gru_backward, dt, 0, T, N, C, H, ptr(P[0]), ptr(P[1]), ptr(P[2]), ptr(P[3]), g, g + row,
-                                              ptr(x), slot0(y), ptr(S[0]), gh, ptr(dx), ptr(D[0]), ptr(D[1]), ptr(D[2]),
+                                              ptr(x), ptr(hs), ptr(S[0]), gh, ptr(dx), ptr(D[0]), ptr(D[1]), ptr(D[2]),
                                               ptr(D[3]), dg, dg + row, ptr(dh), ptr(dp), ptr(dq), ptr(S[1]), ptr(S[2]),
                                               ptr(S[3]), ptr(S[4]), ptr(mask), s);
         break;
@@ -368,7 +395,7 @@ struct RnnNode : public torch::autograd::Function<RnnNode> {
         // gamma is [2,H]; its second row takes no part and has a zero gradient
         cuda_ok(cudaMemsetAsync(D[3].data_ptr(), 0, D[3].numel() * D[3].element_size(), (cudaStream_t)s));
         CALL(layer_norm_indrnn_backward, dt, 0, T, N, C, H, ptr(P[0]), ptr(P[1]), ptr(P[2]), ptr(P[3]), ptr(x),
-                                                 slot0(y), gh, ptr(dx), ptr(D[0]), ptr(D[1]), ptr(D[2]), ptr(D[3]),
+                                                 ptr(hs), gh, ptr(dx), ptr(D[0]), ptr(D[1]), ptr(D[2]), ptr(D[3]),
                                                  ptr(dh), ptr(ws), ptr(S[0]), ptr(S[1]), ptr(mask), s);
       }
     }
