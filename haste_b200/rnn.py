@@ -17,6 +17,7 @@ Differences, all additive:
   * The layers run on CUDA only; there is no CPU fallback.
 """
 import torch
+import torch.autograd.forward_ad as _forward_ad
 import torch.nn as nn
 import torch.nn.functional as F
 
@@ -30,6 +31,7 @@ def _empty_mask(x):
 
 
 _native_forward = None
+_tracing_state = torch._C._get_tracing_state
 
 
 def _load_native():
@@ -303,11 +305,13 @@ class BaseRNN(nn.Module):
         return R * scale
 
     def _native_applies(self, input, lengths):
-        """The compiled host path takes every call but three: with a data-parallel hook the
+        """The compiled host path takes every call but a few: with a data-parallel hook the
         gradients go to its bucket, `lengths` with gradients index the state slots, and an empty
-        input returns its initial state."""
+        input returns its initial state.  Nor does it show the tracer and forward-mode AD what it
+        does: there the autograd functions say what can be recorded or differentiated."""
         return (self._dp is None and (lengths is None or not torch.is_grad_enabled())
-                and input.numel() > 0)
+                and input.numel() > 0 and _forward_ad._current_level < 0
+                and _tracing_state() is None)
 
     def _native_call(self, input, state, lengths, zoneout_mask=None, dropconnect_mask=None):
         """One call of the layer through torch_ext/native.cc.  A small batch's call is bound by
