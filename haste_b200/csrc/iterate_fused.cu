@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(IT_THREADS, 1) step_fma_kernel(const StepParam
   const Share sh(p, cluster);
   extern __shared__ __align__(16) float smem[];
   float* red = smem;
-  float* xs = smem + PARTS * kSlots * RB * U;  // [k][row]
+  float* xs = smem + PARTS * kSlots * RB * U;  // [k][row], and a line of zeros behind the last k
   const int N = p.N, C = p.C, H = p.H;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int u0 = (blockIdx.x / sh.KS) * U;
@@ -194,13 +194,13 @@ __global__ void __launch_bounds__(IT_THREADS, 1) step_fma_kernel(const StepParam
       }
     };
     fetch(first);  // on its way while x and h are staged
-    for (int kk = tid; kk < n_k; kk += IT_THREADS) {
+    for (int kk = tid; kk <= n_k; kk += IT_THREADS) {
       const int k = c0 + kk;
       float a[RB];
 #pragma unroll
       for (int row = 0; row < RB; ++row) {
         a[row] = 0.f;
-        if (row < N)
+        if (row < N && kk < n_k)
           a[row] = k < nx ? ld(x + (long long)row * C + sh.x0 + k) : ld(hp + (long long)row * H + sh.h0 + k - nx);
       }
 #pragma unroll
@@ -211,7 +211,8 @@ __global__ void __launch_bounds__(IT_THREADS, 1) step_fma_kernel(const StepParam
       if (kb != first) fetch(kb);
 #pragma unroll
       for (int e = 0; e < UNR; ++e) {
-        const int kk = min(kb + e * KR * PARTS, hi - 1);  // beyond the end the weights are zeros
+        int kk = kb + e * KR * PARTS;
+        if (kk >= hi) kk = n_k;  // zeros, like the weights
         float a[RB];
         if constexpr (RB == 4) {
           const float4 t = *reinterpret_cast<const float4*>(xs + kk * RB);
@@ -428,15 +429,45 @@ __global__ void __launch_bounds__(IT_THREADS, 1) step_mma_kernel(const StepParam
       }
     }
   }
-  // accumulator: units lane / 4 (+ 8), rows 2 * (lane % 4) (+ 1)
-  const int unit = mt * 16 + (lane >> 2), r0 = 2 * (lane & 3);
+  // An infinity, or a value that bf16 rounds to one, leaves inf - inf in the lower planes where the
+  // FMA form saturates the gate: a CTA that finds a sum not finite adds up its share again as that
+  // form does.
+  bool again = false;
+  if constexpr (P > 1) {
+    bool finite = true;
 #pragma unroll
-  for (int n = 0; n < NT; ++n) {
-    float* to = red + ((kp * kSlots + slot) * ROWS + n * 8 + r0) * U + unit;
-    to[0] = acc[n][0];
-    to[U] = acc[n][1];
-    to[8] = acc[n][2];
-    to[U + 8] = acc[n][3];
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) finite = finite && fabsf(acc[n][i]) <= 3.402823466e38f;
+    again = __syncthreads_or(!finite) != 0;
+    if (again) {
+      constexpr int SUMS = kSlots * ROWS * U;
+      for (int i = tid; i < SUMS; i += IT_THREADS) {
+        const int sl = i / (ROWS * U), row = i / U % ROWS, j = u0 + i % U, col = (GRU && sl == 3 ? 2 : sl) * H + j;
+        float sum = 0.f;
+        if (row < N && j < H) {
+          if (!GRU || sl != 3)
+            for (int k = sh.x0; k < sh.x0 + nx; ++k) sum = fmaf(x[(long long)row * C + k], W[(long long)k * G * H + col], sum);
+          if (!GRU || sl != 2)
+            for (int k = sh.h0; k < sh.h0 + sh.nh; ++k)
+              sum = fmaf(hp[(long long)row * H + k], R[(long long)k * G * H + col], sum);
+        }
+        red[i] = sum;
+        for (int part = 1; part < PARTS; ++part) red[part * SUMS + i] = 0.f;
+      }
+    }
+  }
+  if (!again) {
+    // accumulator: units lane / 4 (+ 8), rows 2 * (lane % 4) (+ 1)
+    const int unit = mt * 16 + (lane >> 2), r0 = 2 * (lane & 3);
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      float* to = red + ((kp * kSlots + slot) * ROWS + n * 8 + r0) * U + unit;
+      to[0] = acc[n][0];
+      to[U] = acc[n][1];
+      to[8] = acc[n][2];
+      to[U + 8] = acc[n][3];
+    }
   }
   finish<T, GRU, U>(p, cluster, sh, red, PARTS, u0);
 }
@@ -474,7 +505,7 @@ int launch_step_v(StepParams& p, cudaStream_t s) {
   if (p.N <= IT_FMA_ROWS) {
     p.rows = p.N == 1 ? 1 : 4;
     p.chunk = std::min(ceil_div(p.C, KS) + ceil_div(p.H, KS), IT_XS_BYTES / (p.rows * 4));
-    const size_t smem = (size_t)(4 * kSlots * p.rows * U + p.chunk * p.rows) * sizeof(float);
+    const size_t smem = (size_t)(4 * kSlots * p.rows * U + (p.chunk + 1) * p.rows) * sizeof(float);
     return launch(p.N == 1 ? step_fma_kernel<T, GRU, 1, VEC> : step_fma_kernel<T, GRU, 4, VEC>, p, groups, KS, smem, s);
   }
   const int nt = p.N <= 8 ? 1 : (p.N <= 16 ? 2 : (p.N <= 32 ? 4 : 8));

@@ -180,3 +180,42 @@ def test_single_step_sizes(cell, N, C, H, dtype):
     tol = 3e-6 if dtype == torch.float32 else 1e-2
     for a, ref in zip(got, want):
         torch.testing.assert_close(a.double(), ref, rtol=tol, atol=tol)
+
+
+@pytest.mark.parametrize("where", ["input", "weight"])
+@pytest.mark.parametrize("N,C,H", [(1, 300, 40), (3, 40, 64), (5, 300, 33), (8, 16, 250), (33, 130, 64), (64, 40, 48)])
+@pytest.mark.parametrize("cell", ["LSTM", "GRU"])
+def test_single_step_with_infinite_values(cell, N, C, H, where):
+    """fp32: an infinity, or a value beyond bf16, saturates its gates whatever the batch, and what it
+    does not touch stays as exact as ever."""
+    import haste_b200
+    torch.manual_seed(N + H)
+    layer = getattr(haste_b200, cell)(C, H).cuda().eval()
+    x = torch.randn(1, N, C, device="cuda")
+    state = torch.randn(1, N, H, device="cuda")
+    state = (state, torch.randn_like(state)) if cell == "LSTM" else state
+    with torch.no_grad():
+        if where == "input":
+            x[0, N // 2, 7], x[0, N - 1, C - 1] = 3.4e38, float("-inf")
+            x[0, 0, 3] = float("inf")
+            if N == 1:
+                x[0, 0, :C - 1] = torch.randn(C - 1, device="cuda")
+        else:
+            layer.kernel[5, H // 2] = float("inf")
+        y, final = layer(x, state)
+        d = lambda t: t.double()
+        W, R, b = d(layer.kernel), d(layer.recurrent_kernel), d(layer.bias)
+        if cell == "LSTM":
+            h, c = d(state[0][0]), d(state[1][0])
+            i, g, f, o = (d(x[0]) @ W + h @ R + b).chunk(4, 1)
+            c = f.sigmoid() * c + i.sigmoid() * g.tanh()
+            want, got = [o.sigmoid() * c.tanh(), c], [y[0], final[1][0]]
+        else:
+            h = d(state[0])
+            zx, rx, gx = (d(x[0]) @ W + b).chunk(3, 1)
+            zh, rh, gh = (h @ R + d(layer.recurrent_bias)).chunk(3, 1)
+            z, r = (zx + zh).sigmoid(), (rx + rh).sigmoid()
+            want, got = [z * h + (1 - z) * (gx + r * gh).tanh()], [y[0]]
+    for a, ref in zip(got, want):
+        assert not ref.isnan().any()
+        torch.testing.assert_close(a.double(), ref.view_as(a), rtol=3e-6, atol=3e-6)
