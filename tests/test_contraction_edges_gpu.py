@@ -43,3 +43,18 @@ def test_column_sums_and_scans(T, N, H, dtype):
     assert_close(out["h"], ref_out["h"], tol, "h")
     for k, r in ref_g.items():
         assert_close(g[k], r, tol, "d" + k)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("M,K,N", [(8, 512, 2048), (16, 512, 2048), (24, 6400, 1024), (31, 1999, 193), (31, 67, 2051)])
+@pytest.mark.parametrize("transposed", [False, True])
+def test_few_rows_are_fp32_grade(M, K, N, transposed, dtype):
+    """Fewer than 32 rows: as exact as fp32 FMAs.  Bound: products dropped below 2^-24, fp32 sums of
+    chunks, an fp32 (fp16) result: 1e-6 (2^-11) of the result in the 2-norm; two planes leave 4e-6."""
+    torch.manual_seed(M + N)
+    a = torch.randn(K, M, device="cuda").to(dtype).t() if transposed else torch.randn(M, K, device="cuda").to(dtype)
+    b = torch.randn(K, N, device="cuda").to(dtype)
+    want = a.double() @ b.double()
+    got = ops.gemm(a, b).double()
+    bound = 1e-6 if dtype == torch.float32 else 2.0 ** -11
+    assert (got - want).norm() < bound * want.norm()
