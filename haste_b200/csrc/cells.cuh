@@ -158,9 +158,18 @@ int exchange_probe(int N, int H, int steps, float* us_per_step, cudaStream_t s);
 // Per-step contraction (M = batch rows).  Small products are launch-bound and stay on the
 // CUDA-core kernel; from 2^26 multiply-adds up the tensor-core kernel pays for its set-up
 // (operand split and tensor maps) even with a partly empty 128-row tile.
+inline bool tensor_core_step(long long M, long long N, long long K) { return M >= 32 && M * N * K >= (1LL << 26); }
 inline int gemm_small(const GemmDesc& g, cudaStream_t s) {
-  if (g.M >= 32 && (long long)g.M * g.N * g.K >= (1LL << 26)) return gemm(g, s);
-  return gemm_simt(g, s);
+  return tensor_core_step(g.M, g.N, g.K) ? gemm(g, s) : gemm_simt(g, s);
+}
+// fp32 LSTM / GRU layers of 512 to 1024 units whose step product would be fp32 FMAs if the grid
+// recurrence did not take it, with two planes: their input projection is made exact (six products), so
+// that the outputs as a whole are no less exact than by that path.  Relative error against fp64, step
+// by step / grid / grid with this: LSTM, T = 100, 16 rows, H = 640 h 4.6e-6 / 5.2e-6 / 2.4e-6, dx 5.3 /
+// 6.0 / 5.3, dR 5.4 / 6.6 / 4.6; 31 rows, H = 1024 4.6 / 5.1 / 2.4.  (The bias gradient, a sum over all
+// rows and steps, keeps the planes of R: 2.0 / 3.6 / 3.2.)  1 to 3 % of a pass, 6 % of GRU inference.
+inline int wide_few_rows(int dtype, int N, int GH, int H) {
+  return dtype == HASTE_B200_F32 && H > 512 && H <= 1024 && !tensor_core_step(N, GH, H);
 }
 
 // fp32 [rows, width] -> planes for several contractions, in the scratch the recurrence kernels would

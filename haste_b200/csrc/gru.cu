@@ -195,6 +195,7 @@ int gru_forward(const GruFwd& a, cudaStream_t s) {
   HB_REQUIRE(a.tmp_Wx && a.tmp_Rh, "null pointer");
   GemmDesc g{a.dtype, a.dtype, (int)TN, 3 * a.H, a.C, a.x, a.C, 1, a.W, 3LL * a.H, 1, a.tmp_Wx,
              3LL * a.H, 0};
+  g.precise = wide_few_rows(a.dtype, a.N, 3 * a.H, a.H);
   {
     ProfScope p(PH_PROJ, s);
     HB_TRY(gemm(g, s));

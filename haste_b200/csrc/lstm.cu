@@ -168,6 +168,7 @@ int lstm_forward(const LstmFwd& a, cudaStream_t s) {
   // v = x . W for all steps at once
   GemmDesc g{a.dtype, a.dtype, (int)TN, 4 * a.H, a.C, a.x, a.C, 1, a.W, 4LL * a.H, 1, a.v,
              4LL * a.H, 0};
+  g.precise = wide_few_rows(a.dtype, a.N, 4 * a.H, a.H);
   {
     ProfScope p(PH_PROJ, s);
     HB_TRY(gemm(g, s));
