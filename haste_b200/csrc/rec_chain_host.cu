@@ -27,12 +27,7 @@ bool aligned(std::initializer_list<const void*> ptrs, int H, int dtype) {
 // 90 rows, twelve, 8.1 / 6.4).
 constexpr int kGridChains = 12, kGruChainsBeforeTc = 6, kLstmChainsBeforeTc = 8;
 
-// A handful of steps of a wide fp32 / fp16 layer stays on the step-wise path (as
-// tests/test_parity_gpu.py expects of it).
-constexpr int kWideSteps = 8;
-
-bool gl_geometry(int dtype, int T, int N, int H, int most, GlGeometry* g) {
-  if (dtype != HASTE_B200_BF16 && H > 512 && T < kWideSteps) return false;
+bool gl_geometry(int dtype, int N, int H, int most, GlGeometry* g) {
   g->KS16 = ceil_div(H, 16);
   const int ks = ceil_div(g->KS16, GL_WARPS);
   if (ks > 8) return false;
@@ -92,7 +87,7 @@ int run_fwd(ChainParams& p, int dtype, int grid_most, ClRun cl, GlRun gl, cudaSt
     if (st_ != HASTE_B200_ERR_UNSUPPORTED) return st_;
   }
   GlGeometry g;
-  if (!gl_geometry(dtype, p.T, p.N, p.H, grid_most, &g)) return HASTE_B200_ERR_UNSUPPORTED;
+  if (!gl_geometry(dtype, p.N, p.H, grid_most, &g)) return HASTE_B200_ERR_UNSUPPORTED;
   p.CTAS = g.nHS; p.CH = g.CH; p.K16 = g.KS16;
   HB_TRY(gl_scratch(&p, (size_t)2 * ceil_div(p.N, 8) * g.KS16 * 128, 0, nullptr, s));
   return gl(dtype, p, g, s);
@@ -114,7 +109,7 @@ int run_bwd(ChainParams& p, int dtype, int grid_most, int gates, void* db, void*
     if (st_ != HASTE_B200_ERR_UNSUPPORTED) return st_;
   }
   GlGeometry g;
-  if (!gl_geometry(dtype, p.T, p.N, p.H, grid_most, &g)) return HASTE_B200_ERR_UNSUPPORTED;
+  if (!gl_geometry(dtype, p.N, p.H, grid_most, &g)) return HASTE_B200_ERR_UNSUPPORTED;
   p.CTAS = g.nHS; p.CH = g.CH; p.K16 = ceil_div(g.nHS * g.NMT, 4);
   HB_TRY(gl_scratch(&p, (size_t)2 * tiles * g.nHS * g.nHS * g.NMT * 32, (size_t)g.nRG * 8 * p.H, &p.db_part, s));
   HB_TRY(gl(dtype, p, g, s));

@@ -237,10 +237,10 @@ def test_float16_is_rejected_outside_the_gru():
 
 @pytest.mark.parametrize("cell", ["lstm", "gru", "layer_norm_lstm", "layer_norm_gru"])
 def test_hidden_size_beyond_the_persistent_kernels_falls_back_and_stays_correct(cell):
-    """fp32 H > 512 does not fit the register-resident recurrence; the step-wise path takes
-    over without the caller noticing anything but the launch count."""
+    """fp32 H > 1024 (LayerNorm cells: 512) does not fit the register-resident recurrences; the
+    step-wise path takes over without the caller noticing anything but the launch count."""
     from haste_b200 import _C
-    T, N, C, H = 5, 6, 24, 640
+    T, N, C, H = 5, 6, 24, 1032
     d = oracle.make_inputs(cell, T, N, C, H, seed=H, zoneout=0.1)
     ref_out, ref_grads = oracle.forward_backward(cell, d, zoneout=0.1)
     n0 = _C.launch_count()

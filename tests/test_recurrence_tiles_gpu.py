@@ -62,6 +62,18 @@ def test_grid_recurrence_reduced_precision(cell, dtype, tol, shape):
     _check(cell, *shape, dtype, tol, 0.25)
 
 
+@pytest.mark.parametrize("shape", [(1, 3, 513), (2, 64, 640), (4, 6, 1024), (7, 17, 900)],
+                         ids=lambda s: "T%d_N%d_H%d" % s)
+@pytest.mark.parametrize("cell", ["lstm", "gru"])
+def test_short_sequences_of_wide_layers_take_the_recurrence(cell, shape):
+    """A few steps of an fp32 layer beyond 512 units: right, and one launch for the recurrence of
+    each pass, so that the launches do not grow with the steps."""
+    from haste_b200 import _C
+    n0 = _C.launch_count()
+    _check(cell, *shape, torch.float32, TOL_F32, 0.25)
+    assert _C.launch_count() - n0 <= 14
+
+
 # tensor-core recurrence: two 64-row tiles per CTA with a ragged second one, a last slice of eight units, rings whose stage
 # count is no multiple of the issuers, fewer k-blocks than issuers have turns
 @pytest.mark.parametrize("T,N,H,sms", [(40, 90, 1024, 74), (40, 65, 1024, 74), (60, 128, 768, 74), (8, 700, 320, 0),
