@@ -11,8 +11,8 @@
 // (G = 3 for the GRU; G = 4 for the LSTM, where "dq" is the gate gradient in the cache's place.)
 // A step is bound by its chain - counter, TMA, MMA issue (65 cycles each), tensor-memory read, gate
 // math, publish - and, with many rows per CTA, by the stream of h or dq at 64 bytes per clock and SM.
-// GRU, H = 1024, us per step forward / backward: 128 rows 6.5 / 9.8, 256 rows 7.5 / 11.9 (one 128-row tile
-// per CTA before: 7.6 / 13.3).  Two directions of 200 steps side by side, chain kernels -> this: GRU 90
+// GRU, H = 1024, us per step forward / backward: 128 rows 6.8 / 10.3, 256 rows 7.8 / 12.1 (with one 128-row
+// tile per CTA 7.6 / 13.3, then with the faster gate functions below).  Two directions of 200 steps side by side, chain kernels -> this: GRU 90
 // rows 8.2 -> 5.0 ms, LSTM 90 rows 8.1 -> 6.4, LSTM 178 rows H = 808 9.4 -> 6.9.
 //
 // * Grid = (H / 16 hidden slices) x (row groups), one cooperative launch per layer pass; a
@@ -32,6 +32,9 @@
 //   waits for all of them (acquire) before it loads step t's operand.  CTAs of different row
 //   groups never wait for each other, and with several tiles per CTA the wait for one tile
 //   hides behind the contraction of the others.
+// * The gate functions are the accurate ones of rec_chain.cuh.  One MUFU.TANH each (relative error
+//   2^-11) would take 0.3 us off a forward step of the GRU, but then 0.17 % of the stored states are
+//   another bf16 than the exact step gives, against 0.02 %.
 // * Every wait - counter or mbarrier - is bounded; on expiry the grid's abort flag and the
 //   process error word are set, all roles leave their loops, tensor memory is released and
 //   the host reports HASTE_B200_ERR_TIMEOUT.
@@ -51,15 +54,6 @@ namespace {
 
 using namespace tc;
 typedef __nv_bfloat16 bf16;
-
-// Gate functions of the GRU here (the LSTM uses those of rec_chain.cuh): one MUFU.TANH each (relative error 2^-11, a
-// fraction of a bf16 ulp; the parity bar of bf16 storage is 2e-2).
-__device__ __forceinline__ float tanh_fast(float x) {
-  float y;
-  asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ float sigmoid_fast(float x) { return fmaf(0.5f, tanh_fast(0.5f * x), 0.5f); }
 
 constexpr int UC = 16;                 // hidden units per CTA
 constexpr int BK = 64;                 // K elements per TMA box / swizzle row (128 bytes)
@@ -553,10 +547,10 @@ tc_recurrence_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p
 #pragma unroll
               for (int u = 0; u < 8; ++u) {
                 const float hprev = bfq(hp[hf], u);
-                const float z = sigmoid_fast(bfq(in0[hf], u) + s0[u] + s_bias[uo + u] + s_bias[48 + uo + u]);
-                const float rr = sigmoid_fast(bfq(in1[hf], u) + s1[u] + s_bias[16 + uo + u] + s_bias[64 + uo + u]);
+                const float z = rec::chain_sigmoid(bfq(in0[hf], u) + s0[u] + s_bias[uo + u] + s_bias[48 + uo + u]);
+                const float rr = rec::chain_sigmoid(bfq(in1[hf], u) + s1[u] + s_bias[16 + uo + u] + s_bias[64 + uo + u]);
                 const float qg = s2[u] + s_bias[80 + uo + u];
-                const float g = tanh_fast(bfq(in2[hf], u) + rr * qg + s_bias[32 + uo + u]);
+                const float g = rec::chain_tanh(bfq(in2[hf], u) + rr * qg + s_bias[32 + uo + u]);
                 float x = z * hprev + (1.0f - z) * g;
                 if (p.has_zoneout)
                   x = p.training ? zoneout<true>(x, hprev, p.zoneout_prob, bfq(mk[hf], u))
