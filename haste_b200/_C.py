@@ -43,12 +43,15 @@ SIGNATURES = {
     "haste_b200_set_recurrence_path": [_i],
     "haste_b200_set_gemm_path": [_i],
     "haste_b200_set_sm_budget": [_i],
+    "haste_b200_exchange_sm_budget": [_i],
     "haste_b200_set_assign_gradients": [_i],
+    "haste_b200_exchange_assign_gradients": [_i],
     "haste_b200_sync_check": [_p],
     "haste_b200_profile_enable": [_i],
     "haste_b200_profile_read": [_p, _i],
 }
-OTHER_SYMBOLS = ["haste_b200_last_error", "haste_b200_version", "haste_b200_launch_count"]
+OTHER_SYMBOLS = ["haste_b200_last_error", "haste_b200_version", "haste_b200_launch_count",
+                 "haste_b200_sm_budget"]
 
 _lib = None
 
@@ -114,6 +117,16 @@ def set_recurrence_path(path):
 def set_sm_budget(sms):
     """SMs one persistent recurrence launch may occupy (0 = all); see the header."""
     call("haste_b200_set_sm_budget", int(sms))
+
+
+def exchange_sm_budget(sms):
+    """Sets the budget of this thread's calls (0: the process's holds) and returns what it was."""
+    return lib().haste_b200_exchange_sm_budget(int(sms))
+
+
+def sm_budget():
+    """The budget that holds for this thread's calls."""
+    return lib().haste_b200_sm_budget()
 
 
 def set_gemm_path(path):

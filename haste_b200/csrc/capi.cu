@@ -11,7 +11,8 @@ static std::atomic<int> g_rec_path{HASTE_B200_PATH_AUTO};
 static std::atomic<int> g_gemm_path{HASTE_B200_GEMM_AUTO};
 static std::atomic<int> g_sm_budget{0};
 int recurrence_path() { return g_rec_path.load(); }
-int sm_budget() { return g_sm_budget.load(); }
+static thread_local int t_sm_budget = 0;  // in front of the process's while not 0
+int sm_budget() { return t_sm_budget ? t_sm_budget : g_sm_budget.load(); }
 int gemm_path() { return g_gemm_path.load(); }
 static thread_local bool g_assign = false;
 bool assign_gradients() { return g_assign; }
@@ -66,9 +67,20 @@ int haste_b200_set_sm_budget(int sms) {
   g_sm_budget.store(sms);
   return HASTE_B200_OK;
 }
+int haste_b200_sm_budget(void) { return sm_budget(); }
+int haste_b200_exchange_sm_budget(int sms) {
+  const int was = t_sm_budget;
+  t_sm_budget = sms > 0 ? sms : 0;
+  return was;
+}
 int haste_b200_set_assign_gradients(int on) {
   g_assign = on != 0;
   return HASTE_B200_OK;
+}
+int haste_b200_exchange_assign_gradients(int on) {
+  const int was = g_assign;
+  g_assign = on != 0;
+  return was;
 }
 int haste_b200_set_gemm_path(int path) {
   if (path < 0 || path > 3) return HASTE_B200_ERR_INVALID;

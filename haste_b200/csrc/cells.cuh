@@ -177,7 +177,7 @@ inline int wide_few_rows(int dtype, int N, int GH, int H) {
 int split_once(const void* src, long long rows, int width, bool wanted, GradPlanes* planes, long long* ld, bool* have,
                cudaStream_t s);
 
-// Process-wide knobs (set through the C ABI).
+// Knobs of the process (set through the C ABI); the budget also of a thread, in front of it.
 int recurrence_path();
 int sm_budget();  // 0: the whole GPU; else the SMs one recurrence launch may occupy
 int gemm_path();

@@ -41,19 +41,20 @@ def _load_native():
 
 
 class _sm_budget:
-    """While active, one persistent recurrence launch occupies at most `sms` SMs (0: no
-    limit), so that the two directions of a bidirectional level are co-resident."""
+    """While active, one persistent recurrence launch of this thread occupies at most `sms` SMs
+    (0: whatever the process has set), so that the two directions of a bidirectional level are
+    co-resident."""
 
     def __init__(self, sms):
         self.sms = sms
 
     def __enter__(self):
         if self.sms:
-            _C.set_sm_budget(self.sms)
+            self.was = _C.exchange_sm_budget(self.sms)
 
     def __exit__(self, *exc):
         if self.sms:
-            _C.set_sm_budget(0)
+            _C.exchange_sm_budget(self.was)
 
 
 def _bucket(ctx):

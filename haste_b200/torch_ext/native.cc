@@ -36,7 +36,7 @@ bool has_c(int cell) { return cell == LSTM || cell == LN_LSTM; }
 // The library functions, resolved once from the shared object that the ctypes binding has loaded
 // (so that both use one copy of it and its settings).
 #define HB_FUNCTIONS(X)                                                                              \
-  X(last_error) X(set_sm_budget) X(set_assign_gradients) X(lstm_forward) X(lstm_backward)            \
+  X(last_error) X(exchange_sm_budget) X(exchange_assign_gradients) X(lstm_forward) X(lstm_backward)  \
   X(gru_forward) X(gru_backward) X(indrnn_forward) X(indrnn_backward) X(layer_norm_lstm_forward)     \
   X(layer_norm_lstm_backward) X(layer_norm_gru_forward) X(layer_norm_gru_backward)                   \
   X(layer_norm_indrnn_forward) X(layer_norm_indrnn_backward) X(lstm_forward_iterate)                 \
@@ -93,14 +93,15 @@ int lib_dtype(const Tensor& x, int cell) {
 
 void* ptr(const Tensor& t) { return t.defined() && t.numel() ? t.data_ptr() : nullptr; }
 
+// Settings of this thread's calls, put back as they were.
 struct SmBudget {
-  int sms;
-  explicit SmBudget(int n) : sms(n) { if (sms) lib.set_sm_budget(sms); }
-  ~SmBudget() { if (sms) lib.set_sm_budget(0); }
+  int sms, was;
+  explicit SmBudget(int n) : sms(n), was(sms ? lib.exchange_sm_budget(sms) : 0) {}
+  ~SmBudget() { if (sms) lib.exchange_sm_budget(was); }
 };
 struct AssignGradients {
-  AssignGradients() { lib.set_assign_gradients(1); }
-  ~AssignGradients() { lib.set_assign_gradients(0); }
+  int was = lib.exchange_assign_gradients(1);
+  ~AssignGradients() { lib.exchange_assign_gradients(was); }
 };
 
 void check(const Tensor& x, at::ArrayRef<Tensor> ts) {

@@ -72,8 +72,13 @@ int haste_b200_set_recurrence_path(int path);
 /* Limits the number of SMs one persistent recurrence launch of the calling process occupies
  * (0 = the whole GPU, the default).  With half the GPU per launch the two directions of a
  * bidirectional layer, issued on two streams, are co-resident and run concurrently.  Honoured by
- * the tensor-core GRU recurrence; no reference counterpart. */
+ * the LSTM and GRU recurrences and by the LayerNorm ones on clusters; no reference counterpart. */
 int haste_b200_set_sm_budget(int sms);
+/* The same for the calls of this thread alone, in front of the process's setting while not 0.
+ * Returns what it was, so that a caller who sets it for a call can put it back. */
+int haste_b200_exchange_sm_budget(int sms);
+/* The budget that holds for this thread's calls. */
+int haste_b200_sm_budget(void);
 enum { HASTE_B200_GEMM_AUTO = 0, HASTE_B200_GEMM_SIMT = 1, HASTE_B200_GEMM_TCGEN05 = 2,
        HASTE_B200_GEMM_TCGEN05_SINGLE = 3 /* tensor cores, never the CTA-pair kernel */ };
 int haste_b200_set_gemm_path(int path);
@@ -101,6 +106,7 @@ int haste_b200_profile_read(float* ms, int n);
  * gradients, dh and dc instead of accumulating into them, so that a caller with fresh buffers need
  * not zero them first.  Off by default (the reference's contract). */
 int haste_b200_set_assign_gradients(int on);
+int haste_b200_exchange_assign_gradients(int on); /* the same; returns what it was */
 
 /* ---- LSTM -------------------------------------------------------------- */
 /* Replaces lstm::ForwardPass<T>::Run  (lib/haste/lstm.h:118-129,

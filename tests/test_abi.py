@@ -59,3 +59,34 @@ def test_version_and_error_calls_work_without_gpu(built_lib):
     assert b"invalid argument" in L.haste_b200_last_error()
     with pytest.raises(_C.HasteError):
         _C.call("haste_b200_set_gemm_path", 17)
+
+
+def test_a_threads_sm_budget_is_its_own_and_put_back(built_lib):
+    """What a layer sets for its call neither reaches another thread nor outlives the call, and a
+    budget that the caller has set for the process stays."""
+    import threading
+    from haste_b200 import _C, rnn
+    _C.set_sm_budget(100)
+    try:
+        with rnn._sm_budget(74):
+            assert _C.sm_budget() == 74
+            seen = []
+            t = threading.Thread(target=lambda: seen.append(_C.sm_budget()))
+            t.start()
+            t.join()
+            assert seen == [100]
+            with rnn._sm_budget(37):
+                assert _C.sm_budget() == 37
+            with rnn._sm_budget(0):
+                assert _C.sm_budget() == 74
+            assert _C.sm_budget() == 74
+        assert _C.sm_budget() == 100
+    finally:
+        _C.set_sm_budget(0)
+    assert _C.sm_budget() == 0
+
+
+def test_assigning_gradients_is_put_back(built_lib):
+    from haste_b200 import _C
+    exchange = _C.lib().haste_b200_exchange_assign_gradients
+    assert exchange(1) == 0 and exchange(1) == 1 and exchange(0) == 1 and exchange(0) == 0

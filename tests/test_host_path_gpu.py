@@ -66,3 +66,19 @@ def test_inference_call(cell, T, N, H, zoneout, dtype):
             got, want = [_run(layer, x, state, None, g, **kw) for g in (False, True)]
             for a, b in zip(got, want):
                 torch.testing.assert_close(a, b, rtol=tol, atol=tol)
+
+
+def test_settings_of_the_caller_survive_a_call():
+    from haste_b200 import _C
+    exchange = _C.lib().haste_b200_exchange_assign_gradients
+    layer = haste_b200.GRU(8, 16).cuda()
+    layer._sm_budget = 74
+    x = torch.randn(3, 2, 8, device="cuda", requires_grad=True)
+    _C.set_sm_budget(100)
+    exchange(1)
+    try:
+        layer(x)[0].sum().backward()  # (the backward pass runs on a thread of autograd's)
+        assert _C.sm_budget() == 100
+    finally:
+        _C.set_sm_budget(0)
+        assert exchange(0) == 1
