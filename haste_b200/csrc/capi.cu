@@ -1,6 +1,8 @@
 // extern "C" surface of libhaste_b200.so (declared in include/haste_b200.h).
 // Each function packs its arguments into the driver's argument block and forwards.
 #include <atomic>
+#include <map>
+#include <mutex>
 
 #include "cells.cuh"
 
@@ -33,7 +35,23 @@ int report_timeout() {
                      "results are incomplete", code, d[0], d[1], d[2], (unsigned)d[3]);
   return HASTE_B200_ERR_TIMEOUT;
 }
-#define HB_ENTRY() HB_TRY(report_timeout())
+
+// Calls on one stream share its scratch (util.cuh), so all launches of one call go out before the next
+// call's: another thread's would put its own zeroing between a zeroing and its kernel, or free a block
+// that has grown too small under launches that still name it.
+std::mutex& stream_mutex(void* stream) {
+  static std::mutex mu;
+  static auto* of = new std::map<void*, std::mutex>;  // (kept to the end: threads may outlive statics)
+  static thread_local std::map<void*, std::mutex>::value_type* last = nullptr;
+  if (!last || last->first != stream) {
+    std::lock_guard<std::mutex> lk(mu);
+    last = &*of->try_emplace(stream).first;
+  }
+  return last->second;
+}
+#define HB_ENTRY()           \
+  HB_TRY(report_timeout()); \
+  const std::lock_guard<std::mutex> call_lock(stream_mutex(stream))
 }  // namespace
 
 extern "C" {

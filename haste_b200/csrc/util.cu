@@ -134,7 +134,9 @@ void profile_read(float* ms, int n) {
 namespace {
 struct Block { void* p = nullptr; size_t n = 0; };
 std::mutex g_ws_mu;
-std::map<std::tuple<int, cudaStream_t, int>, Block> g_ws;
+// (device, stream, slot, and for the handle that names another stream in every thread the thread)
+std::map<std::tuple<int, cudaStream_t, int, const void*>, Block> g_ws;
+thread_local char t_self;
 }  // namespace
 
 void* workspace(cudaStream_t stream, size_t bytes, int slot) {
@@ -144,7 +146,8 @@ void* workspace(cudaStream_t stream, size_t bytes, int slot) {
     return nullptr;
   }
   std::lock_guard<std::mutex> lk(g_ws_mu);
-  Block& b = g_ws[std::make_tuple(dev, stream, slot)];
+  const void* thread = stream == cudaStreamPerThread ? &t_self : nullptr;
+  Block& b = g_ws[std::make_tuple(dev, stream, slot, thread)];
   if (b.n >= bytes && b.p) return b.p;
   if (b.p) {
     // Work already queued on this stream may still read the old block.

@@ -20,9 +20,9 @@ int* device_error_word();
 int take_error_word(int* detail = nullptr);  // detail: 4 ints of kernel-specific context
 
 // Library-owned scratch.  One grow-only buffer per (device, stream, slot), so
-// calls issued on different streams never share scratch.  The pointer stays
-// valid until the next larger request on the same stream.  Returns nullptr
-// (and sets the last error) if the allocation fails.
+// calls issued on different streams never share scratch; calls on one stream are let
+// in one at a time (capi.cu).  The pointer stays valid until the next larger request
+// on the same stream.  Returns nullptr (and sets the last error) if the allocation fails.
 void* workspace(cudaStream_t stream, size_t bytes, int slot = 0);
 
 // Bump allocator over one workspace() block; every sub-buffer is 256-byte aligned.

@@ -22,7 +22,8 @@
  *     (x_t [C,T,N], W_t [G*H,C], R_t [G*H,H]); zero means they are passed in their
  *     forward layout (x [T,N,C], W [C,G*H], R [H,G*H]) and no copy is made.
  *   - `stream` is a cudaStream_t (NULL = default stream).  All work is issued on
- *     it, in order; nothing blocks the host.
+ *     it, in order; nothing blocks the host.  Any number of threads may call, on the same
+ *     stream too: a call's launches go out together.
  *   - Return value: HASTE_B200_OK or an error code; haste_b200_last_error()
  *     returns a thread-local message.  No exceptions cross this boundary.
  */
