@@ -644,9 +644,6 @@ class LayerNormIndRNN(BaseRNN):
         return self._permute(h[1:]), state
 
 
-_reversed_index = {}
-
-
 class _FlipTime(torch.autograd.Function):
     """Time reversal of a `[T, ...]` tensor as a row gather (whole `[N, F]` slabs copied with
     wide accesses; `torch.flip`'s element-indexed kernel runs at a fifth of the copy bandwidth
@@ -661,12 +658,22 @@ class _FlipTime(torch.autograd.Function):
         return _flip_rows(g)
 
 
+_reversed_index = {}  # (steps, device, stream) -> index; the oldest goes when there are 64
+
+
 def _flip_rows(x):
-    T = x.shape[0]
-    key = (T, x.device)
+    """The index is kept for the stream that made it, where later uses are ordered behind it; a graph
+    makes its own, which nothing outside the graph reads."""
+    T, device = x.shape[0], x.get_device()
+    key = (T, device, torch._C._cuda_getCurrentRawStream(device))
     idx = _reversed_index.get(key)
-    if idx is None:
-        idx = _reversed_index[key] = torch.arange(T - 1, -1, -1, device=x.device)
+    capturing = torch.cuda.is_current_stream_capturing()
+    if idx is None or capturing:
+        idx = torch.arange(T - 1, -1, -1, device=x.device)
+        if not capturing:
+            if len(_reversed_index) >= 64:
+                _reversed_index.pop(next(iter(_reversed_index)), None)
+            _reversed_index[key] = idx
     return x.contiguous().index_select(0, idx)
 
 
