@@ -52,9 +52,6 @@ void set_last_error(const char* fmt, ...);
 // ---------------------------------------------------------------------------
 // Storage types: fp32, or bf16 storage with all arithmetic in fp32.
 // ---------------------------------------------------------------------------
-template <typename T> struct is_bf16 { static constexpr bool value = false; };
-template <> struct is_bf16<__nv_bfloat16> { static constexpr bool value = true; };
-
 __device__ __forceinline__ float ld(const float* p) { return *p; }
 __device__ __forceinline__ float ld(const __nv_bfloat16* p) { return __bfloat162float(*p); }
 __device__ __forceinline__ float ld(const __half* p) { return __half2float(*p); }

@@ -258,11 +258,6 @@ __global__ void __launch_bounds__(IT_THREADS, 1) step_fma_kernel(const StepParam
 }
 
 // ---------------------------------------------------------------- mma form: 8 .. 64 rows
-__device__ __forceinline__ void ldm4(uint32_t (&r)[4], const void* at) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"((uint32_t)__cvta_generic_to_shared(at)));
-}
 __device__ __forceinline__ void ldm2(uint32_t (&r)[2], const void* at) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];"
                : "=r"(r[0]), "=r"(r[1])

@@ -66,8 +66,7 @@ int gl_fwd(ChainParams& p, const GlGeometry& g, cudaStream_t s) {
   if (g.NMT == nmt && ksw <= k) return gl_fwd_go<G, nmt, k, SPLIT, T>(p, g, s);
   HB_GL(4, 2) HB_GL(4, 4)
   if constexpr (SPLIT == 1) { HB_GL(4, 6) HB_GL(4, 8) }
-  HB_GL(2, 4) HB_GL(2, 6) HB_GL(2, 8)
-  HB_GL(1, 4)
+  else { HB_GL(2, 6) HB_GL(2, 8) }  // (as gl_geometry chooses NMT)
 #undef HB_GL
   return HASTE_B200_ERR_UNSUPPORTED;
 }
@@ -88,8 +87,7 @@ int gl_bwd(ChainParams& p, const GlGeometry& g, cudaStream_t s) {
   if (g.NMT == nmt && tpw <= k) return gl_bwd_go<G, nmt, k, SPLIT, T>(p, g, s);
   HB_GL(4, 2) HB_GL(4, 4)
   if constexpr (SPLIT == 1) { HB_GL(4, 6) HB_GL(4, 8) }
-  HB_GL(2, 4) HB_GL(2, 6) HB_GL(2, 8)
-  HB_GL(1, 4)
+  else { HB_GL(2, 6) HB_GL(2, 8) }  // (as gl_geometry chooses NMT)
 #undef HB_GL
   return HASTE_B200_ERR_UNSUPPORTED;
 }

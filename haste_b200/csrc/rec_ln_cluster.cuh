@@ -661,7 +661,7 @@ __global__ void __launch_bounds__(NW * 32, 1) ln_cl_bwd_kernel(const __grid_cons
   // inputs of a (step, chain), fetched one ahead: gates 4, h.R G, dh_new, mask, then LSTM dc_new, c
   // before, LN(c), GRU h before; statistics of h.R, LSTM those of c
   constexpr int NI = 4 + G + 2 + (G == 4 ? 3 : 1) + (G == 4 ? 4 : 2);
-  constexpr int I_RH = 4, I_DH = 4 + G, I_M = I_DH + 1, I_S = I_M + 1, I_C1 = I_S + (G == 4 ? 3 : 1), I_C3 = I_C1 + 2;
+  constexpr int I_RH = 4, I_DH = 4 + G, I_M = I_DH + 1, I_S = I_M + 1, I_C1 = I_S + (G == 4 ? 3 : 1);
   float nx[NI];
   auto fetch_inputs = [&](int ti, int ch) {
     const int n = (tile0 + ch) * 8 + row, t = p.T - 1 - ti;
@@ -694,7 +694,6 @@ __global__ void __launch_bounds__(NW * 32, 1) ln_cl_bwd_kernel(const __grid_cons
       }
     }
   };
-  (void)I_C3;
   // stash: 0..G-1 gate gradients, 4..4+G-1 h.R - mean, 8 its 1/sigma; LSTM before stage B: 9 dc
   // arriving, 10 c before, 11 c - mean, 12 its 1/sigma, 13 gamma_h d(LN c), 0..2 gates i, g, f, 3 d_o
   fetch_inputs(0, 0);

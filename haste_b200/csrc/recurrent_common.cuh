@@ -73,17 +73,7 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ float ldcg_f(const float* p) { return __ldcg(p); }
-__device__ __forceinline__ float ldcg_f(const __nv_bfloat16* p) {
-  return __bfloat162float(__ldcg(p));
-}
-
 // Polling loads: relaxed, gpu scope, so that every poll is served by L2.
-__device__ __forceinline__ uint32_t ld_relaxed_u32(const uint32_t* p) {
-  uint32_t v;
-  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
 __device__ __forceinline__ uint4 ld_relaxed_u32x4(const uint32_t* p) {
   uint4 v;
   asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];"
@@ -116,9 +106,6 @@ __device__ __forceinline__ uint32_t xword_encode(float x, uint32_t tag) {
 }
 __device__ __forceinline__ float xword_value(uint32_t w) {
   return __uint_as_float(w << 16) + __uint_as_float(w & 0xBFFF0000u);
-}
-__device__ __forceinline__ bool xword_ready(uint32_t w, uint32_t tag) {
-  return ((w >> 30) & 1u) == tag;
 }
 
 // Tagged fp32 word: the value with its lowest mantissa bit replaced by the tag (22 explicit

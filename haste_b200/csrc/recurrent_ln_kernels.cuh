@@ -91,9 +91,6 @@ struct LnBwdParams {
 template <int SPLIT> __device__ __forceinline__ uint32_t hword_encode(float x, uint32_t tag) {
   return SPLIT == 2 ? fword_encode(x, tag) : xword_encode(x, tag);
 }
-template <int SPLIT> __device__ __forceinline__ bool hword_ready(uint32_t w, uint32_t tag) {
-  return SPLIT == 2 ? fword_ready(w, tag) : xword_ready(w, tag);
-}
 // Gate functions of the LayerNorm cells.  With fp32 storage the accurate expf / tanhf: three
 // normalisations per step amplify a relative error of 1e-6 (the ex2.approx-based fast forms)
 // a hundredfold over a few dozen steps, which is most of the distance between these kernels
