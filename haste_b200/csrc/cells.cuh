@@ -125,7 +125,7 @@ struct GradPlanes {
 // Chain recurrences (rec_chain_host.cu): on a thread-block cluster or the whole grid, H up to
 // 1024.  Forward: the input projection is already in a.v (LSTM) / a.tmp_Wx (GRU).  Backward:
 // complete - dh and dc are read and written in place (dc_new may be null), the bias gradients
-// added.  `few` (GRU): leave batches to the tensor-core recurrence where that is faster.
+// added.  `few`: leave batches to the tensor-core recurrence where that is faster.
 int lstm_forward_chain(const LstmFwd& a, bool few, cudaStream_t s);
 int lstm_backward_chain(const LstmBwd& a, const GradPlanes& planes, bool few, cudaStream_t s);
 int gru_forward_chain(const GruFwd& a, bool few, cudaStream_t s);

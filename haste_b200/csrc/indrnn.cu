@@ -16,8 +16,7 @@ constexpr int AHEAD = 8;  // steps whose inputs are loaded together
 
 // Piped: a group's loads are issued before the group in front of it is computed.  With few (batch,
 // unit) pairs the GPU has too little in flight to hide a group's latency behind other threads, and
-// the scan took T / 8 latencies; with many, the registers cost more threads than that wins.  The
-// line lies where the pairs no longer fit in half of the resident threads (see scan_blocks).
+// the scan took T / 8 latencies; with many, the registers cost more threads than that wins (ScanShape).
 template <typename T, bool Training, bool Zoneout, bool Piped>
 __global__ void __launch_bounds__(128) indrnn_scan_fwd(int T_, long long NH, int H, const T* __restrict__ Wx,
                                 const T* __restrict__ u, const T* __restrict__ b,
@@ -132,14 +131,14 @@ __global__ void __launch_bounds__(128) indrnn_scan_bwd(int T_, long long NH, int
   db_part[idx] = db;
 }
 
-// Threads per block and whether the piped form runs: half of 2048 threads on every SM.
+// The piped form runs while the pairs fit in a quarter of the 2048 threads that an SM holds.  400 steps
+// with zoneout, us forward / backward, plain -> piped: 8 192 pairs 51 / 45 -> 41 / 41; 32 768 72 / 72 ->
+// 56 / 60; 75 776, where the line lies on 148 SMs, 88 / 94 -> 78 / 87; 98 304 99 / 111 -> 93 / 123.
+// (Blocks of 32 threads, to spread few pairs over more SMs, measured the same as 128 everywhere.)
 struct ScanShape {
-  int blocks, threads;
+  int blocks, threads = 128;
   bool piped;
-  explicit ScanShape(long long NH)
-      : threads(NH < 64LL * 4 * sm_count() ? 32 : 128), piped(NH <= 1024LL * sm_count() / 2) {
-    blocks = ceil_div(NH, threads);
-  }
+  explicit ScanShape(long long NH) : blocks(ceil_div(NH, 128)), piped(NH <= 512LL * sm_count()) {}
 };
 
 template <typename T, bool Piped>

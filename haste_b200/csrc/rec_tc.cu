@@ -638,16 +638,14 @@ struct TcGeometry {
   size_t ring, smem;
 };
 
-// Shapes this path takes: bf16, H a multiple of 8 up to 1024 (the resident slice of R and a
-// useful ring must fit shared memory), at least 64 batch rows (below that the register
-// kernels are faster) and at most two row tiles per CTA: every CTA of a row group streams
-// the group's whole h (or dq), H / 16 copies of it per step out of L2, which is what bounds
-// the step from a few hundred rows per GPU on - there the per-step contraction + pointwise
-// launches of the step-wise path, with their full-size tiles, are faster (measured at
-// H = 1024: forward 9.4 / 10.3 / 11.8 us per step at 128 / 256 / 512 rows against 9.3
-// (register kernel) / 18.4 / 20.5 us; backward 20.6 / 22.4 / 30.4 against 16.4 / 18.6 / 24.6).
-// `half` asks for the geometry under the SM budget (concurrent directions); without it, or
-// when the budget would need more than two tiles per CTA, the whole GPU is used.
+// Shapes this path takes: bf16, H a multiple of 8 up to 1024 (the resident slice of R and a useful ring
+// must fit shared memory), at least 64 batch rows and at most two row tiles per CTA: every CTA of a row
+// group streams the group's whole h (or dq), H / 16 copies of it per step out of L2, so that a third and
+// a fourth tile cost as much again, where the step-wise path's full-size contractions grow little.  GRU,
+// H = 1024, us per step forward / backward, this / step by step: 128 rows 7.0 / 10.5 and 19.3 / 18.5, 256
+// rows 8.0 / 12.6 and 22.6 / 18.6, 512 rows 10.4 / 17.2 and 20.5 / 22.7; 1024 rows step by step 30.4 / 30.2.
+// LSTM: 256 rows 10.2 / 20.1 and 16.5 / 21.8, 512 rows 14.3 / 33.2 and 20.5 / 28.3.
+// (Where the chain kernels take a batch themselves: rec_chain_host.cu.)
 bool tc_geometry_for(int G, int N, int H, bool fwd, int sms, TcGeometry* g) {
   const int K = fwd ? H : G * H;
   const size_t r_bytes = (size_t)ceil_div(K, BK) * (fwd ? G * UC : UC) * 128;
@@ -671,6 +669,7 @@ bool tc_geometry_for(int G, int N, int H, bool fwd, int sms, TcGeometry* g) {
     const size_t stage = (size_t)rb * 128, pad = A_STAGE - stage;
     int stages = (int)(((size_t)MAX_SMEM - fixed - pad) / stage);
     if (stages > 16) stages = 16;
+    if (stages < NI) return false;  // every issuer owns a stage
     g->stages = stages;
     g->ring = stages * stage + pad;
     g->smem = fixed + g->ring;
@@ -679,17 +678,13 @@ bool tc_geometry_for(int G, int N, int H, bool fwd, int sms, TcGeometry* g) {
   return false;
 }
 
-// `budgeted` reports whether the geometry honours the SM budget (then the two directions of a
-// bidirectional layer are co-resident).
-bool tc_geometry(int G, int N, int H, bool fwd, TcGeometry* g, bool* budgeted) {
-  *budgeted = false;
+// Under an SM budget (concurrent directions) the geometry within it, so that the two directions are
+// co-resident; where that would need more than two tiles per CTA, the whole GPU.
+bool tc_geometry(int G, int N, int H, bool fwd, TcGeometry* g) {
   if (H % 8 != 0 || H < 64 || H > 1024 || N < 64) return false;
   const int budget = sm_budget();
-  if (budget > 0 && budget < sm_count() && tc_geometry_for(G, N, H, fwd, budget, g)) {
-    *budgeted = true;
-    return true;
-  }
-  return tc_geometry_for(G, N, H, fwd, sm_count(), g);
+  return (budget > 0 && budget < sm_count() && tc_geometry_for(G, N, H, fwd, budget, g)) ||
+         tc_geometry_for(G, N, H, fwd, sm_count(), g);
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -753,20 +748,18 @@ int tc_scratch(int tiles, TcParams* p, cudaStream_t s) {
 
 bool lstm_tc_takes(int dtype, int N, int H, bool fwd) {
   TcGeometry g;
-  bool budgeted = false;
   return dtype == HASTE_B200_BF16 && recurrence_path() != HASTE_B200_PATH_STEPWISE &&
          recurrence_path() != HASTE_B200_PATH_NO_TENSOR_CORE && encode_fn() &&
-         tc_geometry(4, N, H, fwd, &g, &budgeted);
+         tc_geometry(4, N, H, fwd, &g);
 }
 
 // Forward: x.W is already in a.tmp_Wx.  HASTE_B200_ERR_UNSUPPORTED (nothing touched) when the
 // shape is not this path's.
 int gru_forward_tc(const GruFwd& a, cudaStream_t s) {
   TcGeometry g;
-  bool budgeted = false;
   if (a.dtype != HASTE_B200_BF16 || recurrence_path() == HASTE_B200_PATH_STEPWISE ||
       recurrence_path() == HASTE_B200_PATH_NO_TENSOR_CORE || a.h_out ||
-      !encode_fn() || !tc_geometry(3, a.N, a.H, true, &g, &budgeted))
+      !encode_fn() || !tc_geometry(3, a.N, a.H, true, &g))
     return HASTE_B200_ERR_UNSUPPORTED;
   if (!aligned16(a.R) || !aligned16(a.tmp_Wx) || !aligned16(a.h) || !aligned16(a.v) ||
       !aligned16(a.zoneout_mask) || !aligned16(a.bx) || !aligned16(a.br))
@@ -791,10 +784,9 @@ int gru_forward_tc(const GruFwd& a, cudaStream_t s) {
 // (the caller adds dq_0 . R^T).  Bias gradients are NOT summed here.
 int gru_backward_tc(const GruBwd& a, float* dh_carry, cudaStream_t s) {
   TcGeometry g;
-  bool budgeted = false;
   if (a.dtype != HASTE_B200_BF16 || recurrence_path() == HASTE_B200_PATH_STEPWISE ||
       recurrence_path() == HASTE_B200_PATH_NO_TENSOR_CORE || a.iterate ||
-      !encode_fn() || !tc_geometry(3, a.N, a.H, false, &g, &budgeted))
+      !encode_fn() || !tc_geometry(3, a.N, a.H, false, &g))
     return HASTE_B200_ERR_UNSUPPORTED;
   if (!aligned16(a.R) || !aligned16(a.h) || !aligned16(a.v) || !aligned16(a.dh_new) ||
       !aligned16(a.dp) || !aligned16(a.dq) || !aligned16(a.zoneout_mask) || !aligned16(dh_carry))
@@ -817,8 +809,7 @@ int gru_backward_tc(const GruBwd& a, float* dh_carry, cudaStream_t s) {
 // LSTM, in the same way: x.W is in a.v; c_carry (fp32 [N,H]) holds c_0.
 int lstm_forward_tc(const LstmFwd& a, float* c_carry, cudaStream_t s) {
   TcGeometry g;
-  bool budgeted = false;
-  if (!lstm_tc_takes(a.dtype, a.N, a.H, true) || !tc_geometry(4, a.N, a.H, true, &g, &budgeted) || !aligned16(a.R) ||
+  if (!lstm_tc_takes(a.dtype, a.N, a.H, true) || !tc_geometry(4, a.N, a.H, true, &g) || !aligned16(a.R) ||
       !aligned16(a.h) || !aligned16(a.c) || !aligned16(a.v) || !aligned16(a.zoneout_mask) || !aligned16(c_carry))
     return HASTE_B200_ERR_UNSUPPORTED;
   CUtensorMap map;
@@ -838,8 +829,7 @@ int lstm_forward_tc(const LstmFwd& a, float* c_carry, cudaStream_t s) {
 // v: gates in, gate gradients out.  dh_carry, dc_carry as dh_carry of gru_backward_tc.
 int lstm_backward_tc(const LstmBwd& a, float* dh_carry, float* dc_carry, cudaStream_t s) {
   TcGeometry g;
-  bool budgeted = false;
-  if (!lstm_tc_takes(a.dtype, a.N, a.H, false) || !tc_geometry(4, a.N, a.H, false, &g, &budgeted) || !aligned16(a.R) ||
+  if (!lstm_tc_takes(a.dtype, a.N, a.H, false) || !tc_geometry(4, a.N, a.H, false, &g) || !aligned16(a.R) ||
       !aligned16(a.c) || !aligned16(a.v) || !aligned16(a.dh_new) || !aligned16(a.dc_new) ||
       !aligned16(a.zoneout_mask) || !aligned16(dh_carry) || !aligned16(dc_carry))
     return HASTE_B200_ERR_UNSUPPORTED;

@@ -285,7 +285,7 @@ LnBwdParams ln_lstm_params(const LnLstmBwd& a, float* dh_carry, float* dc_carry,
 }
 }  // namespace
 
-// The cluster kernels, up to 256 units: dh and dc come back complete, and the bias and LayerNorm
+// The cluster kernels, up to 320 units: dh and dc come back complete, and the bias and LayerNorm
 // gradients of h.R and c go into the caller's tensors (added or assigned).
 int layer_norm_lstm_backward_cluster(const LnLstmBwd& a, float* dh_carry, float* dc_carry, cudaStream_t s) {
   LnBwdParams p = ln_lstm_params(a, dh_carry, dc_carry, GradPlanes{});

@@ -75,7 +75,7 @@ struct LnBwdParams {
   float* dgRh_part;       // [N,4H] per-row partial sums of dgamma_Rh (reduced by the host)
   float* dgh_part;        // [N,H]  per-row partial sums of dgamma_h
   float* dbh_part;        // [N,H]  per-row partial sums of dbeta_h
-  uint32_t* exch;         // tagged partial dh, as in rec_bwd_kernel
+  uint32_t* exch;         // tagged partial dh [2][nBS][dst CTA][src CTA][rows][16]
   uint32_t* sbuf;         // [2 stats][2 parity][nBS][rows][nHS][2]
   Sync sync;
   __nv_bfloat16* gpl;     // optional bf16 planes of d(x.W-side gate gradient) (dv)
@@ -1166,7 +1166,7 @@ int run_ln_bwd(LnBwdParams& p, const Geometry& g, cudaStream_t s) {
   return HASTE_B200_ERR_UNSUPPORTED;
 }
 
-// Clusters (rec_ln_cluster.cuh): HASTE_B200_ERR_UNSUPPORTED beyond 256 units.
+// Clusters (rec_ln_cluster.cuh): HASTE_B200_ERR_UNSUPPORTED beyond 320 units.
 int run_ln_cl_fwd_f32(const LnFwdParams& p, cudaStream_t s);
 int run_ln_cl_fwd_bf16(const LnFwdParams& p, cudaStream_t s);
 int run_lngru_cl_fwd_f32(const LnFwdParams& p, cudaStream_t s);
