@@ -385,12 +385,12 @@ def main():
         "weight_grad": 2.0 * T * N * 4 * H * (C + H),
         "input_grad": 2.0 * T * N * C * 4 * H,
     }
-    # DRAM bytes per time step of the fp32 N=64 H=512 recurrence launches, from one ncu
-    # capture of each kernel at T=200 (dram__bytes_read.sum + dram__bytes_write.sum over
-    # the 200 steps).  Every step touches its own slice of the activations once, so a
-    # launch's traffic is this times T.
-    ncu_bytes_per_step = {"recurrence_fwd": (109.424896e6 + 103.794944e6) / 200,
-                          "recurrence_bwd": (188.525568e6 + 169.723648e6) / 200}
+    # DRAM bytes per time step of the fp32 N=64 H=512 recurrence launches (gl_fwd_kernel,
+    # gl_bwd_kernel), from one ncu capture of each at T=200 (dram__bytes_read.sum +
+    # dram__bytes_write.sum over the 200 steps).  Every step touches its own slice of the
+    # activations once, so a launch's traffic is this times T.
+    ncu_bytes_per_step = {"recurrence_fwd": (109.582336e6 + 105.076736e6) / 200,
+                          "recurrence_bwd": (193.671424e6 + 167.135744e6) / 200}
     dom = max(phases, key=phases.get)
     if dom in alg_bytes:
         ach = alg_bytes[dom] / (phases[dom] * 1e-3) / 1e9
@@ -398,8 +398,8 @@ def main():
         roof = {"kernel": dom, "bound": "hbm", "achieved": ach, "peak": peaks["hbm_gbs"],
                 "unit": "GB/s", "frac": ach / peaks["hbm_gbs"],
                 "traffic": ncu_bytes_per_step[dom] * T if captured else None,
-                "traffic_source": ("ncu capture of this kernel at T=200 (dram bytes read + "
-                                   "written), scaled by T") if captured else None,
+                "traffic_source": ("ncu capture of gl_fwd_kernel / gl_bwd_kernel at T=200 (dram "
+                                   "bytes read + written), scaled by T") if captured else None,
                 "algorithmic_bytes": alg_bytes[dom],
                 "peak_source": peak_src,
                 "us_per_timestep": phases[dom] * 1e3 / T}
