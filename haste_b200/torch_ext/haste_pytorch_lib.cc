@@ -15,6 +15,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <algorithm>
+#include <utility>
 #include <vector>
 
 #include "haste_b200.h"
@@ -76,12 +78,27 @@ Dims dims_bwd(const Tensor& x_t, const Tensor& h) {  // x_t [C,T,N]
   return {(int)x_t.size(1), (int)x_t.size(2), (int)x_t.size(0), (int)h.size(2)};
 }
 
+// The library takes pointers and sizes, so what the tensors hold is said here: G gates, the weights, the
+// mask where it is read (it may be empty) and (tensor, values) of the rest.
+void holds(const Dims& d, int64_t G, const Tensor& kernel, const Tensor& recurrent, const Tensor* mask,
+           std::initializer_list<std::pair<const Tensor*, int64_t>> rest) {
+  const int64_t H = d.H;
+  bool ok = kernel.numel() == d.C * G * H && recurrent.numel() == (G > 1 ? H * G * H : H);
+  if (mask && mask->numel()) ok = ok && mask->numel() == (int64_t)d.T * d.N * H;
+  for (const auto& [t, n] : rest) ok = ok && t->numel() == n;
+  TORCH_CHECK(ok, "haste_b200: the tensors do not fit one another's sizes");
+}
+const Tensor* read(bool training, float zoneout_prob, const Tensor& mask) {
+  return training && zoneout_prob != 0.0f ? &mask : nullptr;
+}
+
 // ---------------------------------------------------------------- LSTM
 std::vector<Tensor> lstm_forward(bool training, float zoneout_prob, Tensor x, Tensor h0, Tensor c0,
                                  Tensor kernel, Tensor recurrent_kernel, Tensor bias,
                                  Tensor zoneout_mask) {
   check({&x, &h0, &c0, &kernel, &recurrent_kernel, &bias, &zoneout_mask});
   const Dims d = dims_fwd(x, recurrent_kernel.size(0));
+  holds(d, 4, kernel, recurrent_kernel, read(training, zoneout_prob, zoneout_mask), {{&bias, 4 * d.H}});
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor h = at::empty({d.T + 1, d.N, d.H}, x.options());
   Tensor c = at::empty({d.T + 1, d.N, d.H}, x.options());
@@ -102,6 +119,9 @@ std::vector<Tensor> lstm_backward(Tensor x_t, Tensor kernel_t, Tensor recurrent_
   check({&x_t, &kernel_t, &recurrent_kernel_t, &bias, &zoneout_mask, &h, &c, &cache, &dh_new,
          &dc_new});
   const Dims d = dims_bwd(x_t, h);
+  const int64_t rows = (int64_t)d.T * d.N, seq = (rows + d.N) * d.H;
+  holds(d, 4, kernel_t, recurrent_kernel_t, &zoneout_mask,
+        {{&h, seq}, {&c, seq}, {&cache, rows * 4 * d.H}, {&dh_new, seq}, {&dc_new, seq}});
   const c10::cuda::CUDAGuard guard(h.device());
   Tensor dx = at::empty({d.T, d.N, d.C}, h.options());
   Tensor dW = at::zeros({d.C, 4 * d.H}, h.options());
@@ -122,6 +142,8 @@ std::vector<Tensor> gru_forward(bool training, float zoneout_prob, Tensor x, Ten
                                 Tensor recurrent_bias, Tensor zoneout_mask) {
   check({&x, &h0, &kernel, &recurrent_kernel, &bias, &recurrent_bias, &zoneout_mask});
   const Dims d = dims_fwd(x, recurrent_kernel.size(0));
+  holds(d, 3, kernel, recurrent_kernel, read(training, zoneout_prob, zoneout_mask),
+        {{&bias, 3 * d.H}, {&recurrent_bias, 3 * d.H}});
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor h = at::empty({d.T + 1, d.N, d.H}, x.options());
   h[0].copy_(h0);
@@ -142,6 +164,8 @@ std::vector<Tensor> gru_backward(Tensor x_t, Tensor kernel_t, Tensor recurrent_k
   check({&x_t, &kernel_t, &recurrent_kernel_t, &bias, &recurrent_bias, &zoneout_mask, &h, &cache,
          &dh_new});
   const Dims d = dims_bwd(x_t, h);
+  const int64_t rows = (int64_t)d.T * d.N, seq = (rows + d.N) * d.H;
+  holds(d, 3, kernel_t, recurrent_kernel_t, &zoneout_mask, {{&h, seq}, {&cache, rows * 4 * d.H}, {&dh_new, seq}});
   const c10::cuda::CUDAGuard guard(h.device());
   Tensor dx = at::empty({d.T, d.N, d.C}, h.options());
   Tensor dW = at::zeros({d.C, 3 * d.H}, h.options());
@@ -164,6 +188,7 @@ Tensor indrnn_forward(bool training, float zoneout_prob, Tensor x, Tensor h0, Te
                       Tensor recurrent_scale, Tensor bias, Tensor zoneout_mask) {
   check({&x, &h0, &kernel, &recurrent_scale, &bias, &zoneout_mask});
   const Dims d = dims_fwd(x, kernel.size(1));
+  holds(d, 1, kernel, recurrent_scale, read(training, zoneout_prob, zoneout_mask), {{&bias, d.H}});
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor h = at::empty({d.T + 1, d.N, d.H}, x.options());
   h[0].copy_(h0);
@@ -179,6 +204,8 @@ std::vector<Tensor> indrnn_backward(Tensor x_t, Tensor kernel_t, Tensor recurren
                                     Tensor bias, Tensor zoneout_mask, Tensor h, Tensor dh_new) {
   check({&x_t, &kernel_t, &recurrent_scale, &bias, &zoneout_mask, &h, &dh_new});
   const Dims d = dims_bwd(x_t, h);
+  const int64_t seq = (int64_t)(d.T + 1) * d.N * d.H;
+  holds(d, 1, kernel_t, recurrent_scale, &zoneout_mask, {{&h, seq}, {&dh_new, seq}});
   const c10::cuda::CUDAGuard guard(h.device());
   Tensor dx = at::empty({d.T, d.N, d.C}, h.options());
   Tensor dW = at::zeros({d.C, d.H}, h.options());
@@ -213,6 +240,8 @@ std::vector<Tensor> layer_norm_lstm_forward(bool training, float zoneout_prob, T
   check({&x, &h0, &c0, &kernel, &recurrent_kernel, &bias, &gamma, &gamma_h, &beta_h,
          &zoneout_mask});
   const Dims d = dims_fwd(x, recurrent_kernel.size(0));
+  holds(d, 4, kernel, recurrent_kernel, read(training, zoneout_prob, zoneout_mask),
+        {{&bias, 4 * d.H}, {&gamma, 8 * d.H}, {&gamma_h, d.H}, {&beta_h, d.H}});
   const c10::cuda::CUDAGuard guard(x.device());
   const auto so = saved_options(x);
   Tensor h = at::empty({d.T + 1, d.N, d.H}, x.options());
@@ -247,6 +276,12 @@ std::vector<Tensor> layer_norm_lstm_backward(
   check({&act_Wx, &act_Wx_norm, &act_Wx_norm_cache, &act_Rh, &act_Rh_cache, &act_c_norm,
          &act_c_norm_cache});
   const Dims d = dims_bwd(x_t, h);
+  const int64_t rows = (int64_t)d.T * d.N, seq = (rows + d.N) * d.H;
+  holds(d, 4, kernel_t, recurrent_kernel_t, &zoneout_mask,
+        {{&gamma, 8 * d.H}, {&gamma_h, d.H}, {&beta_h, d.H}, {&h, seq}, {&c, seq}, {&dh_new, seq},
+         {&dc_new, seq}, {&act_Wx, rows * 4 * d.H}, {&act_Wx_norm, rows * 4 * d.H},
+         {&act_Wx_norm_cache, rows * 2}, {&act_Rh, rows * 4 * d.H}, {&act_Rh_cache, rows * 2},
+         {&act_c_norm, rows * d.H}, {&act_c_norm_cache, rows * 2}});
   const c10::cuda::CUDAGuard guard(h.device());
   Tensor dx = at::empty({d.T, d.N, d.C}, h.options());
   Tensor dW = at::zeros({d.C, 4 * d.H}, h.options());
@@ -275,6 +310,8 @@ std::vector<Tensor> layer_norm_gru_forward(bool training, float zoneout_prob, Te
                                            Tensor zoneout_mask) {
   check({&x, &h0, &kernel, &recurrent_kernel, &bias, &recurrent_bias, &gamma, &zoneout_mask});
   const Dims d = dims_fwd(x, recurrent_kernel.size(0));
+  holds(d, 3, kernel, recurrent_kernel, read(training, zoneout_prob, zoneout_mask),
+        {{&bias, 3 * d.H}, {&recurrent_bias, 3 * d.H}, {&gamma, 6 * d.H}});
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor h = at::empty({d.T + 1, d.N, d.H}, x.options());
   h[0].copy_(h0);
@@ -303,6 +340,10 @@ std::vector<Tensor> layer_norm_gru_backward(Tensor x_t, Tensor kernel_t, Tensor 
   check({&x_t, &kernel_t, &recurrent_kernel_t, &bias, &recurrent_bias, &gamma, &zoneout_mask, &h,
          &cache, &act_Wx, &act_Wx_norm_cache, &act_Rh, &act_Rh_norm_cache, &dh_new});
   const Dims d = dims_bwd(x_t, h);
+  const int64_t rows = (int64_t)d.T * d.N, seq = (rows + d.N) * d.H;
+  holds(d, 3, kernel_t, recurrent_kernel_t, &zoneout_mask,
+        {{&gamma, 6 * d.H}, {&h, seq}, {&cache, rows * 4 * d.H}, {&dh_new, seq}, {&act_Wx, rows * 3 * d.H},
+         {&act_Wx_norm_cache, rows * 2}, {&act_Rh, rows * 3 * d.H}, {&act_Rh_norm_cache, rows * 2}});
   const c10::cuda::CUDAGuard guard(h.device());
   Tensor dx = at::empty({d.T, d.N, d.C}, h.options());
   Tensor dW = at::zeros({d.C, 3 * d.H}, h.options());
@@ -329,6 +370,8 @@ std::vector<Tensor> layer_norm_indrnn_forward(bool training, float zoneout_prob,
                                               Tensor bias, Tensor gamma, Tensor zoneout_mask) {
   check({&x, &h0, &kernel, &recurrent_scale, &bias, &gamma, &zoneout_mask});
   const Dims d = dims_fwd(x, kernel.size(1));
+  holds(d, 1, kernel, recurrent_scale, read(training, zoneout_prob, zoneout_mask),
+        {{&bias, d.H}, {&gamma, std::max<int64_t>(gamma.numel(), d.H)}});
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor h = at::empty({d.T + 1, d.N, d.H}, x.options());
   h[0].copy_(h0);
@@ -351,6 +394,10 @@ std::vector<Tensor> layer_norm_indrnn_backward(Tensor x_t, Tensor kernel_t, Tens
   check({&x_t, &kernel_t, &recurrent_scale, &bias, &gamma, &zoneout_mask, &h, &act_Wx,
          &act_Wx_norm_cache, &dh_new});
   const Dims d = dims_bwd(x_t, h);
+  const int64_t rows = (int64_t)d.T * d.N, seq = (rows + d.N) * d.H;
+  holds(d, 1, kernel_t, recurrent_scale, &zoneout_mask,
+        {{&gamma, std::max<int64_t>(gamma.numel(), d.H)}, {&h, seq}, {&dh_new, seq}, {&act_Wx, rows * d.H},
+         {&act_Wx_norm_cache, rows * 2}});
   const c10::cuda::CUDAGuard guard(h.device());
   Tensor dx = at::empty({d.T, d.N, d.C}, h.options());
   Tensor dW = at::zeros({d.C, d.H}, h.options());

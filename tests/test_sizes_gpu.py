@@ -48,3 +48,45 @@ def test_backward_op():
         short[i] = new(T, N, H - 1) if i == 4 else args[i][1:].contiguous()
         _refused(lambda: ops.lstm_backward(*short, transposed=False))
     ops.lstm_backward(*args, transposed=False)
+
+
+@pytest.mark.parametrize("cell", ["lstm", "gru", "indrnn", "layer_norm_lstm", "layer_norm_gru", "layer_norm_indrnn"])
+def test_compiled_extension(cell):
+    """haste_pytorch_lib: one tensor after another a value short (initial states are copied by torch,
+    which checks them)."""
+    import importlib.util
+    import haste_oracle as oracle
+    from haste_b200 import build
+    spec = importlib.util.spec_from_file_location("haste_pytorch_lib", build.TORCH_EXT)
+    lib = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(lib)
+    d = oracle.make_inputs(cell, T, N, C, H, seed=1, zoneout=0.2)
+    t = {k: v.float().cuda().contiguous() for k, v in d.items() if v is not None}
+    has_c = "lstm" in cell
+    names = {"lstm": ["W", "R", "b"], "gru": ["W", "R", "bx", "br"], "indrnn": ["W", "u", "b"],
+             "layer_norm_lstm": ["W", "R", "b", "gamma", "gamma_h", "beta_h"],
+             "layer_norm_gru": ["W", "R", "bx", "br", "gamma"], "layer_norm_indrnn": ["W", "u", "b", "gamma"]}[cell]
+    forward, backward = getattr(lib, cell + "_forward"), getattr(lib, cell + "_backward")
+    states = [t["h0"], t["c0"]] if has_c else [t["h0"]]
+    fwd = [t["x"], *states, *[t[n] for n in names], t["mask"]]
+    out = forward(True, 0.2, *fwd)
+    out = list(out) if isinstance(out, (list, tuple)) else [out]
+    turned = [t[n].t().contiguous() if n in ("W", "R") else t[n] for n in names]
+    bwd = [t["x"].permute(2, 0, 1).contiguous(), *turned, t["mask"], *out, t["dh"]] + ([t["dc"]] if has_c else [])
+    short = lambda a: a.reshape(-1)[:-1].clone().view(*([1] * (a.dim() - 1)), -1)
+    read = lambda n: not (n == "gamma" and cell == "layer_norm_indrnn")
+    for i, n in enumerate(names):
+        if read(n) and n not in ("R", "u") and not (n == "W" and "indrnn" in cell):
+            bad = list(fwd)
+            bad[1 + len(states) + i] = short(bad[1 + len(states) + i])
+            _refused(lambda: forward(True, 0.2, *bad))
+    _refused(lambda: forward(True, 0.2, *fwd[:-1], short(fwd[-1])))
+    for i in range(1, len(bwd)):
+        n = names[i - 1] if i <= len(names) else ""
+        h = len(names) + 2
+        if i == h or not read(n) or n in ("b", "bx", "br"):
+            continue  # the sizes come from h; biases are not read; the second row of gamma neither
+        bad = list(bwd)
+        bad[i] = short(bad[i])
+        _refused(lambda: backward(*bad))
+    backward(*bwd)
