@@ -832,7 +832,7 @@ const char* refusal(const GemmDesc& g) {
   // Small problems are launch-bound either way; keep them on the generic kernel.
   if ((long long)g.M * g.N * g.K < (1LL << 21) || g.M < 8 || g.N < 32)
     return "problem too small for the tensor-core path";
-  if (g.dtype != HASTE_B200_BF16 && g.M < 32) return "few rows: fp32 sums";  // gemm.cu
+  if (g.dtype != HASTE_B200_BF16 && g.M < 32 && gemm_path() == HASTE_B200_GEMM_AUTO) return "few rows: fp32 sums";  // gemm.cu
   if ((g.a_cs != 1 && g.a_rs != 1) || (g.b_rs != 1 && g.b_cs != 1)) return "operand has no unit stride";
   return nullptr;
 }
