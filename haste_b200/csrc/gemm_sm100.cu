@@ -41,6 +41,7 @@ constexpr int UK = 16;                       // K of one tcgen05.mma (bf16)
 constexpr int TILE_BYTES = BM * BK * 2;      // one operand plane of one stage (A or B): 16 KiB
 constexpr int THREADS = 192;                 // warp 0 TMA, warp 1 MMA, warps 2..5 epilogue
 constexpr int NACC = 4;                      // fp32 accumulators of BN columns in tensor memory
+constexpr int EPI_TILE = 32 * 32 * 4;         // shared memory of an epilogue warp
 constexpr int TMEM_COLS = NACC * BN;         // (all 512 columns: one CTA per SM)
 
 struct Params {
@@ -48,6 +49,7 @@ struct Params {
   int a_mn_major, b_mn_major;  // 0: K contiguous, 1: M/N contiguous
   int tiles_m, tiles_n, splits, kb_per_split, kb_total;
   int c_is_bf16, accumulate;   // direct epilogue only; c_is_bf16: 0 fp32, 1 bf16, 2 fp16 output
+  int wide;                    // C's rows take stores of four values
   void* c;
   long long ldc;
   float* partial;              // non-null: write fp32 partial tiles [split][M][partial_ld]
@@ -62,7 +64,7 @@ struct Cfg {
   static constexpr int PLANES = NPROD == 1 ? 1 : (NPROD == 3 ? 2 : 3);
   static constexpr int STAGE_BYTES = 2 * PLANES * TILE_BYTES;
   static constexpr int STAGES = NPROD == 1 ? 6 : (NPROD == 3 ? 3 : 2);
-  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;  // + a tile per epilogue warp
   // fp32 storage: the tensor core adds every MMA result into the fp32 accumulator with
   // truncation, a bias of about half an ulp per accumulation that always points the same way;
   // over the few hundred accumulations of a long K it reaches 1e-5 of the result (measured:
@@ -76,95 +78,78 @@ struct Cfg {
   static constexpr int CHUNK = NPROD == 1 ? 0 : (NPROD == 3 ? 4 : 2);
 };
 
-// Stores 32 consecutive columns (starting at nb) of row m of the result: r holds the fp32 bit
-// patterns.  Partial tile of a K split, or the final C in fp32 / bf16 / fp16, optionally
-// accumulating into what C holds.
-__device__ __forceinline__ void store_chunk(const Params& p, int sp, int m, int nb,
-                                      const uint32_t (&r)[32]) {
-  if (m < p.M && nb < p.N) {
-    if (p.partial) {  // rows of whole chunks, 16-byte aligned
-      float* dst = p.partial + ((long long)sp * p.M + m) * p.partial_ld + nb;
-#pragma unroll
-      for (int j = 0; j < 32; j += 4)
-        *reinterpret_cast<float4*>(dst + j) =
-            make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
-                        __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
-    } else if (p.c_is_bf16) {
-      __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.c) + (long long)m * p.ldc + nb;
-      if (nb + 32 <= p.N && (p.ldc & 7) == 0 &&
-          (reinterpret_cast<uintptr_t>(p.c) & 15) == 0) {
-        // 16-byte stores: eight bf16 per store, four per 32-column chunk
-#pragma unroll
-        for (int j = 0; j < 32; j += 8) {
-          float v[8];
-#pragma unroll
-          for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[j + e]);
-          if (p.accumulate) {
-            const uint4 old = *reinterpret_cast<const uint4*>(dst + j);
-            const uint32_t ow[4] = {old.x, old.y, old.z, old.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              if (p.c_is_bf16 == 2) {
-                const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&ow[e]));
-                v[2 * e] += f.x;
-                v[2 * e + 1] += f.y;
-              } else {
-                v[2 * e] += __uint_as_float(ow[e] << 16);
-                v[2 * e + 1] += __uint_as_float(ow[e] & 0xFFFF0000u);
-              }
-            }
-          }
-          uint32_t w[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            if (p.c_is_bf16 == 2) {
-              __half2 t2 = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
-              w[e] = *reinterpret_cast<uint32_t*>(&t2);
-            } else {
-              __nv_bfloat162 t2 = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
-              w[e] = *reinterpret_cast<uint32_t*>(&t2);
-            }
-          }
-          *reinterpret_cast<uint4*>(dst + j) = make_uint4(w[0], w[1], w[2], w[3]);
+// Rows 0 .. rows - 1 of a 32 x 32 tile in shared memory (laid out by store_chunk) to dst, whose first
+// column is column n0 of the result, with `cols` columns to go.
+template <bool ADD, typename TC>
+__device__ __forceinline__ void store_tile(const float4* tile, TC* dst, long long ld_dst, int rows, int cols, bool wide) {
+  const int lane = threadIdx.x & 31;
+  if (wide) {
+    const int u = lane & 7;
+    if (u * 4 >= cols) return;
+#pragma unroll 4
+    for (int r = lane >> 3; r < rows; r += 4) {
+      float4 x = tile[r * 8 + (u ^ (r & 7))];
+      TC* to = dst + r * ld_dst + u * 4;
+      if constexpr (sizeof(TC) == 4) {
+        if (ADD) {
+          const float4 c = *reinterpret_cast<const float4*>(to);
+          x.x += c.x; x.y += c.y; x.z += c.z; x.w += c.w;
         }
+        *reinterpret_cast<float4*>(to) = x;
       } else {
-        for (int j = 0; j < 32 && nb + j < p.N; ++j) {
-          float v = __uint_as_float(r[j]);
-          if (p.c_is_bf16 == 2) {
-            __half* hd = reinterpret_cast<__half*>(dst);
-            if (p.accumulate) v += __half2float(hd[j]);
-            hd[j] = __float2half_rn(v);
-          } else {
-            if (p.accumulate) v += __bfloat162float(dst[j]);
-            dst[j] = __float2bfloat16_rn(v);
-          }
+        __align__(8) TC o[4];
+        if (ADD) {
+          *reinterpret_cast<uint2*>(o) = *reinterpret_cast<const uint2*>(to);
+          x.x += ld(o); x.y += ld(o + 1); x.z += ld(o + 2); x.w += ld(o + 3);
         }
+        st(o, x.x); st(o + 1, x.y); st(o + 2, x.z); st(o + 3, x.w);
+        *reinterpret_cast<uint2*>(to) = *reinterpret_cast<const uint2*>(o);
       }
-    } else {
-      float* dst = reinterpret_cast<float*>(p.c) + (long long)m * p.ldc + nb;
-      if (nb + 32 <= p.N && (p.ldc & 3) == 0 &&
-          (reinterpret_cast<uintptr_t>(p.c) & 15) == 0) {
-#pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-          float4 o = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
-                                 __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
-          if (p.accumulate) {
-            const float4 c0 = *reinterpret_cast<const float4*>(dst + j);
-            o.x += c0.x; o.y += c0.y; o.z += c0.z; o.w += c0.w;
-          }
-          *reinterpret_cast<float4*>(dst + j) = o;
-        }
-      } else {
-        for (int j = 0; j < 32 && nb + j < p.N; ++j) {
-          float v = __uint_as_float(r[j]);
-          if (p.accumulate) v += dst[j];
-          dst[j] = v;
-        }
-      }
+    }
+  } else {
+    if (lane >= cols) return;
+    const float* at = reinterpret_cast<const float*>(tile) + (lane & 3);
+#pragma unroll 4
+    for (int r = 0; r < rows; ++r) {
+      const float x = at[(r * 8 + ((lane >> 2) ^ (r & 7))) * 4];
+      TC* to = dst + r * ld_dst + lane;
+      st(to, ADD ? x + ld(to) : x);
     }
   }
 }
+template <typename TC>
+__device__ __forceinline__ void store_tile_c(const Params& p, const float4* tile, int m0, int n0) {
+  TC* dst = static_cast<TC*>(p.c) + m0 * p.ldc + n0;
+  const int rows = min(32, p.M - m0), cols = min(32, p.N - n0);
+  const bool wide = p.wide && (cols & 3) == 0;
+  if (p.accumulate) store_tile<true, TC>(tile, dst, p.ldc, rows, cols, wide);
+  else store_tile<false, TC>(tile, dst, p.ldc, rows, cols, wide);
+}
 
+// A warp stores 32 rows (m0 ..) x 32 columns (n0 ..) of the result; lane r holds row r.  The tile goes
+// through shared memory (`buf`, 4 KB of the warp's own), because a store instruction is paid per line
+// it touches: 8 lanes per row write whole 128-byte lines, four per instruction instead of 32, and
+// where C's rows start anywhere a warp still writes one row at a time.  The 16-byte pieces of a row
+// are rotated by the row so that both sides touch all banks.
+// (Row by row from the lanes, the epilogue bounded outputs with a short K and cost the others their last
+// tile; before / now: bf16 64000 x 3072, K = 512 412 / 234 us, 4096^3 112 / 97; fp32 64000 x 2048, K = 512
+// 424 / 346, 256000 x 1024, K = 1024 1691 / 1475, 12321 x 750, K = 161 54 / 34, which went through a padded tile.)
+__device__ __forceinline__ void store_chunk(const Params& p, int sp, int m0, int n0, const float* v, uint8_t* buf) {
+  if (m0 >= p.M || n0 >= p.N) return;  // the same for the whole warp
+  const int lane = threadIdx.x & 31;
+  float4* tile = reinterpret_cast<float4*>(buf);
+  __syncwarp();  // the tile before has been read
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    tile[lane * 8 + (j ^ (lane & 7))] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+  __syncwarp();
+  if (p.partial)  // rows of whole chunks
+    store_tile<false, float>(tile, p.partial + ((long long)sp * p.M + m0) * p.partial_ld + n0, p.partial_ld,
+                             min(32, p.M - m0), 32, true);
+  else if (p.c_is_bf16 == 0) store_tile_c<float>(p, tile, m0, n0);
+  else if (p.c_is_bf16 == 1) store_tile_c<__nv_bfloat16>(p, tile, m0, n0);
+  else store_tile_c<__half>(p, tile, m0, n0);
+}
 template <int NPROD>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
@@ -310,6 +295,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
   } else {
     // ------------------------------------------------------------------ epilogue
     const int quad = warp & 3;  // tensor-memory lane quadrant this warp may read
+    uint8_t* tile = aligned + C::STAGES * C::STAGE_BYTES + 256 + (warp - 2) * EPI_TILE;
     uint32_t acc_phase = 0;  // one parity bit per accumulator
     int cidx = 0;
     bool ok = true;
@@ -320,7 +306,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
       const int kb0 = sp * p.kb_per_split;
       const int kb1 = min(p.kb_total, kb0 + p.kb_per_split);
       const int nchunks = C::CHUNK ? (kb1 - kb0 + C::CHUNK - 1) / C::CHUNK : 1;
-      const int m = tm * BM + quad * 32 + lane;
+      const int m0 = tm * BM + quad * 32;
       const int n0 = tn * BN;
       // running sums of this thread's row of the tile (only with chunked hand-over)
       float sum[C::CHUNK ? BN : 1];
@@ -350,7 +336,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
             uint32_t r[32];
             tc_ld32(taddr + ch * 32, r);
             tc_wait_ld();
-            store_chunk(p, sp, m, n0 + ch * 32, r);
+            float v[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+            store_chunk(p, sp, m0, n0 + ch * 32, v, tile);
           }
         }
         tc_fence_before();
@@ -359,12 +348,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
       if (!ok) break;
       if (C::CHUNK) {
 #pragma unroll
-        for (int ch = 0; ch < BN / 32; ++ch) {
-          uint32_t r[32];
-#pragma unroll
-          for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(sum[(C::CHUNK ? ch * 32 : 0) + j]);
-          store_chunk(p, sp, m, n0 + ch * 32, r);
-        }
+        for (int ch = 0; ch < BN / 32; ++ch)
+          store_chunk(p, sp, m0, n0 + ch * 32, sum + (C::CHUNK ? ch * 32 : 0), tile);
       }
     }
   }
@@ -545,6 +530,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
   } else {
     // ------------------------------------------------------------------ epilogue (both CTAs)
     const int quad = warp & 3;         // tensor-memory lane quadrant this warp may read
+    uint8_t* tile = aligned + C::STAGES * C::STAGE_BYTES + 256 + (warp - 2) * EPI_TILE;
     const int half = (warp - 2) >> 2;  // which 128 columns of the accumulator
     uint32_t acc_phase = 0;  // one parity bit per accumulator
     int cidx = 0;
@@ -556,7 +542,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       const int kb0 = sp * p.kb_per_split;
       const int kb1 = min(p.kb_total, kb0 + p.kb_per_split);
       const int nchunks = C::CHUNK ? (kb1 - kb0 + C::CHUNK - 1) / C::CHUNK : 1;
-      const int m = tm * PBM + (int)rank * BM + quad * 32 + lane;
+      const int m0 = tm * PBM + (int)rank * BM + quad * 32;
       const int n0 = tn * PBN + half * BN;
       float sum[C::CHUNK ? BN : 1];
 #pragma unroll
@@ -585,7 +571,10 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
             uint32_t r[32];
             tc_ld32(taddr + ch * 32, r);
             tc_wait_ld();
-            store_chunk(p, sp, m, n0 + ch * 32, r);
+            float v[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+            store_chunk(p, sp, m0, n0 + ch * 32, v, tile);
           }
         }
         tc_fence_before();
@@ -595,12 +584,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       if (!ok) break;
       if (C::CHUNK) {
 #pragma unroll
-        for (int ch = 0; ch < BN / 32; ++ch) {
-          uint32_t r[32];
-#pragma unroll
-          for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(sum[(C::CHUNK ? ch * 32 : 0) + j]);
-          store_chunk(p, sp, m, n0 + ch * 32, r);
-        }
+        for (int ch = 0; ch < BN / 32; ++ch)
+          store_chunk(p, sp, m0, n0 + ch * 32, sum + (C::CHUNK ? ch * 32 : 0), tile);
       }
     }
   }
@@ -765,18 +750,24 @@ constexpr int kMaxDevices = 64;
 std::atomic<bool> g_attr_set[kMaxDevices];
 std::atomic<int> g_max_pairs[kMaxDevices];  // 0: not asked yet, -1: no clusters, else the count
 
+template <int NPROD>
+constexpr int single_smem() { return Cfg<NPROD>::SMEM + 4 * EPI_TILE; }
+template <int NPROD>
+constexpr int pair_smem() { return Cfg<NPROD>::SMEM + PAIR_EPI_WARPS * EPI_TILE; }
+static_assert(pair_smem<1>() <= 232448 && pair_smem<3>() <= 232448 && pair_smem<6>() <= 232448, "shared memory per CTA");
+
 int set_kernel_attributes() {
   int dev = 0;
   HB_CUDA_OK(cudaGetDevice(&dev));
   if (dev >= 0 && dev < kMaxDevices && g_attr_set[dev].load(std::memory_order_acquire))
     return HASTE_B200_OK;
   const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  HB_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<1>, attr, Cfg<1>::SMEM));
-  HB_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<3>, attr, Cfg<3>::SMEM));
-  HB_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<6>, attr, Cfg<6>::SMEM));
-  HB_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<1>, attr, Cfg<1>::SMEM));
-  HB_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<3>, attr, Cfg<3>::SMEM));
-  HB_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<6>, attr, Cfg<6>::SMEM));
+  HB_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<1>, attr, single_smem<1>()));
+  HB_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<3>, attr, single_smem<3>()));
+  HB_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_kernel<6>, attr, single_smem<6>()));
+  HB_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<1>, attr, pair_smem<1>()));
+  HB_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<3>, attr, pair_smem<3>()));
+  HB_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<6>, attr, pair_smem<6>()));
   if (dev >= 0 && dev < kMaxDevices) g_attr_set[dev].store(true, std::memory_order_release);
   return HASTE_B200_OK;
 }
@@ -793,7 +784,7 @@ int max_pairs() {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(2 * sm_count());
       cfg.blockDim = dim3(PAIR_THREADS);
-      cfg.dynamicSmemBytes = Cfg<6>::SMEM;
+      cfg.dynamicSmemBytes = pair_smem<6>();
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
       attr[0].val.clusterDim.x = 2;
@@ -916,13 +907,8 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
   const int planes = f32 ? (g.precise ? 3 : 2) : 1;
   const size_t a_plane = a_copy ? Arena::pad((size_t)a_rows * a_ld * 2) : 0;
   const size_t b_plane = b_copy ? Arena::pad((size_t)b_rows * b_ld * 2) : 0;
-  // The epilogue stores a row per lane in 16-byte pieces.  Element by element - a C whose rows do
-  // not start on 16 bytes - each store touches 32 lines and the epilogue took five times the MMAs
-  // ([12321 x 161] . [161 x 750] in fp32: 56 us), so such a C goes through a padded fp32 tile as
-  // the parts of a K split do, and the reduction writes it row by row.
-  const bool c_rows = (g.ldc % (g.dtype_c == HASTE_B200_F32 ? 4 : 8)) == 0 && ((uintptr_t)g.c & 15) == 0;
   const int part_ld = (N + 31) & ~31;
-  const bool via_partial = splits > 1 || (!c_rows && M >= 64 && (long long)M * (part_ld / 4) < (1LL << 31));
+  const bool via_partial = splits > 1;
   const size_t part_bytes = via_partial ? Arena::pad((size_t)splits * M * part_ld * 4) : 0;
   const size_t bytes = planes * (a_plane + b_plane) + part_bytes + 1024;
   Arena ws;
@@ -971,6 +957,7 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
   p.c_is_bf16 = g.dtype_c == HASTE_B200_BF16 ? 1 : (g.dtype_c == HASTE_B200_F16 ? 2 : 0);
   p.accumulate = g.accumulate;
   p.c = g.c; p.ldc = g.ldc;
+  p.wide = (g.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(g.c) & (4 * dtype_size(g.dtype_c) - 1)) == 0;
   p.partial = partial;
   p.partial_ld = part_ld;
   p.err = err;
@@ -989,23 +976,23 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     if (planes == 3) {
-      cfg.dynamicSmemBytes = Cfg<6>::SMEM;
+      cfg.dynamicSmemBytes = pair_smem<6>();
       HB_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_tcgen05_pair_kernel<6>, m_a, m_b, p));
     } else if (planes == 2) {
-      cfg.dynamicSmemBytes = Cfg<3>::SMEM;
+      cfg.dynamicSmemBytes = pair_smem<3>();
       HB_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_tcgen05_pair_kernel<3>, m_a, m_b, p));
     } else {
-      cfg.dynamicSmemBytes = Cfg<1>::SMEM;
+      cfg.dynamicSmemBytes = pair_smem<1>();
       HB_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_tcgen05_pair_kernel<1>, m_a, m_b, p));
     }
   } else {
     const int grid = min(sms, tiles_m * tiles_n * splits);
     if (planes == 3)
-      gemm_tcgen05_kernel<6><<<grid, THREADS, Cfg<6>::SMEM, stream>>>(m_a, m_b, p);
+      gemm_tcgen05_kernel<6><<<grid, THREADS, single_smem<6>(), stream>>>(m_a, m_b, p);
     else if (planes == 2)
-      gemm_tcgen05_kernel<3><<<grid, THREADS, Cfg<3>::SMEM, stream>>>(m_a, m_b, p);
+      gemm_tcgen05_kernel<3><<<grid, THREADS, single_smem<3>(), stream>>>(m_a, m_b, p);
     else
-      gemm_tcgen05_kernel<1><<<grid, THREADS, Cfg<1>::SMEM, stream>>>(m_a, m_b, p);
+      gemm_tcgen05_kernel<1><<<grid, THREADS, single_smem<1>(), stream>>>(m_a, m_b, p);
   }
   HB_LAUNCH_OK();
   count_launch(1);
