@@ -10,6 +10,8 @@
 //   (hi.hi + hi.lo + lo.hi).  The dropped lo.lo term and the plane rounding leave a
 //   relative error near 2^-17 per product, far inside the 1e-4 parity bar, at 3/16 of
 //   the fp32 CUDA-core cost.
+// * fp32 storage, large contractions whose error a LayerNorm or a long recurrence would amplify: two
+//   fp16 planes per operand, scaled by row and column (see split_f16_kernel), three products.
 // * Either operand may be K-major or MN-major (every transpose the cells need), chosen
 //   from its strides; no data is ever transposed in memory.
 // * Persistent kernel: one CTA per SM walks (tile, k-split) work items.  Warp 0 issues
@@ -52,6 +54,9 @@ struct Params {
   int wide;                    // C's rows take stores of four values
   void* c;
   long long ldc;
+  const int* a_exp;            // fp16 planes: the result's row m, column n is to be scaled by
+  const signed char* b_exp;    // 2^(a_exp[m] + b_exp[n]); null otherwise
+  int chunk;                   // k-blocks per hand-over of the accumulator (Cfg::CHUNK != 0)
   float* partial;              // non-null: write fp32 partial tiles [split][M][partial_ld]
   int partial_ld;              // N rounded up to whole 32-column chunks
   int* err;
@@ -78,17 +83,45 @@ struct Cfg {
   static constexpr int CHUNK = NPROD == 1 ? 0 : (NPROD == 3 ? 4 : 2);
 };
 
-// Rows 0 .. rows - 1 of a 32 x 32 tile in shared memory (laid out by store_chunk) to dst, whose first
-// column is column n0 of the result, with `cols` columns to go.
-template <bool ADD, typename TC>
-__device__ __forceinline__ void store_tile(const float4* tile, TC* dst, long long ld_dst, int rows, int cols, bool wide) {
+__device__ __forceinline__ float exp2_int(int e) {  // 2^e, -126 <= e <= 127
+  return __uint_as_float((uint32_t)(e + 127) << 23);
+}
+
+// The powers of two that fp16 planes leave in a tile: of this lane's row, and of the four columns that the
+// lane stores of each 32-column chunk.  Loaded before the products are there.
+struct TileScale {
+  int row;
+  int cols[BN / 32];
+  __device__ __forceinline__ void load(const Params& p, int m0, int n0) {
+    const int lane = threadIdx.x & 31;
+    row = m0 + lane < p.M ? p.a_exp[m0 + lane] : 0;
+#pragma unroll
+    for (int c = 0; c < BN / 32; ++c)
+      cols[c] = *reinterpret_cast<const int*>(p.b_exp + n0 + c * 32 + (lane & 7) * 4);
+  }
+};
+// Rows 0 .. rows - 1 of a 32 x 32 tile in shared memory (laid out by store_chunk) to dst, `cols` columns wide.
+// `ea`, `eb`: see TileScale and store_chunk.
+template <bool SCALED, bool ADD, typename TC>
+__device__ __forceinline__ void store_tile(const float4* tile, TC* dst, long long ld_dst, int rows, int cols, bool wide,
+                                           int ea, int eb) {
   const int lane = threadIdx.x & 31;
   if (wide) {
     const int u = lane & 7;
-    if (u * 4 >= cols) return;
+    float4 fb = make_float4(1.f, 1.f, 1.f, 1.f);
+    if (SCALED)
+      fb = make_float4(exp2_int((signed char)eb), exp2_int((signed char)(eb >> 8)), exp2_int((signed char)(eb >> 16)),
+                       exp2_int(eb >> 24));
 #pragma unroll 4
-    for (int r = lane >> 3; r < rows; r += 4) {
+    for (int i = 0; i < 8; ++i) {
+      const int r = i * 4 + (lane >> 3), e = SCALED ? __shfl_sync(0xffffffffu, ea, r) : 0;
+      if (r >= rows || u * 4 >= cols) continue;
       float4 x = tile[r * 8 + (u ^ (r & 7))];
+      if (SCALED) {
+        const float f1 = exp2_int(e >> 1), f2 = exp2_int(e - (e >> 1));
+        x.x = x.x * f1 * fb.x * f2; x.y = x.y * f1 * fb.y * f2;
+        x.z = x.z * f1 * fb.z * f2; x.w = x.w * f1 * fb.w * f2;
+      }
       TC* to = dst + r * ld_dst + u * 4;
       if constexpr (sizeof(TC) == 4) {
         if (ADD) {
@@ -107,23 +140,28 @@ __device__ __forceinline__ void store_tile(const float4* tile, TC* dst, long lon
       }
     }
   } else {
-    if (lane >= cols) return;
+    // column `lane`, whose power its quad's lane has
+    const int e4 = SCALED ? __shfl_sync(0xffffffffu, eb, lane >> 2) : 0;
+    const float fb = SCALED ? exp2_int((signed char)(e4 >> 8 * (lane & 3))) : 1.f;
     const float* at = reinterpret_cast<const float*>(tile) + (lane & 3);
 #pragma unroll 4
     for (int r = 0; r < rows; ++r) {
-      const float x = at[(r * 8 + ((lane >> 2) ^ (r & 7))) * 4];
+      const int e = SCALED ? __shfl_sync(0xffffffffu, ea, r) : 0;
+      if (lane >= cols) continue;
+      float x = at[(r * 8 + ((lane >> 2) ^ (r & 7))) * 4];
+      if (SCALED) x = x * exp2_int(e >> 1) * fb * exp2_int(e - (e >> 1));
       TC* to = dst + r * ld_dst + lane;
       st(to, ADD ? x + ld(to) : x);
     }
   }
 }
-template <typename TC>
-__device__ __forceinline__ void store_tile_c(const Params& p, const float4* tile, int m0, int n0) {
+template <bool SCALED, typename TC>
+__device__ __forceinline__ void store_tile_c(const Params& p, const float4* tile, int m0, int n0, int ea, int eb) {
   TC* dst = static_cast<TC*>(p.c) + m0 * p.ldc + n0;
   const int rows = min(32, p.M - m0), cols = min(32, p.N - n0);
   const bool wide = p.wide && (cols & 3) == 0;
-  if (p.accumulate) store_tile<true, TC>(tile, dst, p.ldc, rows, cols, wide);
-  else store_tile<false, TC>(tile, dst, p.ldc, rows, cols, wide);
+  if (p.accumulate) store_tile<SCALED, true, TC>(tile, dst, p.ldc, rows, cols, wide, ea, eb);
+  else store_tile<SCALED, false, TC>(tile, dst, p.ldc, rows, cols, wide, ea, eb);
 }
 
 // A warp stores 32 rows (m0 ..) x 32 columns (n0 ..) of the result; lane r holds row r.  The tile goes
@@ -134,7 +172,12 @@ __device__ __forceinline__ void store_tile_c(const Params& p, const float4* tile
 // (Row by row from the lanes, the epilogue bounded outputs with a short K and cost the others their last
 // tile; before / now: bf16 64000 x 3072, K = 512 412 / 234 us, 4096^3 112 / 97; fp32 64000 x 2048, K = 512
 // 424 / 346, 256000 x 1024, K = 1024 1691 / 1475, 12321 x 750, K = 161 54 / 34, which went through a padded tile.)
-__device__ __forceinline__ void store_chunk(const Params& p, int sp, int m0, int n0, const float* v, uint8_t* buf) {
+// fp16 planes: row m, column n times 2^(a_exp[m] + b_exp[n]), the row's power in two halves around the
+// column's, so that no step leaves the range of a float unless the result does.  (b_exp is readable up
+// to whole tiles.)
+template <bool SCALED>
+__device__ __forceinline__ void store_chunk(const Params& p, int sp, int m0, int n0, const float* v, uint8_t* buf,
+                                            int ea = 0, int eb = 0) {
   if (m0 >= p.M || n0 >= p.N) return;  // the same for the whole warp
   const int lane = threadIdx.x & 31;
   float4* tile = reinterpret_cast<float4*>(buf);
@@ -144,12 +187,13 @@ __device__ __forceinline__ void store_chunk(const Params& p, int sp, int m0, int
     tile[lane * 8 + (j ^ (lane & 7))] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
   __syncwarp();
   if (p.partial)  // rows of whole chunks
-    store_tile<false, float>(tile, p.partial + ((long long)sp * p.M + m0) * p.partial_ld + n0, p.partial_ld,
-                             min(32, p.M - m0), 32, true);
-  else if (p.c_is_bf16 == 0) store_tile_c<float>(p, tile, m0, n0);
-  else if (p.c_is_bf16 == 1) store_tile_c<__nv_bfloat16>(p, tile, m0, n0);
-  else store_tile_c<__half>(p, tile, m0, n0);
+    store_tile<SCALED, false, float>(tile, p.partial + ((long long)sp * p.M + m0) * p.partial_ld + n0, p.partial_ld,
+                                     min(32, p.M - m0), 32, true, ea, eb);
+  else if (p.c_is_bf16 == 0) store_tile_c<SCALED, float>(p, tile, m0, n0, ea, eb);
+  else if (p.c_is_bf16 == 1) store_tile_c<SCALED, __nv_bfloat16>(p, tile, m0, n0, ea, eb);
+  else store_tile_c<SCALED, __half>(p, tile, m0, n0, ea, eb);
 }
+
 template <int NPROD>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
@@ -238,7 +282,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |
+      const uint32_t type = p.a_exp ? 0u : 1u;  // fp16 or bf16 operands
+      const uint32_t idesc = (1u << 4) | (type << 7) | (type << 10) |
                              ((uint32_t)p.a_mn_major << 15) | ((uint32_t)p.b_mn_major << 16) |
                              ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
       // K-major: 8-row groups 1024 B apart, a K step of 16 elements is 32 B along the row.
@@ -262,7 +307,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
           acc_phase ^= 1u << acc;
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + acc * BN;
-          const int kend = C::CHUNK ? min(kb1, kb + C::CHUNK) : kb1;
+          const int kend = C::CHUNK ? min(kb1, kb + p.chunk) : kb1;
           uint32_t first = 1;
           for (; kb < kend; ++kb) {
             if (!mbar_wait(full_bar(stage), phase, abort_flag, p.err, 3)) { ok = false; break; }
@@ -305,9 +350,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
       const int sp = item / (p.tiles_n * p.tiles_m);
       const int kb0 = sp * p.kb_per_split;
       const int kb1 = min(p.kb_total, kb0 + p.kb_per_split);
-      const int nchunks = C::CHUNK ? (kb1 - kb0 + C::CHUNK - 1) / C::CHUNK : 1;
+      const int nchunks = C::CHUNK ? (kb1 - kb0 + p.chunk - 1) / p.chunk : 1;
       const int m0 = tm * BM + quad * 32;
       const int n0 = tn * BN;
+      const bool scaled = NPROD == 3 && p.a_exp;
+      TileScale scale;
+      if (scaled) scale.load(p, m0, n0);
       // running sums of this thread's row of the tile (only with chunked hand-over)
       float sum[C::CHUNK ? BN : 1];
 #pragma unroll
@@ -339,7 +387,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
             float v[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-            store_chunk(p, sp, m0, n0 + ch * 32, v, tile);
+            store_chunk<false>(p, sp, m0, n0 + ch * 32, v, tile);
           }
         }
         tc_fence_before();
@@ -348,8 +396,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
       if (!ok) break;
       if (C::CHUNK) {
 #pragma unroll
-        for (int ch = 0; ch < BN / 32; ++ch)
-          store_chunk(p, sp, m0, n0 + ch * 32, sum + (C::CHUNK ? ch * 32 : 0), tile);
+        for (int ch = 0; ch < BN / 32; ++ch) {
+          const float* v = sum + (C::CHUNK ? ch * 32 : 0);
+          if (scaled) store_chunk<true>(p, sp, m0, n0 + ch * 32, v, tile, scale.row, scale.cols[ch]);
+          else store_chunk<false>(p, sp, m0, n0 + ch * 32, v, tile);
+        }
       }
     }
   }
@@ -478,7 +529,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (CTA 0 only)
     if (lane == 0 && rank == 0) {
-      const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) |
+      const uint32_t type = p.a_exp ? 0u : 1u;  // fp16 or bf16 operands
+      const uint32_t idesc = (1u << 4) | (type << 7) | (type << 10) |
                              ((uint32_t)p.a_mn_major << 15) | ((uint32_t)p.b_mn_major << 16) |
                              ((uint32_t)(PBN >> 3) << 17) | ((uint32_t)(PBM >> 4) << 24);
       const uint32_t a_lbo = p.a_mn_major ? TILE_BYTES / 2 : 16, a_kstep = p.a_mn_major ? 2048 : 32;
@@ -499,7 +551,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
           acc_phase ^= 1u << acc;
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + acc * PBN;
-          const int kend = C::CHUNK ? min(kb1, kb + C::CHUNK) : kb1;
+          const int kend = C::CHUNK ? min(kb1, kb + p.chunk) : kb1;
           uint32_t first = 1;
           for (; kb < kend; ++kb) {
             if (!mbar_wait_cluster(full_bar(stage), phase, abort_flag, p.err, 13)) { ok = false; break; }
@@ -541,9 +593,12 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       const int sp = item / (p.tiles_n * p.tiles_m);
       const int kb0 = sp * p.kb_per_split;
       const int kb1 = min(p.kb_total, kb0 + p.kb_per_split);
-      const int nchunks = C::CHUNK ? (kb1 - kb0 + C::CHUNK - 1) / C::CHUNK : 1;
+      const int nchunks = C::CHUNK ? (kb1 - kb0 + p.chunk - 1) / p.chunk : 1;
       const int m0 = tm * PBM + (int)rank * BM + quad * 32;
       const int n0 = tn * PBN + half * BN;
+      const bool scaled = NPROD == 3 && p.a_exp;
+      TileScale scale;
+      if (scaled) scale.load(p, m0, n0);
       float sum[C::CHUNK ? BN : 1];
 #pragma unroll
       for (int j = 0; j < (C::CHUNK ? BN : 1); ++j) sum[j] = 0.f;
@@ -574,7 +629,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
             float v[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-            store_chunk(p, sp, m0, n0 + ch * 32, v, tile);
+            store_chunk<false>(p, sp, m0, n0 + ch * 32, v, tile);
           }
         }
         tc_fence_before();
@@ -584,8 +639,11 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       if (!ok) break;
       if (C::CHUNK) {
 #pragma unroll
-        for (int ch = 0; ch < BN / 32; ++ch)
-          store_chunk(p, sp, m0, n0 + ch * 32, sum + (C::CHUNK ? ch * 32 : 0), tile);
+        for (int ch = 0; ch < BN / 32; ++ch) {
+          const float* v = sum + (C::CHUNK ? ch * 32 : 0);
+          if (scaled) store_chunk<true>(p, sp, m0, n0 + ch * 32, v, tile, scale.row, scale.cols[ch]);
+          else store_chunk<false>(p, sp, m0, n0 + ch * 32, v, tile);
+        }
       }
     }
   }
@@ -663,13 +721,149 @@ __global__ void split_planes_kernel(const SplitJob job0, const SplitJob job1) {
   }
 }
 
+// ---- two fp16 planes per fp32 operand ---------------------------------------------------------
+// x 2^s = p0 + p1, p0 and p1 the fp16 roundings of x 2^s and of what is left: 22 .. 23 bits of x where
+// three bf16 planes keep 24, for three products instead of six and two thirds of the operand bytes.
+// s makes the largest value of a row of A (a column of B) 2^14 .. 2^15, so that values down to 2^-17 of
+// it keep all their bits and smaller ones an absolute error of 2^-40 of it; the epilogue takes the
+// powers out again.
+// k-blocks per hand-over of the accumulator: 24 truncated accumulations, half of the bf16 planes' (relative
+// error of 16384 x 1024 x 1024 against fp64: six bf16 products 1.17e-6, these 6.2e-7, with twice the chunk
+// 1.07e-6 and 2 % less time).
+constexpr int kF16Chunk = 2;
+constexpr int F16_THREADS = 512, F16_ROW_QUADS = 8 * 32;  // quads of a row that a warp holds in registers
+
+__device__ __forceinline__ int f16_shift(float most) {  // non-finite rows are non-finite either way
+  if (!(most > 0.f) || isinf(most)) return 0;
+  int e;
+  frexpf(most, &e);  // most = f 2^e, 0.5 <= f < 1
+  return max(-126, min(126, 15 - e));
+}
+__device__ __forceinline__ float abs_max4(float m, const float4& v) {
+  return fmaxf(fmaxf(fmaxf(m, fabsf(v.x)), fmaxf(fabsf(v.y), fabsf(v.z))), fabsf(v.w));
+}
+__device__ __forceinline__ float4 load_quad(const float* row, int c, int cols, int vec_ok) {
+  if (vec_ok && c + 3 < cols) return *reinterpret_cast<const float4*>(row + c);
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (c < cols) v.x = row[c];
+  if (c + 1 < cols) v.y = row[c + 1];
+  if (c + 2 < cols) v.z = row[c + 2];
+  if (c + 3 < cols) v.w = row[c + 3];
+  return v;
+}
+__device__ __forceinline__ void store_f16_quad(__half* dst, long long plane_stride, const float4& v, float4 scale) {
+  const float x[4] = {v.x * scale.x, v.y * scale.y, v.z * scale.z, v.w * scale.w};
+  const __half2 a = __floats2half2_rn(x[0], x[1]), b = __floats2half2_rn(x[2], x[3]);
+  const __half2 c = __floats2half2_rn(x[0] - __low2float(a), x[1] - __high2float(a));
+  const __half2 d = __floats2half2_rn(x[2] - __low2float(b), x[3] - __high2float(b));
+  *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+  *reinterpret_cast<uint2*>(dst + plane_stride) =
+      make_uint2(*reinterpret_cast<const uint32_t*>(&c), *reinterpret_cast<const uint32_t*>(&d));
+}
+// A warp takes 8 / QL rows at a time, of which it holds QL quads per lane; longer rows are read twice.
+template <int QL>
+__device__ __forceinline__ void split_f16_rows(const SplitJob& a, int* __restrict__ a_exp) {
+  constexpr int RW = 8 / QL;
+  const int lane = threadIdx.x & 31, quads = (int)(a.ld_dst / 4), step = gridDim.x * (F16_THREADS / 32) * RW;
+  for (int r0 = (blockIdx.x * (F16_THREADS / 32) + (threadIdx.x >> 5)) * RW; r0 < a.rows; r0 += step) {
+    float4 v[RW][QL];
+    float most[RW];
+#pragma unroll
+    for (int k = 0; k < RW; ++k) {
+      const float* src = static_cast<const float*>(a.src) + (r0 + k) * a.ld_src;
+      most[k] = 0.f;
+#pragma unroll
+      for (int i = 0; i < QL; ++i)
+        v[k][i] = load_quad(src, (lane + 32 * i) * 4, r0 + k < a.rows ? a.cols : 0, a.vec_ok);
+    }
+#pragma unroll
+    for (int k = 0; k < RW; ++k) {
+#pragma unroll
+      for (int i = 0; i < QL; ++i) most[k] = abs_max4(most[k], v[k][i]);
+      if (QL == 8) {
+        const float* src = static_cast<const float*>(a.src) + r0 * a.ld_src;
+        for (int q = F16_ROW_QUADS + lane; q < quads; q += 32) most[k] = abs_max4(most[k], load_quad(src, q * 4, a.cols, a.vec_ok));
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) most[k] = fmaxf(most[k], __shfl_xor_sync(0xffffffffu, most[k], o));
+    }
+#pragma unroll
+    for (int k = 0; k < RW; ++k) {
+      if (r0 + k >= a.rows) break;
+      __half* dst = reinterpret_cast<__half*>(a.dst) + (r0 + k) * a.ld_dst;
+      const int s = f16_shift(most[k]);
+      const float f = exp2_int(s);
+      const float4 scale = make_float4(f, f, f, f);
+      if (lane == 0) a_exp[r0 + k] = -s;
+#pragma unroll
+      for (int i = 0; i < QL; ++i)
+        if (lane + 32 * i < quads) store_f16_quad(dst + (lane + 32 * i) * 4, a.plane_stride, v[k][i], scale);
+      if (QL == 8) {
+        const float* src = static_cast<const float*>(a.src) + r0 * a.ld_src;
+        for (int q = F16_ROW_QUADS + lane; q < quads; q += 32)
+          store_f16_quad(dst + q * 4, a.plane_stride, load_quad(src, q * 4, a.cols, a.vec_ok), scale);
+      }
+    }
+  }
+}
+// blockIdx.y = 0: `a`, scaled by row, a warp per row or few; 1: `b`, scaled by column, 32 columns per block (its
+// second reading comes from L2).  Bound by HBM: 256000 x 1024 takes one reading and one writing.
+__global__ void __launch_bounds__(F16_THREADS) split_f16_kernel(const SplitJob a, int* __restrict__ a_exp, const SplitJob b,
+                                                                signed char* __restrict__ b_exp) {
+  if (blockIdx.y == 0) {
+    const int quads = (int)(a.ld_dst / 4);
+    if (quads <= 32) split_f16_rows<1>(a, a_exp);
+    else if (quads <= 64) split_f16_rows<2>(a, a_exp);
+    else if (quads <= 128) split_f16_rows<4>(a, a_exp);
+    else split_f16_rows<8>(a, a_exp);
+  } else {
+    __shared__ float4 part[F16_THREADS];
+    const int q = threadIdx.x & 7, ry = threadIdx.x >> 3;
+    constexpr int RY = F16_THREADS / 8;
+    for (int c0 = blockIdx.x * 32; c0 < (int)b.ld_dst; c0 += gridDim.x * 32) {
+      const int c = c0 + q * 4;
+      const float* src = static_cast<const float*>(b.src);
+      float4 most = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+      for (int r = ry; r < b.rows; r += RY) {
+        const float4 v = load_quad(src + r * b.ld_src, c, b.cols, b.vec_ok);
+        most = make_float4(fmaxf(most.x, fabsf(v.x)), fmaxf(most.y, fabsf(v.y)), fmaxf(most.z, fabsf(v.z)),
+                           fmaxf(most.w, fabsf(v.w)));
+      }
+      __syncthreads();  // the columns before have been read
+      part[threadIdx.x] = most;
+      __syncthreads();
+      for (int h = RY / 2; h > 0; h >>= 1) {
+        if (ry < h) {
+          const float4 o = part[threadIdx.x + h * 8];
+          float4& m = part[threadIdx.x];
+          m = make_float4(fmaxf(m.x, o.x), fmaxf(m.y, o.y), fmaxf(m.z, o.z), fmaxf(m.w, o.w));
+        }
+        __syncthreads();
+      }
+      most = part[q];
+      const int4 s = make_int4(f16_shift(most.x), f16_shift(most.y), f16_shift(most.z), f16_shift(most.w));
+      const float4 scale = make_float4(exp2_int(s.x), exp2_int(s.y), exp2_int(s.z), exp2_int(s.w));
+      if (c < (int)b.ld_dst) {
+        if (ry == 0) *reinterpret_cast<char4*>(b_exp + c) = make_char4(-s.x, -s.y, -s.z, -s.w);
+#pragma unroll 4
+        for (int r = ry; r < b.rows; r += RY)
+          store_f16_quad(reinterpret_cast<__half*>(b.dst) + r * b.ld_dst + c, b.plane_stride,
+                         load_quad(src + r * b.ld_src, c, b.cols, b.vec_ok), scale);
+      }
+    }
+  }
+}
+
 // `dtype` of the sources.  __half: its 11 significant bits split exactly into two planes.  bf16: one
 // plane, a copy with rows that TMA can address.  jobs: one or two.
+bool wide_rows(const SplitJob& job, int dtype) {
+  return (job.ld_src & 3) == 0 && (reinterpret_cast<uintptr_t>(job.src) & (dtype == HASTE_B200_F32 ? 15 : 7)) == 0;
+}
 int launch_split(SplitJob* jobs, int n, int dtype, int planes, cudaStream_t stream) {
   long long most = 0;
   for (int i = 0; i < n; ++i) {
-    jobs[i].vec_ok = (jobs[i].ld_src & 3) == 0 &&
-                     (reinterpret_cast<uintptr_t>(jobs[i].src) & (dtype == HASTE_B200_F32 ? 15 : 7)) == 0;
+    jobs[i].vec_ok = wide_rows(jobs[i], dtype);
     most = std::max(most, (long long)jobs[i].rows * (jobs[i].ld_dst / 4));
   }
   const dim3 grid(min(ceil_div(most, 256), 8 * sm_count()), n);
@@ -679,6 +873,16 @@ int launch_split(SplitJob* jobs, int n, int dtype, int planes, cudaStream_t stre
   else if (dtype == HASTE_B200_F16) split_planes_kernel<2, __half><<<grid, 256, 0, stream>>>(a, b);
   else if (planes == 3) split_planes_kernel<3, float><<<grid, 256, 0, stream>>>(a, b);
   else split_planes_kernel<2, float><<<grid, 256, 0, stream>>>(a, b);
+  HB_LAUNCH_OK();
+  count_launch(1);
+  return HASTE_B200_OK;
+}
+
+int launch_split_f16(SplitJob* jobs, int* a_exp, signed char* b_exp, cudaStream_t stream) {
+  for (int i = 0; i < 2; ++i) jobs[i].vec_ok = wide_rows(jobs[i], HASTE_B200_F32);
+  const int per_warp = (int)(8 / max(1LL, min(8LL, (jobs[0].ld_dst + 127) / 128)));  // about what split_f16_rows takes
+  const int blocks = max(ceil_div(jobs[0].rows, F16_THREADS / 32 * per_warp), ceil_div(jobs[1].cols, 32));
+  split_f16_kernel<<<dim3(min(blocks, 4 * sm_count()), 2), F16_THREADS, 0, stream>>>(jobs[0], a_exp, jobs[1], b_exp);
   HB_LAUNCH_OK();
   count_launch(1);
   return HASTE_B200_OK;
@@ -827,6 +1031,14 @@ const char* refusal(const GemmDesc& g) {
   if ((g.a_cs != 1 && g.a_rs != 1) || (g.b_rs != 1 && g.b_cs != 1)) return "operand has no unit stride";
   return nullptr;
 }
+// fp32-accurate products go through two fp16 planes where half the products save more than the rows' and
+// columns' scales cost (us with the splits and a LayerNorm over the result, six bf16 products / these:
+// 65536 x 1024 x 1024 1354 / 1165, 16384 x 512 x 1024 290 / 278, 65536 x 512 x 256 359 / 330; but
+// 16384 x 256 x 1024 253 / 257, 4096 x 1024 x 1024 108 / 113, 65536 x 192 x 1024 920 / 933; M x K x N).
+bool f16_planes(const GemmDesc& g) {
+  return g.precise && g.dtype == HASTE_B200_F32 && g.a_cs == 1 && g.b_cs == 1 && g.b_rs != 1 && g.K >= 256 &&
+         (double)g.M * g.N * g.K >= 8e9;
+}
 }  // namespace
 
 bool gemm_reads_planes(const GemmDesc& g) { return gemm_path() != HASTE_B200_GEMM_SIMT && !refusal(g); }
@@ -844,6 +1056,7 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
   const bool a_k = g.a_cs == 1, b_k = g.b_rs == 1;
 
   const int M = g.M, N = g.N, K = g.K;
+  const bool f16 = f16_planes(g);
   Operand A, B;
   A.mn_major = !a_k;
   B.mn_major = !b_k;
@@ -875,7 +1088,7 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
     // + the traffic of the partial tiles (written once, read once by the reduction).
     const int tiles = tiles_m * tiles_n;
     const int max_splits = min(kb_total / 4, 64);
-    const double products = g.dtype == HASTE_B200_BF16 ? 1.0 : (g.precise ? 6.0 : 3.0);
+    const double products = g.dtype == HASTE_B200_BF16 ? 1.0 : (g.precise && !f16 ? 6.0 : 3.0);
     // us per K block and work unit (measured: the single-CTA kernel is bound by its operand
     // loads, the pair kernel by the tensor pipe)
     const double t_kb = pair ? 0.27 * products : (products == 1.0 ? 0.27 : 0.17 * products);
@@ -904,13 +1117,14 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
   const bool b_copy = f32 ? !b_pre : (b_ld_src % 8) != 0 || ((uintptr_t)g.b & 15) != 0;
   const long long a_ld = a_pre ? g.a_pl_ld : (a_copy ? ((a_cols + 7) & ~7LL) : a_ld_src);
   const long long b_ld = b_pre ? g.b_pl_ld : (b_copy ? ((b_cols + 7) & ~7LL) : b_ld_src);
-  const int planes = f32 ? (g.precise ? 3 : 2) : 1;
+  const int planes = f32 ? (g.precise && !f16 ? 3 : 2) : 1;
   const size_t a_plane = a_copy ? Arena::pad((size_t)a_rows * a_ld * 2) : 0;
   const size_t b_plane = b_copy ? Arena::pad((size_t)b_rows * b_ld * 2) : 0;
   const int part_ld = (N + 31) & ~31;
   const bool via_partial = splits > 1;
   const size_t part_bytes = via_partial ? Arena::pad((size_t)splits * M * part_ld * 4) : 0;
-  const size_t bytes = planes * (a_plane + b_plane) + part_bytes + 1024;
+  const size_t a_exps = f16 ? Arena::pad((size_t)M * 4) : 0, b_exps = f16 ? Arena::pad((size_t)tiles_n * PBN) : 0;
+  const size_t bytes = planes * (a_plane + b_plane) + part_bytes + a_exps + b_exps + 1024;
   Arena ws;
   HB_TRY(make_arena(&ws, stream, bytes, /*slot=*/1));
   int* err = device_error_word();
@@ -931,7 +1145,16 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
   };
   if (a_copy && !through_scratch(g.a, a_ld_src, a_rows, a_cols, a_plane, a_ld, &A)) return unsupported("scratch arena");
   if (b_copy && !through_scratch(g.b, b_ld_src, b_rows, b_cols, b_plane, b_ld, &B)) return unsupported("scratch arena");
-  if (n_jobs) HB_TRY(launch_split(jobs, n_jobs, g.dtype, planes, stream));
+  int* a_exp = nullptr;
+  signed char* b_exp = nullptr;
+  if (f16) {
+    a_exp = ws.take<int>(a_exps / 4);
+    b_exp = ws.take<signed char>(b_exps);
+    if (!a_exp || !b_exp) return unsupported("scratch arena");
+    HB_TRY(launch_split_f16(jobs, a_exp, b_exp, stream));
+  } else if (n_jobs) {
+    HB_TRY(launch_split(jobs, n_jobs, g.dtype, planes, stream));
+  }
   A.ld = a_ld;
   B.ld = b_ld;
   float* partial = nullptr;
@@ -958,6 +1181,8 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
   p.accumulate = g.accumulate;
   p.c = g.c; p.ldc = g.ldc;
   p.wide = (g.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(g.c) & (4 * dtype_size(g.dtype_c) - 1)) == 0;
+  p.a_exp = a_exp; p.b_exp = b_exp;
+  p.chunk = f16 ? kF16Chunk : (planes == 3 ? Cfg<6>::CHUNK : Cfg<3>::CHUNK);
   p.partial = partial;
   p.partial_ld = part_ld;
   p.err = err;
