@@ -1082,7 +1082,9 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
   const int tiles_m = ceil_div(M, pair ? PBM : BM), tiles_n = ceil_div(N, pair ? PBN : BN);
   const int kb_total = ceil_div(K, BK);
   int splits = 1;
-  if (tiles_m * tiles_n < units && kb_total >= 8) {
+  // (With K of 8192 and more also where a second or third wave would be nearly empty: 2048 x 3072 is 96 tiles
+  // for 74 pairs; us at K = 64000 one split / three 734 / 601, 2000 x 2600, K = 20000 260 / 222.)
+  if (kb_total >= 8 && tiles_m * tiles_n < (kb_total >= 128 ? 4 : 1) * units) {
     // Split K so that the work items fill whole waves of the persistent grid: pick the split
     // count with the smallest estimated time = (waves / splits) x K blocks x time per K block
     // + the traffic of the partial tiles (written once, read once by the reduction).

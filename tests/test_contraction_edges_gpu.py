@@ -58,3 +58,18 @@ def test_few_rows_are_fp32_grade(M, K, N, transposed, dtype):
     got = ops.gemm(a, b).double()
     bound = 1e-6 if dtype == torch.float32 else 2.0 ** -11
     assert (got - want).norm() < bound * want.norm()
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 2e-5), (torch.bfloat16, 1e-2)])
+@pytest.mark.parametrize("M,K,N", [(2048, 20000, 3072), (2000, 8200, 2601), (5000, 8192, 900)])
+def test_long_sums_over_more_than_one_wave(M, K, N, dtype, tol):
+    """Weight gradients of wide layers: more tiles than the GPU holds at once, K split all the same.  The bounds
+    are those of the edges above."""
+    torch.manual_seed(K)
+    a, b = torch.randn(K, M, device="cuda").to(dtype).t(), torch.randn(K, N, device="cuda").to(dtype)
+    c = torch.randn(M, N, device="cuda").to(dtype)
+    want = a.double() @ b.double()
+    scale = want.abs().max().item()
+    assert (ops.gemm(a, b).double() - want).abs().max().item() < tol * scale
+    added = ops.gemm(a, b, out=c.clone(), accumulate=True)
+    assert (added.double() - want - c.double()).abs().max().item() < tol * scale
