@@ -137,19 +137,13 @@ int lstm_forward_tc(const LstmFwd& a, float* c_carry, cudaStream_t s);
 int lstm_backward_tc(const LstmBwd& a, float* dh_carry, float* dc_carry, cudaStream_t s);
 int gru_forward_tc(const GruFwd& a, cudaStream_t s);
 int gru_backward_tc(const GruBwd& a, float* dh_carry, cudaStream_t s);
-// LayerNormLSTM: forward expects LN(x.W) in a.act_Wx_norm; backward adds the LayerNorm
-// parameter gradients of the recurrence into the fp32 accumulators acc = [dgamma_Rh 4H |
-// dgamma_h H | dbeta_h H]; planes.p / p2 receive the gate gradient and d(h.R).
+// LayerNorm cells (recurrent_host.cu): forward expects LN(x.W) in a.act_Wx_norm / a.tmp_Wx_norm; backward is
+// complete - fp32 carries read and written in place, bias and LayerNorm gradients of h.R and c added or
+// assigned - and leaves d(h.R) in a.act_Rh.
 int layer_norm_lstm_forward_persistent(const LnLstmFwd& a, cudaStream_t s);
-int layer_norm_lstm_backward_cluster(const LnLstmBwd& a, float* dh_carry, float* dc_carry, cudaStream_t s);
-int layer_norm_lstm_backward_persistent(const LnLstmBwd& a, float* dh_carry, float* dc_carry,
-                                        float* acc, const GradPlanes& planes, cudaStream_t s);
-// LayerNormGRU: forward expects LN(x.W) in a.tmp_Wx_norm; backward adds dgamma_Rh into the
-// fp32 accumulator acc [3H] and leaves d(h.R) in a.act_Rh.
+int layer_norm_lstm_backward_persistent(const LnLstmBwd& a, float* dh_carry, float* dc_carry, cudaStream_t s);
 int layer_norm_gru_forward_persistent(const LnGruFwd& a, cudaStream_t s);
-int layer_norm_gru_backward_cluster(const LnGruBwd& a, float* dh_carry, cudaStream_t s);
-int layer_norm_gru_backward_persistent(const LnGruBwd& a, float* dh_carry, float* acc,
-                                       const GradPlanes& planes, cudaStream_t s);
+int layer_norm_gru_backward_persistent(const LnGruBwd& a, float* dh_carry, cudaStream_t s);
 
 // Exchange-only probe (recurrent_host.cu): device microseconds per step of the forward
 // recurrence's hand-off alone, for the tiling (N, H) would get.

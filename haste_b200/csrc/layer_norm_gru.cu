@@ -137,7 +137,7 @@ int layer_norm_gru_backward(const LnGruBwd& a, cudaStream_t s) {
     HB_CUDA_OK(cudaMemsetAsync(dh_carry, 0, NH * 4, s));
     HB_CUDA_OK(cudaMemsetAsync(a.dgamma_Wx, 0, 3 * H * es, s));  // LayerNorm 1 below adds
   }
-  int st_ = layer_norm_gru_backward_cluster(a, dh_carry, s);
+  int st_ = layer_norm_gru_backward_persistent(a, dh_carry, s);
   const bool done = st_ == HASTE_B200_OK;  // biases and gamma_Rh included
   bool use_acc = false;
   if (st_ == HASTE_B200_ERR_UNSUPPORTED) {
@@ -146,16 +146,11 @@ int layer_norm_gru_backward(const LnGruBwd& a, cudaStream_t s) {
       HB_CUDA_OK(cudaMemsetAsync(a.dbr, 0, 3 * H * es, s));
       HB_CUDA_OK(cudaMemsetAsync(a.dgamma_Rh, 0, 3 * H * es, s));
     }
-    // Persistent recurrence first; it adds dgamma_Rh into `acc`.
-    HB_CUDA_OK(cudaMemsetAsync(acc, 0, 3 * H * sizeof(float), s));
-    st_ = layer_norm_gru_backward_persistent(a, dh_carry, acc, GradPlanes{}, s);
-    use_acc = st_ == HASTE_B200_OK;
-  }
-  if (st_ == HASTE_B200_ERR_UNSUPPORTED) {
     void* dgamma1 = a.dgamma_Rh;
     if (bf) {
       dgamma1 = acc;
       use_acc = true;
+      HB_CUDA_OK(cudaMemsetAsync(acc, 0, 3 * H * sizeof(float), s));
     }
     st_ = bf ? backward_steps<__nv_bfloat16>(a, dh_carry, dgamma1, lns, s)
              : backward_steps<float>(a, dh_carry, dgamma1, lns, s);

@@ -457,7 +457,7 @@ int backward_core(const LnLstmBwd& a, cudaStream_t s) {
   }
 
   if (profile_enabled()) profile_mark(PH_REC_BWD, true, s);
-  int st_ = layer_norm_lstm_backward_cluster(a, dh_carry, dc_carry, s);
+  int st_ = layer_norm_lstm_backward_persistent(a, dh_carry, dc_carry, s);
   const bool done = st_ == HASTE_B200_OK;  // bias, gamma_Rh, gamma_h, beta_h included
   bool use_acc = false;
   if (st_ == HASTE_B200_ERR_UNSUPPORTED) {
@@ -467,12 +467,6 @@ int backward_core(const LnLstmBwd& a, cudaStream_t s) {
       HB_CUDA_OK(cudaMemsetAsync(a.dgamma_h, 0, H * es, s));
       HB_CUDA_OK(cudaMemsetAsync(a.dbeta_h, 0, H * es, s));
     }
-    // Persistent recurrence first; it adds its LayerNorm parameter gradients into `acc`.
-    HB_CUDA_OK(cudaMemsetAsync(acc, 0, 6 * H * sizeof(float), s));
-    st_ = layer_norm_lstm_backward_persistent(a, dh_carry, dc_carry, acc, GradPlanes{}, s);
-    use_acc = st_ == HASTE_B200_OK;
-  }
-  if (st_ == HASTE_B200_ERR_UNSUPPORTED) {
     void* dgamma1 = a.dgamma_Rh;
     void* dgamma_h = a.dgamma_h;
     void* dbeta_h = a.dbeta_h;
@@ -481,6 +475,7 @@ int backward_core(const LnLstmBwd& a, cudaStream_t s) {
       dgamma_h = acc + 4 * H;
       dbeta_h = acc + 5 * H;
       use_acc = true;
+      HB_CUDA_OK(cudaMemsetAsync(acc, 0, 6 * H * sizeof(float), s));
     }
     st_ = bf ? backward_steps<__nv_bfloat16>(a, dh_carry, dc_carry, dgamma1, dgamma_h, dbeta_h,
                                              HASTE_B200_F32, lns, s)

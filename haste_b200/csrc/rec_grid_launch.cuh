@@ -15,7 +15,8 @@ struct GlGeometry {
 };
 
 // One CTA per SM, all resident (cooperative launch).  `attr_set`: per kernel and device.
-inline int gl_launch(void (*kernel)(ChainParams), ChainParams& p, int grid, size_t smem, std::atomic<int>* attr_set,
+template <typename P>
+int gl_launch(void (*kernel)(P), P& p, int grid, size_t smem, std::atomic<int>* attr_set,
                      cudaStream_t s) {
   int dev = 0;
   HB_CUDA_OK(cudaGetDevice(&dev));

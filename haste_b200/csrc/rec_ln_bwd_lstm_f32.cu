@@ -1,12 +1,14 @@
 // Instantiates the persistent LayerNormLSTM bwd recurrence kernels for f32 storage
 // (one translation unit per combination so that they compile in parallel).
-#include "rec_ln_cluster.cuh"
+#include "rec_ln_grid.cuh"
 
 namespace hb {
 namespace rec {
-int run_ln_bwd_f32(LnBwdParams& p, const Geometry& g, cudaStream_t s) { return run_ln_bwd<4, 2, float>(p, g, s); }
 int run_ln_cl_bwd_f32(const LnBwdParams& p, float* db_part, int* row_groups, cudaStream_t s) {
   return run_ln_cl_bwd<4, 2, float>(p, db_part, row_groups, s);
+}
+int run_ln_grid_bwd_f32(const LnBwdParams& p, float* db_part, const LnGridGeometry& g, int wide, cudaStream_t s) {
+  return run_ln_grid_bwd<4, 2, float>(p, db_part, g, wide, s);
 }
 }  // namespace rec
 }  // namespace hb

@@ -2,7 +2,7 @@
 //
 // A LayerNorm step is a chain of hand-offs: besides the new state, the row statistics of h.R (and,
 // LSTM, of the cell state) have to meet from all columns before any of them can go on.  Through L2
-// (recurrent_ln_kernels.cuh) each hand-off costs 1.3 .. 1.5 us; here the layer's row group lives in
+// (rec_ln_grid.cuh) each hand-off costs 0.9 .. 1 us; here the layer's row group lives in
 // one cluster - 16 or 20 hidden units per CTA, R in registers, chains of eight rows, as in
 // rec_cluster_kernels.cuh, whose layouts and tagged words these kernels use - and a hand-off is a
 // store into the peers' shared memory.  The statistics of a CTA's warps meet in its own
@@ -13,7 +13,7 @@
 // normalised gates of every chain, ...), so that one chain's hand-off is under way while the others
 // compute; what a chain carries from stage to stage waits in shared memory.
 //
-// Arithmetic is that of recurrent_ln_kernels.cuh: fp32 storage multiplies three bf16 planes per
+// Arithmetic: fp32 storage multiplies three bf16 planes per
 // operand (all products down to 2^-16 of the largest, smallest terms in accumulators of their own)
 // and exchanges fp32 words; statistics are (mean, M2) pairs combined by Chan's formula forward and
 // plain sums backward.  Waits are bounded; a warp that gives up says so at the next barrier of its
@@ -23,7 +23,7 @@
 #include <atomic>
 
 #include "rec_cluster_launch.cuh"
-#include "recurrent_ln_kernels.cuh"
+#include "rec_ln_common.cuh"
 
 namespace hb {
 namespace rec {

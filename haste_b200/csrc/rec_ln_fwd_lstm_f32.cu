@@ -1,10 +1,12 @@
 // Instantiates the persistent LayerNormLSTM fwd recurrence kernels for f32 storage
 // (one translation unit per combination so that they compile in parallel).
-#include "rec_ln_cluster.cuh"
+#include "rec_ln_grid.cuh"
 
 namespace hb {
 namespace rec {
-int run_ln_fwd_f32(LnFwdParams& p, const Geometry& g, cudaStream_t s) { return run_ln_fwd<4, 2, float>(p, g, s); }
 int run_ln_cl_fwd_f32(const LnFwdParams& p, cudaStream_t s) { return run_ln_cl_fwd<4, 2, float>(p, s); }
+int run_ln_grid_fwd_f32(const LnFwdParams& p, const LnGridGeometry& g, int wide, cudaStream_t s) {
+  return run_ln_grid_fwd<4, 2, float>(p, g, wide, s);
+}
 }  // namespace rec
 }  // namespace hb

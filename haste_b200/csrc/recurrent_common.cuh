@@ -33,14 +33,6 @@ constexpr int WARPS = 8;
 constexpr int THREADS = WARPS * 32;
 constexpr long long SPIN_LIMIT_CYCLES = 4000000000LL;
 
-// Timing experiments (attributing step time to waits, contraction, prefetch) are compiled in
-// only with -DHASTE_B200_TIMING_EXPERIMENTS; the shipped kernels carry none of their branches.
-#ifdef HASTE_B200_TIMING_EXPERIMENTS
-#define HB_DBG(p, bit) (((p).dbg & (bit)) != 0)
-#else
-#define HB_DBG(p, bit) false
-#endif
-
 struct Sync {
   int* abort_flag;  // device-global
   int* err;         // process error word (pinned host memory)
@@ -60,11 +52,6 @@ __device__ __forceinline__ void split_bf16(float x, float& hi, float& lo) {
   hi = __bfloat162float(__float2bfloat16_rn(x));
   lo = x - hi;
 }
-__device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&a)[4]) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3])
-               : "r"(addr));
-}
 __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0,
                                          uint32_t b1) {
   asm volatile(
@@ -80,6 +67,19 @@ __device__ __forceinline__ uint4 ld_relaxed_u32x4(const uint32_t* p) {
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "l"(p)
                : "memory");
+  return v;
+}
+
+// The same under a condition, without a branch; else four times `other`.
+__device__ __forceinline__ uint4 ld_relaxed_u32x4_if(bool ok, const uint32_t* p, uint32_t other) {
+  uint4 v = make_uint4(other, other, other, other);
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.u32 p, %5, 0;\n\t"
+      "@p ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}"
+      : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
+      : "l"(p), "r"((uint32_t)ok)
+      : "memory");
   return v;
 }
 
@@ -138,37 +138,6 @@ __device__ __forceinline__ void raise_abort(const Sync& s, int* s_abort, int cod
     e[0] = code;
   }
   __threadfence_system();
-}
-
-// ---------------------------------------------------------------------------------------
-// Host-side launch helpers shared by the instantiation files
-// ---------------------------------------------------------------------------------------
-struct Geometry {
-  int nHS, nBS, MT;
-};
-
-template <typename K>
-int launch_coop(K kernel, int grid, size_t smem, void* params, cudaStream_t s) {
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return HASTE_B200_ERR_UNSUPPORTED;
-  }
-  int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, THREADS, smem);
-  if (e != cudaSuccess || per_sm * sm_count() < grid) {
-    cudaGetLastError();
-    return HASTE_B200_ERR_UNSUPPORTED;
-  }
-  void* args[] = {params};
-  e = cudaLaunchCooperativeKernel((const void*)kernel, dim3(grid), dim3(THREADS), args, smem, s);
-  if (e != cudaSuccess) {
-    set_last_error("cooperative launch failed: %s", cudaGetErrorString(e));
-    cudaGetLastError();
-    return HASTE_B200_ERR_CUDA;
-  }
-  count_launch(1);
-  return HASTE_B200_OK;
 }
 
 }  // namespace rec

@@ -1,9 +1,8 @@
-// Host side of the LayerNorm recurrence kernels (recurrent_ln_kernels.cuh) - tiling choice,
+// Host side of the LayerNorm recurrence kernels (rec_ln_cluster.cuh, rec_ln_grid.cuh) - tiling choice,
 // exchange-buffer scratch and the entry points the cell drivers call - and the exchange probe.
-#include <cstdio>
-#include <cstdlib>
+#include <initializer_list>
 
-#include "recurrent_ln_kernels.cuh"
+#include "rec_ln_common.cuh"
 
 namespace hb {
 namespace rec {
@@ -11,57 +10,40 @@ namespace rec {
 
 namespace {
 
-constexpr int MAX_MT = 4;
+// The grid kernels' tiling: as many row groups as the SMs have room for, one CTA per SM, the rest of the rows
+// as chains.  Under an SM budget (two directions side by side) within it first: four chains per CTA cost a
+// third to a half more than two, not twice as much (see rec_ln_grid.cuh), so both directions at once take
+// 9.5 / 10.6 us per step where one after the other takes 14.0 / 13.8 (LayerNormLSTM fp32, 64 rows, H = 512).
+constexpr int kLnGridChains = 8;
 
-// Picks the batch tiling: as many CTAs as fit on the GPU at once (one CTA per SM).
-bool pick_geometry(int N, int H, Geometry* g) {
-  const int nHS = ceil_div(H, U);
-  const int sms = sm_count();
-  for (int mt = 1; mt <= MAX_MT; ++mt) {
-    const int nBS = ceil_div(N, 16 * mt);
-    if ((long long)nHS * nBS <= sms) {
-      g->nHS = nHS; g->nBS = nBS; g->MT = mt;
-      return true;
-    }
+bool ln_grid_geometry(int dtype, int N, int H, LnGridGeometry* g) {
+  // R's slice must fit the registers: two planes with fp32 storage, one with bf16
+  if (H > (dtype == HASTE_B200_BF16 ? 1024 : 512)) return false;
+  g->nHS = ceil_div(H, 16);
+  const int tiles = ceil_div(N, 8), sms = sm_count(), budget = sm_budget();
+  for (int use : {budget, sms}) {
+    if (use < g->nHS || use > sms) continue;
+    g->nRG = min(tiles, use / g->nHS);
+    g->CH = ceil_div(tiles, g->nRG);
+    g->nRG = ceil_div(tiles, g->CH);
+    if (g->CH <= kLnGridChains) return true;
   }
   return false;
 }
-
-bool supported(int dtype, int N, int H, Geometry* g) {
-  if (recurrence_path() == HASTE_B200_PATH_STEPWISE) return false;
-  // R slice must fit the register file (two bf16 planes for fp32 and fp16 storage, one for bf16)
-  if (dtype != HASTE_B200_BF16 && H > 512) return false;
-  if (dtype == HASTE_B200_BF16 && H > 1024) return false;
-  return pick_geometry(N, H, g);
+// Whole-quad accesses: every row of every array starts on a multiple of four elements.
+int wide_rows(std::initializer_list<const void*> ptrs, int H, int dtype) {
+  uintptr_t a = 0;
+  for (const void* q : ptrs) a |= reinterpret_cast<uintptr_t>(q);
+  return H % 4 == 0 && a % (4 * dtype_size(dtype)) == 0;
 }
 
-// Timing-experiment builds only (-DHASTE_B200_TIMING_EXPERIMENTS): the environment variable
-// HASTE_B200_TIMING_EXPERIMENT=<bits> switches parts of the persistent kernels off to attribute
-// step time to them; results of such a run are wrong by construction and the library says so
-// on stderr.  The shipped library reads no environment variable and compiles the switches out.
-int debug_skip() {
-#ifdef HASTE_B200_TIMING_EXPERIMENTS
-  static int v = -1;
-  if (v < 0) {
-    const char* e = getenv("HASTE_B200_TIMING_EXPERIMENT");
-    v = e ? atoi(e) : 0;
-    if (v != 0)
-      fprintf(stderr, "haste_b200: HASTE_B200_TIMING_EXPERIMENT=%d - parts of the recurrence "
-                      "kernels are switched off, results are wrong\n", v);
-  }
-  return v;
-#else
-  return 0;
-#endif
-}
-
-// Zeroed scratch: abort flag followed by `words` exchange words.
-int make_scratch(size_t words, Sync* sync, uint32_t** xwords, cudaStream_t s) {
+// Zeroed scratch: abort flag followed by `words` exchange words; then `floats` that need no zeroing.
+int make_scratch(size_t words, Sync* sync, uint32_t** xwords, cudaStream_t s, size_t floats = 0) {
   Arena ws;
   const size_t bytes = Arena::pad(4096) + Arena::pad(words * 4);
-  HB_TRY(make_arena(&ws, s, bytes + 512, /*slot=*/2));
+  HB_TRY(make_arena(&ws, s, bytes + floats * 4 + 512, /*slot=*/2));
   int* flag = ws.take<int>(1024);
-  uint32_t* x = ws.take<uint32_t>(words);
+  uint32_t* x = ws.take<uint32_t>(words + floats);
   HB_REQUIRE(flag && x, "scratch arena");
   HB_CUDA_OK(cudaMemsetAsync(flag, 0, bytes, s));
   sync->abort_flag = flag;
@@ -185,12 +167,24 @@ using namespace rec;
 
 namespace {
 
-// The cluster kernels (rec_ln_cluster.cuh), where they take the shape.
-int cluster_forward(LnFwdParams& p, int (*run)(const LnFwdParams&, cudaStream_t), cudaStream_t s) {
+typedef int (*ClFwd)(const LnFwdParams&, cudaStream_t);
+typedef int (*GridFwd)(const LnFwdParams&, const LnGridGeometry&, int, cudaStream_t);
+typedef int (*ClBwd)(const LnBwdParams&, float*, int*, cudaStream_t);
+typedef int (*GridBwd)(const LnBwdParams&, float*, const LnGridGeometry&, int, cudaStream_t);
+
+// The cluster kernels where they take the shape, else the grid kernels.
+int run_forward(LnFwdParams& p, int dtype, int wide, ClFwd cluster, GridFwd grid, cudaStream_t s) {
   if (recurrence_path() == HASTE_B200_PATH_STEPWISE) return HASTE_B200_ERR_UNSUPPORTED;
   p.sync.err = device_error_word();
   HB_REQUIRE(p.sync.err, "error word");
-  return run(p, s);
+  const int cl = cluster(p, s);
+  if (cl != HASTE_B200_ERR_UNSUPPORTED) return cl;
+  LnGridGeometry g;
+  if (!ln_grid_geometry(dtype, p.N, p.H, &g)) return HASTE_B200_ERR_UNSUPPORTED;
+  const size_t tiles = ceil_div(p.N, 8), xwords = 2 * tiles * g.nHS * 128, swords = 4 * tiles * g.nHS * 16;
+  HB_TRY(make_scratch(xwords + swords, &p.sync, &p.xbuf, s));
+  p.sbuf = p.xbuf + xwords;
+  return grid(p, g, wide, s);
 }
 // Sums of the row groups' partial parameter gradients, into the caller's tensors: bias (as
 // bias_grad_finish), gains of h.R and, LSTM, gain and offset of the cell state.
@@ -225,21 +219,39 @@ __global__ void ln_grad_finish(int G, const float* db_part, const float* dgRh_pa
   if (d2) st(d2, accumulate ? s + ld(d2) : s);
 }
 
-int cluster_backward(LnBwdParams& p, int gates, int dtype, const LnGrads& out,
-                     int (*run)(const LnBwdParams&, float*, int*, cudaStream_t), cudaStream_t s) {
-  if (recurrence_path() == HASTE_B200_PATH_STEPWISE || p.H > 320) return HASTE_B200_ERR_UNSUPPORTED;
+int run_backward(LnBwdParams& p, int gates, int dtype, int wide, const LnGrads& out, ClBwd cluster, GridBwd grid,
+                 cudaStream_t s) {
+  if (recurrence_path() == HASTE_B200_PATH_STEPWISE) return HASTE_B200_ERR_UNSUPPORTED;
   p.sync.err = device_error_word();
   HB_REQUIRE(p.sync.err, "error word");
   const int H = p.H;
   const size_t tiles = ceil_div(p.N, 8);
-  float* part = static_cast<float*>(workspace(s, tiles * 10 * H * sizeof(float), /*slot=*/2));
-  if (!part) return HASTE_B200_ERR_CUDA;
-  float* db_part = part + tiles * 6 * H;
-  p.dgRh_part = part;
-  p.dgh_part = part + tiles * 4 * H;
-  p.dbh_part = part + tiles * 5 * H;
-  int rows = 0;
-  HB_TRY(run(p, db_part, &rows, s));
+  // partial parameter gradients: rows x (gains of h.R, gain and offset of c, gates)
+  float* db_part = nullptr;
+  auto partials = [&](float* part, size_t rows) {
+    p.dgRh_part = part;
+    p.dgh_part = part + rows * 4 * H;
+    p.dbh_part = part + rows * 5 * H;
+    db_part = part + rows * 6 * H;
+  };
+  int rows = 0, st_ = HASTE_B200_ERR_UNSUPPORTED;
+  if (H <= 320) {
+    float* part = static_cast<float*>(workspace(s, tiles * 10 * H * sizeof(float), /*slot=*/2));
+    if (!part) return HASTE_B200_ERR_CUDA;
+    partials(part, tiles);
+    st_ = cluster(p, db_part, &rows, s);
+  }
+  if (st_ == HASTE_B200_ERR_UNSUPPORTED) {
+    LnGridGeometry g;
+    if (!ln_grid_geometry(dtype, p.N, H, &g)) return HASTE_B200_ERR_UNSUPPORTED;
+    rows = 2 * g.nRG;
+    const size_t xwords = 2 * tiles * g.nHS * g.nHS * 128, swords = 4 * tiles * g.nHS * 16;
+    HB_TRY(make_scratch(xwords + swords, &p.sync, &p.exch, s, (size_t)rows * 10 * H));
+    p.sbuf = p.exch + xwords;
+    partials(reinterpret_cast<float*>(p.sbuf + swords), rows);
+    st_ = grid(p, db_part, g, wide, s);
+  }
+  if (st_ != HASTE_B200_OK) return st_;
   const int blocks = ceil_div((gates == 4 ? 10LL : 7LL) * H, 128), add = assign_gradients() ? 0 : 1;
   if (dtype == HASTE_B200_F32)
     ln_grad_finish<float><<<blocks, 128, 0, s>>>(gates, db_part, p.dgRh_part, p.dgh_part, p.dbh_part, rows, H, out, add);
@@ -253,147 +265,51 @@ int cluster_backward(LnBwdParams& p, int gates, int dtype, const LnGrads& out,
 
 }  // namespace
 
-// ---- LayerNormLSTM (recurrent_ln_kernels.cuh) ------------------------------------------
-// Forward: LN(x.W) is already in a.act_Wx_norm.  Four source slices per thread in the
-// statistic exchange limit the kernels to 64 hidden slices, which `supported` guarantees.
+// ---- LayerNormLSTM: LN(x.W) is already in a.act_Wx_norm ---------------------------------
 int layer_norm_lstm_forward_persistent(const LnLstmFwd& a, cudaStream_t s) {
   const bool zo = a.zoneout_prob != 0.0f && a.zoneout_mask != nullptr;
-  LnFwdParams p{a.T, a.N, a.H, 0, 0, 0, a.training, zo ? 1 : 0, a.zoneout_prob, a.R, a.b,
-                nullptr, a.act_Wx_norm, a.gamma_Rh, a.gamma_h, a.beta_h, a.act_Wx_norm, a.act_Rh, a.cache_Rh,
-                a.act_c_norm, a.cache_c, a.h, a.c, a.zoneout_mask, nullptr, nullptr, Sync{}, debug_skip()};
-  const int cl = cluster_forward(p, a.dtype == HASTE_B200_F32 ? run_ln_cl_fwd_f32 : run_ln_cl_fwd_bf16, s);
-  if (cl != HASTE_B200_ERR_UNSUPPORTED) return cl;
-  Geometry g;
-  if (!supported(a.dtype, a.N, a.H, &g) || g.nHS > 64) return HASTE_B200_ERR_UNSUPPORTED;
-  p.Hx = (a.H + 3) & ~3;
-  p.nHS = g.nHS;
-  p.MT = g.MT;
-  const size_t xwords = (size_t)2 * a.N * p.Hx;
-  const size_t swords = (size_t)2 * 2 * g.nBS * g.MT * 16 * g.nHS * 2;
-  HB_TRY(make_scratch(xwords + swords + 64, &p.sync, &p.xbuf, s));
-  p.sbuf = p.xbuf + ((xwords + 63) & ~size_t(63));
-  return a.dtype == HASTE_B200_F32 ? run_ln_fwd_f32(p, g, s) : run_ln_fwd_bf16(p, g, s);
+  LnFwdParams p{a.T, a.N, a.H, a.training, zo ? 1 : 0, a.zoneout_prob, a.R, a.b, nullptr, a.act_Wx_norm, a.gamma_Rh,
+                a.gamma_h, a.beta_h, a.act_Wx_norm, a.act_Rh, a.cache_Rh, a.act_c_norm, a.cache_c, a.h, a.c,
+                a.zoneout_mask, nullptr, nullptr, Sync{}};
+  const int wide = wide_rows({a.act_Wx_norm, a.act_Rh, a.act_c_norm, a.h, a.c, a.zoneout_mask}, a.H, a.dtype);
+  return a.dtype == HASTE_B200_F32 ? run_forward(p, a.dtype, wide, run_ln_cl_fwd_f32, run_ln_grid_fwd_f32, s)
+                                   : run_forward(p, a.dtype, wide, run_ln_cl_fwd_bf16, run_ln_grid_fwd_bf16, s);
 }
 
-namespace {
-LnBwdParams ln_lstm_params(const LnLstmBwd& a, float* dh_carry, float* dc_carry, const GradPlanes& planes) {
-  return LnBwdParams{a.T, a.N, a.H, 0, 0, a.zoneout_mask ? 1 : 0, a.transposed_inputs, a.R,
-                     a.gamma_Rh, a.gamma_h, a.c, nullptr, nullptr, nullptr, a.act_Wx_norm, a.act_Rh,
-                     a.cache_Rh, a.act_c_norm,
-                     a.cache_c, a.dh_new, a.dc_new, a.zoneout_mask, dh_carry, dc_carry, nullptr, nullptr, nullptr,
-                     nullptr, nullptr, Sync{}, planes.p, planes.p2, planes.stride, debug_skip()};
-}
-}  // namespace
-
-// The cluster kernels, up to 320 units: dh and dc come back complete, and the bias and LayerNorm
-// gradients of h.R and c go into the caller's tensors (added or assigned).
-int layer_norm_lstm_backward_cluster(const LnLstmBwd& a, float* dh_carry, float* dc_carry, cudaStream_t s) {
-  LnBwdParams p = ln_lstm_params(a, dh_carry, dc_carry, GradPlanes{});
-  return cluster_backward(p, 4, a.dtype, LnGrads{a.db, nullptr, a.dgamma_Rh, a.dgamma_h, a.dbeta_h},
-                          a.dtype == HASTE_B200_F32 ? run_ln_cl_bwd_f32 : run_ln_cl_bwd_bf16, s);
+// dh and dc come back complete, and the bias and LayerNorm gradients of h.R and c go into the caller's
+// tensors (added or assigned).
+int layer_norm_lstm_backward_persistent(const LnLstmBwd& a, float* dh_carry, float* dc_carry, cudaStream_t s) {
+  LnBwdParams p{a.T, a.N, a.H, a.zoneout_mask ? 1 : 0, a.transposed_inputs, a.R, a.gamma_Rh, a.gamma_h, a.c, nullptr,
+                nullptr, nullptr, a.act_Wx_norm, a.act_Rh, a.cache_Rh, a.act_c_norm, a.cache_c, a.dh_new, a.dc_new,
+                a.zoneout_mask, dh_carry, dc_carry, nullptr, nullptr, nullptr, nullptr, nullptr, Sync{}};
+  const LnGrads out{a.db, nullptr, a.dgamma_Rh, a.dgamma_h, a.dbeta_h};
+  const int wide = wide_rows({a.act_Wx_norm, a.act_Rh, a.act_c_norm, a.c, a.dh_new, a.dc_new, a.zoneout_mask}, a.H, a.dtype);
+  return a.dtype == HASTE_B200_F32 ? run_backward(p, 4, a.dtype, wide, out, run_ln_cl_bwd_f32, run_ln_grid_bwd_f32, s)
+                                   : run_backward(p, 4, a.dtype, wide, out, run_ln_cl_bwd_bf16, run_ln_grid_bwd_bf16, s);
 }
 
-// Backward.  `acc` holds fp32 accumulators [dgamma_Rh 4H | dgamma_h H | dbeta_h H] that the
-// per-row-group partial sums of the kernel are added into (fixed order).  As for the plain
-// LSTM, the recurrent contribution of step 0 to dh is added here by one small contraction.
-int layer_norm_lstm_backward_persistent(const LnLstmBwd& a, float* dh_carry, float* dc_carry,
-                                        float* acc, const GradPlanes& planes, cudaStream_t s) {
-  const int H = a.H;
-  LnBwdParams p = ln_lstm_params(a, dh_carry, dc_carry, planes);
-  Geometry g;
-  if (!supported(a.dtype, a.N, a.H, &g) || g.nHS > 64) return HASTE_B200_ERR_UNSUPPORTED;
-  p.nHS = g.nHS;
-  p.MT = g.MT;
-  const size_t ewords = ((size_t)2 * g.nBS * g.nHS * g.nHS * g.MT * 16 * U + 63) & ~size_t(63);
-  const size_t swords = ((size_t)2 * 2 * g.nBS * g.MT * 16 * g.nHS * 2 + 63) & ~size_t(63);
-  const int prow = g.nBS * 16;
-  const size_t pwords = (size_t)prow * 6 * H;
-  const size_t cwords = colsum_scratch_floats(prow, 4 * H);
-  HB_TRY(make_scratch(ewords + swords + pwords + cwords + 64, &p.sync, &p.exch, s));
-  p.sbuf = p.exch + ewords;
-  float* part = reinterpret_cast<float*>(p.sbuf + swords);
-  float* cs = part + pwords;
-  p.dgRh_part = part;
-  p.dgh_part = part + (size_t)prow * 4 * H;
-  p.dbh_part = part + (size_t)prow * 5 * H;
-  int st_ = a.dtype == HASTE_B200_F32 ? run_ln_bwd_f32(p, g, s) : run_ln_bwd_bf16(p, g, s);
-  if (st_ != HASTE_B200_OK) return st_;
-  HB_TRY(colsum(HASTE_B200_F32, part, 4LL * H, prow, 4 * H, HASTE_B200_F32, acc, 1, cs, s));
-  HB_TRY(colsum(HASTE_B200_F32, part + (size_t)prow * 4 * H, H, prow, H, HASTE_B200_F32,
-                acc + 4 * H, 1, cs, s));
-  HB_TRY(colsum(HASTE_B200_F32, part + (size_t)prow * 5 * H, H, prow, H, HASTE_B200_F32,
-                acc + 5 * H, 1, cs, s));
-  GemmDesc gd{a.dtype, HASTE_B200_F32, a.N, H, 4 * H, a.act_Rh, 4LL * H, 1, a.R,
-              a.transposed_inputs ? H : 1, a.transposed_inputs ? 1 : 4LL * H, dh_carry, H, 1};
-  gd.precise = 1;
-  // (once per pass, not once per step: the CUDA-core kernel would take 92 us for 45 rows, H = 296)
-  return gemm(gd, s);
-}
-
-// ---- LayerNormGRU (the G = 3 instantiation of the same kernels) ---------------------------
-// Forward: LN(x.W) is already in a.tmp_Wx_norm.
+// ---- LayerNormGRU (the G = 3 instantiations): LN(x.W) is already in a.tmp_Wx_norm --------
 int layer_norm_gru_forward_persistent(const LnGruFwd& a, cudaStream_t s) {
   const bool zo = a.zoneout_prob != 0.0f && a.zoneout_mask != nullptr;
-  LnFwdParams p{a.T, a.N, a.H, 0, 0, 0, a.training, zo ? 1 : 0, a.zoneout_prob, a.R, a.bx,
-                a.br, a.tmp_Wx_norm, a.gamma_Rh, nullptr, nullptr, a.v, a.act_Rh, a.cache_Rh,
-                nullptr, nullptr, a.h, nullptr, a.zoneout_mask, nullptr, nullptr, Sync{}};
-  const int cl = cluster_forward(p, a.dtype == HASTE_B200_F32 ? run_lngru_cl_fwd_f32 : run_lngru_cl_fwd_bf16, s);
-  if (cl != HASTE_B200_ERR_UNSUPPORTED) return cl;
-  Geometry g;
-  if (!supported(a.dtype, a.N, a.H, &g) || g.nHS > 64) return HASTE_B200_ERR_UNSUPPORTED;
-  p.Hx = (a.H + 3) & ~3;
-  p.nHS = g.nHS;
-  p.MT = g.MT;
-  const size_t xwords = (size_t)2 * a.N * p.Hx;
-  const size_t swords = (size_t)2 * 2 * g.nBS * g.MT * 16 * g.nHS * 2;
-  HB_TRY(make_scratch(xwords + swords + 64, &p.sync, &p.xbuf, s));
-  p.sbuf = p.xbuf + ((xwords + 63) & ~size_t(63));
-  return a.dtype == HASTE_B200_F32 ? run_lngru_fwd_f32(p, g, s) : run_lngru_fwd_bf16(p, g, s);
+  LnFwdParams p{a.T, a.N, a.H, a.training, zo ? 1 : 0, a.zoneout_prob, a.R, a.bx, a.br, a.tmp_Wx_norm, a.gamma_Rh,
+                nullptr, nullptr, a.v, a.act_Rh, a.cache_Rh, nullptr, nullptr, a.h, nullptr, a.zoneout_mask, nullptr,
+                nullptr, Sync{}};
+  const int wide = wide_rows({a.tmp_Wx_norm, a.v, a.act_Rh, a.h, a.zoneout_mask}, a.H, a.dtype);
+  return a.dtype == HASTE_B200_F32 ? run_forward(p, a.dtype, wide, run_lngru_cl_fwd_f32, run_lngru_grid_fwd_f32, s)
+                                   : run_forward(p, a.dtype, wide, run_lngru_cl_fwd_bf16, run_lngru_grid_fwd_bf16, s);
 }
 
-namespace {
-LnBwdParams ln_gru_params(const LnGruBwd& a, float* dh_carry, const GradPlanes& planes) {
-  return LnBwdParams{a.T, a.N, a.H, 0, 0, a.zoneout_mask ? 1 : 0, a.transposed_inputs, a.R,
-                     a.gamma_Rh, nullptr, nullptr, a.h, a.dp, a.dq, const_cast<void*>(a.v), a.act_Rh,
-                     a.cache_Rh, nullptr, nullptr, a.dh_new, nullptr, a.zoneout_mask, dh_carry, nullptr,
-                     nullptr, nullptr, nullptr, nullptr, nullptr, Sync{}, planes.p, planes.p2, planes.stride};
-}
-}  // namespace
-
-int layer_norm_gru_backward_cluster(const LnGruBwd& a, float* dh_carry, cudaStream_t s) {
-  LnBwdParams p = ln_gru_params(a, dh_carry, GradPlanes{});
-  return cluster_backward(p, 3, a.dtype, LnGrads{a.dbx, a.dbr, a.dgamma_Rh, nullptr, nullptr},
-                          a.dtype == HASTE_B200_F32 ? run_lngru_cl_bwd_f32 : run_lngru_cl_bwd_bf16, s);
-}
-
-// Backward.  `acc` is the fp32 accumulator [3H] for dgamma_Rh.  a.act_Rh is overwritten with
-// d(h.R); a.dp / a.dq receive the gradients w.r.t. the normalised projections (+ biases).
-int layer_norm_gru_backward_persistent(const LnGruBwd& a, float* dh_carry, float* acc,
-                                       const GradPlanes& planes, cudaStream_t s) {
-  const int H = a.H;
-  LnBwdParams p = ln_gru_params(a, dh_carry, planes);
-  Geometry g;
-  if (!supported(a.dtype, a.N, a.H, &g) || g.nHS > 64) return HASTE_B200_ERR_UNSUPPORTED;
-  p.nHS = g.nHS;
-  p.MT = g.MT;
-  const size_t ewords = ((size_t)2 * g.nBS * g.nHS * g.nHS * g.MT * 16 * U + 63) & ~size_t(63);
-  const size_t swords = ((size_t)2 * 2 * g.nBS * g.MT * 16 * g.nHS * 2 + 63) & ~size_t(63);
-  const int prow = g.nBS * 16;
-  const size_t pwords = (size_t)prow * 3 * H;
-  const size_t cwords = colsum_scratch_floats(prow, 3 * H);
-  HB_TRY(make_scratch(ewords + swords + pwords + cwords + 64, &p.sync, &p.exch, s));
-  p.sbuf = p.exch + ewords;
-  float* part = reinterpret_cast<float*>(p.sbuf + swords);
-  float* cs = part + pwords;
-  p.dgRh_part = part;
-  int st_ = a.dtype == HASTE_B200_F32 ? run_lngru_bwd_f32(p, g, s) : run_lngru_bwd_bf16(p, g, s);
-  if (st_ != HASTE_B200_OK) return st_;
-  HB_TRY(colsum(HASTE_B200_F32, part, 3LL * H, prow, 3 * H, HASTE_B200_F32, acc, 1, cs, s));
-  GemmDesc gd{a.dtype, HASTE_B200_F32, a.N, H, 3 * H, a.act_Rh, 3LL * H, 1, a.R,
-              a.transposed_inputs ? H : 1, a.transposed_inputs ? 1 : 3LL * H, dh_carry, H, 1};
-  gd.precise = 1;
-  // (once per pass, not once per step: the CUDA-core kernel would take 92 us for 45 rows, H = 296)
-  return gemm(gd, s);
+// a.act_Rh is overwritten with d(h.R); a.dp / a.dq receive the gradients w.r.t. the normalised projections
+// (+ biases).
+int layer_norm_gru_backward_persistent(const LnGruBwd& a, float* dh_carry, cudaStream_t s) {
+  LnBwdParams p{a.T, a.N, a.H, a.zoneout_mask ? 1 : 0, a.transposed_inputs, a.R, a.gamma_Rh, nullptr, nullptr, a.h,
+                a.dp, a.dq, const_cast<void*>(a.v), a.act_Rh, a.cache_Rh, nullptr, nullptr, a.dh_new, nullptr,
+                a.zoneout_mask, dh_carry, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, Sync{}};
+  const LnGrads out{a.dbx, a.dbr, a.dgamma_Rh, nullptr, nullptr};
+  const int wide = wide_rows({a.v, a.act_Rh, a.h, a.dp, a.dq, a.dh_new, a.zoneout_mask}, a.H, a.dtype);
+  return a.dtype == HASTE_B200_F32
+             ? run_backward(p, 3, a.dtype, wide, out, run_lngru_cl_bwd_f32, run_lngru_grid_bwd_f32, s)
+             : run_backward(p, 3, a.dtype, wide, out, run_lngru_cl_bwd_bf16, run_lngru_grid_bwd_bf16, s);
 }
 
 }  // namespace hb

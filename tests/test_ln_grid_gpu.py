@@ -1,0 +1,57 @@
+"""LayerNorm recurrences over the whole grid (beyond 320 units, or many rows): the edges of their tiles,
+chains and scales against the fp64 oracle."""
+import pytest
+import torch
+
+import haste_oracle as oracle
+from haste_b200 import _C
+from helpers import TOL_BF16, TOL_F32, assert_close, run_cuda
+
+pytestmark = pytest.mark.gpu
+
+
+def check(cell, d, tol, dtype=torch.float32, grad=1.0):
+    if dtype == torch.bfloat16:
+        d = {k: (v.to(dtype).to(torch.float64) if v is not None else None) for k, v in d.items()}
+    ref_out, ref_g = oracle.forward_backward(cell, d, zoneout=0.2)
+    out, g = run_cuda(cell, d, zoneout=0.2, dtype=dtype)
+    assert_close(out["h"], ref_out["h"], tol, "h")
+    for k, r in ref_g.items():
+        assert_close(g[k].double() / grad, r / grad, tol, "d" + k)
+
+
+# slices of 16 units with a ragged last one, rows that are no multiple of 4, one to eight chains per CTA
+@pytest.mark.parametrize("T,N,H", [(1, 1, 321), (2, 8, 336), (5, 9, 353), (6, 3, 384), (4, 17, 400), (5, 33, 497),
+                                   (7, 41, 510), (4, 70, 512), (3, 130, 511), (3, 250, 512), (4, 150, 300)])
+@pytest.mark.parametrize("cell", ["layer_norm_lstm", "layer_norm_gru"])
+def test_tiles_f32(cell, T, N, H):
+    check(cell, oracle.make_inputs(cell, T, N, 12, H, seed=H + N, zoneout=0.2), TOL_F32)
+
+
+# half of the GPU, and one row group of many chains (fewer slots for partial tiles than chains)
+@pytest.mark.parametrize("budget,N,H", [(74, 64, 512), (74, 100, 340), (40, 60, 512), (33, 64, 500), (24, 50, 370)])
+@pytest.mark.parametrize("cell", ["layer_norm_lstm", "layer_norm_gru"])
+def test_sm_budget(cell, budget, N, H):
+    was = _C.exchange_sm_budget(budget)
+    try:
+        check(cell, oracle.make_inputs(cell, 5, N, 12, H, seed=H, zoneout=0.2), TOL_F32)
+    finally:
+        _C.exchange_sm_budget(was)
+
+
+# states of 2 and more take a scale of their own; gradients of any size take theirs from a bound
+@pytest.mark.parametrize("state,grad", [(1.0, 1e-12), (3.0, 1.0), (500.0, 1e9), (1e-4, 1.0)])
+@pytest.mark.parametrize("cell", ["layer_norm_lstm", "layer_norm_gru"])
+def test_scales(cell, state, grad):
+    d = oracle.make_inputs(cell, 4, 21, 12, 400, seed=7, zoneout=0.2)
+    d["h0"] = d["h0"] * state
+    d["h0"][3] = 0.0
+    for k in ("dh", "dc"):
+        if k in d:
+            d[k] = d[k] * grad
+    check(cell, d, TOL_F32, grad=grad)
+
+
+@pytest.mark.parametrize("N,H", [(9, 330), (20, 512), (13, 777), (70, 1000), (30, 1024)])
+def test_tiles_bf16(N, H):
+    check("layer_norm_gru", oracle.make_inputs("layer_norm_gru", 5, N, 16, H, seed=H, zoneout=0.2), TOL_BF16, torch.bfloat16)
