@@ -17,7 +17,7 @@ bool aligned(std::initializer_list<const void*> ptrs, int H, int dtype) {
   return H % 4 == 0 && a % (4 * dtype_size(dtype)) == 0;
 }
 
-// Grid tiling: NMT quads of hidden units per CTA such that its slice of R fits the registers, as
+// Grid tiling: NMT quads of hidden units per CTA such that its slice of R fits on chip, as
 // many row groups as there are SMs for, the rest of the rows as chains - at most `most` of them: a
 // chain adds 0.7 .. 2 us to a step (H = 512 .. 1024), which the step-wise path (about 20 us plus the
 // product) undercuts from a dozen on, and beyond six the tensor-core GRU recurrence (6 us
@@ -27,23 +27,35 @@ bool aligned(std::initializer_list<const void*> ptrs, int H, int dtype) {
 // 90 rows, twelve, 8.1 / 6.4).
 constexpr int kGridChains = 12, kGruChainsBeforeTc = 6, kLstmChainsBeforeTc = 8;
 
-bool gl_geometry(int dtype, int N, int H, int most, GlGeometry* g) {
+// fp32 and fp16 storage beyond 512 units: two quads per CTA keep both planes of R in registers, four put the
+// second plane into shared memory and so take half the CTAs per row group.  Half the CTAs read (backward:
+// add up) each state, and twice the row groups share the chains; but a chain's product takes twice as long, so
+// the chains must be enough to fill that time (LSTM fp32, us per step, two quads / four: forward H = 1024 24
+// rows, three chains 3.2 / 3.8, 32 rows, four 4.2 / 3.8, 64 rows 8.2 / 7.0, H = 768 64 rows 7.3 / 4.5; backward
+// H = 1024 16 rows 3.8 / 4.0, 24 rows 5.9 / 4.9, 32 rows 6.4 / 5.0, 64 rows 12.8 / 8.8, 90 rows 24.4 / 12.3).
+constexpr int kFourQuadsFwd = 4, kFourQuadsBwd = 3;
+
+bool gl_geometry(int dtype, int N, int H, bool bwd, int most, GlGeometry* g) {
   g->KS16 = ceil_div(H, 16);
   const int ks = ceil_div(g->KS16, GL_WARPS);
   if (ks > 8) return false;
   const int tiles = ceil_div(N, 8), sms = sm_count(), budget = sm_budget();
-  g->NMT = (dtype == HASTE_B200_BF16 || ks <= 4) ? 4 : 2;
-  g->nHS = ceil_div(H, 4 * g->NMT);
-  if (g->nHS > sms) return false;
   // Under an SM budget (two directions side by side) first within it; if that takes too many chains,
   // the whole GPU for one direction after the other still beats the step-wise path (bf16 LSTM, two
   // directions of 139 rows, H = 696: 18 chains within the budget, 6 without).
   for (int use : {budget, sms}) {
-    if (use < g->nHS || use > sms) continue;
-    g->nRG = min(tiles, use / g->nHS);
-    g->CH = ceil_div(tiles, g->nRG);
-    g->nRG = ceil_div(tiles, g->CH);
-    if (g->CH <= most) return true;
+    if (use > sms) continue;
+    for (int nmt : {2, 4}) {
+      if (nmt == 2 && (dtype == HASTE_B200_BF16 || ks <= 4)) continue;
+      g->NMT = nmt;
+      g->nHS = ceil_div(H, 4 * nmt);
+      if (use < g->nHS) continue;
+      g->nRG = min(tiles, use / g->nHS);
+      g->CH = ceil_div(tiles, g->nRG);
+      g->nRG = ceil_div(tiles, g->CH);
+      if (nmt == 2 && g->CH >= (bwd ? kFourQuadsBwd : kFourQuadsFwd)) continue;
+      if (g->CH <= most) return true;
+    }
     if (most < kGridChains) break;  // the tensor-core recurrence comes next, within the budget too
   }
   return false;
@@ -87,7 +99,7 @@ int run_fwd(ChainParams& p, int dtype, int grid_most, ClRun cl, GlRun gl, cudaSt
     if (st_ != HASTE_B200_ERR_UNSUPPORTED) return st_;
   }
   GlGeometry g;
-  if (!gl_geometry(dtype, p.N, p.H, grid_most, &g)) return HASTE_B200_ERR_UNSUPPORTED;
+  if (!gl_geometry(dtype, p.N, p.H, false, grid_most, &g)) return HASTE_B200_ERR_UNSUPPORTED;
   p.CTAS = g.nHS; p.CH = g.CH; p.K16 = g.KS16;
   HB_TRY(gl_scratch(&p, (size_t)2 * ceil_div(p.N, 8) * g.KS16 * 128, 0, nullptr, s));
   return gl(dtype, p, g, s);
@@ -109,7 +121,7 @@ int run_bwd(ChainParams& p, int dtype, int grid_most, int gates, void* db, void*
     if (st_ != HASTE_B200_ERR_UNSUPPORTED) return st_;
   }
   GlGeometry g;
-  if (!gl_geometry(dtype, p.N, p.H, grid_most, &g)) return HASTE_B200_ERR_UNSUPPORTED;
+  if (!gl_geometry(dtype, p.N, p.H, true, grid_most, &g)) return HASTE_B200_ERR_UNSUPPORTED;
   p.CTAS = g.nHS; p.CH = g.CH; p.K16 = ceil_div(g.nHS * g.NMT, 4);
   HB_TRY(gl_scratch(&p, (size_t)2 * tiles * g.nHS * g.nHS * g.NMT * 32, (size_t)g.nRG * 8 * p.H, &p.db_part, s));
   HB_TRY(gl(dtype, p, g, s));

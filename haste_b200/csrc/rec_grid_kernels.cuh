@@ -36,6 +36,11 @@ constexpr int GL_FWD_P = 192, GL_FWD_F = 64, GL_BWD_P = 176, GL_BWD_F = 80;
 static_assert(GL_FWD_P + GL_FWD_F == 256 && GL_BWD_P + GL_BWD_F == 256,
               "the split must be what the block was launched with");
 
+// Layers beyond 512 units of fp32 or fp16 storage, 16 units per CTA: R's second plane lies in shared memory
+// (128 KB at 1024 units) because both do not fit the registers.
+template <int NMT, int TILES, int SPLIT>
+constexpr bool gl_lo_in_smem() { return SPLIT == 2 && NMT == 4 && TILES > 4; }
+
 template <int N>
 __device__ __forceinline__ void reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N>
@@ -54,9 +59,12 @@ template <int G, int NMT, int KSW, int SPLIT, typename T>
 __global__ void __launch_bounds__(GL_THREADS, 1) gl_fwd_kernel(const __grid_constant__ ChainParams p) {
   constexpr int U = 4 * NMT, GROUPS = GL_WARPS / NMT;
   constexpr int PART = GL_WARPS * NMT * 32;
+  constexpr bool LO = gl_lo_in_smem<NMT, KSW, SPLIT>();
+  constexpr int RP = LO ? 1 : SPLIT;  // planes of R in registers
   extern __shared__ __align__(16) uint8_t smem[];
   float4* part = reinterpret_cast<float4*>(smem);                                // [ring][warp][NMT][lane]
-  float* carry = reinterpret_cast<float*>(part + p.ring * PART);                 // [CH][h, c][NMT * 32]
+  uint4* lo = reinterpret_cast<uint4*>(part + p.ring * PART);                    // LO: [warp][NMT][KSW][lane]
+  float* carry = reinterpret_cast<float*>(lo + (LO ? PART * KSW : 0));           // [CH][h, c][NMT * 32]
   uint64_t* barp = reinterpret_cast<uint64_t*>(carry + p.CH * 2 * NMT * 32);     // full[ring], empty[ring]
   const uint32_t pbar = smem_u32(barp);
   uint8_t* io_base = reinterpret_cast<uint8_t*>(barp + 2 * p.ring);              // per finishing warp
@@ -84,13 +92,21 @@ __global__ void __launch_bounds__(GL_THREADS, 1) gl_fwd_kernel(const __grid_cons
   if (w < GL_WARPS) {
     // ------------------------------------------------------------------ product warps
     reg_inc<GL_FWD_P>();
-    uint32_t wf[SPLIT][NMT][KSW][4];
+    uint32_t wf[RP][NMT][KSW][4];
+    lo += w * NMT * KSW * 32 + lane;  // this lane's
 #pragma unroll
     for (int mt = 0; mt < NMT; ++mt)
 #pragma unroll
       for (int s = 0; s < KSW; ++s)
-        fwd_weights<G, SPLIT, T>(p, u0 + 4 * mt + (gq >> 1), gq & 1, ((w * KSW + s) * 4 + q) * 4, true,
-                                 wf[0][mt][s], wf[SPLIT - 1][mt][s]);
+      {
+        uint32_t l[4];
+        fwd_weights<G, SPLIT, T>(p, u0 + 4 * mt + (gq >> 1), gq & 1, ((w * KSW + s) * 4 + q) * 4, true, wf[0][mt][s], l);
+        if (LO) lo[(mt * KSW + s) * 32] = make_uint4(l[0], l[1], l[2], l[3]);
+        else if (SPLIT == 2) {
+#pragma unroll
+          for (int a = 0; a < 4; ++a) wf[RP - 1][mt][s][a] = l[a];
+        }
+      }
     // words of h_t for the rows of one chain, this warp's K range.  Quads and rows that do not
     // exist count as ready.
     const int kq = w * KSW * 4 + q;  // first quad of this lane
@@ -137,7 +153,10 @@ __global__ void __launch_bounds__(GL_THREADS, 1) gl_fwd_kernel(const __grid_cons
 #pragma unroll
             for (int mt = 0; mt < NMT; ++mt) mma_bf16(acc[mt], wf[0][mt][s], bl[0], bl[1]);
 #pragma unroll
-            for (int mt = 0; mt < NMT; ++mt) mma_bf16(acc[mt], wf[SPLIT - 1][mt][s], bh[0], bh[1]);
+            for (int mt = 0; mt < NMT; ++mt) {
+              if (LO) mma_bf16(acc[mt], lo[(mt * KSW + s) * 32], bh[0], bh[1]);
+              else mma_bf16(acc[mt], wf[RP - 1][mt][s], bh[0], bh[1]);
+            }
           }
         }
         // partial tile into the ring.  (A ring of two slots per chain needs no look at `empty`:
@@ -226,9 +245,12 @@ __global__ void __launch_bounds__(GL_THREADS, 1) gl_bwd_kernel(const __grid_cons
   constexpr int U = 4 * NMT;
   constexpr int KSB = (G * NMT + 3) / 4;  // k-steps of the CTA's own gate columns
   constexpr int SP = 4 / NMT;             // parts the sources of a gather are split into
+  constexpr bool LO = gl_lo_in_smem<NMT, TPW, SPLIT>();
+  constexpr int RP = LO ? 1 : SPLIT;
   extern __shared__ __align__(16) uint8_t smem[];
   uint8_t* gsm = smem;                                                    // [ring][KSB][512]
-  float* red = reinterpret_cast<float*>(gsm + GL_GRING * KSB * 512);      // [2 groups][2][SP][NMT * 32]
+  uint4* lo = reinterpret_cast<uint4*>(gsm + GL_GRING * KSB * 512);       // LO: [warp][TPW][KSB][lane]
+  float* red = reinterpret_cast<float*>(lo + (LO ? GL_WARPS * TPW * KSB * 32 : 0));  // [2 groups][2][SP][NMT * 32]
   float* carry = red + 4 * SP * NMT * 32;                                 // [CH][dh, dc, c][NMT * 32]
   uint64_t* barp = reinterpret_cast<uint64_t*>(carry + p.CH * 3 * NMT * 32);
   const uint32_t gbar = smem_u32(barp);                                   // full, empty, parts met (a group each)
@@ -261,7 +283,8 @@ __global__ void __launch_bounds__(GL_THREADS, 1) gl_bwd_kernel(const __grid_cons
     // destinations at a time); tile row m is unit m & 1 (+ 2 for m >= 8) of quad (m & 7) / 2
     reg_inc<GL_BWD_P>();
     const int rot = hs % p.K16;
-    uint32_t wf[SPLIT][TPW][KSB][4];
+    uint32_t wf[RP][TPW][KSB][4];
+    lo += w * TPW * KSB * 32 + lane;
     uint32_t doff[TPW];  // word offset of this lane's piece, ~0: nothing to store
 #pragma unroll
     for (int i = 0; i < TPW; ++i) {
@@ -273,7 +296,13 @@ __global__ void __launch_bounds__(GL_THREADS, 1) gl_bwd_kernel(const __grid_cons
 #pragma unroll
       for (int kk = 0; kk < KSB; ++kk) {
         const int lq = kk * 4 + q, gate = lq / NMT, wq = lq - gate * NMT;
-        bwd_weights<G, SPLIT, T>(p, Q * 4 + (gq & 1), gate, u0 + 4 * wq, live, wf[0][i][kk], wf[SPLIT - 1][i][kk]);
+        uint32_t l[4];
+        bwd_weights<G, SPLIT, T>(p, Q * 4 + (gq & 1), gate, u0 + 4 * wq, live, wf[0][i][kk], l);
+        if (LO) lo[(i * KSB + kk) * 32] = make_uint4(l[0], l[1], l[2], l[3]);
+        else if (SPLIT == 2) {
+#pragma unroll
+          for (int a = 0; a < 4; ++a) wf[RP - 1][i][kk][a] = l[a];
+        }
       }
     }
     bool alive = true;
@@ -304,7 +333,10 @@ __global__ void __launch_bounds__(GL_THREADS, 1) gl_bwd_kernel(const __grid_cons
                 if (i0 + i < TPW) mma_bf16(acc[i], wf[0][(i0 + i) % TPW][kk], y[kk].z, y[kk].w);
 #pragma unroll
               for (int i = 0; i < 4; ++i)
-                if (i0 + i < TPW) mma_bf16(acc[i], wf[SPLIT - 1][(i0 + i) % TPW][kk], y[kk].x, y[kk].y);
+                if (i0 + i < TPW) {
+                  if (LO) mma_bf16(acc[i], lo[((i0 + i) * KSB + kk) * 32], y[kk].x, y[kk].y);
+                  else mma_bf16(acc[i], wf[RP - 1][(i0 + i) % TPW][kk], y[kk].x, y[kk].y);
+                }
             }
           }
 #pragma unroll

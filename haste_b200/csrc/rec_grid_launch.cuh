@@ -51,7 +51,8 @@ template <int G, int NMT, int KSW, int SPLIT, typename T>
 int gl_fwd_go(ChainParams& p, const GlGeometry& g, cudaStream_t s) {
   static std::atomic<int> set[kChainMaxDevices];
   const size_t slot = (size_t)GL_WARPS * NMT * 512 + 16;
-  const size_t rest = (size_t)g.CH * 2 * NMT * 128 + (size_t)GL_WARPS * IoBytes<T>::WARP;
+  const size_t rest = (size_t)g.CH * 2 * NMT * 128 + (size_t)GL_WARPS * IoBytes<T>::WARP +
+                      (gl_lo_in_smem<NMT, KSW, SPLIT>() ? (size_t)GL_WARPS * NMT * KSW * 512 : 0);
   // two slots per chain where they fit, else as many as do
   const int fit = rest >= (size_t)kGlMaxSmem ? 0 : (int)(((size_t)kGlMaxSmem - rest) / slot);
   p.ring = min(2 * g.CH, fit);
@@ -65,9 +66,8 @@ int gl_fwd(ChainParams& p, const GlGeometry& g, cudaStream_t s) {
   const int ksw = ceil_div(g.KS16, GL_WARPS);
 #define HB_GL(nmt, k) \
   if (g.NMT == nmt && ksw <= k) return gl_fwd_go<G, nmt, k, SPLIT, T>(p, g, s);
-  HB_GL(4, 2) HB_GL(4, 4)
-  if constexpr (SPLIT == 1) { HB_GL(4, 6) HB_GL(4, 8) }
-  else { HB_GL(2, 6) HB_GL(2, 8) }  // (as gl_geometry chooses NMT)
+  HB_GL(4, 2) HB_GL(4, 4) HB_GL(4, 6) HB_GL(4, 8)
+  if constexpr (SPLIT == 2) { HB_GL(2, 6) HB_GL(2, 8) }
 #undef HB_GL
   return HASTE_B200_ERR_UNSUPPORTED;
 }
@@ -76,7 +76,7 @@ template <int G, int NMT, int TPW, int SPLIT, typename T>
 int gl_bwd_go(ChainParams& p, const GlGeometry& g, cudaStream_t s) {
   static std::atomic<int> set[kChainMaxDevices];
   constexpr int KSB = (G * NMT + 3) / 4, SP = 4 / NMT;
-  const size_t smem = (size_t)GL_GRING * KSB * 512 + (size_t)4 * SP * NMT * 128 + (size_t)g.CH * 3 * NMT * 128 +
+  const size_t smem = (size_t)GL_GRING * KSB * 512 + (gl_lo_in_smem<NMT, TPW, SPLIT>() ? (size_t)GL_WARPS * TPW * KSB * 512 : 0) + (size_t)4 * SP * NMT * 128 + (size_t)g.CH * 3 * NMT * 128 +
                       (2 * GL_GRING + 2) * 8 + (size_t)GL_WARPS * IoBytes<T>::WARP;
   return gl_launch(gl_bwd_kernel<G, NMT, TPW, SPLIT, T>, p, g.nHS * g.nRG, smem, set, s);
 }
@@ -86,9 +86,8 @@ int gl_bwd(ChainParams& p, const GlGeometry& g, cudaStream_t s) {
   const int tpw = ceil_div(g.KS16, GL_WARPS);
 #define HB_GL(nmt, k) \
   if (g.NMT == nmt && tpw <= k) return gl_bwd_go<G, nmt, k, SPLIT, T>(p, g, s);
-  HB_GL(4, 2) HB_GL(4, 4)
-  if constexpr (SPLIT == 1) { HB_GL(4, 6) HB_GL(4, 8) }
-  else { HB_GL(2, 6) HB_GL(2, 8) }  // (as gl_geometry chooses NMT)
+  HB_GL(4, 2) HB_GL(4, 4) HB_GL(4, 6) HB_GL(4, 8)
+  if constexpr (SPLIT == 2) { HB_GL(2, 6) HB_GL(2, 8) }
 #undef HB_GL
   return HASTE_B200_ERR_UNSUPPORTED;
 }

@@ -60,6 +60,10 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint4& a, uint32_t b0, uint32_t b1) {
+  const uint32_t f[4] = {a.x, a.y, a.z, a.w};
+  mma_bf16(d, f, b0, b1);
+}
 // Polling loads: relaxed, gpu scope, so that every poll is served by L2.
 __device__ __forceinline__ uint4 ld_relaxed_u32x4(const uint32_t* p) {
   uint4 v;

@@ -109,3 +109,18 @@ def test_tensor_core_gru_gates_are_exact(N, H):
         z, r = (zx + zh).sigmoid(), (rx + rh).sigmoid()
         want = (z * h + (1 - z) * (gx + r * gh).tanh()).bfloat16()
     assert (y != want).double().mean() < 6e-4
+
+
+# beyond 512 units with more rows: sixteen units per CTA, R's second plane in shared memory
+@pytest.mark.parametrize("shape", [(5, 24, 513), (6, 31, 1024), (5, 45, 777), (4, 64, 640), (4, 100, 530), (3, 190, 1021)],
+                         ids=lambda s: "T%d_N%d_H%d" % s)
+@pytest.mark.parametrize("cell,dtype,tol", [("lstm", torch.float32, TOL_F32), ("gru", torch.float32, TOL_F32),
+                                            ("gru", torch.float16, TOL_F16)])
+@pytest.mark.parametrize("budget", [0, 74])
+def test_grid_recurrence_of_wide_layers(cell, dtype, tol, shape, budget):
+    from haste_b200 import _C
+    was = _C.exchange_sm_budget(budget)
+    try:
+        _check(cell, *shape, dtype, tol, 0.25, transposed=shape[1] % 2 == 0)
+    finally:
+        _C.exchange_sm_budget(was)
