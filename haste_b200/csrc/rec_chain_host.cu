@@ -44,7 +44,7 @@ bool gl_geometry(int dtype, int N, int H, bool bwd, int most, GlGeometry* g) {
   // the whole GPU for one direction after the other still beats the step-wise path (bf16 LSTM, two
   // directions of 139 rows, H = 696: 18 chains within the budget, 6 without).
   for (int use : {budget, sms}) {
-    if (use > sms) continue;
+    if (use < g->KS16 || use > sms) continue;  // (four quads take the fewest CTAs: one per 16 units)
     for (int nmt : {2, 4}) {
       if (nmt == 2 && (dtype == HASTE_B200_BF16 || ks <= 4)) continue;
       g->NMT = nmt;
