@@ -97,8 +97,8 @@ __device__ __forceinline__ void load_bias(const ChainParams& p, int unit, float 
 }
 
 // The cell's gradient: gate values gv, gradients of h and c -> gate gradients dg (LSTM d(i,g,f,o);
-// GRU dp_z, dp_r, dp_g, dq_g), carried gradients.
-template <int G>
+// GRU dp_z, dp_r, dp_g, dq_g), carried gradients.  TANH: `cnew` is already tanh(c).
+template <int G, bool TANH = false>
 __device__ __forceinline__ void cell_bwd(const float (&gv)[4], float prev /* c or h before */, float cnew,
                                          float dh_total, float dcv, bool zo, float m, float& dh_c,
                                          float& dc_c, float (&dg)[4]) {
@@ -108,7 +108,7 @@ __device__ __forceinline__ void cell_bwd(const float (&gv)[4], float prev /* c o
     dh_total = m * dh_total;
   }
   if (G == 4) {
-    const float c_tanh = chain_tanh(cnew);
+    const float c_tanh = TANH ? cnew : chain_tanh(cnew);
     const float dc_total = dcv + dc_c + d_tanh(c_tanh) * (gv[3] * dh_total);
     dg[0] = d_sigmoid(gv[0]) * (gv[1] * dc_total);
     dg[1] = d_tanh(gv[1]) * (gv[0] * dc_total);

@@ -7,13 +7,14 @@
 //
 //   forward   gates[rows, G*16] = h_{t-1}[rows, 0:H] . R[0:H, slice]            K = H
 //   backward  dh_rec[rows, 16]  = dq_{t+1}[rows, 0:GH] . R[slice, 0:GH]^T       K = GH
+//   (long K: four CTAs, a quarter of K and 64 units each - tc_geometry_for)
 //
 // (G = 3 for the GRU; G = 4 for the LSTM, where "dq" is the gate gradient in the cache's place.)
 // A step is bound by its chain - counter, TMA, MMA issue (65 cycles each), tensor-memory read, gate
 // math, publish - and, with many rows per CTA, by the stream of h or dq at 64 bytes per clock and SM.
-// GRU, H = 1024, us per step forward / backward: 128 rows 6.8 / 10.3, 256 rows 7.8 / 12.1 (with one 128-row
-// tile per CTA 7.6 / 13.3, then with the faster gate functions below).  Two directions of 200 steps side by side, chain kernels -> this: GRU 90
-// rows 8.2 -> 5.0 ms, LSTM 90 rows 8.1 -> 6.4, LSTM 178 rows H = 808 9.4 -> 6.9.
+// GRU, H = 1024, us per step forward / backward: 128 rows 6.9 / 8.0, 256 rows 7.9 / 10.4 (with one 128-row
+// tile per CTA 7.9 / 11.5).  Two directions of 200 steps side by side, chain kernels -> this: GRU 90
+// rows 8.2 -> 5.0 ms, LSTM 90 rows 8.1 -> 6.4, LSTM 178 rows H = 808 9.4 -> 6.9 (with all of K per CTA, below).
 //
 // * Grid = (H / 16 hidden slices) x (row groups), one cooperative launch per layer pass; a
 //   CTA owns 16 hidden units for MT tiles of RB (64 or 128) batch rows.
@@ -46,6 +47,8 @@
 // (lib/gru_forward_gpu.cu.cc:214-308,345-363, lib/gru_backward_gpu.cu.cc:252-320) for
 // bf16 batches of about a hundred rows and more; math as in lib/gru_forward_gpu.cu.cc:27-85
 // and lib/gru_backward_gpu.cu.cc:26-96.
+#include <atomic>
+
 #include "rec_chain.cuh"
 #include "tcgen05.cuh"
 
@@ -58,12 +61,15 @@ typedef __nv_bfloat16 bf16;
 constexpr int UC = 16;                 // hidden units per CTA
 constexpr int BK = 64;                 // K elements per TMA box / swizzle row (128 bytes)
 constexpr int A_STAGE = 128 * BK * 2;  // one streamed stage: 128 rows x 128 bytes
-#ifndef HB_TC_NI
-#define HB_TC_NI 4
-#endif
-constexpr int NI = HB_TC_NI;           // MMA-issuing warps (k-blocks go to them in turn)
-constexpr int TC_THREADS = 32 * (1 + NI + 4);  // warp 0 TMA, warps 1..NI MMA, then 4 epilogue warps
+constexpr int PL = 4;                  // lanes that issue the TMA loads (k-blocks go to them in turn)
+// MMA-issuing warps (likewise).  Four, but two where a CTA has a quarter of the k-blocks: their instructions
+// still hide behind the stream, and there is half as much tensor memory to read.
+template <int CL> constexpr int issuers() { return CL > 1 ? 2 : 4; }
+// warp 0 TMA, then the issuers, then 4 epilogue warps
+template <int CL> constexpr int tc_threads() { return 32 * (1 + issuers<CL>() + 4); }
 constexpr int MAX_SMEM = 227 * 1024;
+constexpr int CLUSTER = 4;             // CTAs that share out a long K (backward)
+constexpr int XCH = 4 * (CLUSTER - 1) * 4 * 512;  // bytes of partial dh a CTA takes: [warp][source][4 units][row][4]
 
 struct TcParams {
   int T, N, H, nHS, MT, RB, training, has_zoneout, r_transposed;
@@ -109,6 +115,11 @@ __device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int* p) {
 }
 __device__ __forceinline__ void red_release_add(unsigned int* p, unsigned int v) {
   asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t add_acq_rel_cta(uint32_t p, uint32_t v) {
+  uint32_t old;
+  asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(p), "r"(v) : "memory");
+  return old;
 }
 __device__ __forceinline__ void fence_proxy_async_all() {
   asm volatile("fence.proxy.async;" ::: "memory");
@@ -187,13 +198,14 @@ __device__ __forceinline__ uint32_t swz_off(int n, int kk) {
   return (uint32_t)((n >> 3) * 1024 + (n & 7) * 128 + ((((kk >> 3) ^ (n & 7)) & 7) << 4) + (kk & 7) * 2);
 }
 
-// The ring's stages belong to NI lanes / issuers for good: `own` has stages own, own + NI, ...  (If
+// The ring's stages belong to M lanes / issuers for good: `own` has stages own, own + M, ...  (If
 // they took k-blocks in turn whatever the stage, one of them a whole ring ahead of another would
 // take a phase of a stage for the one two further on, which a barrier's parity does not tell
 // apart.)  From one block of `own` to its next.
+template <int M>
 __device__ __forceinline__ void next_block(int& stage, uint32_t& phase, int& kb, int own, int stages) {
-  stage += NI;
-  kb += NI;
+  stage += M;
+  kb += M;
   if (stage >= stages) {
     kb += stages + own - stage;
     stage = own;
@@ -201,35 +213,53 @@ __device__ __forceinline__ void next_block(int& stage, uint32_t& phase, int& kb,
   }
 }
 
-// G: gates, 3 GRU, 4 LSTM.
-template <int G, bool FWD>
-__global__ void __launch_bounds__(TC_THREADS, 1)
+// 16 bytes into another CTA's shared memory, counted on its barrier when they have arrived.
+__device__ __forceinline__ void st_async_f4(uint32_t addr, uint32_t bar, float a, float b, float c, float d) {
+  asm volatile(
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr),
+      "f"(a), "f"(b), "f"(c), "f"(d), "r"(bar)
+      : "memory");
+}
+
+// G: gates, 3 GRU, 4 LSTM.  CL: CTAs of a cluster that share out K (backward).
+template <int G, bool FWD, int CL>
+__global__ void __launch_bounds__(tc_threads<CL>(), 1)
 tc_recurrence_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p, const int stages) {
+  constexpr int NI = issuers<CL>(), TC_THREADS = tc_threads<CL>();
+  constexpr bool SPLIT = CL > 1;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* aligned = smem_raw + (base - smem_u32(smem_raw));
   const int H = p.H, N = p.N;
-  constexpr int NB = FWD ? G * UC : UC;  // columns of the step product
+  constexpr int NB = FWD ? G * UC : CL * UC;  // columns of the step product
   const int K = FWD ? H : G * H;
-  const int KB = (K + BK - 1) / BK;  // (TMA fills what lies beyond K with zeros)
+  const int hs = blockIdx.x % p.nHS, rg = blockIdx.x / p.nHS;
+  const int rank = hs % CL;  // in the cluster
+  // this CTA's k-blocks: all or a share of them (TMA fills what lies beyond K with zeros)
+  const int KBT = (K + BK - 1) / BK, KBS = (KBT + CL - 1) / CL;
+  const int kb0 = SPLIT ? rank * KBS : 0, KB = SPLIT ? max(0, min(KBS, KBT - kb0)) : KBT;
   constexpr int R_TILE = NB * 128;  // bytes of the resident operand per k-block
-  const uint32_t r_bytes = (uint32_t)KB * R_TILE;
+  const uint32_t r_bytes = (uint32_t)KBS * R_TILE;
   const uint32_t ring = base + r_bytes;  // r_bytes is a multiple of 1024
   uint8_t* ring_ptr = aligned + r_bytes;
   // (a 64-row stage is read by the 128-row MMA together with the stage behind it - rows whose
   // results nobody uses - so the ring is padded by half a tile at its end)
-  uint64_t* bars = reinterpret_cast<uint64_t*>(ring_ptr + p.ring_bytes);
+  float4* xch = reinterpret_cast<float4*>(ring_ptr + p.ring_bytes);  // SPLIT: the other CTAs' partial dh
+  uint64_t* bars = reinterpret_cast<uint64_t*>(ring_ptr + p.ring_bytes + (SPLIT ? XCH : 0));
   const uint32_t bar0 = smem_u32(bars);
   auto full_bar = [&](int s) { return bar0 + 8u * s; };
   auto empty_bar = [&](int s) { return bar0 + 8u * (stages + s); };
   auto accf_bar = [&](int a) { return bar0 + 8u * (2 * stages + a); };
   auto acce_bar = [&](int a) { return bar0 + 8u * (2 * stages + 2 + a); };
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * stages + 4);
+  // SPLIT, per epilogue warp: partial dh has come; what went out has been read
+  auto xfull_bar = [&](int w) { return bar0 + 8u * (2 * stages + 4 + w); };
+  auto xfree_bar = [&](int w) { return bar0 + 8u * (2 * stages + 8 + w); };
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * stages + (SPLIT ? 12 : 4));
   volatile int* s_abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const uint32_t s_done = smem_u32(tmem_slot + 2);  // [2 tiles] epilogue warps that have stored
   float* s_bias = reinterpret_cast<float*>(tmem_slot + 4);  // forward: [2][48] bx, br
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int hs = blockIdx.x % p.nHS, rg = blockIdx.x / p.nHS;
   const int u0 = hs * UC;
   // two 64-row tiles per CTA: the second one's rows are rows 64..127 of its MMAs and belong to
   // epilogue warps of their own, so that the tiles are two chains that only share the streams
@@ -247,7 +277,12 @@ tc_recurrence_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p
       mbar_init(accf_bar(a), NI);
       mbar_init(acce_bar(a), halves ? 64 : 128);
     }
+    for (int w = 0; SPLIT && w < 4; ++w) {
+      mbar_init(xfull_bar(w), 1);
+      mbar_init(xfree_bar(w), CL - 1);
+    }
     *s_abort = 0;
+    if (SPLIT) tmem_slot[2] = tmem_slot[3] = 0u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -283,21 +318,22 @@ tc_recurrence_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p
       s_bias[i] = u0 + u < H ? __bfloat162float((which ? p.br : p.bx)[gate * H + u0 + u]) : 0.f;
     }
   } else {
-    // B^T[n = unit j][k = gate column c] = R[u0 + j][c]   (R_t[c][u0 + j] when transposed)
+    // B^T[n = unit j of the cluster][k = gate column c] = R[c0 + j][c]   (R_t[c][c0 + j] when transposed)
+    const int c0 = u0 - rank * UC, k0 = kb0 * BK, kn = min(K - k0, KB * BK);
     if (!p.r_transposed) {
-      for (int item = threadIdx.x; item < 16 * (K / 8); item += TC_THREADS) {
-        const int j = item / (K / 8), c8 = (item % (K / 8)) * 8;
-        if (u0 + j >= H) continue;
-        const uint4 w = *reinterpret_cast<const uint4*>(p.R + (size_t)(u0 + j) * K + c8);
+      for (int item = threadIdx.x; item < NB * (KB * BK / 8); item += TC_THREADS) {
+        const int j = item / (KB * BK / 8), c8 = (item % (KB * BK / 8)) * 8;
+        if (c0 + j >= H || c8 >= kn) continue;
+        const uint4 w = *reinterpret_cast<const uint4*>(p.R + (size_t)(c0 + j) * K + k0 + c8);
         uint8_t* tile = aligned + (size_t)(c8 / BK) * R_TILE;
         *reinterpret_cast<uint4*>(tile + swz_off(j, c8 % BK)) = w;  // one whole 16-byte chunk
       }
     } else {
-      for (int item = threadIdx.x; item < K * 2; item += TC_THREADS) {
-        const int c = item / 2, uo = item % 2 * 8;
-        if (u0 + uo >= H) continue;
+      for (int item = threadIdx.x; item < KB * BK * (NB / 8); item += TC_THREADS) {
+        const int c = item / (NB / 8), uo = item % (NB / 8) * 8;
+        if (c0 + uo >= H || c >= kn) continue;
         float x[8];
-        ld8(p.R + (size_t)c * H + u0 + uo, x);
+        ld8(p.R + (size_t)(k0 + c) * H + c0 + uo, x);
         uint8_t* tile = aligned + (size_t)(c / BK) * R_TILE;
 #pragma unroll
         for (int j = 0; j < 8; ++j)
@@ -310,18 +346,18 @@ tc_recurrence_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (SPLIT) cluster_sync_all();  // the others' barriers are initialised before anything arrives on them
   const uint32_t tmem_base = *tmem_slot;
 
   const int tiles_total = (N + p.RB - 1) / p.RB;
-  // per step: the epilogue warps of every CTA
-  const unsigned int arrivals = (unsigned int)p.nHS * (halves ? 2u : 4u);
+  // per step: the epilogue warps of every CTA; SPLIT: the last of them
+  const unsigned int arrivals = (unsigned int)p.nHS * (SPLIT ? 1u : halves ? 2u : 4u);
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
     // PL lanes issue the k-blocks (lane l fills stages l, l + PL, ...): a cp.async.bulk.tensor
     // holds its issuing thread for about 0.1 us, which would otherwise be the rate of the whole
     // ring.
-    constexpr int PL = NI;
     constexpr unsigned PMASK = (1u << PL) - 1u;
     if (lane < PL) {
       int stage = lane, kb = lane;  // this lane's next stage, and its k-block counted from this tile
@@ -345,8 +381,8 @@ tc_recurrence_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p
           while (kb < KB) {
             if (!mbar_wait(empty_bar(stage), phase ^ 1u, s_abort, p.err, 52)) { ok = false; break; }
             mbar_expect_tx(full_bar(stage), box_bytes);
-            tma_load_3d(ring + stage * p.stage_bytes, &map_a, full_bar(stage), kb * BK, row, 0);
-            next_block(stage, phase, kb, lane, stages);
+            tma_load_3d(ring + stage * p.stage_bytes, &map_a, full_bar(stage), (kb0 + kb) * BK, row, 0);
+            next_block<PL>(stage, phase, kb, lane, stages);
           }
           kb -= KB;
           ok = __all_sync(PMASK, ok);  // all producer lanes leave together
@@ -392,7 +428,7 @@ tc_recurrence_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p
             tc_mma_bf16(d_tmem, ad + 4, bd + 4, idesc, 1u);
             tc_mma_bf16(d_tmem, ad + 6, bd + 6, idesc, 1u);
             tc_commit(empty_bar(stage));
-            next_block(stage, phase, kb, iss, stages);
+            next_block<NI>(stage, phase, kb, iss, stages);
           }
           kb -= KB;
           if (iss == 0) HB_STAMP(p, it, mt, 3);  // last MMA issued
@@ -405,6 +441,7 @@ tc_recurrence_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p
     const int quad = warp & 3;
     const int r = (halves ? quad & 1 : quad) * 32 + lane;  // row of the tile
     uint32_t acc_phase[2] = {0, 0};
+    uint32_t x_phase = 0;
     int n_acc = 0;
     bool ok = true;
     const long long NH = (long long)N * H;
@@ -419,10 +456,11 @@ tc_recurrence_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p
         const long long o0 = (long long)n * H + u0;
         // The 16 units are handled in two halves of 8 and the step inputs stay packed (bf16
         // pairs) until they are used, so that the live state of a thread stays within its
-        // share of the register file (nine warps per CTA).
+        // share of the register file (nine warps per CTA, seven where K is shared out).
         // ---- inputs that do not depend on the recurrence: issued before the wait below
         uint4 in0[2], in1[2], in2[2], in3[2], hp[2], mk[2], dhn[2], cn[2], dcn[2];
         float carry[2][8];  // backward: dh; LSTM forward: c
+        float dc0[2][8], c_tanh[2][8];  // LSTM backward
         if (valid) {
 #pragma unroll
           for (int hf = 0; hf < 2; ++hf) {
@@ -449,6 +487,22 @@ tc_recurrence_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p
               dhn[hf] = ldq(p.dh_new + (long long)(t + 1) * NH + o0 + uo);
               if (p.has_zoneout) mk[hf] = ldq(p.mask + (long long)t * NH + o0 + uo);
               ld_carry(p.dh_carry + o0 + uo, carry[hf]);
+              if (G == 4) ld_carry(p.c_carry + o0 + uo, dc0[hf]);
+            }
+          }
+        }
+        // ---- backward: what can be done without the step product (the accurate tanh of an LSTM's c takes 2000 cycles)
+        if (!FWD && valid) {
+#pragma unroll
+          for (int hf = 0; hf < 2; ++hf) {
+            if (u0 + hf * 8 >= H) break;
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+              carry[hf][u] += bfq(dhn[hf], u);
+              if (G == 4) {
+                if (p.dc_new) dc0[hf][u] += bfq(dcn[hf], u);
+                c_tanh[hf][u] = rec::chain_tanh(bfq(cn[hf], u));
+              }
             }
           }
         }
@@ -471,16 +525,89 @@ tc_recurrence_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p
           if (warp == NI + 1 && lane == 0) HB_STAMP(p, it, mt, 4);  // accumulator complete
         }
         const uint32_t taddr = tmem_base + acc * NI * ACC_COLS + ((uint32_t)(quad * 32) << 16);
+        const bool takes = halves || quad * 32 < p.RB;  // some of the warp's rows are in the tile
+        float rec_dh[16];  // backward: the step product
+        if (!FWD && have_acc) {
+          constexpr int XG = G == 4 && !SPLIT ? 2 : NI;  // accumulators in flight (registers)
+          // columns of 16 units, summed over the issuers
+          auto columns = [&](int col, float (&x)[16]) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) x[i] = 0.f;
+#pragma unroll
+            for (int g0 = 0; g0 < NI; g0 += XG) {
+              uint32_t b[XG][16];
+#pragma unroll
+              for (int k = 0; k < XG; ++k) {
+                if (have >> (g0 + k) & 1u) {
+                  tc_ld16(taddr + (g0 + k) * ACC_COLS + col, b[k]);
+                } else {
+#pragma unroll
+                  for (int i = 0; i < 16; ++i) b[k][i] = 0u;
+                }
+              }
+              tc_wait_ld();
+#pragma unroll
+              for (int k = 0; k < XG; ++k)
+#pragma unroll
+                for (int i = 0; i < 16; ++i) x[i] += __uint_as_float(b[k][i]);
+            }
+          };
+          // the other CTAs' units go to them, to the warp with the same rows; then this CTA's own
+          // (a second row tile's partial sums take the place of the first one's)
+          if (SPLIT && takes && p.MT > 1 && !halves) {
+            bool free_ = mbar_wait_cluster(xfree_bar(quad), x_phase ^ 1u, s_abort, p.err, 56);
+            free_ = __all_sync(0xffffffffu, free_);
+            if (!free_) { ok = false; break; }
+          }
+          const uint32_t xat = smem_u32(xch) + (uint32_t)(quad * (CL - 1) * 4 * 512 + lane * 16);
+          if (SPLIT && takes && lane == 0) mbar_expect_tx(xfull_bar(quad), (CL - 1) * 32 * 64);
+#pragma unroll 1
+          for (int d = 1; takes && d < CL; ++d) {
+            const uint32_t to = (uint32_t)(rank + d) % CL;
+            const uint32_t at = mapa_u32(xat + (uint32_t)(CL - 1 - d) * 2048, to), bar = mapa_u32(xfull_bar(quad), to);
+            float x[16];
+            columns((int)to * UC, x);
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+              st_async_f4(at + c * 512, bar, x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
+          }
+          columns(rank * UC, rec_dh);
+          tc_fence_before();
+          mbar_arrive(acce_bar(acc));  // the accumulator buffer is free
+          if (warp == NI + 1 && lane == 0) HB_STAMP(p, it, mt, 5);
+        }
+        if (SPLIT && have_acc && takes) {
+          bool got = mbar_wait_cluster(xfull_bar(quad), x_phase, s_abort, p.err, 57);
+          got = __all_sync(0xffffffffu, got);
+          if (!got) { ok = false; break; }
+          x_phase ^= 1u;
+          const float4* x = xch + quad * (CL - 1) * 4 * 32 + lane;
+#pragma unroll
+          for (int d = 0; d < CL - 1; ++d)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const float4 v = x[(d * 4 + c) * 32];
+              float* y = rec_dh + c * 4;
+              y[0] += v.x; y[1] += v.y; y[2] += v.z; y[3] += v.w;
+            }
+          if (p.MT > 1 && !halves) {
+            __syncwarp();
+            if (lane < CL - 1) mbar_arrive_cluster(mapa_u32(xfree_bar(quad), (uint32_t)((rank + 1 + lane) % CL)));
+          }
+        }
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
           const int uo = hf * 8;
           // this half's columns of the accumulators (one per issuer), summed
           float s0[8], s1[8], s2[8], s3[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) s0[i] = s1[i] = s2[i] = s3[i] = 0.f;
-          if (have_acc) {
+          for (int i = 0; i < 8; ++i) {
+            s0[i] = !FWD && have_acc ? rec_dh[hf * 8 + i] : 0.f;
+            s1[i] = s2[i] = s3[i] = 0.f;
+          }
+          if (FWD) {
             // the issuers' accumulators, GRP of them per wait (all loads of a group in flight)
-            constexpr int GRP = FWD ? (G == 4 ? 1 : 2) : NI;
+            constexpr int GRP = G == 4 ? 1 : 2;
 #pragma unroll
             for (int g0 = 0; g0 < NI; g0 += GRP) {
               uint32_t b0[GRP][8], b1[GRP][8], b2[GRP][8], b3[GRP][8];
@@ -489,11 +616,9 @@ tc_recurrence_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p
                 const int i2 = g0 + k;
                 if (i2 < NI && (have >> i2 & 1u)) {
                   tc_ld8(taddr + i2 * ACC_COLS + uo, b0[k]);
-                  if (FWD) {
-                    tc_ld8(taddr + i2 * ACC_COLS + 16 + uo, b1[k]);
-                    tc_ld8(taddr + i2 * ACC_COLS + 32 + uo, b2[k]);
-                    if (G == 4) tc_ld8(taddr + i2 * ACC_COLS + 48 + uo, b3[k]);
-                  }
+                  tc_ld8(taddr + i2 * ACC_COLS + 16 + uo, b1[k]);
+                  tc_ld8(taddr + i2 * ACC_COLS + 32 + uo, b2[k]);
+                  if (G == 4) tc_ld8(taddr + i2 * ACC_COLS + 48 + uo, b3[k]);
                 }
               }
               tc_wait_ld();
@@ -504,11 +629,9 @@ tc_recurrence_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p
 #pragma unroll
                   for (int i = 0; i < 8; ++i) {
                     s0[i] += __uint_as_float(b0[k][i]);
-                    if (FWD) {
-                      s1[i] += __uint_as_float(b1[k][i]);
-                      s2[i] += __uint_as_float(b2[k][i]);
-                      if (G == 4) s3[i] += __uint_as_float(b3[k][i]);
-                    }
+                    s1[i] += __uint_as_float(b1[k][i]);
+                    s2[i] += __uint_as_float(b2[k][i]);
+                    if (G == 4) s3[i] += __uint_as_float(b3[k][i]);
                   }
                 }
               }
@@ -563,28 +686,26 @@ tc_recurrence_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p
                 st8(vt, vz); st8(vt + H, vr); st8(vt + 2 * H, vg); st8(vt + 3 * H, vq);
               }
             } else if (G == 4) {
-              float di[8], dg[8], df[8], d_o[8], dcc[8];
-              ld_carry(p.c_carry + o0 + uo, dcc);  // the carried gradient of c
+              float di[8], dg[8], df[8], d_o[8];
 #pragma unroll
               for (int u = 0; u < 8; ++u) {
                 const float gv[4] = {bfq(in0[hf], u), bfq(in1[hf], u), bfq(in2[hf], u), bfq(in3[hf], u)};
                 float d[4];
-                const float dh_total = bfq(dhn[hf], u) + carry[hf][u] + s0[u];
-                rec::cell_bwd<4>(gv, bfq(hp[hf], u), bfq(cn[hf], u), dh_total, p.dc_new ? bfq(dcn[hf], u) : 0.f,
-                                 p.has_zoneout != 0, p.has_zoneout ? bfq(mk[hf], u) : 1.f, carry[hf][u], dcc[u], d);
+                rec::cell_bwd<4, true>(gv, bfq(hp[hf], u), c_tanh[hf][u], carry[hf][u] + s0[u], 0.f, p.has_zoneout != 0,
+                                       p.has_zoneout ? bfq(mk[hf], u) : 1.f, carry[hf][u], dc0[hf][u], d);
                 di[u] = d[0]; dg[u] = d[1]; df[u] = d[2]; d_o[u] = d[3];
               }
               bf16* vt = p.v + ((long long)t * N + n) * 4 * H + u0 + uo;  // streamed next
               st8(vt, di); st8(vt + H, dg); st8(vt + 2 * H, df); st8(vt + 3 * H, d_o);
               st_carry(p.dh_carry + o0 + uo, carry[hf]);
-              st_carry(p.c_carry + o0 + uo, dcc);
+              st_carry(p.c_carry + o0 + uo, dc0[hf]);
             } else {
               float dpz[8], dpr[8], dpg[8], dqg[8];
 #pragma unroll
               for (int u = 0; u < 8; ++u) {
                 const float z = bfq(in0[hf], u), rr = bfq(in1[hf], u), g = bfq(in2[hf], u),
                             qg = bfq(in3[hf], u);
-                float dh_total = bfq(dhn[hf], u) + carry[hf][u] + s0[u];
+                float dh_total = carry[hf][u] + s0[u];
                 float keep = 0.f;
                 if (p.has_zoneout) {
                   const float m = bfq(mk[hf], u);
@@ -614,8 +735,13 @@ tc_recurrence_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p
         // and publishes all 32 lanes' stores.  (A __threadfence() in front of it cost another
         // 0.5 us per step and changed nothing.)  Only lane 0 waits; the other lanes go on to
         // the next step's loads.  Rows beyond the batch store nothing but still arrive.
+        // SPLIT: the tile's last warp arrives for all of them (GRU, H = 1024, 128 rows 8.4 -> 8.0 us per step;
+        // forward 7.1 -> 6.7, but two tiles per CTA 8.0 -> 9.1).
         __syncwarp();
-        if (lane == 0) red_release_add(p.cnt + tile, 1u);
+        if (lane == 0) {
+          const uint32_t others = halves ? 1u : 3u;
+          if (!SPLIT || (add_acq_rel_cta(s_done + 4 * (uint32_t)mt, 1u) & others) == others) red_release_add(p.cnt + tile, 1u);
+        }
         if (warp == NI + 1 && lane == 0) HB_STAMP(p, it, mt, 7);  // published
       }
     }
@@ -625,6 +751,11 @@ tc_recurrence_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p
   tc_fence_before();
   __syncthreads();
   if (*s_abort) atomicExch(p.abort_flag, 1);
+  if (SPLIT) {  // nobody leaves while another may still write to it
+    if (*s_abort)  // (nor before what is under way has arrived: nobody waits for it then)
+      for (const long long t0 = clock64(); clock64() - t0 < 100000;) {}
+    cluster_sync_all();
+  }
   if (warp == 1) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
                  "r"(TMEM_COLS)
@@ -633,8 +764,38 @@ tc_recurrence_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p
 }
 
 // ---- host side ---------------------------------------------------------------------------
+// How many clusters of the backward kernel with SPLIT the device holds at once; 0: none.
+int max_tc_clusters() {
+  constexpr int kMaxDevices = 64;
+  static std::atomic<int> most[kMaxDevices];  // 0: not asked yet, -1: none
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+  int n = most[dev].load(std::memory_order_acquire);
+  if (n == 0) {
+    n = -1;
+    auto kernel = tc_recurrence_kernel<3, false, CLUSTER>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(sm_count() / CLUSTER * CLUSTER);
+    cfg.blockDim = dim3(tc_threads<CLUSTER>());
+    cfg.dynamicSmemBytes = MAX_SMEM;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = CLUSTER;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0)
+      n = min(clusters, sm_count() / CLUSTER);
+    cudaGetLastError();
+    most[dev].store(n, std::memory_order_release);
+  }
+  return n > 0 ? n : 0;
+}
+
 struct TcGeometry {
-  int nHS, nRG, MT, RB, stages;
+  int nHS, nRG, MT, RB, stages, CL;
   size_t ring, smem;
 };
 
@@ -642,16 +803,21 @@ struct TcGeometry {
 // must fit shared memory), at least 64 batch rows and at most two row tiles per CTA: every CTA of a row
 // group streams the group's whole h (or dq), H / 16 copies of it per step out of L2, so that a third and
 // a fourth tile cost as much again, where the step-wise path's full-size contractions grow little.  GRU,
-// H = 1024, us per step forward / backward, this / step by step: 128 rows 7.0 / 10.5 and 19.3 / 18.5, 256
-// rows 8.0 / 12.6 and 22.6 / 18.6, 512 rows 10.4 / 17.2 and 20.5 / 22.7; 1024 rows step by step 30.4 / 30.2.
-// LSTM: 256 rows 10.2 / 20.1 and 16.5 / 21.8, 512 rows 14.3 / 33.2 and 20.5 / 28.3.
+// H = 1024, us per step forward / backward, this / step by step: 128 rows 7.0 / 8.0 and 19.3 / 18.5, 256
+// rows 8.0 / 10.4 and 22.6 / 18.6, 512 rows 10.2 / 16.2 and 20.5 / 22.7; 1024 rows step by step 30.4 / 30.2.
+// LSTM: 256 rows 9.8 / 10.1 and 16.5 / 21.8, 512 rows 14.0 / 17.8 and 20.5 / 28.3.
 // (Where the chain kernels take a batch themselves: rec_chain_host.cu.)
-bool tc_geometry_for(int G, int N, int H, bool fwd, int sms, TcGeometry* g) {
+bool tc_geometry_of(int G, int N, int H, bool fwd, int CL, int sms, TcGeometry* g) {
   const int K = fwd ? H : G * H;
-  const size_t r_bytes = (size_t)ceil_div(K, BK) * (fwd ? G * UC : UC) * 128;
-  const size_t fixed = 1024 /*alignment*/ + r_bytes + 1024 /*barriers, bias*/;
+  g->CL = CL;
+  const size_t r_bytes = (size_t)ceil_div(ceil_div(K, BK), CL) * (fwd ? G : CL) * UC * 128;
+  const size_t fixed = 1024 /*alignment*/ + r_bytes + (CL > 1 ? XCH : 0) + 1024 /*barriers, bias*/;
   if (fixed + 2 * (size_t)A_STAGE > (size_t)MAX_SMEM) return false;
   g->nHS = ceil_div(H, UC);
+  if (CL > 1) {  // whole clusters, as many as are resident at a time
+    g->nHS = ceil_div(g->nHS, CLUSTER) * CLUSTER;
+    sms = (int)((long long)max_tc_clusters() * sms / sm_count()) * CLUSTER;
+  }
   const int groups_max = sms / g->nHS;
   if (groups_max < 1) return false;
   // 64-row tiles when that still gives one tile per CTA (more CTAs, less to stream per CTA)
@@ -669,13 +835,34 @@ bool tc_geometry_for(int G, int N, int H, bool fwd, int sms, TcGeometry* g) {
     const size_t stage = (size_t)rb * 128, pad = A_STAGE - stage;
     int stages = (int)(((size_t)MAX_SMEM - fixed - pad) / stage);
     if (stages > 16) stages = 16;
-    if (stages < NI) return false;  // every issuer owns a stage
+    if (stages < PL) return false;  // every lane owns a stage
     g->stages = stages;
     g->ring = stages * stage + pad;
     g->smem = fixed + g->ring;
     return true;
   }
   return false;
+}
+
+// Backward, K = G * H: a CTA that streams dq over all of K for its 16 units reads 128 rows at 64 bytes per clock and
+// as long again into the tensor cores (65 cycles per MMA, whatever its columns).  A cluster of four shares out K
+// instead: each CTA streams a quarter of it for the 64 units of all, and the partial dh - 24 KB in and out
+// - travel through distributed shared memory.  That takes 1500 cycles of its own, so short K stays unsplit, and so
+// does what would take more rows per CTA (clusters leave some SMs out).  us per step, all of K / a quarter: GRU
+// H = 1024 128 rows 10.2 / 8.0, half of the GPU 11.9 / 9.8, 178 rows H = 808 19.2 / 13.6, 256 rows H = 640 15.0 / 15.5,
+// H = 512 8.1 / 8.5; LSTM H = 1024 256 rows 19.6 / 10.1 (of that 4 from the tanh of c, now taken before the wait), 128
+// rows on half of the GPU 19.3 / 9.7, H = 512 512 rows 13.1 / 9.9, H = 320 700 rows 8.0 / 9.0.
+constexpr int kSplitK = 2048;
+
+bool tc_geometry_for(int G, int N, int H, bool fwd, int sms, TcGeometry* g) {
+  const bool whole = tc_geometry_of(G, N, H, fwd, 1, sms, g);
+  TcGeometry split;
+  if (!fwd && G * H >= kSplitK && tc_geometry_of(G, N, H, fwd, CLUSTER, sms, &split) &&
+      (!whole || split.MT * split.RB <= g->MT * g->RB)) {
+    *g = split;
+    return true;
+  }
+  return whole;
 }
 
 // Under an SM budget (concurrent directions) the geometry within it, so that the two directions are
@@ -689,9 +876,9 @@ bool tc_geometry(int G, int N, int H, bool fwd, TcGeometry* g) {
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-template <int G, bool FWD>
+template <int G, bool FWD, int CL>
 int launch_tc(const CUtensorMap& map, TcParams& p, const TcGeometry& g, cudaStream_t s) {
-  auto kernel = tc_recurrence_kernel<G, FWD>;
+  auto kernel = tc_recurrence_kernel<G, FWD, CL>;
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)g.smem);
   if (e != cudaSuccess) {
@@ -699,15 +886,27 @@ int launch_tc(const CUtensorMap& map, TcParams& p, const TcGeometry& g, cudaStre
     return HASTE_B200_ERR_UNSUPPORTED;
   }
   int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, TC_THREADS, g.smem);
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, tc_threads<CL>(), g.smem);
   const int grid = g.nHS * g.nRG;
   if (e != cudaSuccess || per_sm * sm_count() < grid) {
     cudaGetLastError();
     return HASTE_B200_ERR_UNSUPPORTED;
   }
   int stages = g.stages;
-  void* args[] = {const_cast<CUtensorMap*>(&map), &p, &stages};
-  e = cudaLaunchCooperativeKernel((const void*)kernel, dim3(grid), dim3(TC_THREADS), args, g.smem, s);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(tc_threads<CL>());
+  cfg.dynamicSmemBytes = g.smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = CL;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = CL > 1 ? 2 : 1;
+  e = cudaLaunchKernelEx(&cfg, kernel, map, static_cast<const TcParams&>(p), static_cast<const int&>(stages));
   if (e != cudaSuccess) {
     set_last_error("cooperative launch failed: %s", cudaGetErrorString(e));
     cudaGetLastError();
@@ -776,7 +975,7 @@ int gru_forward_tc(const GruFwd& a, cudaStream_t s) {
   p.Wx = (const bf16*)a.tmp_Wx; p.mask = (const bf16*)a.zoneout_mask;
   p.h = (bf16*)a.h; p.v = (bf16*)a.v;
   HB_TRY(tc_scratch(ceil_div(a.N, g.RB), &p, s));
-  return launch_tc<3, true>(map, p, g, s);
+  return launch_tc<3, true, 1>(map, p, g, s);
 }
 
 // Backward: dh_carry (fp32 [N,H]) holds the incoming gradient of the final state and receives
@@ -803,7 +1002,7 @@ int gru_backward_tc(const GruBwd& a, float* dh_carry, cudaStream_t s) {
   p.dh_new = (const bf16*)a.dh_new; p.dp = (bf16*)a.dp; p.dq = (bf16*)a.dq;
   p.dh_carry = dh_carry;
   HB_TRY(tc_scratch(ceil_div(a.N, g.RB), &p, s));
-  return launch_tc<3, false>(map, p, g, s);
+  return g.CL > 1 ? launch_tc<3, false, CLUSTER>(map, p, g, s) : launch_tc<3, false, 1>(map, p, g, s);
 }
 
 // LSTM, in the same way: x.W is in a.v; c_carry (fp32 [N,H]) holds c_0.
@@ -823,7 +1022,7 @@ int lstm_forward_tc(const LstmFwd& a, float* c_carry, cudaStream_t s) {
   p.R = (const bf16*)a.R; p.bx = (const bf16*)a.b; p.Wx = (const bf16*)a.v; p.mask = (const bf16*)a.zoneout_mask;
   p.h = (bf16*)a.h; p.c = (bf16*)a.c; p.v = (bf16*)a.v; p.c_carry = c_carry;
   HB_TRY(tc_scratch(ceil_div(a.N, g.RB), &p, s));
-  return launch_tc<4, true>(map, p, g, s);
+  return launch_tc<4, true, 1>(map, p, g, s);
 }
 
 // v: gates in, gate gradients out.  dh_carry, dc_carry as dh_carry of gru_backward_tc.
@@ -844,7 +1043,7 @@ int lstm_backward_tc(const LstmBwd& a, float* dh_carry, float* dc_carry, cudaStr
   p.c = (bf16*)const_cast<void*>(a.c); p.v = (bf16*)a.v; p.dh_new = (const bf16*)a.dh_new;
   p.dc_new = (const bf16*)a.dc_new; p.dh_carry = dh_carry; p.c_carry = dc_carry;
   HB_TRY(tc_scratch(ceil_div(a.N, g.RB), &p, s));
-  return launch_tc<4, false>(map, p, g, s);
+  return g.CL > 1 ? launch_tc<4, false, CLUSTER>(map, p, g, s) : launch_tc<4, false, 1>(map, p, g, s);
 }
 
 #ifdef HASTE_B200_TIMING_EXPERIMENTS

@@ -137,3 +137,18 @@ def test_few_rows_do_not_go_to_the_tensor_cores():
             layer(x)[0].float().sum().backward()
             torch.cuda.synchronize()
         assert not [e.name for e in seen.events() if "tc_recurrence" in e.name]
+
+
+# a quarter of K per CTA of a cluster: two 128-row and two 64-row tiles per CTA, one of either, unequal shares of K, a
+# cluster with units beyond H
+@pytest.mark.parametrize("T,N,H,sms", [(6, 256, 1024, 74), (5, 200, 520, 74), (5, 190, 688, 74), (4, 300, 1016, 0),
+                                        (3, 270, 744, 74), (4, 128, 1024, 0)])
+@pytest.mark.parametrize("cell", ["lstm", "gru"])
+def test_tensor_core_backward_shares_out_k(cell, T, N, H, sms):
+    from haste_b200 import _C
+    _C.set_sm_budget(sms)
+    try:
+        _check(cell, T, N, H, torch.bfloat16, TOL_BF16, 0.25, transposed=N % 4 == 0)
+        _C.sync_check(torch.cuda.current_stream().cuda_stream)
+    finally:
+        _C.set_sm_budget(0)
