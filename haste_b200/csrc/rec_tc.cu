@@ -1,8 +1,8 @@
 // Tensor-core GRU and LSTM recurrences for large batches (bf16 storage), sm_100a.
 //
 // The chain kernels (rec_grid_kernels.cuh) take eight batch rows at a time and pay for every chain
-// of a CTA.  Where they would need more than six (LSTM: eight) - a hundred rows of a wide layer, or
-// half of that on half of the GPU - the step product is a real tile for the 5th-generation tensor
+// of a CTA.  Where they would need more than four to seven (rec_chain_host.cu) - a hundred rows of a wide
+// layer, or half of that on half of the GPU - the step product is a real tile for the 5th-generation tensor
 // cores, and this file runs it there:
 //
 //   forward   gates[rows, G*16] = h_{t-1}[rows, 0:H] . R[0:H, slice]            K = H

@@ -1,5 +1,5 @@
 """Contractions whose rows are not multiples of 16 bytes: operands go through a copy, results
-through a padded tile."""
+leave value by value."""
 import pytest
 import torch
 
