@@ -24,10 +24,11 @@ bool aligned(std::initializer_list<const void*> ptrs, int H, int dtype) {
 // step hardly depends on the rows.  us per step forward / backward, chains / tensor cores.  GRU H = 1024: five chains
 // 5.7 / 8.4 and 6.8 / 7.8, six 6.8 / 8.9 and 6.8 / 7.9; H = 512: six 5.7 / 6.0 and 5.5 / 6.9.  LSTM H = 1024: six
 // 7.1 / 8.8 and 8.3 / 8.7, seven 8.3 / 10.7 and 8.3 / 8.9, eight 9.4 / 11.6 and 8.4 / 9.0; H = 768: seven 7.3 / 10.8 and
-// 8.0 / 11.2; H = 512: eight 7.2 / 8.0 and 6.9 / 7.2 on half of the GPU, 6.9 / 8.1 and 7.1 / 7.7 on all of it.
+// 8.0 / 11.2; H = 512: eight 7.2 / 8.0 and 6.9 / 7.2 on half of the GPU, 6.9 / 8.1 and 7.1 / 7.7 on all of it.  Backward the
+// chains keep more than their time says: they sum the bias gradients before these are rounded to bf16 (GRU 90 rows
+// H = 1000, relative to fp64: 2.6e-3, summed from the rounded gradients 2.85e-3).
 constexpr int kGridChains = 12;
-int gru_chains_before_tc(int H, bool bwd) { return bwd && H > 768 ? 4 : 6; }
-int lstm_chains_before_tc(int H, bool bwd) { return bwd && H > 768 ? 6 : 7; }
+constexpr int kGruChainsBeforeTc = 6, kLstmChainsBeforeTcFwd = 7, kLstmChainsBeforeTcBwd = 8;
 
 // fp32 and fp16 storage beyond 512 units: two quads per CTA keep both planes of R in registers, four put the
 // second plane into shared memory and so take half the CTAs per row group.  Half the CTAs read (backward:
@@ -146,7 +147,7 @@ int lstm_forward_chain(const LstmFwd& a, bool few, cudaStream_t s) {
   p.R = a.R; p.b = a.b; p.gin = a.v; p.gout = a.training ? a.v : nullptr; p.mask = a.zoneout_mask;
   p.h = a.h; p.c = a.c;
   p.wide = aligned({a.v, a.h, a.c, a.zoneout_mask}, a.H, a.dtype);
-  const int most = few && lstm_tc_takes(a.dtype, a.N, a.H, true) ? lstm_chains_before_tc(a.H, false) : kGridChains;
+  const int most = few && lstm_tc_takes(a.dtype, a.N, a.H, true) ? kLstmChainsBeforeTcFwd : kGridChains;
   return run_fwd(p, a.dtype, most, run_cl_fwd_lstm, run_gl_fwd_lstm, s);
 }
 
@@ -159,7 +160,7 @@ int gru_forward_chain(const GruFwd& a, bool few, cudaStream_t s) {
   p.R = a.R; p.b = a.bx; p.b2 = a.br; p.gin = a.tmp_Wx; p.gout = a.training ? a.v : nullptr;
   p.mask = a.zoneout_mask; p.h = a.h;
   p.wide = aligned({a.tmp_Wx, a.v, a.h, a.zoneout_mask}, a.H, a.dtype);
-  return run_fwd(p, a.dtype, few && tc_waits(a.dtype, a.N, a.H) ? gru_chains_before_tc(a.H, false) : kGridChains,
+  return run_fwd(p, a.dtype, few && tc_waits(a.dtype, a.N, a.H) ? kGruChainsBeforeTc : kGridChains,
                  run_cl_fwd_gru, run_gl_fwd_gru, s);
 }
 
@@ -172,7 +173,7 @@ int lstm_backward_chain(const LstmBwd& a, const GradPlanes& planes, bool few, cu
   p.mask = a.zoneout_mask; p.dh = a.dh; p.dc = a.dc;
   p.gpl = planes.p; p.gpl_stride = planes.stride;
   p.wide = aligned({a.v, a.c, a.dh_new, a.dc_new, a.zoneout_mask}, a.H, a.dtype);
-  const int most = few && lstm_tc_takes(a.dtype, a.N, a.H, false) ? lstm_chains_before_tc(a.H, true) : kGridChains;
+  const int most = few && lstm_tc_takes(a.dtype, a.N, a.H, false) ? kLstmChainsBeforeTcBwd : kGridChains;
   return run_bwd(p, a.dtype, most, 4, a.db, nullptr, run_cl_bwd_lstm, run_gl_bwd_lstm, s);
 }
 
@@ -185,7 +186,7 @@ int gru_backward_chain(const GruBwd& a, const GradPlanes& planes, bool few, cuda
   p.mask = a.zoneout_mask; p.dh = a.dh;
   p.gpl = planes.p; p.gpl2 = planes.p2; p.gpl_stride = planes.stride;
   p.wide = aligned({a.v, a.dp, a.dq, a.h, a.dh_new, a.zoneout_mask}, a.H, a.dtype);
-  return run_bwd(p, a.dtype, few && tc_waits(a.dtype, a.N, a.H) ? gru_chains_before_tc(a.H, true) : kGridChains,
+  return run_bwd(p, a.dtype, few && tc_waits(a.dtype, a.N, a.H) ? kGruChainsBeforeTc : kGridChains,
                  3, a.dbx, a.dbr, run_cl_bwd_gru, run_gl_bwd_gru, s);
 }
 

@@ -1,7 +1,7 @@
 // Tensor-core GRU and LSTM recurrences for large batches (bf16 storage), sm_100a.
 //
 // The chain kernels (rec_grid_kernels.cuh) take eight batch rows at a time and pay for every chain
-// of a CTA.  Where they would need more than four to seven (rec_chain_host.cu) - a hundred rows of a wide
+// of a CTA.  Where they would need more than six to eight (rec_chain_host.cu) - a hundred rows of a wide
 // layer, or half of that on half of the GPU - the step product is a real tile for the 5th-generation tensor
 // cores, and this file runs it there:
 //
