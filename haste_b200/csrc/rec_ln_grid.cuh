@@ -21,8 +21,9 @@
 // scaled by a power of two per tile (values reach 2^15 at most), all four products.  That is 22 .. 23
 // bits per operand, where the exchanged words carry 23; three bf16 planes took six products.  (With the
 // gate functions of rec_ln_common.cuh outputs and gradients are as far from fp64 as before or nearer.)
-// A chain whose state reaches 2 (an initial state may) is scaled by what it needs instead.  Backward, the rows of d(h.R) are scaled by a bound on their
-// largest value that falls out of the statistics' meeting.  bf16 storage: one bf16 plane.
+// A chain with a state of 2 or more (an initial state may be) is multiplied in passes (product_by_size).
+// Backward, the rows of d(h.R) are scaled by a bound on their largest value that falls out of the statistics'
+// meeting.  bf16 storage: one bf16 plane.
 #pragma once
 
 #include "rec_grid_launch.cuh"
@@ -131,6 +132,73 @@ __device__ __forceinline__ float scaled_fragments(float (&x)[NS][2][4], uint32_t
       rest[s * 32] = make_uint4(l[0], l[1], l[2], l[3]);
     }
     return pow2(-sh);
+  }
+}
+// The product of a chain with a state of 2 or more (x: this lane's values of row lane >> 2, in shared memory,
+// because the registers are full).  An element is scaled by its own row and size, so that it keeps its 22 bits
+// whatever lies beside it: a first pass takes what is smaller than 2, as the usual product does and with the same
+// result, each further one what is within 2^-16 of the largest value that is left of a row.  Infinities and NaN
+// go with the first pass.
+template <int KSW, int NMT, int KEEP>
+__device__ __forceinline__ void product_by_size(float4* x, const uint32_t (&wf)[NMT][KEEP][4], const uint4* rest,
+                                                const float (&wscale)[NMT], float (&acc)[NMT][4]) {
+  const int q = threadIdx.x & 3;
+  const uint32_t at = smem_u32(x);
+  float least = 0.f, limit = 2.f;  // of what this pass takes
+  int sh = 14;
+  auto takes = [&](float v) {
+    v = fabsf(v);
+    return (v >= least && v < limit) || !(v <= 3.402823466e38f);
+  };
+#pragma unroll 1
+  for (int pass = 0; pass < 32; ++pass) {  // (a float's 277 powers of two are 18 passes)
+    const float f = pow2(sh);
+    auto planes = [&](int s, uint32_t (&hi)[2], uint32_t (&lo)[2]) {
+      float4 v;  // (volatile: made anew for each tile)
+      asm volatile("ld.volatile.shared.v4.f32 {%0,%1,%2,%3}, [%4];"
+                   : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at + s * 512) : "memory");
+      f16_pair(takes(v.x) ? v.x * f : 0.f, takes(v.y) ? v.y * f : 0.f, hi[0], lo[0]);
+      f16_pair(takes(v.z) ? v.z * f : 0.f, takes(v.w) ? v.w * f : 0.f, hi[1], lo[1]);
+    };
+    const float back = pow2(-sh);
+    const float u0 = __shfl_sync(0xffffffffu, back, 8 * q), u1 = __shfl_sync(0xffffffffu, back, 8 * q + 4);
+#pragma unroll
+    for (int mt = 0; mt < NMT; ++mt) {
+      float d[4] = {0.f, 0.f, 0.f, 0.f};  // in the order of the usual product
+#pragma unroll
+      for (int s = 0; s < KSW; ++s) {
+        uint32_t bh[2], bl[2];
+        planes(s, bh, bl);
+        const uint4 a = rest[(mt * KSW + s) * 32];
+        mma_f16(d, wf[mt][s % KEEP], bl[0], bl[1]);
+        mma_f16(d, a, bl[0], bl[1]);
+        mma_f16(d, a, bh[0], bh[1]);
+      }
+#pragma unroll
+      for (int s = 0; s < KSW; ++s) {
+        uint32_t bh[2], bl[2];
+        planes(s, bh, bl);
+        mma_f16(d, wf[mt][s % KEEP], bh[0], bh[1]);
+      }
+      const float f0 = wscale[mt] * u0, f1 = wscale[mt] * u1;
+      acc[mt][0] += d[0] * f0; acc[mt][1] += d[1] * f1;
+      acc[mt][2] += d[2] * f0; acc[mt][3] += d[3] * f1;
+    }
+    float most = 0.f;  // of what is left
+#pragma unroll
+    for (int s = 0; s < KSW; ++s) {
+      float4 v = x[s * 32];
+      v.x = takes(v.x) ? 0.f : v.x; v.y = takes(v.y) ? 0.f : v.y;
+      v.z = takes(v.z) ? 0.f : v.z; v.w = takes(v.w) ? 0.f : v.w;
+      x[s * 32] = v;
+      most = fmaxf(most, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+    }
+    if (!__any_sync(0xffffffffu, most > 0.f)) return;
+    most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, 1));
+    most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, 2));
+    sh = f16_shift_of(most);
+    least = most * (1.0f / 65536.0f);
+    limit = __uint_as_float(0x7f800000u);
   }
 }
 // How many fragments of a tile lie in shared memory.
@@ -464,22 +532,24 @@ __global__ void __launch_bounds__(GL_THREADS, 1) lg_fwd_kernel(const __grid_cons
         float acc[NMT][4];
 #pragma unroll
         for (int mt = 0; mt < NMT; ++mt) acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.f;
-        float unscale = 1.f;
-        if constexpr (SPLIT == 2) {
-          // (the tag lies in bit 0, so bit 30 of `bad` says that some state is 2 or more)
-          int sh = 14;
-          if (__any_sync(0xffffffffu, (bad & 0x40000000u) != 0)) {
-            float most = 0.f;
+        constexpr float kUsual = 1.0f / 16384.0f;  // takes the usual scale of h out again
+        // (the tag lies in bit 0, so bit 30 of `bad` says that some state is 2 or more)
+        const bool apart = SPLIT == 2 && __any_sync(0xffffffffu, (bad & 0x40000000u) != 0);
+        if (__builtin_expect(apart, 0)) {
+          if constexpr (SPLIT == 2) {
+            // (the place of this warp's results: free as below)
+            if (throttle &&
+                !mb_wait_warp(pbar + 8 * (p.ring + slot), phase ^ 1u, p.sync, s_abort, 64)) { alive = false; break; }
+            static_assert(KSW <= NMT, "a lane's values take the place of its results");
+            float4* x = part + slot * PART + w * NMT * 32 + lane;
 #pragma unroll
             for (int s = 0; s < KSW; ++s)
-              most = finite_max(finite_max(finite_max(finite_max(most, fword_value(y[s].x)), fword_value(y[s].y)),
-                                           fword_value(y[s].z)), fword_value(y[s].w));
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
-            sh = f16_shift_of(most);
+              x[s * 32] = make_float4(fword_value(y[s].x), fword_value(y[s].y), fword_value(y[s].z), fword_value(y[s].w));
+            product_by_size<KSW, NMT, KEEP>(x, wf, rest, wscale, acc);
+            fetch(t2 & 1, tag_of(t2), ch2, y, 0, KSW);
           }
-          const float f = pow2(sh);
-          unscale = pow2(-sh);
+        } else if constexpr (SPLIT == 2) {
+          constexpr float f = 1.0f / kUsual;
           uint32_t bh[KSW][2], bl[KSW][2];
 #pragma unroll
           for (int s = 0; s < KSW; ++s) {
@@ -503,6 +573,10 @@ __global__ void __launch_bounds__(GL_THREADS, 1) lg_fwd_kernel(const __grid_cons
           for (int s = 0; s < KSW; ++s)
 #pragma unroll
             for (int mt = 0; mt < NMT; ++mt) mma_f16(acc[mt], wf[mt][s % KEEP], bh[s][0], bh[s][1]);
+#pragma unroll
+          for (int mt = 0; mt < NMT; ++mt)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[mt][i] *= wscale[mt] * kUsual;
         } else {
 #pragma unroll
           for (int s = 0; s < KSW; ++s) {
@@ -526,10 +600,7 @@ __global__ void __launch_bounds__(GL_THREADS, 1) lg_fwd_kernel(const __grid_cons
             !mb_wait_warp(pbar + 8 * (p.ring + slot), phase ^ 1u, p.sync, s_abort, 64)) { alive = false; break; }
         float4* pw = part + slot * PART + w * NMT * 32 + lane;
 #pragma unroll
-        for (int mt = 0; mt < NMT; ++mt) {
-          const float f = SPLIT == 2 ? wscale[mt] * unscale : 1.f;
-          pw[mt * 32] = make_float4(acc[mt][0] * f, acc[mt][1] * f, acc[mt][2] * f, acc[mt][3] * f);
-        }
+        for (int mt = 0; mt < NMT; ++mt) pw[mt * 32] = make_float4(acc[mt][0], acc[mt][1], acc[mt][2], acc[mt][3]);
         __syncwarp();
         if (lane == 0) mb_arrive(pbar + 8 * slot);
         next_slot();

@@ -55,3 +55,20 @@ def test_scales(cell, state, grad):
 @pytest.mark.parametrize("N,H", [(9, 330), (20, 512), (13, 777), (70, 1000), (30, 1024)])
 def test_tiles_bf16(N, H):
     check("layer_norm_gru", oracle.make_inputs("layer_norm_gru", 5, N, 16, H, seed=H, zoneout=0.2), TOL_BF16, torch.bfloat16)
+
+
+# One row of a large state among ordinary ones: the others come out bit for bit as without it, and within the bar.
+# (The forward pass alone: the large row's gradients are not finite beyond 1e19, and parameter gradients sum over rows.)
+@pytest.mark.parametrize("large", [1e6, 1e9, 1e30, float("inf"), float("nan")])
+@pytest.mark.parametrize("whole_row", [True, False])
+@pytest.mark.parametrize("cell,N,H", [("layer_norm_lstm", 9, 400), ("layer_norm_gru", 21, 512), ("layer_norm_gru", 150, 300)])
+def test_a_large_row_stays_to_itself(cell, N, H, whole_row, large):
+    d = oracle.make_inputs(cell, 6, N, 12, H, seed=9, zoneout=0.2)
+    d["h0"] = d["h0"].clamp(-1.5, 1.5)
+    plain = run_cuda(cell, d, zoneout=0.2, backward=False)[0]["h"]
+    d["h0"][5, slice(None) if whole_row else 37] = large
+    got = run_cuda(cell, d, zoneout=0.2, backward=False)[0]["h"]
+    others = [n for n in range(N) if n != 5]
+    assert torch.equal(got[:, others], plain[:, others])
+    ref = oracle.forward_backward(cell, d, zoneout=0.2)[0]["h"]
+    assert_close(got[:, others], ref[:, others], TOL_F32, "h")
