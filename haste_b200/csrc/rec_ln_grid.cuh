@@ -526,6 +526,23 @@ __global__ void __launch_bounds__(GL_THREADS, 1) lg_fwd_kernel(const __grid_cons
           fetch(t & 1, wt, ch, y, 0, KSW);
         }
         if (!alive) break;
+        // The first step multiplies the initial state as the caller has it: its words, which say that the others
+        // are there too, lack the last bit.
+        uint32_t bits = ~1u;  // of a word that are the value
+        if constexpr (SPLIT == 2) {
+          if (t == 0) {
+            bits = ~0u;
+            const T* h0 = static_cast<const T*>(p.h) + (long long)((tile0 + ch) * 8 + gq) * H;
+#pragma unroll
+            for (int s = 0; s < KSW; ++s) {
+              const int k = (kq + s * 4) * 4;
+              const bool rok = ch * 8 < nrow;
+              y[s] = make_uint4(rok && k < H ? __float_as_uint(ld(h0 + k)) : 0u, rok && k + 1 < H ? __float_as_uint(ld(h0 + k + 1)) : 0u,
+                                rok && k + 2 < H ? __float_as_uint(ld(h0 + k + 2)) : 0u, rok && k + 3 < H ? __float_as_uint(ld(h0 + k + 3)) : 0u);
+            }
+          }
+        }
+        auto value = [&](uint32_t word) { return __uint_as_float(word & bits); };
         // the next chain's words are on their way while this one's are multiplied (beyond the last step: words
         // that nobody waits for)
         const int ch2 = ch + 1 < ch_n ? ch + 1 : 0, t2 = ch + 1 < ch_n ? t : t + 1;
@@ -544,7 +561,7 @@ __global__ void __launch_bounds__(GL_THREADS, 1) lg_fwd_kernel(const __grid_cons
             float4* x = part + slot * PART + w * NMT * 32 + lane;
 #pragma unroll
             for (int s = 0; s < KSW; ++s)
-              x[s * 32] = make_float4(fword_value(y[s].x), fword_value(y[s].y), fword_value(y[s].z), fword_value(y[s].w));
+              x[s * 32] = make_float4(value(y[s].x), value(y[s].y), value(y[s].z), value(y[s].w));
             product_by_size<KSW, NMT, KEEP>(x, wf, rest, wscale, acc);
             fetch(t2 & 1, tag_of(t2), ch2, y, 0, KSW);
           }
@@ -553,8 +570,8 @@ __global__ void __launch_bounds__(GL_THREADS, 1) lg_fwd_kernel(const __grid_cons
           uint32_t bh[KSW][2], bl[KSW][2];
 #pragma unroll
           for (int s = 0; s < KSW; ++s) {
-            f16_pair(fword_value(y[s].x) * f, fword_value(y[s].y) * f, bh[s][0], bl[s][0]);
-            f16_pair(fword_value(y[s].z) * f, fword_value(y[s].w) * f, bh[s][1], bl[s][1]);
+            f16_pair(value(y[s].x) * f, value(y[s].y) * f, bh[s][0], bl[s][0]);
+            f16_pair(value(y[s].z) * f, value(y[s].w) * f, bh[s][1], bl[s][1]);
           }
           // the small products first
 #pragma unroll

@@ -72,3 +72,20 @@ def test_a_large_row_stays_to_itself(cell, N, H, whole_row, large):
     assert torch.equal(got[:, others], plain[:, others])
     ref = oracle.forward_backward(cell, d, zoneout=0.2)[0]["h"]
     assert_close(got[:, others], ref[:, others], TOL_F32, "h")
+
+
+def test_the_first_step_takes_the_whole_initial_state():
+    """Initial states 1 and 1 + 2^-23, R of one 1 per column: h.R is h0 itself, and a gain of 1000 over the root of
+    LayerNorm's epsilon makes 0.038 of the last bit.  The row's mean may be off by 2^-22 (its words have 23 bits): 0.075 in all
+    gates alike, which moves the slopes of sigmoid and tanh by less than a tenth."""
+    cell, N, H = "layer_norm_gru", 3, 336
+    d = oracle.make_inputs(cell, 1, N, 12, H, seed=1)
+    for k in ("W", "bx", "br"):
+        d[k] = torch.zeros_like(d[k])
+    d["h0"] = (1 + 2.0 ** -23 * (torch.arange(H) % 2)).double().expand(N, H).contiguous()
+    d["R"] = torch.eye(H, dtype=torch.float64).repeat(1, 3)
+    d["gamma"] = torch.full_like(d["gamma"], 1000.0)
+    step = lambda h: (h[1, :, 1::2].double().mean() - h[1, :, 0::2].double().mean()).item()
+    want = step(oracle.forward_backward(cell, d)[0]["h"])
+    got = step(run_cuda(cell, d, backward=False)[0]["h"].cpu())
+    assert abs(got - want) < 0.1 * abs(want)
