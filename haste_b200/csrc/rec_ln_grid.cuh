@@ -144,6 +144,10 @@ __device__ __forceinline__ void product_by_size(float4* x, const uint32_t (&wf)[
                                                 const float (&wscale)[NMT], float (&acc)[NMT][4]) {
   const int q = threadIdx.x & 3;
   const uint32_t at = smem_u32(x);
+  bool some = false;
+#pragma unroll
+  for (int s = 0; s < KSW; ++s) some |= x[s * 32].x != 0.f || x[s * 32].y != 0.f || x[s * 32].z != 0.f || x[s * 32].w != 0.f;
+  if (!__any_sync(0xffffffffu, some)) return;  // (the usual initial state)
   float least = 0.f, limit = 2.f;  // of what this pass takes
   int sh = 14;
   auto takes = [&](float v) {
@@ -204,6 +208,19 @@ __device__ __forceinline__ void product_by_size(float4* x, const uint32_t (&wf)[
 // How many fragments of a tile lie in shared memory.
 template <int SPLIT, int NS>
 constexpr int frag_rest() { return SPLIT == 2 ? NS : NS - LgRegs<NS>::KEEP; }
+
+// Whether a phase has ended, without waiting.
+__device__ __forceinline__ bool mb_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 
 // Barrier of a group's four warps; true if any of them has given up.
 __device__ __forceinline__ bool group_barrier_or(int grp, bool flag) {
@@ -433,8 +450,8 @@ __global__ void __launch_bounds__(GL_THREADS, 1) lg_fwd_kernel(const __grid_cons
   float2* meet = reinterpret_cast<float2*>(consts + (3 * G + 2) * 16);         // [2 groups][2][quad][8]
   float2* found = meet + 2 * 2 * NMT * 8;                                      // [2 groups][2][8] mean, 1/sigma
   uint64_t* barp = reinterpret_cast<uint64_t*>(found + 2 * 2 * 8);             // full[ring], empty[ring]
-  const uint32_t pbar = smem_u32(barp);
-  uint8_t* io_base = reinterpret_cast<uint8_t*>(barp + 2 * p.ring);
+  const uint32_t pbar = smem_u32(barp), obar = pbar + 16 * p.ring;             // and, per chain: h has left
+  uint8_t* io_base = reinterpret_cast<uint8_t*>(barp + 2 * p.ring + ((p.CH + 1) & ~1));
   __shared__ int s_abort_;
   volatile int* s_abort = &s_abort_;
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
@@ -448,6 +465,7 @@ __global__ void __launch_bounds__(GL_THREADS, 1) lg_fwd_kernel(const __grid_cons
       mb_init(pbar + 8 * i, GL_WARPS);
       mb_init(pbar + 8 * (p.ring + i), NMT);
     }
+    for (int i = 0; i < p.CH; ++i) mb_init(obar + 8 * i, NMT);
   }
   for (int i = tid; i < (3 * G + 2) * 16; i += GL_THREADS) {
     const int a = i / 16, unit = u0 + (i & 15);
@@ -511,9 +529,20 @@ __global__ void __launch_bounds__(GL_THREADS, 1) lg_fwd_kernel(const __grid_cons
       return SPLIT == 2 ? rt : rt << 30;
     };
     fetch(0, tag_of(0), 0, y, 0, KSW);
+    // Product warps that poll all the time fill the way to L2 for the statistics and for the words themselves.  So
+    // after a first look they wait until this CTA's own h of the chain has left; the others' leaves at about
+    // that time.  bf16 storage, whose next look falls behind the whole product, does not even take that first look before
+    // (us per step, polling / this: LayerNormGRU bf16 8 rows H = 512 4.2 / 3.7, 32 rows H = 1024 7.1 / 5.8, 128 rows 18.2 /
+    // 16.1; LayerNormLSTM fp32 64 rows H = 512 7.7 / 7.1; LayerNormGRU fp32 128 rows 8.0 / 7.9, without the first look 8.8).
+    constexpr bool kAskAhead = SPLIT == 2;
+    bool asked = true;
     for (int t = 0; t < p.T && alive; ++t) {
       const uint32_t wt = tag_of(t);
       for (int ch = 0; ch < ch_n; ++ch) {
+        if (!asked) {
+          if (!mb_wait_warp(obar + 8 * ch, (t - 1) & 1, p.sync, s_abort, 74)) { alive = false; break; }
+          fetch(t & 1, wt, ch, y, 0, KSW);
+        }
         long long t0 = 0;
         unsigned int spins = 0;
         uint32_t bad;
@@ -522,36 +551,27 @@ __global__ void __launch_bounds__(GL_THREADS, 1) lg_fwd_kernel(const __grid_cons
 #pragma unroll
           for (int s = 0; s < KSW; ++s) bad |= stale4(y[s], wt);
           if (__all_sync(0xffffffffu, (bad & TAGBIT) == 0)) break;
+          if (kAskAhead && spins == 0 && t > 0 && !mb_wait_warp(obar + 8 * ch, (t - 1) & 1, p.sync, s_abort, 74)) {
+            alive = false;
+            break;
+          }
           if (__any_sync(0xffffffffu, !may_spin(spins, t0, p.sync, s_abort, 63))) { alive = false; break; }
           fetch(t & 1, wt, ch, y, 0, KSW);
         }
         if (!alive) break;
-        // The first step multiplies the initial state as the caller has it: its words, which say that the others
-        // are there too, lack the last bit.
-        uint32_t bits = ~1u;  // of a word that are the value
-        if constexpr (SPLIT == 2) {
-          if (t == 0) {
-            bits = ~0u;
-            const T* h0 = static_cast<const T*>(p.h) + (long long)((tile0 + ch) * 8 + gq) * H;
-#pragma unroll
-            for (int s = 0; s < KSW; ++s) {
-              const int k = (kq + s * 4) * 4;
-              const bool rok = ch * 8 < nrow;
-              y[s] = make_uint4(rok && k < H ? __float_as_uint(ld(h0 + k)) : 0u, rok && k + 1 < H ? __float_as_uint(ld(h0 + k + 1)) : 0u,
-                                rok && k + 2 < H ? __float_as_uint(ld(h0 + k + 2)) : 0u, rok && k + 3 < H ? __float_as_uint(ld(h0 + k + 3)) : 0u);
-            }
-          }
-        }
-        auto value = [&](uint32_t word) { return __uint_as_float(word & bits); };
         // the next chain's words are on their way while this one's are multiplied (beyond the last step: words
         // that nobody waits for)
         const int ch2 = ch + 1 < ch_n ? ch + 1 : 0, t2 = ch + 1 < ch_n ? t : t + 1;
+        auto fetch_next = [&]() {
+          asked = kAskAhead || t2 == 0 || __all_sync(0xffffffffu, mb_test(obar + 8 * ch2, (t2 - 1) & 1));
+          if (asked) fetch(t2 & 1, tag_of(t2), ch2, y, 0, KSW);
+        };
         float acc[NMT][4];
 #pragma unroll
         for (int mt = 0; mt < NMT; ++mt) acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.f;
         constexpr float kUsual = 1.0f / 16384.0f;  // takes the usual scale of h out again
         // (the tag lies in bit 0, so bit 30 of `bad` says that some state is 2 or more)
-        const bool apart = SPLIT == 2 && __any_sync(0xffffffffu, (bad & 0x40000000u) != 0);
+        const bool apart = SPLIT == 2 && __any_sync(0xffffffffu, (bad & 0x40000000u) != 0 || t == 0);
         if (__builtin_expect(apart, 0)) {
           if constexpr (SPLIT == 2) {
             // (the place of this warp's results: free as below)
@@ -561,17 +581,27 @@ __global__ void __launch_bounds__(GL_THREADS, 1) lg_fwd_kernel(const __grid_cons
             float4* x = part + slot * PART + w * NMT * 32 + lane;
 #pragma unroll
             for (int s = 0; s < KSW; ++s)
-              x[s * 32] = make_float4(value(y[s].x), value(y[s].y), value(y[s].z), value(y[s].w));
+              x[s * 32] = make_float4(fword_value(y[s].x), fword_value(y[s].y), fword_value(y[s].z), fword_value(y[s].w));
+            // The first step multiplies the initial state as the caller has it: its words, which say that the
+            // others are there too, lack the last bit.
+            if (t == 0 && ch * 8 < nrow) {
+              const T* h0 = static_cast<const T*>(p.h) + (long long)((tile0 + ch) * 8 + gq) * H;
+#pragma unroll
+              for (int i = 0; i < KSW * 4; ++i) {
+                const int k = (kq + (i >> 2) * 4) * 4 + (i & 3);
+                if (k < H) reinterpret_cast<float*>(x + (i >> 2) * 32)[i & 3] = ld(h0 + k);
+              }
+            }
             product_by_size<KSW, NMT, KEEP>(x, wf, rest, wscale, acc);
-            fetch(t2 & 1, tag_of(t2), ch2, y, 0, KSW);
+            fetch_next();
           }
         } else if constexpr (SPLIT == 2) {
           constexpr float f = 1.0f / kUsual;
           uint32_t bh[KSW][2], bl[KSW][2];
 #pragma unroll
           for (int s = 0; s < KSW; ++s) {
-            f16_pair(value(y[s].x) * f, value(y[s].y) * f, bh[s][0], bl[s][0]);
-            f16_pair(value(y[s].z) * f, value(y[s].w) * f, bh[s][1], bl[s][1]);
+            f16_pair(fword_value(y[s].x) * f, fword_value(y[s].y) * f, bh[s][0], bl[s][0]);
+            f16_pair(fword_value(y[s].z) * f, fword_value(y[s].w) * f, bh[s][1], bl[s][1]);
           }
           // the small products first
 #pragma unroll
@@ -585,7 +615,7 @@ __global__ void __launch_bounds__(GL_THREADS, 1) lg_fwd_kernel(const __grid_cons
               mma_f16(acc[mt], a, bh[s][0], bh[s][1]);
             }
           }
-          fetch(t2 & 1, tag_of(t2), ch2, y, 0, KSW);
+          fetch_next();
 #pragma unroll
           for (int s = 0; s < KSW; ++s)
 #pragma unroll
@@ -609,7 +639,7 @@ __global__ void __launch_bounds__(GL_THREADS, 1) lg_fwd_kernel(const __grid_cons
               }
             }
           }
-          fetch(t2 & 1, tag_of(t2), ch2, y, 0, KSW);
+          fetch_next();
         }
         // (a slot per chain needs no look at `empty`: h of the next step took the statistics of this one,
         // which left after the group's barrier, and the partials are read before it)
@@ -870,6 +900,8 @@ __global__ void __launch_bounds__(GL_THREADS, 1) lg_fwd_kernel(const __grid_cons
           h_new = uok ? round_to_storage<T>(h_new) : 0.f;
           if (t + 1 < p.T && n0 + row < N)
             gl_publish(xdst + ((size_t)((t + 1) & 1) * tiles + tile) * xtile, hword_encode<SPLIT>(h_new, stat_tag(t + 1)));
+          __syncwarp();
+          if (lane == 0) mb_arrive(obar + 8 * ch);
           look_ahead(k, i);
           // ---- off the chain
           sh[0] = h_new;
@@ -1407,7 +1439,7 @@ int lg_fwd_go(LnGridFwd& p, int nRG, cudaStream_t s) {
   static std::atomic<int> set[kChainMaxDevices];
   const size_t slot = (size_t)GL_WARPS * 4 * 512 + 16;
   const size_t rest = (size_t)GL_WARPS * 4 * frag_rest<SPLIT, KSW>() * 512 + (size_t)p.CH * LG_FWD_STASH * 512 +
-                      (3 * G + 2) * 64 + 2 * 2 * (4 + 1) * 8 * 8 + (size_t)GL_WARPS * LnIo<T, 2>::WARP;
+                      (3 * G + 2) * 64 + 2 * 2 * (4 + 1) * 8 * 8 + (size_t)((p.CH + 1) & ~1) * 8 + (size_t)GL_WARPS * LnIo<T, 2>::WARP;
   p.ring = min(p.CH, (int)(((size_t)kGlMaxSmem - rest) / slot));
   p.throttle = p.ring < p.CH;  // (a group's four warps have read their partials before its statistics leave)
   return gl_launch(lg_fwd_kernel<G, KSW, SPLIT, T>, p, p.CTAS * nRG, p.ring * slot + rest, set, s);
