@@ -45,7 +45,10 @@ struct LnGridBwd : LnBwdParams {
 // plane); the second plane and fragments beyond the fourth (bf16 storage, beyond 512 units) lie in shared
 // memory.  P: registers per thread of the product warps; the finishing warps get the rest of 256.  (With all
 // of R in registers they had 80, and spilled: LayerNormLSTM fp32, 64 rows, H = 512, two directions at a
-// time, us per step forward / backward 11.3 / 13.1 -> 10.6 / 10.5.)
+// time, us per step forward / backward 11.3 / 13.1 -> 10.6 / 10.5.)  Backward beyond 512 units every warp keeps the 128 of
+// the launch: with 104 the finishing warps bounded the step (us for a backward call of 60 steps with 104 / 128, LayerNormGRU
+// bf16 H = 1024: 8 rows 785 / 721, 128 rows 2213 / 1770; H = 1001 128 rows 2504 / 2079; LayerNormLSTM H = 1024 128 rows
+// 2896 / 2275).
 template <int N>
 struct LgRegs {
   static constexpr int KEEP = N < 4 ? N : 4, P = N <= 2 ? 112 : (N == 3 ? 120 : (N == 4 ? 136 : 152)), F = 256 - P;
@@ -971,7 +974,7 @@ __global__ void __launch_bounds__(GL_THREADS, 1) lg_bwd_kernel(const __grid_cons
 
   if (w < GL_WARPS) {
     // ------------------------------------------------------------------ product warps (as gl_bwd_kernel)
-    reg_product<TPW>();
+    if (TPW <= 4) reg_product<TPW>();
     const int rot = hs % p.K16;
     constexpr int KEEP = LgRegs<TPW>::KEEP, REST = frag_rest<SPLIT, TPW>();  // tiles
     uint32_t wf[KEEP][KSB][4];
@@ -1079,7 +1082,7 @@ __global__ void __launch_bounds__(GL_THREADS, 1) lg_bwd_kernel(const __grid_cons
   } else {
     // ------------------------------------------------------------------ finishing warps: quad f & 3 of the
     // chains grp, grp + 2, ...; lanes as in the cluster kernels
-    reg_finish<TPW>();
+    if (TPW <= 4) reg_finish<TPW>();
     const int f = w - GL_WARPS, grp = f >> 2, quad = f & 3, gt = quad * 32 + lane;
     const int sub = lane >> 3, c8 = lane & 7;
     const int row = 2 * (c8 & 3) + (sub & 1), ul = (c8 >> 2) + 2 * (sub >> 1);
