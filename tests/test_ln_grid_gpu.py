@@ -5,7 +5,7 @@ import torch
 
 import haste_oracle as oracle
 from haste_b200 import _C
-from helpers import TOL_BF16, TOL_F32, assert_close, run_cuda
+from helpers import TOL_BF16, TOL_BF16_ALL_STORAGE_LN_LSTM, TOL_F32, assert_close, run_cuda
 
 pytestmark = pytest.mark.gpu
 
@@ -89,3 +89,27 @@ def test_the_first_step_takes_the_whole_initial_state():
     want = step(oracle.forward_backward(cell, d)[0]["h"])
     got = step(run_cuda(cell, d, backward=False)[0]["h"].cpu())
     assert abs(got - want) < 0.1 * abs(want)
+
+
+# all-bf16 LayerNormLSTM: fragments of R in shared memory beyond 512 units, two statistic sources per lane, rows that
+# start anywhere.  Against the oracle at that mode's bar, and against the step-wise path, which rounds tensors of
+# the same kind and so lies within the same distance; a slip of layout is of order 1.
+@pytest.mark.parametrize("N,H", [(9, 330), (13, 777), (70, 1000), (30, 1024)])
+def test_tiles_bf16_lstm(N, H):
+    d = oracle.make_inputs("layer_norm_lstm", 3, N, 16, H, seed=H, zoneout=0.2)
+    d = {k: (v.to(torch.bfloat16).double() if v is not None else None) for k, v in d.items()}
+    ref_out, ref_g = oracle.forward_backward("layer_norm_lstm", d, zoneout=0.2)
+    run = lambda: run_cuda("layer_norm_lstm", d, zoneout=0.2, dtype=torch.bfloat16,
+                           fwd_kwargs={"saved_dtype": torch.bfloat16})
+    out, g = run()
+    _C.set_recurrence_path(_C.PATH_STEPWISE)
+    try:
+        step_out, step_g = run()
+    finally:
+        _C.set_recurrence_path(_C.PATH_AUTO)
+    bar = TOL_BF16_ALL_STORAGE_LN_LSTM
+    assert_close(out["h"], ref_out["h"], bar, "h")
+    assert_close(out["h"], step_out["h"], bar, "h, step by step")
+    for k, r in ref_g.items():
+        assert_close(g[k].double(), r, bar, "d" + k)
+        assert_close(g[k].double(), step_g[k].double(), bar, "d%s, step by step" % k)
