@@ -57,6 +57,7 @@ struct Params {
   const int* a_exp;            // fp16 planes: the result's row m, column n is to be scaled by
   const signed char* b_exp;    // 2^(a_exp[m] + b_exp[n]); null otherwise
   int chunk;                   // k-blocks per hand-over of the accumulator (Cfg::CHUNK != 0)
+  const int* uneven;           // fp16 planes: points to whether bf16 planes have taken their place
   float* partial;              // non-null: write fp32 partial tiles [split][M][partial_ld]
   int partial_ld;              // N rounded up to whole 32-column chunks
   int* err;
@@ -194,10 +195,9 @@ __device__ __forceinline__ void store_chunk(const Params& p, int sp, int m0, int
   else store_tile_c<SCALED, __half>(p, tile, m0, n0, ea, eb);
 }
 
-template <int NPROD>
-__global__ void __launch_bounds__(THREADS, 1)
-gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
-                    const __grid_constant__ CUtensorMap map_b, const Params p) {
+// UNEVEN: bf16 planes in the place of fp16 planes, handed over as often per product.
+template <int NPROD, bool UNEVEN = false>
+__device__ __forceinline__ void gemm_tile(const CUtensorMap& map_a, const CUtensorMap& map_b, const Params& p) {
   using C = Cfg<NPROD>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -213,6 +213,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int chunk = NPROD == 6 ? C::CHUNK / (UNEVEN ? 2 : 1) : p.chunk;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
@@ -282,7 +283,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (lane == 0) {
-      const uint32_t type = p.a_exp ? 0u : 1u;  // fp16 or bf16 operands
+      const uint32_t type = NPROD == 3 && p.a_exp ? 0u : 1u;  // fp16 or bf16 operands
       const uint32_t idesc = (1u << 4) | (type << 7) | (type << 10) |
                              ((uint32_t)p.a_mn_major << 15) | ((uint32_t)p.b_mn_major << 16) |
                              ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
@@ -307,7 +308,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
           acc_phase ^= 1u << acc;
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + acc * BN;
-          const int kend = C::CHUNK ? min(kb1, kb + p.chunk) : kb1;
+          const int kend = C::CHUNK ? min(kb1, kb + chunk) : kb1;
           uint32_t first = 1;
           for (; kb < kend; ++kb) {
             if (!mbar_wait(full_bar(stage), phase, abort_flag, p.err, 3)) { ok = false; break; }
@@ -350,7 +351,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
       const int sp = item / (p.tiles_n * p.tiles_m);
       const int kb0 = sp * p.kb_per_split;
       const int kb1 = min(p.kb_total, kb0 + p.kb_per_split);
-      const int nchunks = C::CHUNK ? (kb1 - kb0 + p.chunk - 1) / p.chunk : 1;
+      const int nchunks = C::CHUNK ? (kb1 - kb0 + chunk - 1) / chunk : 1;
       const int m0 = tm * BM + quad * 32;
       const int n0 = tn * BN;
       const bool scaled = NPROD == 3 && p.a_exp;
@@ -415,6 +416,21 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a,
   }
 }
 
+template <int NPROD>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                    const __grid_constant__ Params p) {
+  gemm_tile<NPROD>(map_a, map_b, p);
+}
+// fp16 planes, or the bf16 planes that have taken their place.
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_tcgen05_f16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                        const __grid_constant__ CUtensorMap bf_a, const __grid_constant__ CUtensorMap bf_b,
+                        const __grid_constant__ Params p) {
+  if (*p.uneven) gemm_tile<6, true>(bf_a, bf_b, p);
+  else gemm_tile<3>(map_a, map_b, p);
+}
+
 // ---- the same contraction on CTA pairs ------------------------------------------------------
 // The single-CTA kernel above runs at (shared-memory ring bytes) / (load latency): a 128 x 128
 // tile needs 32 KB of operands per 64-wide k-block and product, about twice what the ring can
@@ -437,10 +453,8 @@ constexpr int PAIR_EPI_WARPS = 8;
 // (Ten warps put three on two of the SM's four sub-partitions, 16384 registers each, so 168
 // registers per thread is the most a 320-thread CTA can have; the epilogue therefore drains the
 // accumulator 16 columns at a time.)
-template <int NPROD>
-__global__ void __launch_bounds__(PAIR_THREADS, 1)
-gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
-                         const __grid_constant__ CUtensorMap map_b, const Params p) {
+template <int NPROD, bool UNEVEN = false>
+__device__ __forceinline__ void gemm_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, const Params& p) {
   using C = Cfg<NPROD>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -458,6 +472,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 issues the MMAs
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
+  const int chunk = NPROD == 6 ? C::CHUNK / (UNEVEN ? 2 : 1) : p.chunk;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
@@ -529,7 +544,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (CTA 0 only)
     if (lane == 0 && rank == 0) {
-      const uint32_t type = p.a_exp ? 0u : 1u;  // fp16 or bf16 operands
+      const uint32_t type = NPROD == 3 && p.a_exp ? 0u : 1u;  // fp16 or bf16 operands
       const uint32_t idesc = (1u << 4) | (type << 7) | (type << 10) |
                              ((uint32_t)p.a_mn_major << 15) | ((uint32_t)p.b_mn_major << 16) |
                              ((uint32_t)(PBN >> 3) << 17) | ((uint32_t)(PBM >> 4) << 24);
@@ -551,7 +566,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
           acc_phase ^= 1u << acc;
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + acc * PBN;
-          const int kend = C::CHUNK ? min(kb1, kb + p.chunk) : kb1;
+          const int kend = C::CHUNK ? min(kb1, kb + chunk) : kb1;
           uint32_t first = 1;
           for (; kb < kend; ++kb) {
             if (!mbar_wait_cluster(full_bar(stage), phase, abort_flag, p.err, 13)) { ok = false; break; }
@@ -593,7 +608,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       const int sp = item / (p.tiles_n * p.tiles_m);
       const int kb0 = sp * p.kb_per_split;
       const int kb1 = min(p.kb_total, kb0 + p.kb_per_split);
-      const int nchunks = C::CHUNK ? (kb1 - kb0 + p.chunk - 1) / p.chunk : 1;
+      const int nchunks = C::CHUNK ? (kb1 - kb0 + chunk - 1) / chunk : 1;
       const int m0 = tm * PBM + (int)rank * BM + quad * 32;
       const int n0 = tn * PBN + half * BN;
       const bool scaled = NPROD == 3 && p.a_exp;
@@ -661,6 +676,20 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a,
   }
 }
 
+template <int NPROD>
+__global__ void __launch_bounds__(PAIR_THREADS, 1)
+gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                         const __grid_constant__ Params p) {
+  gemm_pair<NPROD>(map_a, map_b, p);
+}
+__global__ void __launch_bounds__(PAIR_THREADS, 1)
+gemm_tcgen05_pair_f16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                             const __grid_constant__ CUtensorMap bf_a, const __grid_constant__ CUtensorMap bf_b,
+                             const __grid_constant__ Params p) {
+  if (*p.uneven) gemm_pair<6, true>(bf_a, bf_b, p);
+  else gemm_pair<3>(map_a, map_b, p);
+}
+
 // x -> `planes` bf16 planes (x = p0 + p1 (+ p2), each the bf16 rounding of what is left),
 // same orientation as the source, leading dimension ld_dst (a multiple of 8), planes
 // `plane_stride` elements apart.  One thread converts 4 consecutive elements of a row:
@@ -675,7 +704,7 @@ struct SplitJob {
   int vec_ok = 0;
 };
 template <int PLANES, typename TS>
-__global__ void split_planes_kernel(const SplitJob job0, const SplitJob job1) {
+__device__ __forceinline__ void split_planes(const SplitJob& job0, const SplitJob& job1) {
   const SplitJob& job = blockIdx.y ? job1 : job0;
   const TS* __restrict__ src = static_cast<const TS*>(job.src);
   __nv_bfloat16* __restrict__ dst = job.dst;
@@ -721,12 +750,30 @@ __global__ void split_planes_kernel(const SplitJob job0, const SplitJob job1) {
   }
 }
 
+template <int PLANES, typename TS>
+__global__ void split_planes_kernel(const SplitJob job0, const SplitJob job1) {
+  split_planes<PLANES, TS>(job0, job1);
+}
+// In the place of fp16 planes, if one of `n` words asks for it; words[n] says so to the product.
+__global__ void split_uneven_kernel(const SplitJob job0, const SplitJob job1, int* words, int n) {
+  int w = 0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) w |= words[i];
+  w = __syncthreads_or(w);
+  if (blockIdx.x + blockIdx.y + threadIdx.x == 0) words[n] = w;
+  if (w) split_planes<3, float>(job0, job1);
+}
+
 // ---- two fp16 planes per fp32 operand ---------------------------------------------------------
 // x 2^s = p0 + p1, p0 and p1 the fp16 roundings of x 2^s and of what is left: 22 .. 23 bits of x where
 // three bf16 planes keep 24, for three products instead of six and two thirds of the operand bytes.
 // s makes the largest value of a row of A (a column of B) 2^14 .. 2^15, so that values down to 2^-17 of
 // it keep all their bits and smaller ones an absolute error of 2^-40 of it; the epilogue takes the
-// powers out again.
+// powers out again.  Such smaller values are one in 20000 of a normal distribution and do not show; but where
+// a few values tower above all others of their row, and meet weights that are small or zero, they are the result.
+// So the splits count them: with more than one in 32 of a row's or column's values other than zero, the
+// operands are split into three bf16 planes after all and multiplied six times (decided on the device; where they
+// are not, the look costs 12 us: 4 in the split, a launch, and a word that the product waits for).  What is left: in up
+// to one value of 32, an error of 2^-40 of the row's or column's largest value.
 // k-blocks per hand-over of the accumulator: 24 truncated accumulations, half of the bf16 planes' (relative
 // error of 16384 x 1024 x 1024 against fp64: six bf16 products 1.17e-6, these 6.2e-7, with twice the chunk
 // 1.07e-6 and 2 % less time).
@@ -751,7 +798,8 @@ __device__ __forceinline__ float4 load_quad(const float* row, int c, int cols, i
   if (c + 3 < cols) v.w = row[c + 3];
   return v;
 }
-__device__ __forceinline__ void store_f16_quad(__half* dst, long long plane_stride, const float4& v, float4 scale) {
+// Returns how many of the values, in either half, are below 0.25 once scaled, zeros among them.
+__device__ __forceinline__ __half2 store_f16_quad(__half* dst, long long plane_stride, const float4& v, float4 scale) {
   const float x[4] = {v.x * scale.x, v.y * scale.y, v.z * scale.z, v.w * scale.w};
   const __half2 a = __floats2half2_rn(x[0], x[1]), b = __floats2half2_rn(x[2], x[3]);
   const __half2 c = __floats2half2_rn(x[0] - __low2float(a), x[1] - __high2float(a));
@@ -759,10 +807,24 @@ __device__ __forceinline__ void store_f16_quad(__half* dst, long long plane_stri
   *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
   *reinterpret_cast<uint2*>(dst + plane_stride) =
       make_uint2(*reinterpret_cast<const uint32_t*>(&c), *reinterpret_cast<const uint32_t*>(&d));
+  const __half2 few = __float2half2_rn(0.25f);
+  return __hadd2(__hlt2(__habs2(a), few), __hlt2(__habs2(b), few));
 }
-// A warp takes 8 / QL rows at a time, of which it holds QL quads per lane; longer rows are read twice.
+// Adds to `score`, which is above zero for a row if more than one in 32 of its values other than zero, scaled
+// by f, lose bits.
+__device__ __forceinline__ void count_small(float x, float f, int& score) {
+  const float v = fabsf(x) * f;
+  score += v > 0.f ? (v < 0.25f ? 31 : -1) : 0;
+}
+__device__ __forceinline__ void count_small4(const float4& x, const float4& f, int (&score)[4]) {
+  count_small(x.x, f.x, score[0]); count_small(x.y, f.y, score[1]);
+  count_small(x.z, f.z, score[2]); count_small(x.w, f.w, score[3]);
+}
+// A warp takes 8 / QL rows at a time, of which it holds QL quads per lane; longer rows are read twice.  Returns whether
+// a row has too many small values.
 template <int QL>
-__device__ __forceinline__ void split_f16_rows(const SplitJob& a, int* __restrict__ a_exp) {
+__device__ __forceinline__ bool split_f16_rows(const SplitJob& a, int* __restrict__ a_exp) {
+  bool uneven = false;
   constexpr int RW = 8 / QL;
   const int lane = threadIdx.x & 31, quads = (int)(a.ld_dst / 4), step = gridDim.x * (F16_THREADS / 32) * RW;
   for (int r0 = (blockIdx.x * (F16_THREADS / 32) + (threadIdx.x >> 5)) * RW; r0 < a.rows; r0 += step) {
@@ -795,29 +857,47 @@ __device__ __forceinline__ void split_f16_rows(const SplitJob& a, int* __restric
       const float f = exp2_int(s);
       const float4 scale = make_float4(f, f, f, f);
       if (lane == 0) a_exp[r0 + k] = -s;
+      int score[4] = {0, 0, 0, 0};
+      __half2 small = __float2half2_rn(0.f);
 #pragma unroll
       for (int i = 0; i < QL; ++i)
-        if (lane + 32 * i < quads) store_f16_quad(dst + (lane + 32 * i) * 4, a.plane_stride, v[k][i], scale);
-      if (QL == 8) {
+        if (lane + 32 * i < quads)
+          small = __hadd2(small, store_f16_quad(dst + (lane + 32 * i) * 4, a.plane_stride, v[k][i], scale));
+      const bool held = QL < 8 || quads <= F16_ROW_QUADS;
+      if (!held) {
         const float* src = static_cast<const float*>(a.src) + r0 * a.ld_src;
-        for (int q = F16_ROW_QUADS + lane; q < quads; q += 32)
-          store_f16_quad(dst + q * 4, a.plane_stride, load_quad(src, q * 4, a.cols, a.vec_ok), scale);
+        for (int q = F16_ROW_QUADS + lane; q < quads; q += 32) {
+          const float4 x = load_quad(src, q * 4, a.cols, a.vec_ok);
+          store_f16_quad(dst + q * 4, a.plane_stride, x, scale);
+          count_small4(x, scale, score);
+        }
+      }
+      // (counted to the end only where zeros may be among the small ones)
+      const int most_small = __reduce_add_sync(0xffffffffu, (int)(__low2float(small) + __high2float(small)));
+      if (!held || 32 * most_small > a.cols - most_small) {
+#pragma unroll
+        for (int i = 0; i < QL; ++i) count_small4(v[k][i], scale, score);
+        uneven |= __reduce_add_sync(0xffffffffu, score[0] + score[1] + score[2] + score[3]) > 0;
       }
     }
   }
+  return uneven;
 }
 // blockIdx.y = 0: `a`, scaled by row, a warp per row or few; 1: `b`, scaled by column, 32 columns per block (its
-// second reading comes from L2).  Bound by HBM: 256000 x 1024 takes one reading and one writing.
+// second reading comes from L2).  Bound by HBM: 256000 x 1024 takes one reading and one writing.  uneven: a word per
+// block, whether its values ask for the bf16 planes.
 __global__ void __launch_bounds__(F16_THREADS) split_f16_kernel(const SplitJob a, int* __restrict__ a_exp, const SplitJob b,
-                                                                signed char* __restrict__ b_exp) {
+                                                                signed char* __restrict__ b_exp, int* __restrict__ uneven) {
+  bool bad = false;
   if (blockIdx.y == 0) {
     const int quads = (int)(a.ld_dst / 4);
-    if (quads <= 32) split_f16_rows<1>(a, a_exp);
-    else if (quads <= 64) split_f16_rows<2>(a, a_exp);
-    else if (quads <= 128) split_f16_rows<4>(a, a_exp);
-    else split_f16_rows<8>(a, a_exp);
+    if (quads <= 32) bad = split_f16_rows<1>(a, a_exp);
+    else if (quads <= 64) bad = split_f16_rows<2>(a, a_exp);
+    else if (quads <= 128) bad = split_f16_rows<4>(a, a_exp);
+    else bad = split_f16_rows<8>(a, a_exp);
   } else {
     __shared__ float4 part[F16_THREADS];
+    __shared__ int scores[32];
     const int q = threadIdx.x & 7, ry = threadIdx.x >> 3;
     constexpr int RY = F16_THREADS / 8;
     for (int c0 = blockIdx.x * 32; c0 < (int)b.ld_dst; c0 += gridDim.x * 32) {
@@ -832,6 +912,7 @@ __global__ void __launch_bounds__(F16_THREADS) split_f16_kernel(const SplitJob a
       }
       __syncthreads();  // the columns before have been read
       part[threadIdx.x] = most;
+      if (threadIdx.x < 32) scores[threadIdx.x] = 0;
       __syncthreads();
       for (int h = RY / 2; h > 0; h >>= 1) {
         if (ry < h) {
@@ -844,15 +925,28 @@ __global__ void __launch_bounds__(F16_THREADS) split_f16_kernel(const SplitJob a
       most = part[q];
       const int4 s = make_int4(f16_shift(most.x), f16_shift(most.y), f16_shift(most.z), f16_shift(most.w));
       const float4 scale = make_float4(exp2_int(s.x), exp2_int(s.y), exp2_int(s.z), exp2_int(s.w));
+      int score[4] = {0, 0, 0, 0};
       if (c < (int)b.ld_dst) {
         if (ry == 0) *reinterpret_cast<char4*>(b_exp + c) = make_char4(-s.x, -s.y, -s.z, -s.w);
 #pragma unroll 4
-        for (int r = ry; r < b.rows; r += RY)
-          store_f16_quad(reinterpret_cast<__half*>(b.dst) + r * b.ld_dst + c, b.plane_stride,
-                         load_quad(src + r * b.ld_src, c, b.cols, b.vec_ok), scale);
+        for (int r = ry; r < b.rows; r += RY) {
+          const float4 x = load_quad(src + r * b.ld_src, c, b.cols, b.vec_ok);
+          store_f16_quad(reinterpret_cast<__half*>(b.dst) + r * b.ld_dst + c, b.plane_stride, x, scale);
+          count_small4(x, scale, score);
+        }
       }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {  // over the warp's rows, then the block's
+        score[i] += __shfl_xor_sync(0xffffffffu, score[i], 8);
+        score[i] += __shfl_xor_sync(0xffffffffu, score[i], 16);
+        if ((threadIdx.x & 31) < 8) atomicAdd(&scores[q * 4 + i], score[i]);
+      }
+      __syncthreads();
+      if (threadIdx.x < 32) bad |= scores[threadIdx.x] > 0;
     }
   }
+  const int any = __syncthreads_or(bad);
+  if (threadIdx.x == 0) uneven[blockIdx.y * gridDim.x + blockIdx.x] = any;
 }
 
 // `dtype` of the sources.  __half: its 11 significant bits split exactly into two planes.  bf16: one
@@ -878,13 +972,18 @@ int launch_split(SplitJob* jobs, int n, int dtype, int planes, cudaStream_t stre
   return HASTE_B200_OK;
 }
 
-int launch_split_f16(SplitJob* jobs, int* a_exp, signed char* b_exp, cudaStream_t stream) {
+// Leaves in *uneven whether the planes are bf16 after all.  `words`: 8 per SM and one.
+int launch_split_f16(SplitJob* jobs, int* a_exp, signed char* b_exp, int* words, const int** uneven, cudaStream_t stream) {
   for (int i = 0; i < 2; ++i) jobs[i].vec_ok = wide_rows(jobs[i], HASTE_B200_F32);
   const int per_warp = (int)(8 / max(1LL, min(8LL, (jobs[0].ld_dst + 127) / 128)));  // about what split_f16_rows takes
   const int blocks = max(ceil_div(jobs[0].rows, F16_THREADS / 32 * per_warp), ceil_div(jobs[1].cols, 32));
-  split_f16_kernel<<<dim3(min(blocks, 4 * sm_count()), 2), F16_THREADS, 0, stream>>>(jobs[0], a_exp, jobs[1], b_exp);
+  const dim3 grid(min(blocks, 4 * sm_count()), 2);
+  split_f16_kernel<<<grid, F16_THREADS, 0, stream>>>(jobs[0], a_exp, jobs[1], b_exp, words);
   HB_LAUNCH_OK();
-  count_launch(1);
+  split_uneven_kernel<<<dim3(sm_count(), 2), 512, 0, stream>>>(jobs[0], jobs[1], words, 2 * grid.x);
+  HB_LAUNCH_OK();
+  count_launch(2);
+  *uneven = words + 2 * grid.x;
   return HASTE_B200_OK;
 }
 
@@ -972,6 +1071,8 @@ int set_kernel_attributes() {
   HB_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<1>, attr, pair_smem<1>()));
   HB_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<3>, attr, pair_smem<3>()));
   HB_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<6>, attr, pair_smem<6>()));
+  HB_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_f16_kernel, attr, max(single_smem<3>(), single_smem<6>())));
+  HB_CUDA_OK(cudaFuncSetAttribute(gemm_tcgen05_pair_f16_kernel, attr, max(pair_smem<3>(), pair_smem<6>())));
   if (dev >= 0 && dev < kMaxDevices) g_attr_set[dev].store(true, std::memory_order_release);
   return HASTE_B200_OK;
 }
@@ -1032,9 +1133,10 @@ const char* refusal(const GemmDesc& g) {
   return nullptr;
 }
 // fp32-accurate products go through two fp16 planes where half the products save more than the rows' and
-// columns' scales cost (us with the splits and a LayerNorm over the result, six bf16 products / these:
-// 65536 x 1024 x 1024 1354 / 1165, 16384 x 512 x 1024 290 / 278, 65536 x 512 x 256 359 / 330; but
-// 16384 x 256 x 1024 253 / 257, 4096 x 1024 x 1024 108 / 113, 65536 x 192 x 1024 920 / 933; M x K x N).
+// columns' scales and the look at their values cost (us with the splits, a LayerNorm and the scan over the result,
+// six bf16 products / these: 256000 x 1024 x 1024 5540 / 4476, 16384 x 1024 x 1024 381 / 343, 65536 x 512 x 256
+// 365 / 342, 16384 x 512 x 1024 297 / 289, 8000 x 1024 x 1024 192 / 189; M x K x N.  Below 8 G multiply-adds, or 256 of
+// K, nothing is left).
 bool f16_planes(const GemmDesc& g) {
   return g.precise && g.dtype == HASTE_B200_F32 && g.a_cs == 1 && g.b_cs == 1 && g.b_rs != 1 && g.K >= 256 &&
          (double)g.M * g.N * g.K >= 8e9;
@@ -1119,14 +1221,15 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
   const bool b_copy = f32 ? !b_pre : (b_ld_src % 8) != 0 || ((uintptr_t)g.b & 15) != 0;
   const long long a_ld = a_pre ? g.a_pl_ld : (a_copy ? ((a_cols + 7) & ~7LL) : a_ld_src);
   const long long b_ld = b_pre ? g.b_pl_ld : (b_copy ? ((b_cols + 7) & ~7LL) : b_ld_src);
-  const int planes = f32 ? (g.precise && !f16 ? 3 : 2) : 1;
+  const int planes = f32 ? (g.precise && !f16 ? 3 : 2) : 1, room = f16 ? 3 : planes;
   const size_t a_plane = a_copy ? Arena::pad((size_t)a_rows * a_ld * 2) : 0;
   const size_t b_plane = b_copy ? Arena::pad((size_t)b_rows * b_ld * 2) : 0;
   const int part_ld = (N + 31) & ~31;
   const bool via_partial = splits > 1;
   const size_t part_bytes = via_partial ? Arena::pad((size_t)splits * M * part_ld * 4) : 0;
   const size_t a_exps = f16 ? Arena::pad((size_t)M * 4) : 0, b_exps = f16 ? Arena::pad((size_t)tiles_n * PBN) : 0;
-  const size_t bytes = planes * (a_plane + b_plane) + part_bytes + a_exps + b_exps + 1024;
+  const size_t words = f16 ? Arena::pad((size_t)(8 * sms + 1) * 4) : 0;
+  const size_t bytes = room * (a_plane + b_plane) + part_bytes + a_exps + b_exps + words + 1024;
   Arena ws;
   HB_TRY(make_arena(&ws, stream, bytes, /*slot=*/1));
   int* err = device_error_word();
@@ -1139,7 +1242,7 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
   int n_jobs = 0;
   auto through_scratch = [&](const void* src, long long ld_src, long long rows, long long cols, size_t plane,
                              long long ld, Operand* o) {
-    __nv_bfloat16* to = ws.take<__nv_bfloat16>(planes * plane / 2);
+    __nv_bfloat16* to = ws.take<__nv_bfloat16>(room * plane / 2);
     jobs[n_jobs++] = SplitJob{src, ld_src, (int)rows, (int)cols, to, ld, (long long)(plane / 2)};
     o->base = to;
     o->plane_stride = plane / 2;
@@ -1149,11 +1252,13 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
   if (b_copy && !through_scratch(g.b, b_ld_src, b_rows, b_cols, b_plane, b_ld, &B)) return unsupported("scratch arena");
   int* a_exp = nullptr;
   signed char* b_exp = nullptr;
+  const int* uneven = nullptr;
   if (f16) {
     a_exp = ws.take<int>(a_exps / 4);
     b_exp = ws.take<signed char>(b_exps);
-    if (!a_exp || !b_exp) return unsupported("scratch arena");
-    HB_TRY(launch_split_f16(jobs, a_exp, b_exp, stream));
+    int* w = ws.take<int>(words / 4);
+    if (!a_exp || !b_exp || !w) return unsupported("scratch arena");
+    HB_TRY(launch_split_f16(jobs, a_exp, b_exp, w, &uneven, stream));
   } else if (n_jobs) {
     HB_TRY(launch_split(jobs, n_jobs, g.dtype, planes, stream));
   }
@@ -1164,15 +1269,6 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
     partial = ws.take<float>(part_bytes / 4);
     if (!partial) return unsupported("scratch arena");
   }
-
-  CUtensorMap m_a, m_b;
-  bool ok = true;
-  // K-major: inner = K, box 64 (k) x 128 rows.  MN-major: inner = M/N, box 64 x 64 (k).
-  ok &= make_map(&m_a, A.base, a_cols, a_rows, A.ld, A.plane_stride, planes, 64,
-                 A.mn_major ? 64 : BM);
-  ok &= make_map(&m_b, B.base, b_cols, b_rows, B.ld, B.plane_stride, planes, 64,
-                 B.mn_major ? 64 : BN);
-  if (!ok) return unsupported("tensor map encoding rejected the operand");
 
   Params p;
   p.M = M; p.N = N; p.K = K;
@@ -1185,11 +1281,20 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
   p.wide = (g.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(g.c) & (4 * dtype_size(g.dtype_c) - 1)) == 0;
   p.a_exp = a_exp; p.b_exp = b_exp;
   p.chunk = f16 ? kF16Chunk : (planes == 3 ? Cfg<6>::CHUNK : Cfg<3>::CHUNK);
+  p.uneven = uneven;
   p.partial = partial;
   p.partial_ld = part_ld;
   p.err = err;
 
   HB_TRY(set_kernel_attributes());
+  // K-major: inner = K, box 64 (k) x 128 rows.  MN-major: inner = M/N, box 64 x 64 (k).
+  CUtensorMap m_a, m_b, bf_a, bf_b;
+  auto maps = [&](CUtensorMap* a, CUtensorMap* b, int n) {
+    return make_map(a, A.base, a_cols, a_rows, A.ld, A.plane_stride, n, 64, A.mn_major ? 64 : BM) &&
+           make_map(b, B.base, b_cols, b_rows, B.ld, B.plane_stride, n, 64, B.mn_major ? 64 : BN);
+  };
+  if (!maps(&m_a, &m_b, planes) || (f16 && !maps(&bf_a, &bf_b, 3)))
+    return unsupported("tensor map encoding rejected the operand");
   if (pair) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * min(pairs, tiles_m * tiles_n * splits));
@@ -1202,7 +1307,10 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (planes == 3) {
+    if (f16) {
+      cfg.dynamicSmemBytes = max(pair_smem<3>(), pair_smem<6>());
+      HB_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_tcgen05_pair_f16_kernel, m_a, m_b, bf_a, bf_b, p));
+    } else if (planes == 3) {
       cfg.dynamicSmemBytes = pair_smem<6>();
       HB_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_tcgen05_pair_kernel<6>, m_a, m_b, p));
     } else if (planes == 2) {
@@ -1214,7 +1322,9 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
     }
   } else {
     const int grid = min(sms, tiles_m * tiles_n * splits);
-    if (planes == 3)
+    if (f16)
+      gemm_tcgen05_f16_kernel<<<grid, THREADS, max(single_smem<3>(), single_smem<6>()), stream>>>(m_a, m_b, bf_a, bf_b, p);
+    else if (planes == 3)
       gemm_tcgen05_kernel<6><<<grid, THREADS, single_smem<6>(), stream>>>(m_a, m_b, p);
     else if (planes == 2)
       gemm_tcgen05_kernel<3><<<grid, THREADS, single_smem<3>(), stream>>>(m_a, m_b, p);

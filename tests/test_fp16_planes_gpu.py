@@ -66,3 +66,28 @@ def test_projection_of_extreme_rows_and_columns():
         keep[1] = r != 2  # 1e-60 is no float
         err = relative(got[r:r + 1], x[r:r + 1], W)[0, keep]
         assert err.square().mean().sqrt().item() < BOUND and err.max().item() < 5 * BOUND, r
+
+
+@pytest.mark.parametrize("M,K,N", [(16384, 512, 1024), (65536, 300, 500), (4096, 2100, 1030), (8200, 1024, 1024)])
+@pytest.mark.parametrize("where", ["row", "column", "nowhere"])
+def test_projection_with_values_that_tower_above_their_row(M, K, N, where):
+    """A feature of 1e7 among others of 1e-3 that meets a weight of zero, or a weight of 1e7 that meets a feature of zero:
+    the result is what the small values make.  Errors relative to the sum of |x| |W|, by the bound above (the
+    bf16 planes are handed over as often; a term's own error, 2^-22, is smaller than the accumulator's)."""
+    g = torch.Generator("cuda").manual_seed(K)
+    x = torch.randn(M, K, device="cuda", generator=g)
+    W = torch.randn(K, N, device="cuda", generator=g) / K ** 0.5
+    if where == "row":
+        x *= 1e-3
+        x[M - 7, 3], x[M - 7, K - 1] = 1e7, -1e7
+        W[3], W[K - 1] = 0.0, 0.0
+    elif where == "column":
+        W *= 1e-3
+        W[5, N - 3], W[K - 1, N - 3] = 1e7, 3e6
+        x[:, 5], x[:, K - 1] = 0.0, 0.0
+    got = projection(x, W)
+    for rows in (slice(0, 64), slice(M - 64, M)):
+        a = x[rows].double()
+        err = (got[rows].double() - a @ W.double()).abs() / (a.abs() @ W.double().abs())
+        assert err.square().mean().sqrt().item() < BOUND and err.max().item() < 5 * BOUND
+        assert err[:, N - 3].max().item() < 5 * BOUND
