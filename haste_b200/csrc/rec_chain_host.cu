@@ -43,13 +43,11 @@ bool gl_geometry(int dtype, int N, int H, bool bwd, int most, GlGeometry* g) {
   const int ks = ceil_div(g->KS16, GL_WARPS);
   if (ks > 8) return false;
   const int tiles = ceil_div(N, 8), sms = sm_count(), budget = sm_budget();
-  // Under an SM budget (two directions side by side) first within it; if that takes too many chains,
-  // the whole GPU for one direction after the other still beats the step-wise path (bf16 LSTM, two
-  // directions of 139 rows, H = 696: 18 chains within the budget, 6 without).
-  for (int use : {budget, sms}) {
-    if (use < g->KS16 || use > sms) continue;  // (four quads take the fewest CTAs: one per 16 units)
+  const bool wide = dtype != HASTE_B200_BF16 && ks > 4;
+  auto within = [&](int use, GlGeometry* g) {
+    if (use < g->KS16) return false;  // (four quads take the fewest CTAs: one per 16 units)
     for (int nmt : {2, 4}) {
-      if (nmt == 2 && (dtype == HASTE_B200_BF16 || ks <= 4)) continue;
+      if (nmt == 2 && !wide) continue;
       g->NMT = nmt;
       g->nHS = ceil_div(H, 4 * nmt);
       if (use < g->nHS) continue;
@@ -59,9 +57,21 @@ bool gl_geometry(int dtype, int N, int H, bool bwd, int most, GlGeometry* g) {
       if (nmt == 2 && g->CH >= (bwd ? kFourQuadsBwd : kFourQuadsFwd)) continue;
       if (g->CH <= most) return true;
     }
-    if (most < kGridChains) break;  // the tensor-core recurrence comes next, within the budget too
+    return false;
+  };
+  // Under an SM budget (two directions side by side) first within it; if that takes too many chains, the whole
+  // GPU for one direction after the other is ahead: of the step-wise path (bf16 LSTM, two directions of 139
+  // rows, H = 696: 18 chains within the budget, 6 without), and for wide fp32 layers, where half of the GPU holds one
+  // row group and all of it two or three, also of twice and three times the chains (budget_pays).
+  if (budget >= g->KS16 && budget <= sms) {
+    GlGeometry whole = *g;
+    if (within(budget, g)) {
+      if (wide && within(sms, &whole) && !budget_pays(bwd, budget, g->CH, whole.CH)) *g = whole;
+      return true;
+    }
+    if (most < kGridChains) return false;  // the tensor-core recurrence comes next, within the budget too
   }
-  return false;
+  return within(sms, g);
 }
 
 // How many chains per CTA the cluster kernels may take before the grid kernels do better (us per

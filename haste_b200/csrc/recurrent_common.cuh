@@ -144,5 +144,21 @@ __device__ __forceinline__ void raise_abort(const Sync& s, int* s_abort, int cod
   __threadfence_system();
 }
 
+// Whether a recurrence with `half` chains per CTA within an SM budget of up to half of the GPU, two directions
+// side by side, is ahead of the whole GPU with `whole` chains for one direction after the other.  Side by side one
+// direction's hand-offs are under way while the other computes, until the chains are enough to fill that time
+// by themselves.  Both directions of 100 steps, us in turn / side by side, forward and backward:
+//   LSTM fp32 H = 1024    16 rows, 2 chains for 2  519 / 461, 1394 / 1136    64 rows, 8 for 4  1483 / 1549, 2897 / 2935
+//        H = 640          32 rows, 4 for 2  635 / 680, 1205 / 1197            48 rows, 6 for 2  652 / 976, 1339 / 1616
+//   GRU fp32 H = 1024     32 rows, 4 for 2  802 / 775, 1641 / 1378            64 rows, 8 for 4  1524 / 1484, 2186 / 2449
+//        H = 640          48 rows, 6 for 2  622 / 867, 1196 / 1618            96 rows, 12 for 4 1186 / 1689, 2021 / 3022
+//   LayerNormLSTM fp32 H = 512  64 rows, 4 for 2  1346 / 1117, 2032 / 1866    128 rows, 8 for 4  2032 / 2014, 3141 / 3403
+//        H = 400          80 rows, 5 for 2  1310 / 1366, 1985 / 2250          96 rows, 6 for 3  1661 / 1473, 2461 / 2448
+//   LayerNormGRU bf16 H = 768   24 rows, 3 for 1  870 / 752, 1272 / 1354      48 rows, 6 for 2  1084 / 1218, 1474 / 1958
+inline bool budget_pays(bool bwd, int budget, int half, int whole) {
+  if (2 * budget > sm_count()) return true;  // a budget for another reason than a second direction
+  return bwd ? half <= 2 * whole && half <= 6 : half <= 2 * whole || half <= 3;
+}
+
 }  // namespace rec
 }  // namespace hb

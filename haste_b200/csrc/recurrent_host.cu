@@ -11,24 +11,26 @@ namespace rec {
 namespace {
 
 // The grid kernels' tiling: as many row groups as the SMs have room for, one CTA per SM, the rest of the rows
-// as chains.  Under an SM budget (two directions side by side) within it first: four chains per CTA cost a
-// third to a half more than two, not twice as much (see rec_ln_grid.cuh), so both directions at once take
-// 9.5 / 10.6 us per step where one after the other takes 14.0 / 13.8 (LayerNormLSTM fp32, 64 rows, H = 512).
+// as chains.  Under an SM budget (two directions side by side) within it first, where that pays (budget_pays).
 constexpr int kLnGridChains = 8;
 
-bool ln_grid_geometry(int dtype, int N, int H, LnGridGeometry* g) {
+bool ln_grid_geometry(int dtype, int N, int H, bool bwd, LnGridGeometry* g) {
   // R's slice must fit the registers: two planes with fp32 storage, one with bf16
   if (H > (dtype == HASTE_B200_BF16 ? 1024 : 512)) return false;
   g->nHS = ceil_div(H, 16);
   const int tiles = ceil_div(N, 8), sms = sm_count(), budget = sm_budget();
-  for (int use : {budget, sms}) {
-    if (use < g->nHS || use > sms) continue;
+  auto within = [&](int use, LnGridGeometry* g) {
+    if (use < g->nHS) return false;
     g->nRG = min(tiles, use / g->nHS);
     g->CH = ceil_div(tiles, g->nRG);
     g->nRG = ceil_div(tiles, g->CH);
-    if (g->CH <= kLnGridChains) return true;
-  }
-  return false;
+    return g->CH <= kLnGridChains;
+  };
+  LnGridGeometry whole = *g;
+  const bool fits = within(sms, &whole);
+  if (budget <= sms && within(budget, g) && (!fits || budget_pays(bwd, budget, g->CH, whole.CH))) return true;
+  *g = whole;
+  return fits;
 }
 // Whole-quad accesses: every row of every array starts on a multiple of four elements.
 int wide_rows(std::initializer_list<const void*> ptrs, int H, int dtype) {
@@ -180,7 +182,7 @@ int run_forward(LnFwdParams& p, int dtype, int wide, ClFwd cluster, GridFwd grid
   const int cl = cluster(p, s);
   if (cl != HASTE_B200_ERR_UNSUPPORTED) return cl;
   LnGridGeometry g;
-  if (!ln_grid_geometry(dtype, p.N, p.H, &g)) return HASTE_B200_ERR_UNSUPPORTED;
+  if (!ln_grid_geometry(dtype, p.N, p.H, false, &g)) return HASTE_B200_ERR_UNSUPPORTED;
   const size_t tiles = ceil_div(p.N, 8), xwords = 2 * tiles * g.nHS * 128, swords = 4 * tiles * g.nHS * 16;
   HB_TRY(make_scratch(xwords + swords, &p.sync, &p.xbuf, s));
   p.sbuf = p.xbuf + xwords;
@@ -243,7 +245,7 @@ int run_backward(LnBwdParams& p, int gates, int dtype, int wide, const LnGrads& 
   }
   if (st_ == HASTE_B200_ERR_UNSUPPORTED) {
     LnGridGeometry g;
-    if (!ln_grid_geometry(dtype, p.N, H, &g)) return HASTE_B200_ERR_UNSUPPORTED;
+    if (!ln_grid_geometry(dtype, p.N, H, true, &g)) return HASTE_B200_ERR_UNSUPPORTED;
     rows = 2 * g.nRG;
     const size_t xwords = 2 * tiles * g.nHS * g.nHS * 128, swords = 4 * tiles * g.nHS * 16;
     HB_TRY(make_scratch(xwords + swords, &p.sync, &p.exch, s, (size_t)rows * 10 * H));
