@@ -33,7 +33,7 @@
 //   waits for all of them (acquire) before it loads step t's operand.  CTAs of different row
 //   groups never wait for each other, and with several tiles per CTA the wait for one tile
 //   hides behind the contraction of the others.
-// * The gate functions are the accurate ones of rec_chain.cuh.  One MUFU.TANH each (relative error
+// * The gate functions are those of rec_chain.cuh (1e-6).  One MUFU.TANH each (relative error
 //   2^-11) would take 0.3 us off a forward step of the GRU, but then 0.17 % of the stored states are
 //   another bf16 than the exact step gives, against 0.02 %.
 // * Every wait - counter or mbarrier - is bounded; on expiry the grid's abort flag and the
@@ -491,7 +491,7 @@ tc_recurrence_kernel(const __grid_constant__ CUtensorMap map_a, const TcParams p
             }
           }
         }
-        // ---- backward: what can be done without the step product (the accurate tanh of an LSTM's c takes 2000 cycles)
+        // ---- backward: what can be done without the step product (the tanh of an LSTM's c takes 2000 cycles)
         if (!FWD && valid) {
 #pragma unroll
           for (int hf = 0; hf < 2; ++hf) {

@@ -119,7 +119,6 @@ __device__ __forceinline__ uint32_t fword_encode(float x, uint32_t tag) {
   return (__float_as_uint(x) & ~1u) | tag;
 }
 __device__ __forceinline__ float fword_value(uint32_t w) { return __uint_as_float(w & ~1u); }
-__device__ __forceinline__ bool fword_ready(uint32_t w, uint32_t tag) { return (w & 1u) == tag; }
 
 // Fast gate functions (ex2.approx based): error ~1e-6 absolute, far inside the parity bar.
 __device__ __forceinline__ float sigmoid_fast(float x) {
