@@ -56,7 +56,6 @@ struct Params {
   long long ldc;
   const int* a_exp;            // fp16 planes: the result's row m, column n is to be scaled by
   const signed char* b_exp;    // 2^(a_exp[m] + b_exp[n]); null otherwise
-  int chunk;                   // k-blocks per hand-over of the accumulator (Cfg::CHUNK != 0)
   const int* uneven;           // fp16 planes: points to whether bf16 planes have taken their place
   float* partial;              // non-null: write fp32 partial tiles [split][M][partial_ld]
   int partial_ld;              // N rounded up to whole 32-column chunks
@@ -88,24 +87,27 @@ __device__ __forceinline__ float exp2_int(int e) {  // 2^e, -126 <= e <= 127
   return __uint_as_float((uint32_t)(e + 127) << 23);
 }
 
-// The powers of two that fp16 planes leave in a tile: of this lane's row, and of the four columns that the
-// lane stores of each 32-column chunk.  Loaded before the products are there.
-struct TileScale {
-  int row;
-  int cols[BN / 32];
-  __device__ __forceinline__ void load(const Params& p, int m0, int n0) {
-    const int lane = threadIdx.x & 31;
-    row = m0 + lane < p.M ? p.a_exp[m0 + lane] : 0;
-#pragma unroll
-    for (int c = 0; c < BN / 32; ++c)
-      cols[c] = *reinterpret_cast<const int*>(p.b_exp + n0 + c * 32 + (lane & 7) * 4);
-  }
-};
-// Rows 0 .. rows - 1 of a 32 x 32 tile in shared memory (laid out by store_chunk) to dst, `cols` columns wide.
-// `ea`, `eb`: see TileScale and store_chunk.
-template <bool SCALED, bool ADD, typename TC>
+// Planes: bf16; two of fp16; three of bf16 in the place of those, handed over as often per product.
+enum { PLAIN, F16_PLANES, UNEVEN };
+
+// The powers of two that fp16 planes leave in a tile: of this lane's row, and of the four columns that the lane
+// stores of the chunk from n0 on.  (Loaded when they are used: the sums fill the registers till then.)
+__device__ __forceinline__ int row_scale(const Params& p, int m0) {
+  const int m = m0 + (threadIdx.x & 31);
+  return m < p.M ? p.a_exp[m] : 0;
+}
+__device__ __forceinline__ int column_scales(const Params& p, int n0) {
+  return *reinterpret_cast<const int*>(p.b_exp + n0 + (threadIdx.x & 7) * 4);
+}
+// Rows 0 .. rows - 1 of a 32 x 32 tile in shared memory (laid out by fill_tile) to dst, `cols` columns wide.
+// `ea`, `eb`: row_scale, column_scales.  Whether C is added to is known to the code where one product is
+// (bf16 64000 x 2048, K = 512 210 us, tested in the loop 220); with several, whose sums fill the registers, two kinds
+// of loops spilled (fp32, the same 386 tested in the loop, 395).
+enum { NEVER, SURELY, EITHER };
+template <bool SCALED, int ADD, typename TC>
 __device__ __forceinline__ void store_tile(const float4* tile, TC* dst, long long ld_dst, int rows, int cols, bool wide,
-                                           int ea, int eb) {
+                                           bool adds, int ea, int eb) {
+  const bool add = ADD == EITHER ? adds : ADD == SURELY;
   const int lane = threadIdx.x & 31;
   if (wide) {
     const int u = lane & 7;
@@ -125,14 +127,14 @@ __device__ __forceinline__ void store_tile(const float4* tile, TC* dst, long lon
       }
       TC* to = dst + r * ld_dst + u * 4;
       if constexpr (sizeof(TC) == 4) {
-        if (ADD) {
+        if (add) {
           const float4 c = *reinterpret_cast<const float4*>(to);
           x.x += c.x; x.y += c.y; x.z += c.z; x.w += c.w;
         }
         *reinterpret_cast<float4*>(to) = x;
       } else {
         __align__(8) TC o[4];
-        if (ADD) {
+        if (add) {
           *reinterpret_cast<uint2*>(o) = *reinterpret_cast<const uint2*>(to);
           x.x += ld(o); x.y += ld(o + 1); x.z += ld(o + 2); x.w += ld(o + 3);
         }
@@ -152,17 +154,17 @@ __device__ __forceinline__ void store_tile(const float4* tile, TC* dst, long lon
       float x = at[(r * 8 + ((lane >> 2) ^ (r & 7))) * 4];
       if (SCALED) x = x * exp2_int(e >> 1) * fb * exp2_int(e - (e >> 1));
       TC* to = dst + r * ld_dst + lane;
-      st(to, ADD ? x + ld(to) : x);
+      st(to, add ? x + ld(to) : x);
     }
   }
 }
-template <bool SCALED, typename TC>
-__device__ __forceinline__ void store_tile_c(const Params& p, const float4* tile, int m0, int n0, int ea, int eb) {
+template <typename TC>
+__device__ __forceinline__ void store_tile_c(const Params& p, const float4* tile, int m0, int n0) {
   TC* dst = static_cast<TC*>(p.c) + m0 * p.ldc + n0;
   const int rows = min(32, p.M - m0), cols = min(32, p.N - n0);
   const bool wide = p.wide && (cols & 3) == 0;
-  if (p.accumulate) store_tile<SCALED, true, TC>(tile, dst, p.ldc, rows, cols, wide, ea, eb);
-  else store_tile<SCALED, false, TC>(tile, dst, p.ldc, rows, cols, wide, ea, eb);
+  if (p.accumulate) store_tile<false, SURELY, TC>(tile, dst, p.ldc, rows, cols, wide, true, 0, 0);
+  else store_tile<false, NEVER, TC>(tile, dst, p.ldc, rows, cols, wide, false, 0, 0);
 }
 
 // A warp stores 32 rows (m0 ..) x 32 columns (n0 ..) of the result; lane r holds row r.  The tile goes
@@ -176,27 +178,53 @@ __device__ __forceinline__ void store_tile_c(const Params& p, const float4* tile
 // fp16 planes: row m, column n times 2^(a_exp[m] + b_exp[n]), the row's power in two halves around the
 // column's, so that no step leaves the range of a float unless the result does.  (b_exp is readable up
 // to whole tiles.)
-template <bool SCALED>
-__device__ __forceinline__ void store_chunk(const Params& p, int sp, int m0, int n0, const float* v, uint8_t* buf,
-                                            int ea = 0, int eb = 0) {
-  if (m0 >= p.M || n0 >= p.N) return;  // the same for the whole warp
+// (A chunk's code stands once in a kernel, in a loop: with four copies of it for every kind of C small contractions
+// waited for their instructions; with cold caches, us, rows from the lanes / four copies / this: 480 x 512, K = 64
+// 8.3 / 15.4 / 8.0, 32 x 4096, K = 1024 10.4 / 13.3 / 10.9.  Except for fp16 planes on pairs, which are never small
+// and also scale what they store: 128000 x 512, K = 512 with the scan 440 us in a loop, 415 without.)
+__device__ __forceinline__ void fill_tile(const float* v, uint8_t* buf) {
   const int lane = threadIdx.x & 31;
   float4* tile = reinterpret_cast<float4*>(buf);
-  __syncwarp();  // the tile before has been read
 #pragma unroll
   for (int j = 0; j < 8; ++j)
     tile[lane * 8 + (j ^ (lane & 7))] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+}
+template <int NPROD, int MODE>
+__device__ __forceinline__ void store_chunk(const Params& p, int sp, int m0, int n0, uint8_t* buf, int ea = 0, int eb = 0) {
+  if (m0 >= p.M || n0 >= p.N) return;  // the same for the whole warp
+  const float4* tile = reinterpret_cast<const float4*>(buf);
   __syncwarp();
-  if (p.partial)  // rows of whole chunks
-    store_tile<SCALED, false, float>(tile, p.partial + ((long long)sp * p.M + m0) * p.partial_ld + n0, p.partial_ld,
-                                     min(32, p.M - m0), 32, true, ea, eb);
-  else if (p.c_is_bf16 == 0) store_tile_c<SCALED, float>(p, tile, m0, n0, ea, eb);
-  else if (p.c_is_bf16 == 1) store_tile_c<SCALED, __nv_bfloat16>(p, tile, m0, n0, ea, eb);
-  else store_tile_c<SCALED, __half>(p, tile, m0, n0, ea, eb);
+  if constexpr (NPROD == 1) {
+    if (p.partial)  // rows of whole chunks
+      store_tile<false, NEVER, float>(tile, p.partial + ((long long)sp * p.M + m0) * p.partial_ld + n0, p.partial_ld,
+                                      min(32, p.M - m0), 32, true, false, 0, 0);
+    else if (p.c_is_bf16 == 0) store_tile_c<float>(p, tile, m0, n0);
+    else if (p.c_is_bf16 == 1) store_tile_c<__nv_bfloat16>(p, tile, m0, n0);
+    else store_tile_c<__half>(p, tile, m0, n0);
+  } else {
+    const int rows = min(32, p.M - m0), cols = min(32, p.N - n0);
+    const bool wide = p.wide && (cols & 3) == 0;
+    const long long at = m0 * p.ldc + n0;
+    if (MODE != PLAIN || p.partial || p.c_is_bf16 == 0) {  // (fp16 planes: fp32 results that are not added to)
+      float* dst = p.partial ? p.partial + ((long long)sp * p.M + m0) * p.partial_ld + n0 : static_cast<float*>(p.c) + at;
+      store_tile<MODE == F16_PLANES, MODE == PLAIN ? EITHER : NEVER>(tile, dst, p.partial ? p.partial_ld : p.ldc, rows,
+                                                                     p.partial ? 32 : cols, p.partial || wide,
+                                                                     !p.partial && p.accumulate, ea, eb);
+    } else if (p.c_is_bf16 == 1) {
+      store_tile<false, EITHER>(tile, static_cast<__nv_bfloat16*>(p.c) + at, p.ldc, rows, cols, wide, p.accumulate, 0, 0);
+    } else {
+      store_tile<false, EITHER>(tile, static_cast<__half*>(p.c) + at, p.ldc, rows, cols, wide, p.accumulate, 0, 0);
+    }
+  }
 }
 
-// UNEVEN: bf16 planes in the place of fp16 planes, handed over as often per product.
-template <int NPROD, bool UNEVEN = false>
+// k-blocks per hand-over of the accumulator.  fp16 planes: 24 truncated accumulations, half of the bf16 planes'
+// (relative error of 16384 x 1024 x 1024 against fp64: six bf16 products 1.17e-6, these 6.2e-7, with twice the chunk
+// 1.07e-6 and 2 % less time).
+template <int NPROD, int MODE>
+constexpr int chunk_of() { return MODE == PLAIN ? Cfg<NPROD>::CHUNK : (MODE == F16_PLANES ? 2 : 1); }
+
+template <int NPROD, int MODE = PLAIN>
 __device__ __forceinline__ void gemm_tile(const CUtensorMap& map_a, const CUtensorMap& map_b, const Params& p) {
   using C = Cfg<NPROD>;
   extern __shared__ uint8_t smem_raw[];
@@ -213,7 +241,7 @@ __device__ __forceinline__ void gemm_tile(const CUtensorMap& map_a, const CUtens
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int chunk = NPROD == 6 ? C::CHUNK / (UNEVEN ? 2 : 1) : p.chunk;
+  constexpr int chunk = chunk_of<NPROD, MODE>();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
@@ -283,7 +311,7 @@ __device__ __forceinline__ void gemm_tile(const CUtensorMap& map_a, const CUtens
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (lane == 0) {
-      const uint32_t type = NPROD == 3 && p.a_exp ? 0u : 1u;  // fp16 or bf16 operands
+      constexpr uint32_t type = MODE == F16_PLANES ? 0u : 1u;  // fp16 or bf16 operands
       const uint32_t idesc = (1u << 4) | (type << 7) | (type << 10) |
                              ((uint32_t)p.a_mn_major << 15) | ((uint32_t)p.b_mn_major << 16) |
                              ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
@@ -351,12 +379,9 @@ __device__ __forceinline__ void gemm_tile(const CUtensorMap& map_a, const CUtens
       const int sp = item / (p.tiles_n * p.tiles_m);
       const int kb0 = sp * p.kb_per_split;
       const int kb1 = min(p.kb_total, kb0 + p.kb_per_split);
-      const int nchunks = C::CHUNK ? (kb1 - kb0 + chunk - 1) / chunk : 1;
+      const int nchunks = C::CHUNK ? (kb1 - kb0 + chunk - 1) / max(chunk, 1) : 1;
       const int m0 = tm * BM + quad * 32;
       const int n0 = tn * BN;
-      const bool scaled = NPROD == 3 && p.a_exp;
-      TileScale scale;
-      if (scaled) scale.load(p, m0, n0);
       // running sums of this thread's row of the tile (only with chunked hand-over)
       float sum[C::CHUNK ? BN : 1];
 #pragma unroll
@@ -388,7 +413,9 @@ __device__ __forceinline__ void gemm_tile(const CUtensorMap& map_a, const CUtens
             float v[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-            store_chunk<false>(p, sp, m0, n0 + ch * 32, v, tile);
+            __syncwarp();  // the tile before has been read
+            fill_tile(v, tile);
+            store_chunk<NPROD, MODE>(p, sp, m0, n0 + ch * 32, tile);
           }
         }
         tc_fence_before();
@@ -396,11 +423,15 @@ __device__ __forceinline__ void gemm_tile(const CUtensorMap& map_a, const CUtens
       }
       if (!ok) break;
       if (C::CHUNK) {
-#pragma unroll
+        const int ea = MODE == F16_PLANES ? row_scale(p, m0) : 0;
+#pragma unroll 1
         for (int ch = 0; ch < BN / 32; ++ch) {
-          const float* v = sum + (C::CHUNK ? ch * 32 : 0);
-          if (scaled) store_chunk<true>(p, sp, m0, n0 + ch * 32, v, tile, scale.row, scale.cols[ch]);
-          else store_chunk<false>(p, sp, m0, n0 + ch * 32, v, tile);
+          const int eb = MODE == F16_PLANES ? column_scales(p, n0 + ch * 32) : 0;
+          __syncwarp();  // the tile before has been read
+#pragma unroll
+          for (int c = 0; c < BN / 32; ++c)
+            if (c == ch) fill_tile(sum + (C::CHUNK ? c * 32 : 0), tile);
+          store_chunk<NPROD, MODE>(p, sp, m0, n0 + ch * 32, tile, ea, eb);
         }
       }
     }
@@ -427,8 +458,8 @@ __global__ void __launch_bounds__(THREADS, 1)
 gemm_tcgen05_f16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                         const __grid_constant__ CUtensorMap bf_a, const __grid_constant__ CUtensorMap bf_b,
                         const __grid_constant__ Params p) {
-  if (*p.uneven) gemm_tile<6, true>(bf_a, bf_b, p);
-  else gemm_tile<3>(map_a, map_b, p);
+  if (*p.uneven) gemm_tile<6, UNEVEN>(bf_a, bf_b, p);
+  else gemm_tile<3, F16_PLANES>(map_a, map_b, p);
 }
 
 // ---- the same contraction on CTA pairs ------------------------------------------------------
@@ -453,7 +484,7 @@ constexpr int PAIR_EPI_WARPS = 8;
 // (Ten warps put three on two of the SM's four sub-partitions, 16384 registers each, so 168
 // registers per thread is the most a 320-thread CTA can have; the epilogue therefore drains the
 // accumulator 16 columns at a time.)
-template <int NPROD, bool UNEVEN = false>
+template <int NPROD, int MODE = PLAIN>
 __device__ __forceinline__ void gemm_pair(const CUtensorMap& map_a, const CUtensorMap& map_b, const Params& p) {
   using C = Cfg<NPROD>;
   extern __shared__ uint8_t smem_raw[];
@@ -472,7 +503,7 @@ __device__ __forceinline__ void gemm_pair(const CUtensorMap& map_a, const CUtens
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();  // 0 issues the MMAs
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
-  const int chunk = NPROD == 6 ? C::CHUNK / (UNEVEN ? 2 : 1) : p.chunk;
+  constexpr int chunk = chunk_of<NPROD, MODE>();
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
@@ -544,7 +575,7 @@ __device__ __forceinline__ void gemm_pair(const CUtensorMap& map_a, const CUtens
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (CTA 0 only)
     if (lane == 0 && rank == 0) {
-      const uint32_t type = NPROD == 3 && p.a_exp ? 0u : 1u;  // fp16 or bf16 operands
+      constexpr uint32_t type = MODE == F16_PLANES ? 0u : 1u;  // fp16 or bf16 operands
       const uint32_t idesc = (1u << 4) | (type << 7) | (type << 10) |
                              ((uint32_t)p.a_mn_major << 15) | ((uint32_t)p.b_mn_major << 16) |
                              ((uint32_t)(PBN >> 3) << 17) | ((uint32_t)(PBM >> 4) << 24);
@@ -608,12 +639,9 @@ __device__ __forceinline__ void gemm_pair(const CUtensorMap& map_a, const CUtens
       const int sp = item / (p.tiles_n * p.tiles_m);
       const int kb0 = sp * p.kb_per_split;
       const int kb1 = min(p.kb_total, kb0 + p.kb_per_split);
-      const int nchunks = C::CHUNK ? (kb1 - kb0 + chunk - 1) / chunk : 1;
+      const int nchunks = C::CHUNK ? (kb1 - kb0 + chunk - 1) / max(chunk, 1) : 1;
       const int m0 = tm * PBM + (int)rank * BM + quad * 32;
       const int n0 = tn * PBN + half * BN;
-      const bool scaled = NPROD == 3 && p.a_exp;
-      TileScale scale;
-      if (scaled) scale.load(p, m0, n0);
       float sum[C::CHUNK ? BN : 1];
 #pragma unroll
       for (int j = 0; j < (C::CHUNK ? BN : 1); ++j) sum[j] = 0.f;
@@ -644,7 +672,9 @@ __device__ __forceinline__ void gemm_pair(const CUtensorMap& map_a, const CUtens
             float v[32];
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-            store_chunk<false>(p, sp, m0, n0 + ch * 32, v, tile);
+            __syncwarp();  // the tile before has been read
+            fill_tile(v, tile);
+            store_chunk<NPROD, MODE>(p, sp, m0, n0 + ch * 32, tile);
           }
         }
         tc_fence_before();
@@ -653,11 +683,15 @@ __device__ __forceinline__ void gemm_pair(const CUtensorMap& map_a, const CUtens
       }
       if (!ok) break;
       if (C::CHUNK) {
-#pragma unroll
+        const int ea = MODE == F16_PLANES ? row_scale(p, m0) : 0;
+#pragma unroll (MODE == F16_PLANES ? BN / 32 : 1)
         for (int ch = 0; ch < BN / 32; ++ch) {
-          const float* v = sum + (C::CHUNK ? ch * 32 : 0);
-          if (scaled) store_chunk<true>(p, sp, m0, n0 + ch * 32, v, tile, scale.row, scale.cols[ch]);
-          else store_chunk<false>(p, sp, m0, n0 + ch * 32, v, tile);
+          const int eb = MODE == F16_PLANES ? column_scales(p, n0 + ch * 32) : 0;
+          __syncwarp();  // the tile before has been read
+#pragma unroll
+          for (int c = 0; c < BN / 32; ++c)
+            if (c == ch) fill_tile(sum + (C::CHUNK ? c * 32 : 0), tile);
+          store_chunk<NPROD, MODE>(p, sp, m0, n0 + ch * 32, tile, ea, eb);
         }
       }
     }
@@ -686,8 +720,8 @@ __global__ void __launch_bounds__(PAIR_THREADS, 1)
 gemm_tcgen05_pair_f16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                              const __grid_constant__ CUtensorMap bf_a, const __grid_constant__ CUtensorMap bf_b,
                              const __grid_constant__ Params p) {
-  if (*p.uneven) gemm_pair<6, true>(bf_a, bf_b, p);
-  else gemm_pair<3>(map_a, map_b, p);
+  if (*p.uneven) gemm_pair<6, UNEVEN>(bf_a, bf_b, p);
+  else gemm_pair<3, F16_PLANES>(map_a, map_b, p);
 }
 
 // x -> `planes` bf16 planes (x = p0 + p1 (+ p2), each the bf16 rounding of what is left),
@@ -772,12 +806,8 @@ __global__ void split_uneven_kernel(const SplitJob job0, const SplitJob job1, in
 // a few values tower above all others of their row, and meet weights that are small or zero, they are the result.
 // So the splits count them: with more than one in 32 of a row's or column's values other than zero, the
 // operands are split into three bf16 planes after all and multiplied six times (decided on the device; where they
-// are not, the look costs 12 us: 4 in the split, a launch, and a word that the product waits for).  What is left: in up
-// to one value of 32, an error of 2^-40 of the row's or column's largest value.
-// k-blocks per hand-over of the accumulator: 24 truncated accumulations, half of the bf16 planes' (relative
-// error of 16384 x 1024 x 1024 against fp64: six bf16 products 1.17e-6, these 6.2e-7, with twice the chunk
-// 1.07e-6 and 2 % less time).
-constexpr int kF16Chunk = 2;
+// are not, the look costs 4 us: a launch, and a word that the product waits for).  What is left: in up to one value of
+// 32, an error of 2^-40 of the row's or column's largest value.
 constexpr int F16_THREADS = 512, F16_ROW_QUADS = 8 * 32;  // quads of a row that a warp holds in registers
 
 __device__ __forceinline__ int f16_shift(float most) {  // non-finite rows are non-finite either way
@@ -1134,12 +1164,12 @@ const char* refusal(const GemmDesc& g) {
 }
 // fp32-accurate products go through two fp16 planes where half the products save more than the rows' and
 // columns' scales and the look at their values cost (us with the splits, a LayerNorm and the scan over the result,
-// six bf16 products / these: 256000 x 1024 x 1024 5540 / 4476, 16384 x 1024 x 1024 381 / 343, 65536 x 512 x 256
-// 365 / 342, 16384 x 512 x 1024 297 / 289, 8000 x 1024 x 1024 192 / 189; M x K x N.  Below 8 G multiply-adds, or 256 of
+// six bf16 products / these: 256000 x 1024 x 1024 5527 / 4448, 16384 x 1024 x 1024 381 / 334, 65536 x 512 x 256
+// 365 / 330, 16384 x 512 x 1024 298 / 278, 8000 x 1024 x 1024 193 / 179; M x K x N.  Below 8 G multiply-adds, or 256 of
 // K, nothing is left).
 bool f16_planes(const GemmDesc& g) {
-  return g.precise && g.dtype == HASTE_B200_F32 && g.a_cs == 1 && g.b_cs == 1 && g.b_rs != 1 && g.K >= 256 &&
-         (double)g.M * g.N * g.K >= 8e9;
+  return g.precise && g.dtype == HASTE_B200_F32 && g.dtype_c == HASTE_B200_F32 && !g.accumulate && g.a_cs == 1 &&
+         g.b_cs == 1 && g.b_rs != 1 && g.K >= 256 && (double)g.M * g.N * g.K >= 8e9;
 }
 }  // namespace
 
@@ -1280,7 +1310,6 @@ int gemm_sm100(const GemmDesc& g, cudaStream_t stream) {
   p.c = g.c; p.ldc = g.ldc;
   p.wide = (g.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(g.c) & (4 * dtype_size(g.dtype_c) - 1)) == 0;
   p.a_exp = a_exp; p.b_exp = b_exp;
-  p.chunk = f16 ? kF16Chunk : (planes == 3 ? Cfg<6>::CHUNK : Cfg<3>::CHUNK);
   p.uneven = uneven;
   p.partial = partial;
   p.partial_ld = part_ld;
