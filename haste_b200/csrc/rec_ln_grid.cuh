@@ -10,8 +10,8 @@
 // chain 1 C' A B - so that the hand-offs of one are under way while another computes.  A bidirectional
 // level runs as two such grids of half the GPU.
 //   LayerNormLSTM fp32, 64 rows, H = 512, us per step forward / backward: 7.4 / 10.7 with 16 rows per CTA as
-// one piece; here 7.0 / 6.9 with two chains per CTA, and 9.5 / 10.6 for both directions of a level side by
-// side with four (one chain: 6.1 / 5.7).  What bounds it then is the finishing warps' own time, about
+// one piece; here 6.5 / 6.9 with two chains per CTA, and 9.5 / 10.6 for both directions of a level side by
+// side with four (one chain: 5.4 / 5.7).  What bounds it then is the finishing warps' own time, about
 // 1200 instructions per warp, chain and step at the latency of dependent ones.
 //
 // The statistics of a CTA's 64 columns meet in its shared memory first (a barrier of the group's four
