@@ -406,7 +406,7 @@ __device__ __forceinline__ void gemm_tile(const CUtensorMap& map_a, const CUtens
           }
         } else {
 #pragma unroll 1
-          for (int ch = 0; ch < BN / 32; ++ch) {
+          for (int ch = 0; ch < BN / 32 && m0 < p.M && n0 + ch * 32 < p.N; ++ch) {
             uint32_t r[32];
             tc_ld32(taddr + ch * 32, r);
             tc_wait_ld();
@@ -423,6 +423,18 @@ __device__ __forceinline__ void gemm_tile(const CUtensorMap& map_a, const CUtens
       }
       if (!ok) break;
       if (C::CHUNK) {
+        // Partial tiles of few rows leave from the lanes: one tile per CTA, and the four trips through shared memory, one
+        // after the other, take 2 us longer than their stores (64 x 2048, K = 512 20.7 / 18.7 us, 32 x 4096, K = 1024
+        // 24.9 / 22.8).
+        if (MODE == PLAIN && p.partial && p.M <= 64) {
+          const int m = m0 + lane;
+          float* dst = p.partial + ((long long)sp * p.M + m) * p.partial_ld + n0;
+#pragma unroll
+          for (int j = 0; j < (C::CHUNK ? BN : 0); j += 4)
+            if (m < p.M && n0 + j < p.partial_ld)
+              *reinterpret_cast<float4*>(dst + j) = make_float4(sum[j], sum[j + 1], sum[j + 2], sum[j + 3]);
+          continue;
+        }
         const int ea = MODE == F16_PLANES ? row_scale(p, m0) : 0;
 #pragma unroll 1
         for (int ch = 0; ch < BN / 32; ++ch) {
@@ -665,7 +677,7 @@ __device__ __forceinline__ void gemm_pair(const CUtensorMap& map_a, const CUtens
           }
         } else {
 #pragma unroll 1
-          for (int ch = 0; ch < BN / 32; ++ch) {
+          for (int ch = 0; ch < BN / 32 && m0 < p.M && n0 + ch * 32 < p.N; ++ch) {
             uint32_t r[32];
             tc_ld32(taddr + ch * 32, r);
             tc_wait_ld();

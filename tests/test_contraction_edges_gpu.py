@@ -73,3 +73,17 @@ def test_long_sums_over_more_than_one_wave(M, K, N, dtype, tol):
     assert (ops.gemm(a, b).double() - want).abs().max().item() < tol * scale
     added = ops.gemm(a, b, out=c.clone(), accumulate=True)
     assert (added.double() - want - c.double()).abs().max().item() < tol * scale
+
+
+@pytest.mark.parametrize("M", [32, 33, 63, 64, 65])
+@pytest.mark.parametrize("K,N", [(512, 2048), (1100, 130), (2048, 1027)])
+def test_partial_tiles_of_few_rows(M, K, N):
+    """Up to 64 rows partial tiles leave from the lanes, beyond through shared memory; the bound is that of the edges above."""
+    torch.manual_seed(M + N)
+    a, b = torch.randn(M, K, device="cuda"), torch.randn(K, N, device="cuda")
+    want = a.double() @ b.double()
+    c = torch.randn(M, N, device="cuda")
+    scale = want.abs().max().item()
+    assert (ops.gemm(a, b).double() - want).abs().max().item() < 2e-5 * scale
+    added = ops.gemm(a, b, out=c.clone(), accumulate=True)
+    assert (added.double() - want - c.double()).abs().max().item() < 2e-5 * scale
