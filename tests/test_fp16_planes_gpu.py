@@ -68,7 +68,8 @@ def test_projection_of_extreme_rows_and_columns():
         assert err.square().mean().sqrt().item() < BOUND and err.max().item() < 5 * BOUND, r
 
 
-@pytest.mark.parametrize("M,K,N", [(16384, 512, 1024), (65536, 300, 500), (4096, 2100, 1030), (8200, 1024, 1024)])
+@pytest.mark.parametrize("M,K,N", [(16384, 512, 1024), (65536, 300, 500), (4096, 2100, 1030), (8200, 1024, 1024),
+                                   (1000, 8200, 1030)])  # the last one: K split
 @pytest.mark.parametrize("where", ["row", "column", "nowhere"])
 def test_projection_with_values_that_tower_above_their_row(M, K, N, where):
     """A feature of 1e7 among others of 1e-3 that meets a weight of zero, or a weight of 1e7 that meets a feature of zero:
